@@ -40,6 +40,7 @@ const KernelTables& kernels() {
     fill_vit_tables(k);
     fill_vit16_tables(k);
     fill_vbin_tables(k);
+    fill_exact_tables(k);
     fill_env_tables(k);
     return k;
   }();

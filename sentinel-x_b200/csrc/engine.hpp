@@ -289,11 +289,17 @@ class HostBytePool {
         return v;
       }
     HostBytes v;
-    v.reserve(bytes);
+    v.reserve(bytes + bytes / 4);  // sizes vary from call to call: grow seldom
     return v;
   }
+  // Page-locked memory is not kept without bound: larger buffers are freed.
+  static constexpr size_t kMaxKept = 256u << 20;
   void give(HostBytes&& v) {
     if (!v.capacity()) return;
+    if (v.capacity() > kMaxKept) {
+      HostBytes().swap(v);
+      return;
+    }
     std::lock_guard<std::mutex> g(mu_);
     free_.push_back(std::move(v));
     if (free_.size() > 2)  // keep the two largest
@@ -428,11 +434,8 @@ struct Slot {
   // Forward/Backward row passes of the block's final pairs, in buffers of
   // their own: the engine thread queues them and moves on to the next block;
   // a host job waits for them, copies the rows out and releases the buffers.
-  DevBuf<PairRec> rrecs;
-  DevBuf<BinRegion> rbins;
-  DevBuf<unsigned> rcnt;
-  DevBuf<int64_t> roff;
-  DevBuf<float> rows_f, rows_b;
+  DevBuf<sxk::RowRec> rrecs;
+  DevBuf<float> rows;
   cudaEvent_t rows_t0 = nullptr, rows_t1 = nullptr;
   cudaStream_t rows_copy = nullptr;  // device-to-host copies of the rows (host job)
   std::shared_ptr<RowsTicket> rows_busy;
@@ -513,6 +516,7 @@ struct sx_engine {
   bool destroyed = false;
   BlockPool target_blocks;  // device memory of freed target sets
   HostBytePool target_bytes;  // host residue buffers of freed target sets
+  HostBytePool row_bytes;     // host copies of the row passes
   // envelope passes of the host domain definition (used by the host pool's
   // driver thread, one batch at a time)
   cudaStream_t env_stream = nullptr;  // the passes' copies; their launches fan out over the slots' streams
@@ -527,8 +531,6 @@ struct sx_engine {
   DevBuf<float> long_scratch, long_out, long_rows_f, long_rows_b;
   DevBuf<int64_t> long_row_off;
   DevBuf<Thresholds> thr;
-  DevBuf<float> rows_f, rows_b;
-  DevBuf<int64_t> row_off;
   DevBuf<float> scores;
   DevBuf<int32_t> slots, plist;
   DevBuf<sxk::AdjPair> adj_pairs;
@@ -550,6 +552,7 @@ struct sx_profiles {
   DevBuf<float4> d_vit;  // Viterbi lane-group images
   DevBuf<uint4> d_qvimg;  // quantized Viterbi images of the packed pre-screen
   DevBuf<float> d_vfb;
+  DevBuf<float> d_x;  // row images of the exact row passes
   DevBuf<double> d_bias;
   // the filter thresholds of the last search options seen (they depend on the
   // profiles' statistics and F1/F2/F3 alone): a stream of searches with one
@@ -596,12 +599,40 @@ struct FinalPair {
   int32_t slot;
 };
 
-// Host copies of one chunk of raw Forward/Backward special rows.
+// Raw Forward/Backward special rows of a chunk of pairs: how the device passes
+// are laid out (records sorted by shape, then longest first) and, once they
+// are done, the rows' host copy.
 struct RowsChunk {
-  std::vector<float> f, b;    // rows of every pair of the chunk, back to back
-  std::vector<int64_t> off;   // offset of pair q's rows in f and b
-  std::vector<size_t> which;  // pair q's index in the caller's list
+  std::vector<sxk::RowRec> recs;
+  std::vector<size_t> which;  // record q's index in the caller's list
+  std::vector<int64_t> boff;  // offset of its Backward rows
+  size_t first[kNumXShapes + 1] = {};  // records of shape s: first[s] .. first[s+1]
+  int longest[kNumXShapes] = {};       // rows of the longest one
+  int64_t floats = 0;
+  // The copy goes to a page-locked buffer of the engine's pool: tens of MB of
+  // rows arrive at the link's rate and no page of fresh memory is touched.
+  HostBytePool* pool = nullptr;
+  HostBytes rows;
+  RowsChunk() = default;
+  RowsChunk(RowsChunk&&) = default;
+  RowsChunk& operator=(RowsChunk&&) = delete;
+  ~RowsChunk() {
+    if (pool) pool->give(std::move(rows));
+  }
+  const float* data() const { return reinterpret_cast<const float*>(rows.data()); }
+  const float* fwd(size_t q) const { return data() + recs[q].row_off; }
+  const float* bwd(size_t q) const { return data() + boff[q]; }
+  void fetch(HostBytePool& from, const float* dev, cudaStream_t s) {
+    const size_t bytes = sizeof(float) * (size_t)floats;
+    pool = &from;
+    rows = from.take(bytes);
+    rows.resize(bytes);
+    CK(cudaMemcpyAsync(rows.data(), dev, bytes, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+  }
 };
+// floats of one pair's rows, both directions
+inline int64_t row_floats(int64_t l) { return 12 * (l + 1); }
 
 // One batch's requests and the places for their results.
 struct EnvSource {
@@ -651,82 +682,10 @@ RegionPassStats region_passes(sx_engine* E, const sx_profiles* P, const sx_targe
                               std::vector<RegionSource>& srcs, int nthr);
 
 // Device Forward and Backward with row output for `pairs`, in chunks bounded
-// by `row_budget` floats per direction; hands each chunk's host copy to
-// consume(RowsChunk&&) as soon as it has arrived.
-template <typename Consume>
+// by the scratch budget; hands each chunk's host copy to consume(RowsChunk&&)
+// as soon as it has arrived.
 void rows_pass(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T, const std::vector<FinalPair>& pairs,
-               Consume&& consume) {
-  if (pairs.empty()) return;
-  const auto& K = kernels();
-  const int64_t row_budget = std::max<int64_t>(scratch_budget(E, E->batch_bytes / 2) / (int64_t)sizeof(float), 1 << 20);
-  size_t i0 = 0;
-  while (i0 < pairs.size()) {
-    // chunk [i0, i1)
-    size_t i1 = i0;
-    int64_t used = 0;
-    while (i1 < pairs.size()) {
-      const int64_t need = 6 * ((int64_t)T->len[pairs[i1].t] + 1);
-      if (i1 > i0 && used + need > row_budget) break;
-      used += need;
-      i1++;
-    }
-    // group by vbin, assign row offsets
-    std::vector<std::vector<size_t>> byb(kNumVbins);
-    for (size_t i = i0; i < i1; i++) byb[P->dp[pairs[i].p].vbin].push_back(i);
-    std::vector<PairRec> recs;
-    RowsChunk c;
-    std::vector<BinRegion> reg(kNumVbins);
-    std::vector<unsigned> cnt(kNumVbins, 0);
-    int64_t ro = 0;
-    for (int b = 0; b < kNumVbins; b++) {
-      reg[b].off = (int64_t)recs.size();
-      reg[b].cap = (uint32_t)byb[b].size();
-      reg[b].pad = 0;
-      cnt[b] = (unsigned)byb[b].size();
-      for (size_t i : byb[b]) {
-        const FinalPair& f = pairs[i];
-        PairRec r{f.p, f.t, f.usc, f.filtersc, f.vsc, 0.f, f.slot, 0};
-        recs.push_back(r);
-        c.off.push_back(ro);
-        c.which.push_back(i);
-        ro += 6 * ((int64_t)T->len[f.t] + 1);
-      }
-    }
-    cudaStream_t s = S.hi.main;
-    S.lists[3].upload(recs.data(), recs.size(), s);
-    E->row_off.upload(c.off.data(), c.off.size(), s);
-    S.bins[3].upload(reg.data(), reg.size(), s);
-    S.counts.alloc(4 * kMaxBins);
-    CK(cudaMemcpyAsync(S.counts.p + 3 * kMaxBins, cnt.data(), sizeof(unsigned) * kNumVbins, cudaMemcpyHostToDevice, s));
-    E->rows_f.alloc((size_t)ro);
-    E->rows_b.alloc((size_t)ro);
-    // rows the kernels never touch are zero
-    CK(cudaMemsetAsync(E->rows_f.p, 0, sizeof(float) * (size_t)ro, s));
-    CK(cudaMemsetAsync(E->rows_b.p, 0, sizeof(float) * (size_t)ro, s));
-    fork_aux(S.hi);
-    for (int b = 0; b < kNumVbins; b++) {
-      if (!cnt[b]) continue;
-      const int blocks = warp_ctas(E->num_sms, cnt[b]);
-      cudaStream_t sa = S.hi.aux[(2 * b) % S.hi.naux], sb = S.hi.aux[(2 * b + 1) % S.hi.naux];
-      K.fwd[b]<<<blocks, 32, 0, sa>>>(S.lists[3].p, S.counts.p + 3 * kMaxBins, S.bins[3].p, b, nullptr, nullptr,
-                                       nullptr, S.overflow.p, P->d_prof.p, E->thr.p, P->d_vfb.p, T->d_res.p,
-                                       T->d_off.p, T->d_len.p, T->d_xsc.p, 0.f, E->rows_f.p, E->row_off.p);
-      K.bwd[b]<<<blocks, 32, 0, sb>>>(S.lists[3].p, S.counts.p + 3 * kMaxBins, S.bins[3].p, b, P->d_prof.p,
-                                       P->d_vfb.p, T->d_res.p, T->d_off.p, T->d_len.p, T->d_xsc.p, E->rows_b.p,
-                                       E->row_off.p);
-      E->stats.kernel_launches += 2;
-    }
-    CK(cudaGetLastError());
-    join_aux(S.hi);
-    c.f.resize((size_t)ro);
-    c.b.resize((size_t)ro);
-    CK(cudaMemcpyAsync(c.f.data(), E->rows_f.p, sizeof(float) * (size_t)ro, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(c.b.data(), E->rows_b.p, sizeof(float) * (size_t)ro, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    consume(std::move(c));
-    i0 = i1;
-  }
-}
+               const std::function<void(RowsChunk&&)>& consume);
 
 // rows_pass with each chunk consumed on the calling thread: sink(i, fwd_rows,
 // bwd_rows) for every pair, spread over the engine's host threads.
@@ -734,8 +693,7 @@ template <typename Sink>
 void rows_pass_sync(sx_engine* E, const sx_profiles* P, const sx_targets* T, const std::vector<FinalPair>& pairs,
                     Sink&& sink) {
   rows_pass(E, E->sl[0], P, T, pairs, [&](RowsChunk&& c) {
-    parallel_for(c.which.size(), E->host_threads,
-                 [&](size_t q) { sink(c.which[q], c.f.data() + c.off[q], c.b.data() + c.off[q]); });
+    parallel_for(c.which.size(), E->host_threads, [&](size_t q) { sink(c.which[q], c.fwd(q), c.bwd(q)); });
   });
 }
 

@@ -1,0 +1,564 @@
+// Forward and Backward in the reference's order of operations
+// (src/hmmer/dp.rs:229-392): the raw special rows of final pairs.
+//
+// A team -- one warp up to 256 columns, a CTA of several warps above -- runs
+// one pair in one direction, thread t holding columns t*C+1 .. t*C+C.  What
+// bounds a pass is the latency of one row, because the B state of a row needs
+// the row's E (Forward) or B (Backward) sum, a sum the reference takes in
+// column order.  Three parts of a row are sequential in the reference:
+//   * the row sum.  It stays sequential, but as one chain of adds over a row
+//     laid out in shared memory (4 cycles a term, loads 16 terms ahead),
+//     not as a baton handed from lane to lane;
+//   * the D chain D[k] = a_k + p_k D[k-1].  Every lane runs its own columns
+//     at once from a guessed carry, then takes the carry its left neighbour
+//     computed and runs them again until no lane's carry changes.  A state
+//     that no lane changes satisfies the sequential recurrence with every
+//     rounding, so the result is the reference's bit for bit; after r rounds
+//     the first r lanes are final, so 32 rounds always suffice.  A wrong
+//     carry fades by the product of p_k, 0.4 a column in a typical model:
+//     a scan of the lanes' transfers gives the first guess and two or three
+//     rounds repair its last bits;
+//   * the descending D chain of Backward, the same way from the other end.
+// Between warps the carry goes through shared memory: each warp runs its D
+// chain from carry 0, publishes its end, takes its neighbour's and repairs its
+// first lanes; a warp whose own end that changed (its 256 columns did not
+// absorb the carry) sets a flag and the CTA repeats the exchange.
+//
+// Measured on B200 against the lane-to-lane baton it replaced (device time of
+// the row passes of one search): marker-set genome (242 pairs, M to 1,500)
+// 45.5 -> 6.9 ms, one profile of M = 100 (50 pairs) 1.99 -> 0.45 ms, 64
+// profiles of M 60-700 (60 pairs) 11.0 -> 2.0 ms.
+//
+// The images hold zeros past column M and where node M has no transition, so
+// the padding columns need no tests: whatever finite value they hold is
+// multiplied by a zero before it reaches a real column.
+#pragma once
+#include "kernels.cuh"
+
+namespace sxk {
+
+// Row image of a profile: kXRows rows of 32 * C * warps floats (its shape's
+// width), column k at index k - 1.
+enum : int {
+  kXMo = 0,    // 25 rows: match odds mo[x][k]
+  kXFwd = 25,  // p_bm[k], p_mm[k-1], p_im[k-1], p_dm[k-1], p_mi[k], p_ii[k], p_md[k-1], p_dd[k-1]
+  kXBwd = 33,  // p_mm[k], p_mi[k], p_md[k], p_im[k], p_ii[k], p_dm[k], p_dd[k], p_bm[k]
+  kXRows = 41
+};
+constexpr int kXMaxWarps = 16;
+
+// One pass over a target: rows of 6 floats (N B E J C, rescale factor) go to
+// row_off (Forward) and row_off + 6 (lr + 1) (Backward).
+struct RowRec {
+  int32_t p, t;
+  int64_t row_off;
+};
+
+struct XShared {  // exchange between the warps of a team
+  float mv[kXMaxWarps];       // last (Forward) or first (Backward) column's new match value
+  float end[kXMaxWarps];      // D at the warp's end of the chain
+  float prev[3][kXMaxWarps];  // M, I, D of the last column
+  int mx[kXMaxWarps];
+  float sum;
+  int flag;
+};
+
+template <bool MULTI>
+__device__ __forceinline__ void team_sync() {
+  if constexpr (MULTI) __syncthreads();
+  else __syncwarp();
+}
+
+template <int C>
+__device__ __forceinline__ void load_cols(const float* __restrict__ p, float (&v)[C]) {
+#pragma unroll
+  for (int q = 0; q < C / 4; q++) {
+    const float4 x = __ldg(reinterpret_cast<const float4*>(p) + q);
+    v[4 * q] = x.x;
+    v[4 * q + 1] = x.y;
+    v[4 * q + 2] = x.z;
+    v[4 * q + 3] = x.w;
+  }
+}
+template <int C>
+__device__ __forceinline__ void store_cols(float* p, const float (&v)[C]) {
+#pragma unroll
+  for (int q = 0; q < C / 4; q++)
+    reinterpret_cast<float4*>(p)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+}
+
+__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_int(a) == __float_as_int(b); }
+
+// t[0] + t[1] + ... + t[n-1] in that order from 0 (n a positive multiple of
+// 16); the loads of the next 16 terms overlap the adds of these.
+__device__ __forceinline__ float ordered_sum(const float* t, int n) {
+  const float4* p = reinterpret_cast<const float4*>(t);
+  float4 a[4];
+#pragma unroll
+  for (int u = 0; u < 4; u++) a[u] = p[u];
+  float s = 0.f;
+  for (int q = 4; q < n / 4; q += 4) {
+    float4 b[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) b[u] = p[q + u];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      s = fadd(fadd(fadd(fadd(s, a[u].x), a[u].y), a[u].z), a[u].w);
+      a[u] = b[u];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; u++) s = fadd(fadd(fadd(fadd(s, a[u].x), a[u].y), a[u].z), a[u].w);
+  return s;
+}
+// The team's sum of its shared row (n terms), known to every thread; the row
+// may be overwritten after the call.
+template <bool MULTI>
+__device__ __forceinline__ float team_sum(const float* t, int n, XShared& sh) {
+  if constexpr (MULTI) {
+    if (threadIdx.x < 32) {
+      const float s = ordered_sum(t, n);
+      if (threadIdx.x == 0) sh.sum = s;
+    }
+    __syncthreads();
+    return sh.sum;
+  } else {
+    const float s = ordered_sum(t, n);
+    __syncwarp();
+    return s;
+  }
+}
+
+// Products of the lanes' p_dd for the guess scan: after the call bs[s] is the
+// product over the 2^s lanes that end at this one (UP: ascending lanes) and
+// `all` the product up to and including this lane; returns the number of scan
+// steps whose factor is not negligible.
+template <bool UP>
+__device__ __forceinline__ int scan_factors(float b, int lane, float (&bs)[5], float& all) {
+  int steps = 5;
+#pragma unroll
+  for (int s = 0; s < 5; s++) {
+    const int o = 1 << s;
+    bs[s] = b;
+    if (steps == 5 && !__any_sync(kFull, b > 1.0e-9f)) steps = s;
+    const float n = UP ? __shfl_up_sync(kFull, b, o) : __shfl_down_sync(kFull, b, o);
+    if (UP ? lane >= o : lane + o < 32) b = b * n;
+  }
+  all = b;
+  return steps;
+}
+template <bool UP>
+__device__ __forceinline__ float scan_guess(float a, int lane, const float (&bs)[5], int steps) {
+#pragma unroll
+  for (int s = 0; s < 5; s++) {
+    if (s >= steps) break;
+    const int o = 1 << s;
+    const float n = UP ? __shfl_up_sync(kFull, a, o) : __shfl_down_sync(kFull, a, o);
+    if (UP ? lane >= o : lane + o < 32) a = fadd(a, fmul(bs[s], n));
+  }
+  return UP ? __shfl_up_sync(kFull, a, 1) : __shfl_down_sync(kFull, a, 1);
+}
+
+// Ascending D chain of a warp from `in` at its first column: rounds from the
+// guessed carries `cin` until no carry changes.
+template <int C>
+__device__ __forceinline__ void settle_up(float (&d)[C], const float (&a)[C], const float (&p)[C], float cin, float in,
+                                          int lane) {
+  for (int it = 0; it < 32; it++) {
+    float v = cin;
+#pragma unroll
+    for (int c = 0; c < C; c++) d[c] = v = fadd(a[c], fmul(v, p[c]));
+    const float up = __shfl_up_sync(kFull, v, 1);
+    const float nc = lane ? up : in;
+    if (__all_sync(kFull, same_bits(nc, cin))) break;
+    cin = nc;
+  }
+}
+// Descending: d[k] = ((a_k + p_k d[k+1]) + e) from `in` past its last column.
+template <int C>
+__device__ __forceinline__ void settle_down(float (&d)[C], const float (&a)[C], const float (&p)[C], float e, float cin,
+                                            float in, int lane) {
+  for (int it = 0; it < 32; it++) {
+    float v = cin;
+#pragma unroll
+    for (int c = C - 1; c >= 0; c--) d[c] = v = fadd(fadd(a[c], fmul(v, p[c])), e);
+    const float dn = __shfl_down_sync(kFull, v, 1);
+    const float nc = lane < 31 ? dn : in;
+    if (__all_sync(kFull, same_bits(nc, cin))) break;
+    cin = nc;
+  }
+}
+
+// Forward (dp.rs:229-298).
+template <int C, bool MULTI>
+__device__ __forceinline__ void exact_forward(const float* __restrict__ img, int M, const uint8_t* __restrict__ s, int L,
+                                              float ploop, float pmove, float pe_loop, float pe_move, float* orow,
+                                              float* T, XShared& sh) {
+  const int lane = threadIdx.x & 31;
+  const int warp = MULTI ? threadIdx.x >> 5 : 0;
+  const int width = (MULTI ? blockDim.x : 32) * C;
+  const int k0 = (MULTI ? threadIdx.x : lane) * C;
+  const bool lead = MULTI ? threadIdx.x == 0 : lane == 0;
+  const int nsum = max(16, (M + 15) & ~15);
+  const float* im = img + k0;
+  float tr[8][C];
+#pragma unroll
+  for (int q = 0; q < 8; q++) load_cols<C>(im + (kXFwd + q) * width, tr[q]);
+  float bs[5], ball, b = 1.f;
+#pragma unroll
+  for (int c = 0; c < C; c++) b = b * tr[7][c];
+  const int steps = scan_factors<true>(b, lane, bs, ball);
+  float bpre = __shfl_up_sync(kFull, ball, 1);
+  if (lane == 0) bpre = 1.f;
+  float mp[C], ip[C], dp[C], eo[C];
+#pragma unroll
+  for (int c = 0; c < C; c++) mp[c] = ip[c] = dp[c] = 0.f;
+  float lm = 0.f, li = 0.f, ld = 0.f;  // the left warp's last column (lane 0)
+  float xn = 1.f, xb = pmove, xj = 0.f, xc = 0.f;
+  if (lead) {
+#pragma unroll
+    for (int q = 0; q < 6; q++) orow[q] = 0.f;
+  }
+  if (MULTI) {
+    if (lead) sh.flag = 0;
+    __syncthreads();
+  }
+  int x = L > 0 ? __ldg(s) : 24, x1 = L > 1 ? __ldg(s + 1) : 24;
+  load_cols<C>(im + x * width, eo);
+  for (int i = 0; i < L; i++) {
+    const int x2 = i + 2 < L ? __ldg(s + i + 2) : 24;
+    float eon[C];
+    load_cols<C>(im + x1 * width, eon);
+    const float ins = x != 24 ? 1.f : 0.f;
+    float mpl = __shfl_up_sync(kFull, mp[C - 1], 1), ipl = __shfl_up_sync(kFull, ip[C - 1], 1);
+    float dpl = __shfl_up_sync(kFull, dp[C - 1], 1);
+    if (lane == 0) {
+      mpl = lm;
+      ipl = li;
+      dpl = ld;
+    }
+    float mv[C], iv[C], a[C], dv[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      float t = fmul(xb, tr[0][c]);
+      t = fadd(t, fmul(c ? mp[c - 1] : mpl, tr[1][c]));
+      t = fadd(t, fmul(c ? ip[c - 1] : ipl, tr[2][c]));
+      t = fadd(t, fmul(c ? dp[c - 1] : dpl, tr[3][c]));
+      mv[c] = fmul(t, eo[c]);
+      iv[c] = fmul(fadd(fmul(mp[c], tr[4][c]), fmul(ip[c], tr[5][c])), ins);
+    }
+    float mcl = __shfl_up_sync(kFull, mv[C - 1], 1);
+    if constexpr (MULTI) {
+      if (lane == 31) sh.mv[warp] = mv[C - 1];
+      __syncthreads();
+      if (lane == 0) mcl = warp ? sh.mv[warp - 1] : 0.f;
+    } else {
+      if (lane == 0) mcl = 0.f;
+    }
+    float end = 0.f;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      a[c] = fmul(c ? mv[c - 1] : mcl, tr[6][c]);
+      end = fadd(a[c], fmul(end, tr[7][c]));
+    }
+    float g = scan_guess<true>(end, lane, bs, steps);
+    if (lane == 0) g = 0.f;
+    settle_up<C>(dv, a, tr[7], g, 0.f, lane);
+    if constexpr (MULTI) {
+      if (lane == 31) sh.end[warp] = dv[C - 1];
+      __syncthreads();
+      if (warp) {
+        const float in = sh.end[warp - 1];
+        const float own = dv[C - 1];
+        float c0 = __shfl_up_sync(kFull, own, 1);
+        c0 = lane ? fadd(c0, fmul(bpre, in)) : in;
+        settle_up<C>(dv, a, tr[7], c0, in, lane);
+        if (lane == 31 && !same_bits(dv[C - 1], own)) sh.flag = 1;
+      }
+    }
+    auto publish = [&]() {
+      float t[C];
+#pragma unroll
+      for (int c = 0; c < C; c++) t[c] = fadd(mv[c], dv[c]);
+      store_cols<C>(T + k0, t);
+      if (MULTI && lane == 31) {
+        sh.prev[0][warp] = mv[C - 1];
+        sh.prev[1][warp] = iv[C - 1];
+        sh.prev[2][warp] = dv[C - 1];
+      }
+      team_sync<MULTI>();
+    };
+    publish();
+    if constexpr (MULTI) {
+      if (sh.flag) {  // a warp's end changed: exchange the ends until none does
+        for (int it = 0; it <= kXMaxWarps; it++) {
+          const float own = dv[C - 1];
+          if (lane == 31) sh.end[warp] = own;
+          __syncthreads();
+          const float in = warp ? sh.end[warp - 1] : 0.f;
+          const float up = __shfl_up_sync(kFull, own, 1);
+          settle_up<C>(dv, a, tr[7], lane ? up : in, in, lane);
+          if (!__syncthreads_or(lane == 31 && !same_bits(dv[C - 1], own))) break;
+        }
+        publish();
+      }
+    }
+    float xe = team_sum<MULTI>(T, nsum, sh);
+    if (MULTI && lead) sh.flag = 0;  // read by all before the sum's barrier, set again after the next row's
+    if (MULTI && lane == 0 && warp) {
+      lm = sh.prev[0][warp - 1];
+      li = sh.prev[1][warp - 1];
+      ld = sh.prev[2][warp - 1];
+    }
+    xj = fadd(fmul(xj, ploop), fmul(xe, pe_loop));
+    xc = fadd(fmul(xc, ploop), fmul(xe, pe_move));
+    xn = fmul(xn, ploop);
+    xb = fadd(fmul(xn, pmove), fmul(xj, pmove));
+    float scale = 0.f;
+    if (xe > 1.0e4f) {
+      const float inv = __fdiv_rn(1.0f, xe);
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        mv[c] = fmul(mv[c], inv);
+        iv[c] = fmul(iv[c], inv);
+        dv[c] = fmul(dv[c], inv);
+      }
+      lm = fmul(lm, inv);
+      li = fmul(li, inv);
+      ld = fmul(ld, inv);
+      xn = fmul(xn, inv);
+      xb = fmul(xb, inv);
+      xj = fmul(xj, inv);
+      xc = fmul(xc, inv);
+      scale = xe;
+      xe = 1.0f;
+    }
+    if (lead) {
+      float* o = orow + 6 * (int64_t)(i + 1);
+      o[0] = xn; o[1] = xb; o[2] = xe; o[3] = xj; o[4] = xc; o[5] = scale;
+    }
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      mp[c] = mv[c];
+      ip[c] = iv[c];
+      dp[c] = dv[c];
+      eo[c] = eon[c];
+    }
+    x = x1;
+    x1 = x2;
+  }
+}
+
+// Backward (dp.rs:301-392): row L (E, C), rows L-1..1 (N B E J C, rescale
+// factor) and the row-0 B sum in slot 1 of row 0.
+template <int C, bool MULTI>
+__device__ __forceinline__ void exact_backward(const float* __restrict__ img, int M, const uint8_t* __restrict__ s,
+                                               int L, float ploop, float pmove, float pe_loop, float pe_move,
+                                               float* orow, float* T, XShared& sh) {
+  const int lane = threadIdx.x & 31;
+  const int warp = MULTI ? threadIdx.x >> 5 : 0;
+  const int nw = MULTI ? blockDim.x >> 5 : 1;
+  const int width = nw * 32 * C;
+  const int k0 = (MULTI ? threadIdx.x : lane) * C;
+  const bool lead = MULTI ? threadIdx.x == 0 : lane == 0;
+  const int nsum = max(16, (M + 15) & ~15);
+  const float* im = img + k0;
+  float tr[8][C];  // mm mi md im ii dm dd bm
+#pragma unroll
+  for (int q = 0; q < 8; q++) load_cols<C>(im + (kXBwd + q) * width, tr[q]);
+  float bs[5], ball, b = 1.f;
+#pragma unroll
+  for (int c = 0; c < C; c++) b = b * tr[6][c];
+  const int steps = scan_factors<false>(b, lane, bs, ball);
+  float bpre = __shfl_down_sync(kFull, ball, 1);  // product over the lanes right of this one
+  if (lane == 31) bpre = 1.f;
+  if (lead) {
+#pragma unroll
+    for (int q = 0; q < 6; q++) orow[q] = 0.f;
+  }
+  if (L <= 0) return;
+  if (MULTI) {
+    if (lead) sh.flag = 0;
+    __syncthreads();
+  }
+  float mn[C], in_[C], al[C], dc[C];
+  // The row's D chain from al = M(i+1) p_dm and e = E: every thread's dc and
+  // the D right of its last column; true if the ends must be exchanged again
+  auto d_chain = [&](float e) -> float {
+    float end = 0.f;
+#pragma unroll
+    for (int c = C - 1; c >= 0; c--) end = fadd(fadd(al[c], fmul(end, tr[6][c])), e);
+    float g = scan_guess<false>(end, lane, bs, steps);
+    if (lane == 31) g = 0.f;
+    settle_down<C>(dc, al, tr[6], e, g, 0.f, lane);
+    float in = 0.f;
+    if constexpr (MULTI) {
+      if (lane == 0) sh.end[warp] = dc[0];
+      __syncthreads();
+      if (warp + 1 < nw) {
+        in = sh.end[warp + 1];
+        const float own = dc[0];
+        float c0 = __shfl_down_sync(kFull, own, 1);
+        c0 = lane < 31 ? fadd(c0, fmul(bpre, in)) : in;
+        settle_down<C>(dc, al, tr[6], e, c0, in, lane);
+        if (lane == 0 && !same_bits(dc[0], own)) sh.flag = 1;
+      }
+    }
+    const float dn = __shfl_down_sync(kFull, dc[0], 1);
+    return lane < 31 ? dn : in;
+  };
+  auto d_again = [&](float e) -> float {  // a warp's end changed
+    float in = 0.f;
+    for (int it = 0; it <= kXMaxWarps; it++) {
+      const float own = dc[0];
+      if (lane == 0) sh.end[warp] = own;
+      __syncthreads();
+      in = warp + 1 < nw ? sh.end[warp + 1] : 0.f;
+      const float dn = __shfl_down_sync(kFull, own, 1);
+      settle_down<C>(dc, al, tr[6], e, lane < 31 ? dn : in, in, lane);
+      if (!__syncthreads_or(lane == 0 && !same_bits(dc[0], own))) break;
+    }
+    const float dn = __shfl_down_sync(kFull, dc[0], 1);
+    return lane < 31 ? dn : in;
+  };
+  // row L
+  float xc = pmove;
+  float xe = fmul(xc, pe_move);
+  float xj = 0.f, xn = 0.f;
+#pragma unroll
+  for (int c = 0; c < C; c++) al[c] = in_[c] = 0.f;
+  float dnr = d_chain(xe);
+  if constexpr (MULTI) {
+    __syncthreads();
+    if (sh.flag) dnr = d_again(xe);
+    __syncthreads();
+    if (lead) sh.flag = 0;
+  }
+#pragma unroll
+  for (int c = 0; c < C; c++) mn[c] = fadd(xe, fmul(c < C - 1 ? dc[c + 1] : dnr, tr[2][c]));
+  if (lead) {
+    float* o = orow + 6 * (int64_t)L;
+    o[0] = 0.f; o[1] = 0.f; o[2] = xe; o[3] = 0.f; o[4] = xc; o[5] = 0.f;
+  }
+  // B sum of row i from M(i+1) and the odds of residue i+1; leaves M(i+1) e in me
+  float me[C];
+  auto b_terms = [&](const float (&eo)[C]) {
+    float bt[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      me[c] = fmul(mn[c], eo[c]);
+      bt[c] = fmul(fmul(mn[c], tr[7][c]), eo[c]);
+    }
+    store_cols<C>(T + k0, bt);
+    if (MULTI && lane == 0) sh.mv[warp] = me[0];
+    team_sync<MULTI>();
+  };
+  int x = __ldg(s + L - 1), x1 = L > 1 ? __ldg(s + L - 2) : 24;
+  float eo[C];
+  load_cols<C>(im + x * width, eo);
+  for (int i = L - 1; i >= 1; i--) {
+    const int x2 = i >= 2 ? __ldg(s + i - 2) : 24;
+    float eon[C];
+    load_cols<C>(im + x1 * width, eon);
+    const float ins = x != 24 ? 1.f : 0.f;
+    b_terms(eo);
+    float me_up = __shfl_down_sync(kFull, me[0], 1);
+    if (lane == 31) me_up = MULTI && warp + 1 < nw ? sh.mv[warp + 1] : 0.f;
+    const float xb = team_sum<MULTI>(T, nsum, sh);
+    xj = fadd(fmul(xj, ploop), fmul(xb, pmove));
+    xc = fmul(xc, ploop);
+    xe = fadd(fmul(xj, pe_loop), fmul(xc, pe_move));
+    xn = fadd(fmul(xn, ploop), fmul(xb, pmove));
+    float iv[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      iv[c] = fmul(in_[c], ins);
+      al[c] = fmul(c < C - 1 ? me[c + 1] : me_up, tr[5][c]);
+    }
+    dnr = d_chain(xe);
+    float rowmax = 0.f;
+    auto cells = [&]() {
+      rowmax = fmaxf(fmaxf(fmaxf(fmaxf(xb, xe), xn), xj), xc);
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        const float mnext = c < C - 1 ? me[c + 1] : me_up, dnext = c < C - 1 ? dc[c + 1] : dnr;
+        mn[c] = fadd(fadd(fadd(fmul(mnext, tr[0][c]), fmul(iv[c], tr[1][c])), xe), fmul(dnext, tr[2][c]));
+        in_[c] = fadd(fmul(mnext, tr[3][c]), fmul(iv[c], tr[4][c]));
+        rowmax = fmaxf(rowmax, mn[c]);
+      }
+      // values are never negative, so their bit patterns order as integers
+      int mx = __reduce_max_sync(kFull, __float_as_int(rowmax));
+      if constexpr (MULTI) {
+        if (lane == 0) sh.mx[warp] = mx;
+        __syncthreads();
+        for (int q = 0; q < nw; q++) mx = max(mx, sh.mx[q]);
+      }
+      rowmax = __int_as_float(mx);
+    };
+    cells();
+    if constexpr (MULTI) {
+      if (sh.flag) {
+        dnr = d_again(xe);  // its barriers also order the reads of sh.mx above before the writes below
+        cells();
+        __syncthreads();
+        if (lead) sh.flag = 0;
+      }
+    }
+    float scale = 0.f, xb_o = xb;
+    if (rowmax > 1.0e4f) {
+      const float inv = __fdiv_rn(1.0f, rowmax);
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        mn[c] = fmul(mn[c], inv);
+        in_[c] = fmul(in_[c], inv);
+      }
+      xb_o = fmul(xb, inv);
+      xe = fmul(xe, inv);
+      xn = fmul(xn, inv);
+      xj = fmul(xj, inv);
+      xc = fmul(xc, inv);
+      scale = rowmax;
+    }
+    if (lead) {
+      float* o = orow + 6 * (int64_t)i;
+      o[0] = xn; o[1] = xb_o; o[2] = xe; o[3] = xj; o[4] = xc; o[5] = scale;
+    }
+#pragma unroll
+    for (int c = 0; c < C; c++) eo[c] = eon[c];
+    x = x1;
+    x1 = x2;
+  }
+  // row 0: the B sum with residue 1
+  b_terms(eo);
+  const float b0 = team_sum<MULTI>(T, nsum, sh);
+  if (lead) orow[1] = b0;
+}
+
+// Forward (blockIdx.y = 0) and Backward (1) rows of n pairs.  MULTI: a CTA per
+// pair; otherwise a warp per pair.  Dynamic shared memory: one row per team.
+template <int C, bool MULTI>
+__global__ void __launch_bounds__(256) exact_rows_kernel(const RowRec* __restrict__ recs, int n,
+                                                         const DevProfile* __restrict__ profs,
+                                                         const float* __restrict__ ximg,
+                                                         const uint8_t* __restrict__ res,
+                                                         const int64_t* __restrict__ toff,
+                                                         const int32_t* __restrict__ tlen,
+                                                         const float4* __restrict__ xsc, float* __restrict__ rows) {
+  extern __shared__ float4 sm_row[];
+  __shared__ XShared sh;
+  const int w = MULTI ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (w >= n) return;  // uniform over the team
+  float* T = reinterpret_cast<float*>(sm_row) + (MULTI ? 0 : (threadIdx.x >> 5) * 32 * C);
+  const RowRec r = recs[w];
+  const DevProfile& P = profs[r.p];
+  const float* img = ximg + P.x_off;
+  const int M = P.m, L = tlen[r.t];
+  const uint8_t* s = res + toff[r.t];
+  const float4 xs = xsc[r.t];
+  if (blockIdx.y == 0)
+    exact_forward<C, MULTI>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off, T, sh);
+  else
+    exact_backward<C, MULTI>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off + 6 * (int64_t)(L + 1), T, sh);
+}
+
+}  // namespace sxk

@@ -1,5 +1,5 @@
-// Instantiations of the warp-chunked kernels (warp-per-pair Viterbi, Forward,
-// the Forward pre-screen, Backward, the adjoint passes), one per column width.
+// Instantiations of the warp-chunked kernels (warp-per-pair Viterbi, the
+// Forward pre-screen, the adjoint passes), one per column width.
 #include "shapes.hpp"
 
 namespace sx {
@@ -8,9 +8,7 @@ template <int I>
 struct VbinTable {
   static void fill(KernelTables& t) {
     t.vit[I] = sxk::viterbi_kernel<kVcBins[I]>;
-    t.fwd[I] = sxk::forward_kernel<kVcBins[I]>;
-    t.fwd_scan[I] = sxk::forward_kernel<kVcBins[I], true>;
-    t.bwd[I] = sxk::backward_kernel<kVcBins[I]>;
+    t.fwd_scan[I] = sxk::forward_scan_kernel<kVcBins[I]>;
     t.adjf[I] = sxk::adjoint_forward_kernel<kVcBins[I]>;
     t.adjb[I] = sxk::adjoint_backward_kernel<kVcBins[I]>;
     VbinTable<I + 1>::fill(t);

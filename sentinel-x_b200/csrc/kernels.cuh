@@ -37,7 +37,8 @@ struct DevProfile {  // 88 bytes
   int32_t qv_shape;  // packed Viterbi pre-screen shape; -1: the profile is not pre-screened
   int64_t qv_off;    // uint4 offset of its quantized Viterbi image
   int32_t qv_cap;    // its row maxima above this (int16 units) pass at once
-  int32_t pad2;
+  int32_t xshape;    // shape of the exact row passes (index into kXShapes)
+  int64_t x_off;     // float offset of its row image
 };
 struct Thresholds {  // per profile, per search: pass iff statistic >= threshold (bits)
   float s1, s2, s3;
@@ -511,34 +512,28 @@ __global__ void __launch_bounds__(256) viterbi_kernel(
 }
 
 // ===========================================================================
-// Forward (src/hmmer/dp.rs:229-298), one warp per pair, probability space with
-// the reference's sparse rescaling.  M and I cells are computed in parallel;
-// the D chain and the row sum xe (both sequential in k in the reference) are
-// evaluated in order by passing a baton from lane to lane, so every rounding
-// matches.  Modes: rows != null writes the raw special rows (N B E J C, rescale
-// factor) per row i = 1..L; otherwise the pair passes when the device estimate
-// of the F3 statistic clears the threshold minus `slack`.
+// Forward pre-screen of F3 (src/hmmer/dp.rs:229-298), one warp per pair,
+// probability space with the reference's sparse rescaling; the pair passes when
+// the device estimate of the F3 statistic clears the threshold minus `slack`.
 //
-// SCAN (the F3 pre-screen only): the D chain is an affine recurrence
-// D[k] = a_k + D[k-1] p_k, so each lane forms its transfer (A, B) over its
-// columns, a Kogge-Stone scan of 5 shuffles composes them across lanes, each
-// lane re-runs its columns from the true carry-in, and the row sum is a
-// butterfly.  A row's dependent depth falls from ~2M to ~6 VC operations.  The
-// rounding differs from the reference's order, so the pass test adds a bound
-// on the difference: for sums and products of non-negative numbers the
-// relative errors of two evaluation orders add up along their longest paths,
-// at most 2^-24 per operation, i.e. |ln F_scan - ln F_ref| <=
-// (L+1)(2M + 6 VC + 64) 2^-24, taken twice.  The pre-screen therefore passes
-// every pair the exact F3 test (on the host, from exact rows) passes.
+// The D chain is an affine recurrence D[k] = a_k + D[k-1] p_k, so each lane
+// forms its transfer (A, B) over its columns, a Kogge-Stone scan of 5 shuffles
+// composes them across lanes, each lane re-runs its columns from the true
+// carry-in, and the row sum is a butterfly.  The rounding differs from the
+// reference's order, so the pass test adds a bound on the difference: for sums
+// and products of non-negative numbers the relative errors of two evaluation
+// orders add up along their longest paths, at most 2^-24 per operation, i.e.
+// |ln F_scan - ln F_ref| <= (L+1)(2M + 6 VC + 64) 2^-24, taken twice.  The
+// pre-screen therefore passes every pair the exact F3 test (on the host, from
+// the exact rows of exact_rows.cuh) passes.
 // ===========================================================================
-template <int VC, bool SCAN = false>
-__global__ void __launch_bounds__(256) forward_kernel(
+template <int VC>
+__global__ void __launch_bounds__(256) forward_scan_kernel(
     const PairRec* __restrict__ in, const unsigned* __restrict__ in_counts, const BinRegion* __restrict__ in_bins,
     int bin, PairRec* __restrict__ out, const BinRegion* __restrict__ out_bins, unsigned* __restrict__ out_counts,
     unsigned* __restrict__ overflow, const DevProfile* __restrict__ profs, const Thresholds* __restrict__ thr,
     const float* __restrict__ vfb, const uint8_t* __restrict__ res, const int64_t* __restrict__ toff,
-    const int32_t* __restrict__ tlen, const float4* __restrict__ xsc, float slack, float* __restrict__ rows,
-    const int64_t* __restrict__ row_off) {
+    const int32_t* __restrict__ tlen, const float4* __restrict__ xsc, float slack) {
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   const unsigned n = min(in_counts[bin], in_bins[bin].cap);
@@ -552,7 +547,6 @@ __global__ void __launch_bounds__(256) forward_kernel(
     const int L = tlen[r.t];
     const float4 xs = xsc[r.t];
     const float ploop = xs.z, pmove = xs.w;
-    float* orow = rows ? rows + row_off[in_bins[bin].off + w] : nullptr;
     TransRows<VC> tr;
     tr.load(img, kRowFwd, lane);
     float mp[VC], ip[VC], dp[VC], eo[VC];
@@ -594,7 +588,7 @@ __global__ void __launch_bounds__(256) forward_kernel(
         pdd[c] = tr.get(img, kRowFwd, 7, c, lane);
       }
       float dcar = 0.f, xe = 0.f;
-      if constexpr (SCAN) {
+      {
         // lane transfer D_out = A + B D_in, then an inclusive scan over lanes
         float A = 0.f, B = 1.f;
 #pragma unroll
@@ -623,21 +617,6 @@ __global__ void __launch_bounds__(256) forward_kernel(
 #pragma unroll
         for (int o = 16; o >= 1; o >>= 1) xl = fadd(xl, __shfl_xor_sync(kFull, xl, o));
         xe = xl;
-      } else {
-        // ordered D chain and row sum: dc[k] = a_k + dc[k-1]*p_dd[k-1]; xe += mv + dc
-        for (int sl = 0; sl < nl; sl++) {
-          if (lane == sl) {
-#pragma unroll
-            for (int c = 0; c < VC; c++) {
-              const float d = fadd(a[c], fmul(dcar, pdd[c]));
-              dv[c] = d;
-              xe = fadd(xe, fadd(mv[c], d));
-              dcar = d;
-            }
-          }
-          dcar = __shfl_sync(kFull, dcar, sl);
-          xe = __shfl_sync(kFull, xe, sl);
-        }
       }
       if (lane >= nl) {
 #pragma unroll
@@ -647,7 +626,6 @@ __global__ void __launch_bounds__(256) forward_kernel(
       xc = fadd(fmul(xc, ploop), fmul(xe, 0.5f));
       xn = fmul(xn, ploop);
       xb = fadd(fmul(xn, pmove), fmul(xj, pmove));
-      float scale = 0.f;
       if (xe > 1.0e4f) {
         const float inv = __fdiv_rn(1.0f, xe);
 #pragma unroll
@@ -661,12 +639,6 @@ __global__ void __launch_bounds__(256) forward_kernel(
         xj = fmul(xj, inv);
         xc = fmul(xc, inv);
         lnscale += log((double)xe);
-        scale = xe;
-        xe = 1.0f;
-      }
-      if (orow && lane == 0) {
-        float* o = orow + 6 * (i + 1);
-        o[0] = xn; o[1] = xb; o[2] = xe; o[3] = xj; o[4] = xc; o[5] = scale;
       }
 #pragma unroll
       for (int c = 0; c < VC; c++) {
@@ -681,214 +653,8 @@ __global__ void __launch_bounds__(256) forward_kernel(
       const float v = fmul(xc, pmove);
       const float fsc = (L > 0 && M > 0) ? (float)((double)(v > 0.f ? logf(v) : SX_NEG_INF) + lnscale) : SX_NEG_INF;
       r.fwd = fsc;
-      const float sl = SCAN ? slack + 2.0f * (float)(L + 1) * (float)(2 * M + 6 * VC + 64) * 5.9604645e-8f / kLn2 : slack;
-      if (!rows && bits_stat(fsc, r.filtersc) >= thr[r.p].s3 - sl) push_pair(r, bin, out, out_bins, out_counts, overflow);
-    }
-  }
-}
-
-// ===========================================================================
-// Backward (src/hmmer/dp.rs:301-392), one warp per pair.  The B sum (ascending
-// in k) and the D chain (descending in k) are sequential in the reference and
-// are evaluated by lane batons; every other cell is parallel.  Writes the raw
-// special rows: row L (E, C), rows L-1..1 (N B E J C, rescale factor) and the
-// row-0 B sum in slot 1 of row 0.
-// ===========================================================================
-template <int VC>
-__global__ void __launch_bounds__(256) backward_kernel(
-    const PairRec* __restrict__ in, const unsigned* __restrict__ in_counts, const BinRegion* __restrict__ in_bins,
-    int bin, const DevProfile* __restrict__ profs, const float* __restrict__ vfb, const uint8_t* __restrict__ res,
-    const int64_t* __restrict__ toff, const int32_t* __restrict__ tlen, const float4* __restrict__ xsc,
-    float* __restrict__ rows, const int64_t* __restrict__ row_off) {
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  const unsigned n = min(in_counts[bin], in_bins[bin].cap);
-  for (unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += warps) {
-    const PairRec r = in[in_bins[bin].off + w];
-    const DevProfile P = profs[r.p];
-    const Img<VC> img{vfb + P.vfb_off};
-    const int M = P.m;
-    const int nl = (M + VC - 1) / VC;
-    const int lM = (M - 1) / VC;  // lane holding column M
-    const uint8_t* s = res + toff[r.t];
-    const int L = tlen[r.t];
-    const float4 xs = xsc[r.t];
-    const float ploop = xs.z, pmove = xs.w;
-    float* orow = rows + row_off[in_bins[bin].off + w];
-    float mn[VC], in_[VC], dn[VC];
-    // row L
-    float xc = pmove;
-    float xe = fmul(xc, 0.5f);
-    float xj = 0.f, xn = 0.f;
-    {
-      float pmd0[VC], pdd0[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        pmd0[c] = img.at(kRowBwd + 2, c, lane);
-        pdd0[c] = img.at(kRowBwd + 6, c, lane);
-      }
-      float dcar = 0.f;
-      for (int sl = lM; sl >= 0; sl--) {
-        if (lane == sl) {
-#pragma unroll
-          for (int c = VC - 1; c >= 0; c--) {
-            const int k = lane * VC + c + 1;
-            if (k > M) {
-              mn[c] = dn[c] = 0.f;
-            } else if (k == M) {
-              mn[c] = dn[c] = xe;
-              dcar = xe;
-            } else {
-              mn[c] = fadd(xe, fmul(dcar, pmd0[c]));
-              dn[c] = fadd(xe, fmul(dcar, pdd0[c]));
-              dcar = dn[c];
-            }
-          }
-        }
-        dcar = __shfl_sync(kFull, dcar, sl);
-      }
-      if (lane > lM) {
-#pragma unroll
-        for (int c = 0; c < VC; c++) mn[c] = dn[c] = 0.f;
-      }
-#pragma unroll
-      for (int c = 0; c < VC; c++) in_[c] = 0.f;
-    }
-    if (lane == 0 && L > 0) {
-      float* o = orow + 6 * L;
-      o[0] = 0.f; o[1] = 0.f; o[2] = xe; o[3] = 0.f; o[4] = xc; o[5] = 0.f;
-    }
-    double lnscale = 0.0;
-    for (int i = L - 1; i >= 1; i--) {
-      const int x = __ldg(s + i);
-      const float ins = x != 24 ? 1.f : 0.f;
-      float eo[VC], me[VC], bt[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        eo[c] = img.at(kRowMo + x, c, lane);
-        me[c] = fmul(mn[c], eo[c]);
-        bt[c] = fmul(fmul(mn[c], img.at(kRowBwd + 7, c, lane)), eo[c]);
-      }
-      // B sum, ascending k
-      float b = 0.f;
-      for (int sl = 0; sl < nl; sl++) {
-        if (lane == sl) {
-#pragma unroll
-          for (int c = 0; c < VC; c++) b = fadd(b, bt[c]);
-        }
-        b = __shfl_sync(kFull, b, sl);
-      }
-      const float xb = b;
-      xj = fadd(fmul(xj, ploop), fmul(xb, pmove));
-      xc = fmul(xc, ploop);
-      xe = fadd(fmul(xj, 0.5f), fmul(xc, 0.5f));
-      xn = fadd(fmul(xn, ploop), fmul(xb, pmove));
-      float rowmax = fmaxf(fmaxf(fmaxf(fmaxf(xb, xe), xn), xj), xc);
-      // mnext[k] = mn[k+1]*eo[k+1]
-      const float me_up = __shfl_down_sync(kFull, me[0], 1);
-      float mnext[VC], iv[VC], mc[VC], ic[VC], dc[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        mnext[c] = c < VC - 1 ? me[c + 1] : (lane < 31 ? me_up : 0.f);
-        iv[c] = fmul(in_[c], ins);
-      }
-      float pdm[VC], pdd[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        pdm[c] = img.at(kRowBwd + 5, c, lane);
-        pdd[c] = img.at(kRowBwd + 6, c, lane);
-      }
-      // D chain, descending k
-      float dcar = 0.f;
-      for (int sl = lM; sl >= 0; sl--) {
-        if (lane == sl) {
-#pragma unroll
-          for (int c = VC - 1; c >= 0; c--) {
-            const int k = lane * VC + c + 1;
-            if (k > M) {
-              dc[c] = 0.f;
-            } else if (k == M) {
-              dc[c] = xe;
-              dcar = xe;
-            } else {
-              dc[c] = fadd(fadd(fmul(mnext[c], pdm[c]), fmul(dcar, pdd[c])), xe);
-              dcar = dc[c];
-            }
-          }
-        }
-        dcar = __shfl_sync(kFull, dcar, sl);
-      }
-      if (lane > lM) {
-#pragma unroll
-        for (int c = 0; c < VC; c++) dc[c] = 0.f;
-      }
-      const float dc_up = __shfl_down_sync(kFull, dc[0], 1);
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        const int k = lane * VC + c + 1;
-        const float dnext = c < VC - 1 ? dc[c + 1] : (lane < 31 ? dc_up : 0.f);
-        if (k < M) {
-          const float mv = fadd(fadd(fadd(fmul(mnext[c], img.at(kRowBwd + 0, c, lane)), fmul(iv[c], img.at(kRowBwd + 1, c, lane))), xe),
-                                fmul(dnext, img.at(kRowBwd + 2, c, lane)));
-          mc[c] = mv;
-          ic[c] = fadd(fmul(mnext[c], img.at(kRowBwd + 3, c, lane)), fmul(iv[c], img.at(kRowBwd + 4, c, lane)));
-          rowmax = fmaxf(rowmax, mv);
-        } else if (k == M) {
-          mc[c] = xe;
-          ic[c] = 0.f;
-        } else {
-          mc[c] = 0.f;
-          ic[c] = 0.f;
-        }
-      }
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) rowmax = fmaxf(rowmax, __shfl_xor_sync(kFull, rowmax, o));
-      float scale = 0.f;
-      float xb_o = xb;
-      if (rowmax > 1.0e4f) {
-        const float inv = __fdiv_rn(1.0f, rowmax);
-#pragma unroll
-        for (int c = 0; c < VC; c++) {
-          mc[c] = fmul(mc[c], inv);
-          ic[c] = fmul(ic[c], inv);
-          dc[c] = fmul(dc[c], inv);
-        }
-        xb_o = fmul(xb, inv);
-        xe = fmul(xe, inv);
-        xn = fmul(xn, inv);
-        xj = fmul(xj, inv);
-        xc = fmul(xc, inv);
-        lnscale += log((double)rowmax);
-        scale = rowmax;
-      }
-      if (lane == 0) {
-        float* o = orow + 6 * i;
-        o[0] = xn; o[1] = xb_o; o[2] = xe; o[3] = xj; o[4] = xc; o[5] = scale;
-      }
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        mn[c] = mc[c];
-        in_[c] = ic[c];
-        dn[c] = dc[c];
-      }
-    }
-    // row 0: B sum with residue 1
-    if (L > 0) {
-      const int x0 = __ldg(s);
-      float bt[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) bt[c] = fmul(fmul(mn[c], img.at(kRowBwd + 7, c, lane)), img.at(kRowMo + x0, c, lane));
-      float b = 0.f;
-      for (int sl = 0; sl < nl; sl++) {
-        if (lane == sl) {
-#pragma unroll
-          for (int c = 0; c < VC; c++) b = fadd(b, bt[c]);
-        }
-        b = __shfl_sync(kFull, b, sl);
-      }
-      if (lane == 0) {
-        orow[0] = 0.f; orow[1] = b; orow[2] = 0.f; orow[3] = 0.f; orow[4] = 0.f; orow[5] = 0.f;
-      }
+      const float sl = slack + 2.0f * (float)(L + 1) * (float)(2 * M + 6 * VC + 64) * 5.9604645e-8f / kLn2;
+      if (bits_stat(fsc, r.filtersc) >= thr[r.p].s3 - sl) push_pair(r, bin, out, out_bins, out_counts, overflow);
     }
   }
 }

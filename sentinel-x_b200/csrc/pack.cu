@@ -70,6 +70,13 @@ int warp_ctas(int num_sms, unsigned n) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)n, (int64_t)num_sms * 32));
 }
 
+// Exact row pass shape of a profile: the narrowest that covers M.
+int choose_xshape(int m) {
+  for (int s = 0; s < kNumXShapes; s++)
+    if (xwidth(s) >= m) return s;
+  return -1;
+}
+
 int choose_vbin(int m) {
   const int need = (m + 31) / 32;
   for (int b = 0; b < kNumVbins; b++)
@@ -197,6 +204,27 @@ void pack_images(const ProfileHost& h, const DevProfile& d, float4* msv, float4*
   }
 }
 
+// Row image of the exact row passes (exact_rows.cuh): kXRows rows of the
+// shape's width, column k at k - 1, zero past column M and for the transitions
+// node M does not have.
+void pack_ximage(const ProfileHost& h, const DevProfile& d, float* out) {
+  const int m = h.m, w = xwidth(d.xshape);
+  float* base = out + d.x_off;
+  auto put = [&](int r, const float* src, int n) {  // columns 1..n from src[0..n)
+    float* o = base + (size_t)r * w;
+    std::copy(src, src + n, o);
+    std::fill(o + n, o + w, 0.0f);
+  };
+  for (int x = 0; x < 25; x++) put(sxk::kXMo + x, h.mo_row(x) + 1, m);
+  const auto& p = h.p;
+  const int fwd[8] = {TBM, TMM, TIM, TDM, TMI, TII, TMD, TDD};
+  const bool at_k[8] = {true, false, false, false, true, true, false, false};  // else the transition out of k - 1
+  for (int q = 0; q < 8; q++)
+    put(sxk::kXFwd + q, p[fwd[q]].data() + (at_k[q] ? 1 : 0), q == 4 || q == 5 ? std::max(m - 1, 0) : m);
+  const int bwd[8] = {TMM, TMI, TMD, TIM, TII, TDM, TDD, TBM};
+  for (int q = 0; q < 8; q++) put(sxk::kXBwd + q, p[bwd[q]].data() + 1, q < 7 ? std::max(m - 1, 0) : m);
+}
+
 // Quantized MSV image of the packed pre-screen (prescreen.cuh): the match
 // scores in units of 2^-9 nat rounded up after adding 2^-12 nat, clamped up to
 // -16 nats (-inf included), -32 nats past column M, in the lane-major chunk
@@ -322,7 +350,7 @@ void pack_profiles(sx_profiles* P) {
   const size_t np = P->h.size();
   P->dp.resize(np);
   P->msv_shape.resize(np);
-  int64_t msv_total = 0, vfb_total = 0, vit_total = 0, q_total = 0, qv_total = 0;
+  int64_t msv_total = 0, vfb_total = 0, vit_total = 0, q_total = 0, qv_total = 0, x_total = 0;
   for (size_t i = 0; i < np; i++) {
     const ProfileHost& h = P->h[i];
     DevProfile& d = P->dp[i];
@@ -331,7 +359,8 @@ void pack_profiles(sx_profiles* P) {
     d.msv_tbm = h.msv_tbm;
     if (is_long(h.m)) {  // no warp-chunked, MSV or Viterbi images: the long kernels read the plain image
       P->msv_shape[i] = -1;
-      d.vbin = d.vshape = -1;
+      d.vbin = d.vshape = d.xshape = -1;
+      d.x_off = x_total;
       d.msv_off = msv_total;
       d.vfb_off = vfb_total;
       d.vit_off = vit_total;
@@ -355,6 +384,9 @@ void pack_profiles(sx_profiles* P) {
     d.q_tbm = (int32_t)std::ceil(((double)h.msv_tbm + std::ldexp(1.0, -17)) * 1048576.0);
     d.vfb_off = vfb_total;
     vfb_total += (int64_t)sxk::kImgRows * 32 * d.vc;
+    d.xshape = choose_xshape(h.m);
+    d.x_off = x_total;
+    x_total += (int64_t)sxk::kXRows * xwidth(d.xshape);
     d.vshape = shape_for(P->eng, 1, h.m);
     if (d.vshape < 0) throw CudaError{SX_EINVAL, "profile '" + h.name + "' too long for the Viterbi shapes"};
     d.vit_off = vit_total;
@@ -368,13 +400,14 @@ void pack_profiles(sx_profiles* P) {
   }
   std::vector<float4> msv((size_t)msv_total);
   std::vector<float4> vit((size_t)std::max<int64_t>(vit_total, 1));
-  std::vector<float> vfb((size_t)vfb_total);
+  std::vector<float> vfb((size_t)vfb_total), ximg((size_t)std::max<int64_t>(x_total, 1));
   std::vector<double> bias(np * 54);
   std::vector<uint2> qimg((size_t)std::max<int64_t>(q_total, 1));
   std::vector<uint4> qvimg((size_t)std::max<int64_t>(qv_total, 1));
   for (size_t i = 0; i < np; i++) {
     if (P->dp[i].vbin >= 0) {
       pack_images(P->h[i], P->dp[i], msv.data(), vit.data(), vfb.data());
+      pack_ximage(P->h[i], P->dp[i], ximg.data());
       // a profile whose rounded scores leave less than half of the int16
       // range as headroom (scores above +16 nats) stays on the exact kernel
       const int emax = pack_qimage(P->h[i], P->dp[i], qimg.data());
@@ -427,6 +460,7 @@ void pack_profiles(sx_profiles* P) {
   P->d_qvimg.upload(qvimg.data(), qvimg.size(), s);
   P->d_vit.upload(vit.data(), vit.size(), s);
   P->d_vfb.upload(vfb.data(), vfb.size(), s);
+  P->d_x.upload(ximg.data(), ximg.size(), s);
   P->d_bias.upload(bias.data(), bias.size(), s);
   CK(cudaStreamSynchronize(s));
 }

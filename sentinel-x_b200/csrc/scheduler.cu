@@ -62,111 +62,115 @@ int64_t scratch_budget(const sx_engine* E, int64_t want) {
 }
 
 
-// Row passes of a block's final pairs queued without waiting: when all of
-// their rows fit one chunk, the kernels go to slot S's high-priority streams
-// with the slot's own row buffers and the call returns a fetch function; a
-// host job calls it, which waits for the kernels, copies the rows out on the
-// slot's copy stream, adds the passes' device time to *dev_ms and releases
-// the buffers.  Returns an empty function when the rows need more than one
-// chunk (the caller then takes the synchronous rows_pass).
-constexpr int kRowsWarps = 8;  // warps (pairs) per CTA of the asynchronous row passes
-std::function<RowsChunk()> rows_pass_async(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T,
-                                           const std::vector<FinalPair>& pairs, std::mutex* ms_mu, double* dev_ms) {
-  const auto& K = kernels();
-  const int64_t row_budget = std::max<int64_t>(scratch_budget(E, E->batch_bytes / 2) / (int64_t)sizeof(float), 1 << 20);
-  int64_t ro = 0;
-  for (const FinalPair& f : pairs) ro += 6 * ((int64_t)T->len[f.t] + 1);
-  if (pairs.empty() || ro > row_budget) return {};
-  if (S.rows_busy) S.rows_busy->wait();  // an earlier block's rows are still being read
-  std::vector<std::vector<size_t>> byb(kNumVbins);
-  for (size_t i = 0; i < pairs.size(); i++) byb[P->dp[pairs[i].p].vbin].push_back(i);
-  // longest first: the warps of a CTA then carry similar lengths, and the
-  // longest chains start first
-  for (auto& v : byb)
-    std::stable_sort(v.begin(), v.end(), [&](size_t a, size_t b) { return T->len[pairs[a].t] > T->len[pairs[b].t]; });
-  std::vector<PairRec> recs;
-  auto c = std::make_shared<RowsChunk>();
-  std::vector<BinRegion> reg(kNumVbins);
-  std::vector<unsigned> cnt(kNumVbins, 0);
-  ro = 0;
-  for (int b = 0; b < kNumVbins; b++) {
-    reg[b].off = (int64_t)recs.size();
-    reg[b].cap = (uint32_t)byb[b].size();
-    reg[b].pad = 0;
-    cnt[b] = (unsigned)byb[b].size();
-    for (size_t i : byb[b]) {
-      const FinalPair& f = pairs[i];
-      recs.push_back({f.p, f.t, f.usc, f.filtersc, f.vsc, 0.f, f.slot, 0});
-      c->off.push_back(ro);
-      c->which.push_back(i);
-      ro += 6 * ((int64_t)T->len[f.t] + 1);
+// The device layout of the row passes of pairs [i0, i1): records grouped by
+// shape, longest first within one, so the warps of a CTA carry similar lengths
+// and the longest chains start first.
+RowsChunk plan_rows(const sx_profiles* P, const sx_targets* T, const std::vector<FinalPair>& pairs, size_t i0, size_t i1) {
+  RowsChunk c;
+  std::vector<std::vector<size_t>> by(kNumXShapes);
+  for (size_t i = i0; i < i1; i++) by[P->dp[pairs[i].p].xshape].push_back(i);
+  for (int s = 0; s < kNumXShapes; s++) {
+    std::stable_sort(by[s].begin(), by[s].end(), [&](size_t a, size_t b) { return T->len[pairs[a].t] > T->len[pairs[b].t]; });
+    c.first[s] = c.recs.size();
+    for (size_t i : by[s]) {
+      const int l = T->len[pairs[i].t];
+      c.recs.push_back({pairs[i].p, pairs[i].t, c.floats});
+      c.which.push_back(i);
+      c.boff.push_back(c.floats + 6 * ((int64_t)l + 1));
+      c.floats += row_floats(l);
+      c.longest[s] = std::max(c.longest[s], l);
     }
   }
+  c.first[kNumXShapes] = c.recs.size();
+  return c;
+}
+
+// Queues the passes of a planned chunk on slot S's high-priority streams, into
+// its own row buffer.  Each launch lasts about its longest chain (rows x
+// columns of its longest pair); the launches go longest first to the
+// least-loaded auxiliary stream, so the long shapes start at once and the
+// short ones queue behind other short ones.
+// The passes are latency-bound chains that run for milliseconds beside the
+// next block's MSV: packed kRowsWarps to a CTA the one-warp teams hold the
+// registers of a few SMs instead of one MSV CTA slot on nearly every SM.
+constexpr int kRowsWarps = 8;
+void queue_rows(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T, const RowsChunk& c) {
+  const auto& K = kernels();
   cudaStream_t s = S.hi.main;
-  S.rrecs.upload(recs.data(), recs.size(), s);
-  S.roff.upload(c->off.data(), c->off.size(), s);
-  S.rbins.upload(reg.data(), reg.size(), s);
-  S.rcnt.upload(cnt.data(), cnt.size(), s);
-  S.rows_f.alloc((size_t)ro);
-  S.rows_b.alloc((size_t)ro);
-  CK(cudaEventRecord(S.rows_t0, s));
-  // rows the kernels never touch are zero
-  CK(cudaMemsetAsync(S.rows_f.p, 0, sizeof(float) * (size_t)ro, s));
-  CK(cudaMemsetAsync(S.rows_b.p, 0, sizeof(float) * (size_t)ro, s));
-  // Each launch lasts about its longest chain (rows x columns of its
-  // longest pair); the launches go longest first to the least-loaded
-  // auxiliary stream, so the long bins start at once and the short ones
-  // queue behind other short ones
-  std::vector<double> load(S.hi.naux, 0.0);
-  auto pick_stream = [&](double est) {
-    const int a = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-    load[a] += est;
-    return S.hi.aux[a];
-  };
+  S.rrecs.upload(c.recs.data(), c.recs.size(), s);
+  S.rows.alloc((size_t)c.floats);
   std::vector<std::pair<double, int>> order;
-  for (int b = 0; b < kNumVbins; b++) {
-    if (!cnt[b]) continue;
-    int64_t longest = 0;
-    for (size_t i : byb[b]) longest = std::max<int64_t>(longest, T->len[pairs[i].t]);
-    order.emplace_back((double)longest * kVcBins[b], b);
-  }
+  for (int x = 0; x < kNumXShapes; x++)
+    if (c.first[x + 1] > c.first[x]) order.emplace_back((double)c.longest[x] * xwidth(x), x);
   std::stable_sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
   fork_aux(S.hi);
-  for (const auto& ob : order) {
-    const int b = ob.second;
-    // The row passes are latency-bound chains that run for milliseconds
-    // beside the next block's MSV: packed kRowsWarps to a CTA they hold the
-    // registers of a few SMs instead of one MSV CTA slot on nearly every SM.
-    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)cnt[b] + kRowsWarps - 1) / kRowsWarps,
-                                                                   (int64_t)E->num_sms * 32 / kRowsWarps));
-    cudaStream_t sa = pick_stream(ob.first), sb = pick_stream(ob.first);
-    K.fwd[b]<<<blocks, 32 * kRowsWarps, 0, sa>>>(S.rrecs.p, S.rcnt.p, S.rbins.p, b, nullptr, nullptr, nullptr, S.overflow.p,
-                                     P->d_prof.p, E->thr.p, P->d_vfb.p, T->d_res.p, T->d_off.p, T->d_len.p,
-                                     T->d_xsc.p, 0.f, S.rows_f.p, S.roff.p);
-    K.bwd[b]<<<blocks, 32 * kRowsWarps, 0, sb>>>(S.rrecs.p, S.rcnt.p, S.rbins.p, b, P->d_prof.p, P->d_vfb.p, T->d_res.p,
-                                     T->d_off.p, T->d_len.p, T->d_xsc.p, S.rows_b.p, S.roff.p);
-    E->stats.kernel_launches += 2;
+  std::vector<double> load(S.hi.naux, 0.0);
+  for (const auto& o : order) {
+    const int x = o.second, n = (int)(c.first[x + 1] - c.first[x]);
+    const XShape& sh = kXShapes[x];
+    const int a = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    load[a] += o.first;
+    const int teams = sh.warps > 1 ? 1 : kRowsWarps;  // per CTA
+    const dim3 grid((unsigned)((n + teams - 1) / teams), 2);
+    K.xrows[x]<<<grid, 32 * teams * sh.warps, sizeof(float) * (size_t)teams * xwidth(x), S.hi.aux[a]>>>(
+        S.rrecs.p + c.first[x], n, P->d_prof.p, P->d_x.p, T->d_res.p, T->d_off.p, T->d_len.p, T->d_xsc.p, S.rows.p);
+    E->stats.kernel_launches++;
   }
   CK(cudaGetLastError());
   join_aux(S.hi);
-  CK(cudaEventRecord(S.rows_t1, s));
+}
+
+int64_t rows_budget(const sx_engine* E) {
+  return std::max<int64_t>(scratch_budget(E, E->batch_bytes) / (int64_t)sizeof(float), 2 << 20);
+}
+
+void rows_pass(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T, const std::vector<FinalPair>& pairs,
+               const std::function<void(RowsChunk&&)>& consume) {
+  const int64_t budget = rows_budget(E);
+  for (size_t i0 = 0, i1 = 0; i0 < pairs.size(); i0 = i1) {
+    int64_t used = 0;
+    for (; i1 < pairs.size(); i1++) {
+      const int64_t need = row_floats(T->len[pairs[i1].t]);
+      if (i1 > i0 && used + need > budget) break;
+      used += need;
+    }
+    RowsChunk c = plan_rows(P, T, pairs, i0, i1);
+    if (S.rows_busy) S.rows_busy->wait();  // an earlier block's rows are still being read
+    queue_rows(E, S, P, T, c);
+    c.fetch(E->row_bytes, S.rows.p, S.hi.main);
+    consume(std::move(c));
+  }
+}
+
+// Row passes of a block's final pairs queued without waiting: when all of
+// their rows fit one chunk, the kernels go to slot S's high-priority streams
+// with the slot's own row buffer and the call returns a fetch function; a
+// host job calls it, which waits for the kernels, copies the rows out on the
+// slot's copy stream, adds the passes' device time to *dev_ms and releases
+// the buffer.  Returns an empty function when the rows need more than one
+// chunk (the caller then takes the synchronous rows_pass).
+std::function<RowsChunk()> rows_pass_async(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T,
+                                           const std::vector<FinalPair>& pairs, std::mutex* ms_mu, double* dev_ms) {
+  int64_t floats = 0;
+  for (const FinalPair& f : pairs) floats += row_floats(T->len[f.t]);
+  if (pairs.empty() || floats > rows_budget(E)) return {};
+  if (S.rows_busy) S.rows_busy->wait();  // an earlier block's rows are still being read
+  auto c = std::make_shared<RowsChunk>(plan_rows(P, T, pairs, 0, pairs.size()));
+  CK(cudaEventRecord(S.rows_t0, S.hi.main));
+  queue_rows(E, S, P, T, *c);
+  CK(cudaEventRecord(S.rows_t1, S.hi.main));
   auto ticket = std::make_shared<RowsTicket>();
   S.rows_busy = ticket;
   Slot* SP = &S;
-  const int device = E->device;
-  return [SP, c, ro, ticket, ms_mu, dev_ms, device]() -> RowsChunk {
-    struct Release {  // the buffers are free again, even if a copy failed
+  return [E, SP, c, ticket, ms_mu, dev_ms]() -> RowsChunk {
+    struct Release {  // the buffer is free again, even if a copy failed
       RowsTicket& t;
       ~Release() { t.set(); }
     } rel{*ticket};
     Slot& S = *SP;
-    CK(cudaSetDevice(device));
+    CK(cudaSetDevice(E->device));
     CK(cudaStreamWaitEvent(S.rows_copy, S.rows_t1, 0));
-    c->f.resize((size_t)ro);
-    c->b.resize((size_t)ro);
-    CK(cudaMemcpyAsync(c->f.data(), S.rows_f.p, sizeof(float) * (size_t)ro, cudaMemcpyDeviceToHost, S.rows_copy));
-    CK(cudaMemcpyAsync(c->b.data(), S.rows_b.p, sizeof(float) * (size_t)ro, cudaMemcpyDeviceToHost, S.rows_copy));
-    CK(cudaStreamSynchronize(S.rows_copy));
+    c->fetch(E->row_bytes, S.rows.p, S.rows_copy);
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, S.rows_t0, S.rows_t1) != cudaSuccess) cudaGetLastError();
     {
@@ -529,7 +533,7 @@ void launch_stage(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets*
         K.fwd_scan[b]<<<warp_ctas(E->num_sms, nin[b]), 32, 0, s>>>(S.lists[2].p, cin, S.bins[2].p, b, S.lists[3].p,
                                                                S.bins[3].p, cout,
                                         S.overflow.p, P->d_prof.p, E->thr.p, P->d_vfb.p, T->d_res.p, T->d_off.p,
-                                        T->d_len.p, T->d_xsc.p, kSlackBits, nullptr, nullptr);
+                                        T->d_len.p, T->d_xsc.p, kSlackBits);
       E->stats.kernel_launches++;
     }
     join_aux(S.hi);
@@ -1101,8 +1105,8 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
               const FinalPair& f = B->finals[i];
               const ProfileHost& h = P->h[f.p];
               const int64_t l = T->len[f.t];
-              const float* fr = ch->f.data() + ch->off[q];
-              const float* br = ch->b.data() + ch->off[q];
+              const float* fr = ch->fwd(q);
+              const float* br = ch->bwd(q);
               const float fwdsc = forward_score_from_rows(h, l, fr);
               if (th[f.p].exact &&
                   std::exp(exp_tail_logsurv((double)((fwdsc - f.filtersc) / kLn2f), h.fwd[0], h.fwd[1])) > o.f3)
@@ -1127,8 +1131,8 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
             const FinalPair& f = B->finals[ch->which[q]];
             const ProfileHost& h = P->h[f.p];
             const int64_t l = T->len[f.t];
-            const float* fr = ch->f.data() + ch->off[q];
-            const float* br = ch->b.data() + ch->off[q];
+            const float* fr = ch->fwd(q);
+            const float* br = ch->bwd(q);
             const float fwdsc = forward_score_from_rows(h, l, fr);
             if (th[f.p].exact &&
                 std::exp(exp_tail_logsurv((double)((fwdsc - f.filtersc) / kLn2f), h.fwd[0], h.fwd[1])) > o.f3)

@@ -300,7 +300,7 @@ int sx_score_prescreens(sx_engine* e, const sx_profiles* p, const sx_targets* t,
           K.fwd_scan[b]<<<warp_ctas(e->num_sms, cnt[b]), 32, 0, s>>>(
               S.lists[2].p, e->counts.p + 2 * kMaxBins, S.bins[2].p, b, S.lists[3].p, S.bins[3].p,
               e->counts.p + 3 * kMaxBins, e->overflow.p, p->d_prof.p, e->thr.p, p->d_vfb.p, t->d_res.p, t->d_off.p,
-              t->d_len.p, t->d_xsc.p, kSlackBits, nullptr, nullptr);
+              t->d_len.p, t->d_xsc.p, kSlackBits);
         }
         CK(cudaGetLastError());
         std::vector<PairRec> out(recs.size());

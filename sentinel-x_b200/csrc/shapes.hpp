@@ -1,7 +1,7 @@
 // Kernel shapes compiled into the library and the per-shape launch tables.
 //
 // The template instantiations live in their own translation units
-// (k_msv.cu, k_msv16.cu, k_vit.cu, k_vit16.cu, k_vbin.cu, k_env.cu) so the library builds in
+// (k_msv.cu, k_msv16.cu, k_vit.cu, k_vit16.cu, k_vbin.cu, k_exact.cu, k_env.cu) so the library builds in
 // parallel; the host translation units launch them through the function-pointer tables
 // filled here.
 #pragma once
@@ -10,6 +10,7 @@
 #include "kernels.cuh"
 #include "adjoint.cuh"
 #include "envelope.cuh"
+#include "exact_rows.cuh"
 #include "prescreen.cuh"
 
 namespace sx {
@@ -76,6 +77,19 @@ constexpr int vit16_threads(const Vit16Shape&) { return 128; }
 constexpr int kVcBins[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
 constexpr int kNumVbins = sizeof(kVcBins) / sizeof(kVcBins[0]);
 
+// Exact row passes (exact_rows.cuh): columns per thread and warps per team; a
+// profile takes the narrowest shape that covers M.  A row's latency is its
+// ordered sum (4 cycles a column whatever the shape) plus the D chain and the
+// exchange between lanes: 4 columns a lane keep the chain's rounds short while
+// one warp suffices, 8 halve the warps (and their barriers) above that.
+struct XShape {
+  int c, warps;
+};
+constexpr XShape kXShapes[] = {{4, 1}, {8, 1}, {8, 2}, {8, 3}, {8, 4}, {8, 6}, {8, 8}};
+constexpr int kNumXShapes = sizeof(kXShapes) / sizeof(kXShapes[0]);
+constexpr int xwidth(int s) { return 32 * kXShapes[s].c * kXShapes[s].warps; }
+static_assert(xwidth(kNumXShapes - 1) == kMaxM, "the exact row passes cover every warp-chunked profile");
+
 typedef void (*MsvFn)(const MsvTile*, const DevProfile*, const Thresholds*, const float4*, const uint8_t*,
                       const int64_t*, const int32_t*, const float4*, const int32_t*, float*, const int32_t*, PairRec*,
                       const BinRegion*, unsigned*, unsigned*, const unsigned*, unsigned, int);
@@ -93,9 +107,9 @@ typedef void (*VitGFn)(const PairRec*, const unsigned*, const BinRegion*, int, P
                        const int32_t*, const float4*, float, float*, unsigned*);
 typedef void (*FwdFn)(const PairRec*, const unsigned*, const BinRegion*, int, PairRec*, const BinRegion*, unsigned*,
                       unsigned*, const DevProfile*, const Thresholds*, const float*, const uint8_t*, const int64_t*,
-                      const int32_t*, const float4*, float, float*, const int64_t*);
-typedef void (*BwdFn)(const PairRec*, const unsigned*, const BinRegion*, int, const DevProfile*, const float*,
-                      const uint8_t*, const int64_t*, const int32_t*, const float4*, float*, const int64_t*);
+                      const int32_t*, const float4*, float);
+typedef void (*XRowsFn)(const sxk::RowRec*, int, const DevProfile*, const float*, const uint8_t*, const int64_t*,
+                        const int32_t*, const float4*, float*);
 typedef void (*AdjFFn)(const sxk::AdjPair*, int, const DevProfile*, const float*, const uint8_t*, const int64_t*,
                        const int32_t*, const float4*, float*, double*, double*);
 typedef void (*AdjBFn)(const sxk::AdjPair*, int, const DevProfile*, const float*, const uint8_t*, const int64_t*,
@@ -112,9 +126,8 @@ struct KernelTables {
   EnvPostFn envp[kNumVbins];
   EnvPassFn regf[kNumVbins];
   VitFn vit[kNumVbins];
-  FwdFn fwd[kNumVbins];
   FwdFn fwd_scan[kNumVbins];  // the F3 pre-screen
-  BwdFn bwd[kNumVbins];
+  XRowsFn xrows[kNumXShapes];  // exact Forward and Backward rows
   AdjFFn adjf[kNumVbins];
   AdjBFn adjb[kNumVbins];
   VitGFn vitg[kNumVitShapes];
@@ -127,6 +140,7 @@ void fill_msv16_tables(KernelTables& t);
 void fill_vit_tables(KernelTables& t);
 void fill_vit16_tables(KernelTables& t);
 void fill_vbin_tables(KernelTables& t);
+void fill_exact_tables(KernelTables& t);
 void fill_env_tables(KernelTables& t);
 
 }  // namespace sx
