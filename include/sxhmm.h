@@ -43,8 +43,8 @@ extern "C" {
 /* Engine options. */
 #define SX_FLAG_PLAIN 1u /* run the plain one-pair-per-block kernels instead of the batched cascade */
 /* Where the envelope rescoring of domain definition runs (default: chosen per
- * profile block; the device when the host's share would not hide behind the
- * device cascade).  Results are identical either way. */
+ * profile block; the device unless the host's share is below what a device
+ * pass costs).  Results are identical either way. */
 #define SX_FLAG_ENV_DEVICE 2u /* always on the device */
 #define SX_FLAG_ENV_HOST 4u   /* always on the host */
 /* Where the stochastic-trace ensembles of multi-domain regions (200 sampled

@@ -34,11 +34,27 @@ struct FanOut {
   }
 };
 
+// Teams per CTA of a one-warp shape: one while every team can have an SM's
+// quarter to itself, packed when there are more.
+int teams_per_cta(const sx_engine* E, int shape, int n) {
+  return kXShapes[shape].warps > 1 || n <= 4 * E->num_sms ? 1 : 8;
+}
+struct TeamLaunch {
+  dim3 grid;
+  unsigned threads;
+  size_t smem;  // one row per team
+};
+TeamLaunch team_launch(const sx_engine* E, int shape, int n, int directions) {
+  const int t = teams_per_cta(E, shape, n);
+  return {dim3((unsigned)((n + t - 1) / t), (unsigned)directions), (unsigned)(32 * t * kXShapes[shape].warps),
+          sizeof(float) * (size_t)t * xwidth(shape)};
+}
+
 // The device passes of a DomainBatch: for every envelope request the
 // full-matrix Forward and Backward (their raw special rows come back to the
 // host), the host's posterior factors, then the posterior / null2 /
-// optimal-accuracy pass.  One warp per envelope; batches bounded by the
-// memory of their matrix planes.  Runs on the host pool's driver thread.
+// optimal-accuracy pass and the insert sums.  One team per envelope; batches
+// bounded by the memory of their matrix planes.  Runs on the host pool's driver thread.
 int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T, std::vector<EnvSource>& srcs,
                         int nthr, PhaseLog* plog) {
   // every request of every batch, as (batch, request)
@@ -64,7 +80,10 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
   std::vector<size_t> order(nr);
   std::iota(order.begin(), order.end(), (size_t)0);
   std::stable_sort(order.begin(), order.end(),
-                   [&](size_t x, size_t y) { return P->dp[req(x).p].vbin < P->dp[req(y).p].vbin; });
+                   [&](size_t x, size_t y) {
+                     const int sx = P->dp[req(x).p].xshape, sy = P->dp[req(y).p].xshape;
+                     return sx != sy ? sx > sy : req(x).j - req(x).i > req(y).j - req(y).i;  // longest chains first
+                   });
   size_t a = 0;
   while (a < nr) {
     size_t b = a;
@@ -72,9 +91,9 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
     std::vector<sxk::EnvRec> recs;
     while (b < nr) {
       const EnvRequest& q = req(order[b]);
-      const int vc = kVcBins[P->dp[q.p].vbin];
+      const int width = xwidth(P->dp[q.p].xshape);
       const int64_t lr = q.j - q.i + 1;
-      const int64_t need = 5 * (lr + 1) * 32 * vc;
+      const int64_t need = sxk::env_plane_floats(lr, width);
       if (b > a && (planes + need) * (int64_t)sizeof(float) > budget) break;
       sxk::EnvRec r{};
       r.p = q.p;
@@ -90,9 +109,10 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
       r.aux_off = aux;
       r.fac_off = fac;
       r.out_off = (int64_t)(b - a) * sxk::kEnvOut;
+      r.width = width;
       planes += need;
       rowsz += 12 * (lr + 1);
-      aux += 8 * (lr + 1);
+      aux += 5 * (lr + 1);
       fac += lr + 1;
       recs.push_back(r);
       b++;
@@ -105,27 +125,25 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
     E->env_aux.alloc((size_t)aux);
     E->env_fac.alloc((size_t)fac);
     E->env_out.alloc(n * sxk::kEnvOut);
-    // one launch per vbin: requests are sorted by vbin
-    auto each_bin = [&](auto&& launch) {
+    // one launch per shape: requests are sorted by shape
+    auto each_shape = [&](auto&& launch) {
       size_t x = 0;
       while (x < n) {
-        const int vb = P->dp[req(order[a + x]).p].vbin;
+        const int sh = P->dp[req(order[a + x]).p].xshape;
         size_t y = x;
-        while (y < n && P->dp[req(order[a + y]).p].vbin == vb) y++;
-        const int cnt = (int)(y - x);
-        launch(vb, (int)x, cnt, (int)std::min<int64_t>(cnt, (int64_t)E->num_sms * 32));
+        while (y < n && P->dp[req(order[a + y]).p].xshape == sh) y++;
+        launch(sh, (int)x, (int)(y - x));
         x = y;
       }
     };
-    // Forward and Backward of every bin at once, each launch on a stream of its own
+    // Forward and Backward of every shape at once, each launch on a stream of its own
     {
       FanOut fan(E, s);
-      each_bin([&](int vb, int x0, int cnt, int blocks) {
-        K.envf[vb]<<<blocks, 32, 0, fan.take()>>>(E->env_recs.p + x0, cnt, P->d_prof.p, P->d_vfb.p, T->d_res.p,
-                                                  T->d_off.p, E->env_planes.p, E->env_rows.p);
-        K.envb[vb]<<<blocks, 32, 0, fan.take()>>>(E->env_recs.p + x0, cnt, P->d_prof.p, P->d_vfb.p, T->d_res.p,
-                                                  T->d_off.p, E->env_planes.p, E->env_rows.p);
-        launches += 2;
+      each_shape([&](int sh, int x0, int cnt) {
+        const TeamLaunch t = team_launch(E, sh, cnt, 2);
+        K.envr[sh]<<<t.grid, t.threads, t.smem, fan.take()>>>(E->env_recs.p + x0, cnt, P->d_prof.p, P->d_x.p, T->d_res.p,
+                                                              T->d_off.p, E->env_planes.p, E->env_rows.p);
+        launches += 1;
       });
       CK(cudaGetLastError());
       fan.join();
@@ -158,12 +176,15 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
     CK(cudaMemcpyAsync(E->env_aux.p, haux.data(), sizeof(float) * (size_t)aux, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(E->env_fac.p, hfac.data(), sizeof(double) * (size_t)fac, cudaMemcpyHostToDevice, s));
     FanOut fan(E, s);
-    each_bin([&](int vb, int x0, int cnt, int blocks) {
-      const size_t psm = sxk::env_post_smem(kVcBins[vb]);
-      CK(cudaFuncSetAttribute((const void*)K.envp[vb], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
-      K.envp[vb]<<<blocks, 32, psm, fan.take()>>>(E->env_recs.p + x0, cnt, P->d_prof.p, P->d_vfb.p, E->env_planes.p,
-                                       E->env_aux.p, E->env_fac.p, E->env_out.p);
-      launches += 1;
+    each_shape([&](int sh, int x0, int cnt) {
+      const TeamLaunch t = team_launch(E, sh, cnt, 1);
+      K.envoa[sh]<<<t.grid, t.threads, t.smem, fan.take()>>>(E->env_recs.p + x0, cnt, P->d_prof.p, P->d_x.p,
+                                                             E->env_planes.p, E->env_aux.p, E->env_fac.p, E->env_out.p);
+      const int ism = 2 * sxk::kInsertRows * xwidth(sh) * (int)sizeof(float);
+      CK(cudaFuncSetAttribute((const void*)sxk::env_insert_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ism));
+      sxk::env_insert_kernel<<<cnt, 32 * (sxk::kInsertRows + 1), ism, fan.take()>>>(
+          E->env_recs.p + x0, cnt, P->d_prof.p, E->env_planes.p, E->env_fac.p, E->env_out.p, xwidth(sh));
+      launches += 2;
     });
     CK(cudaGetLastError());
     fan.join();
@@ -234,7 +255,7 @@ RegionPassStats region_passes(sx_engine* E, const sx_profiles* P, const sx_targe
   std::vector<size_t> order(nr);
   std::iota(order.begin(), order.end(), (size_t)0);
   std::stable_sort(order.begin(), order.end(),
-                   [&](size_t x, size_t y) { return P->dp[reg(x).p].vbin < P->dp[reg(y).p].vbin; });
+                   [&](size_t x, size_t y) { return P->dp[reg(x).p].xshape < P->dp[reg(y).p].xshape; });
   size_t a = 0;
   while (a < nr) {
     size_t b = a;
@@ -289,16 +310,16 @@ RegionPassStats region_passes(sx_engine* E, const sx_profiles* P, const sx_targe
     E->trc_count.alloc(1);
     E->trc_status.alloc(n);
     CK(cudaMemsetAsync(E->trc_count.p, 0, sizeof(int32_t), s));
-    // the region Forward passes, one launch per vbin (regions are sorted by
-    // vbin) on streams of their own, then one trace launch over the batch
+    // the region Forward passes, one launch per shape (regions are sorted by
+    // shape) on streams of their own, then one trace launch over the batch
     FanOut fan(E, s);
     for (size_t x = 0; x < n;) {
-      const int vb = P->dp[reg(order[a + x]).p].vbin;
+      const int sh = P->dp[reg(order[a + x]).p].xshape;
       size_t y = x;
-      while (y < n && P->dp[reg(order[a + y]).p].vbin == vb) y++;
-      const int cnt = (int)(y - x);
-      K.regf[vb]<<<(int)std::min<int64_t>(cnt, (int64_t)E->num_sms * 32), 32, 0, fan.take()>>>(
-          E->env_recs.p + x, cnt, P->d_prof.p, P->d_vfb.p, T->d_res.p, T->d_off.p, E->env_planes.p, E->env_rows.p);
+      while (y < n && P->dp[reg(order[a + y]).p].xshape == sh) y++;
+      const TeamLaunch t = team_launch(E, sh, (int)(y - x), 1);
+      K.regf[sh]<<<t.grid, t.threads, t.smem, fan.take()>>>(E->env_recs.p + x, (int)(y - x), P->d_prof.p, P->d_x.p,
+                                                            T->d_res.p, T->d_off.p, E->env_planes.p, E->env_rows.p);
       st.launches += 1;
       x = y;
     }

@@ -1,22 +1,31 @@
 // Envelope rescoring on the device: the full-matrix passes of
 // rescore_isolated_domain (src/hmmer/pipeline.rs:545-591) for a batch of
-// envelopes, one warp per envelope.
+// envelopes, one team (a warp up to 256 columns, a CTA above) per envelope.
 //
-//   env_forward_kernel   forward_matrix  (src/hmmer/dp.rs:442-513)
-//   env_backward_kernel  backward_matrix (src/hmmer/dp.rs:516-601)
-//   env_post_kernel      decode (dp.rs:1278-1306) fused with the sums of
-//                        null2_from_posterior (dp.rs:1310-1350) and the
-//                        optimal-accuracy DP and traceback (dp.rs:1355-1564)
+//   env_rows_kernel   forward_matrix (src/hmmer/dp.rs:442-513) and
+//                     backward_matrix (dp.rs:516-601), by exact_rows.cuh
+//   env_oa_kernel     decode (dp.rs:1278-1306) fused with the column sums of
+//                     null2_from_posterior (dp.rs:1310-1350) and the
+//                     optimal-accuracy DP and traceback (dp.rs:1355-1564)
+//   env_insert_kernel the ordered sum of the insert posteriors
 //
-// The arithmetic is the reference's, operation for operation (no FMA, the D
-// chains and row sums in order by lane batons), so the matrices, posteriors
-// and coordinates equal the host's bit for bit.  Every log/exp stays on the
-// host: the forward and backward kernels write raw scaled special rows and
-// rescale factors, the host turns them into the per-row posterior factor
-// exp(lnF + lnB - lnZ) and the N/J/C posteriors, and the post kernel reads
-// those back.
+// The arithmetic is the reference's, operation for operation (no FMA, ordered
+// sums in order), so the matrices, posteriors and coordinates equal the
+// host's bit for bit.  Every log/exp stays on the host: env_rows_kernel writes
+// raw scaled special rows and rescale factors, the host turns them into the
+// per-row posterior factor exp(lnF + lnB - lnZ) and the N/J/C posteriors, and
+// the other two read those back.
+//
+// Measured on B200 (wall time of the passes of one search; before: one warp
+// per envelope handing the ordered chains from lane to lane, the insert sum in
+// the optimal-accuracy row loop, the traceback over four planes of floats):
+// marker-set genome (242 envelopes, M to 1,500) Forward/Backward 43.2 -> 8.3
+// ms, posterior/OA 52.8 -> 3.9; Pfam-scale's last block (128) 5.4 -> 1.5 and
+// 5.9 -> 1.0; 64 profiles of M 60-700 (61) 10.4 -> 2.4 and 13.0 -> 1.4.
 #pragma once
-#include "kernels.cuh"
+#include <climits>
+
+#include "exact_rows.cuh"
 
 namespace sxk {
 
@@ -26,728 +35,499 @@ struct EnvRec {
   int32_t p, t;
   int32_t i0, lr;
   float ploop, pmove, pe_loop, pe_move;
-  int64_t plane_off;  // float offset: 5 planes of (lr+1) rows x 32*VC columns (FM FI BM BI OD)
+  int64_t plane_off;  // float offset: 5 planes of (lr+1) rows x width columns (FM FI BM BI OD), then the decisions
   int64_t row_off;    // float offset: forward raw rows 6(lr+1), then backward raw rows 6(lr+1)
-  int64_t aux_off;    // float offset: pn pj pc (inputs), then OA specials xe xn xj xb xc; (lr+1) each
+  int64_t aux_off;    // float offset: pn pj pc (inputs), then OA specials xe xc; (lr+1) each
   int64_t fac_off;    // double offset: posterior factor per row (lr+1)
   int64_t out_off;    // float offset of kEnvOut outputs
+  int32_t width, pad; // columns of a plane row (the profile's exact row shape)
 };
+// floats of an envelope's planes: 5 planes and half a byte of decision per cell
+__host__ __device__ __forceinline__ int64_t env_plane_floats(int64_t lr, int width) {
+  return 5 * (lr + 1) * width + (lr + 1) * (width / 8);
+}
 // Outputs: [0,20) sum_k (sm[k]*norm)*mo[x][k] for x < 20, [20] si (the row-major
 // sum of insert posteriors), [21] found (1/0), [22..25] i0 i1 k0 k1 (as floats).
 constexpr int kEnvOut = 32;
 
-// Plane element of column k (1-based) in the lane-major layout: lane (k-1)/VC,
-// chunk slot (k-1)%VC.
-template <int VC>
-__device__ __forceinline__ int64_t plane_at(int64_t row, int k) {
-  return row * (32 * VC) + (int64_t)(((k - 1) % VC) * 32 + (k - 1) / VC);
-}
-
-// Diagonal layout of a region's M/I/D planes for the stochastic traceback:
-// cell (i, k), 1 <= i <= lr, 1 <= k <= M, at (i - k + M - 1) * M + (k - 1), so
-// the cells of a run of match states, (i, k) -> (i-1, k-1), are adjacent.
-__host__ __device__ __forceinline__ int64_t diag_at(int64_t i, int k, int M) {
-  return (i - k + M - 1) * (int64_t)M + (k - 1);
-}
-__host__ __device__ __forceinline__ int64_t diag_plane(int64_t lr, int M) { return (lr + M - 1) * (int64_t)M; }
-
-// forward_matrix: M/I planes (scaled, after each row's rescaling) and the raw
-// special rows N B E J C scale for rows 1..lr.  DIAG writes the M, I and D
-// planes in the diagonal layout instead (the stochastic traceback's input).
-template <int VC, bool DIAG = false>
-__global__ void __launch_bounds__(32) env_forward_kernel(const EnvRec* __restrict__ recs, int n,
-                                                         const DevProfile* __restrict__ profs,
-                                                         const float* __restrict__ vfb,
-                                                         const uint8_t* __restrict__ res,
-                                                         const int64_t* __restrict__ toff, float* __restrict__ planes,
-                                                         float* __restrict__ rows) {
-  constexpr int RS = 32 * VC;
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += warps) {
-    const EnvRec r = recs[w];
-    const DevProfile P = profs[r.p];
-    const Img<VC> img{vfb + P.vfb_off};
-    const int M = P.m;
-    const int nl = (M + VC - 1) / VC;
-    const uint8_t* s = res + toff[r.t] + r.i0;
-    const int L = r.lr;
-    const float ploop = r.ploop, pmove = r.pmove, pe_loop = r.pe_loop, pe_move = r.pe_move;
-    float* FM = planes + r.plane_off;
-    float* FI = FM + (DIAG ? diag_plane(L, M) : (int64_t)(L + 1) * RS);
-    float* FD = FI + diag_plane(L, M);
-    float* orow = rows + r.row_off;
-    TransRows<VC> tr;
-    tr.load(img, kRowFwd, lane);
-    float mp[VC], ip[VC], dp[VC], eo[VC];
-#pragma unroll
-    for (int c = 0; c < VC; c++) mp[c] = ip[c] = dp[c] = 0.f;
-    float xn = 1.f, xb = pmove, xj = 0.f, xc = 0.f;
-    int x = L > 0 ? __ldg(s) : 24;
-#pragma unroll
-    for (int c = 0; c < VC; c++) eo[c] = img.at(kRowMo + x, c, lane);
-    for (int i = 0; i < L; i++) {
-      const int xnext = (i + 1 < L) ? __ldg(s + i + 1) : 24;
-      float eon[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) eon[c] = img.at(kRowMo + xnext, c, lane);
-      const float ins = x != 24 ? 1.f : 0.f;
-      const float mpl0 = __shfl_up_sync(kFull, mp[VC - 1], 1);
-      const float ipl0 = __shfl_up_sync(kFull, ip[VC - 1], 1);
-      const float dpl0 = __shfl_up_sync(kFull, dp[VC - 1], 1);
-      const float mpl = lane ? mpl0 : 0.f, ipl = lane ? ipl0 : 0.f, dpl = lane ? dpl0 : 0.f;
-      float mv[VC], iv[VC], a[VC], dv[VC], pdd[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        const int k = lane * VC + c + 1;
-        const float mpv = c ? mp[c - 1] : mpl, ipv = c ? ip[c - 1] : ipl, dpv = c ? dp[c - 1] : dpl;
-        float t = fmul(xb, tr.get(img, kRowFwd, 0, c, lane));
-        t = fadd(t, fmul(mpv, tr.get(img, kRowFwd, 1, c, lane)));
-        t = fadd(t, fmul(ipv, tr.get(img, kRowFwd, 2, c, lane)));
-        t = fadd(t, fmul(dpv, tr.get(img, kRowFwd, 3, c, lane)));
-        mv[c] = fmul(t, eo[c]);
-        iv[c] = k < M ? fmul(fadd(fmul(mp[c], tr.get(img, kRowFwd, 4, c, lane)),
-                                  fmul(ip[c], tr.get(img, kRowFwd, 5, c, lane))), ins)
-                      : 0.f;
-      }
-      const float mcl0 = __shfl_up_sync(kFull, mv[VC - 1], 1);
-      const float mcl = lane ? mcl0 : 0.f;
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        a[c] = fmul(c ? mv[c - 1] : mcl, tr.get(img, kRowFwd, 6, c, lane));
-        pdd[c] = tr.get(img, kRowFwd, 7, c, lane);
-      }
-      // ordered D chain and row sum: dc[k] = a_k + dc[k-1]*p_dd[k-1]; xe += mv + dc
-      float dcar = 0.f, xe = 0.f;
-      for (int sl = 0; sl < nl; sl++) {
-        if (lane == sl) {
-#pragma unroll
-          for (int c = 0; c < VC; c++) {
-            const float d = fadd(a[c], fmul(dcar, pdd[c]));
-            dv[c] = d;
-            xe = fadd(xe, fadd(mv[c], d));
-            dcar = d;
-          }
-        }
-        dcar = __shfl_sync(kFull, dcar, sl);
-        xe = __shfl_sync(kFull, xe, sl);
-      }
-      if (lane >= nl) {
-#pragma unroll
-        for (int c = 0; c < VC; c++) dv[c] = 0.f;
-      }
-      xj = fadd(fmul(xj, ploop), fmul(xe, pe_loop));
-      xc = fadd(fmul(xc, ploop), fmul(xe, pe_move));
-      xn = fmul(xn, ploop);
-      xb = fadd(fmul(xn, pmove), fmul(xj, pmove));
-      float scale = 0.f;
-      if (xe > 1.0e4f) {
-        const float inv = __fdiv_rn(1.0f, xe);
-#pragma unroll
-        for (int c = 0; c < VC; c++) {
-          mv[c] = fmul(mv[c], inv);
-          iv[c] = fmul(iv[c], inv);
-          dv[c] = fmul(dv[c], inv);
-        }
-        xn = fmul(xn, inv);
-        xb = fmul(xb, inv);
-        xj = fmul(xj, inv);
-        xc = fmul(xc, inv);
-        scale = xe;
-        xe = 1.0f;
-      }
-      if (lane == 0) {
-        float* o = orow + 6 * (i + 1);
-        o[0] = xn; o[1] = xb; o[2] = xe; o[3] = xj; o[4] = xc; o[5] = scale;
-      }
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        if (DIAG) {
-          const int k = lane * VC + c + 1;
-          if (k <= M) {
-            const int64_t at = diag_at(i + 1, k, M);
-            FM[at] = mv[c];
-            FI[at] = iv[c];
-            FD[at] = dv[c];
-          }
-        } else {
-          FM[(int64_t)(i + 1) * RS + c * 32 + lane] = mv[c];
-          FI[(int64_t)(i + 1) * RS + c * 32 + lane] = iv[c];
-        }
-        mp[c] = mv[c];
-        ip[c] = iv[c];
-        dp[c] = dv[c];
-        eo[c] = eon[c];
-      }
-      x = xnext;
-    }
+// Forward (blockIdx.y = 0) and Backward (1) matrices and raw rows of n
+// envelopes; DIAG: the Forward matrices of regions in the diagonal layout.
+template <int C, bool MULTI, bool DIAG>
+__global__ void __launch_bounds__(256) env_rows_kernel(const EnvRec* __restrict__ recs, int n,
+                                                       const DevProfile* __restrict__ profs,
+                                                       const float* __restrict__ ximg,
+                                                       const uint8_t* __restrict__ res,
+                                                       const int64_t* __restrict__ toff, float* __restrict__ planes,
+                                                       float* __restrict__ rows) {
+  extern __shared__ float4 sm_row[];
+  __shared__ XShared sh;
+  const int w = MULTI ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (w >= n) return;  // uniform over the team
+  float* T = reinterpret_cast<float*>(sm_row) + (MULTI ? 0 : (threadIdx.x >> 5) * 32 * C);
+  const EnvRec r = recs[w];
+  const float* img = ximg + profs[r.p].x_off;
+  const int M = profs[r.p].m;
+  const uint8_t* s = res + toff[r.t] + r.i0;
+  float* pl = planes + r.plane_off;
+  float* orow = rows + r.row_off;
+  if constexpr (DIAG) {
+    exact_forward<C, MULTI, kKeepDiag>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move, orow, pl, T, sh);
+  } else if (blockIdx.y == 0) {
+    exact_forward<C, MULTI, kKeepMI>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move, orow, pl, T, sh);
+  } else {
+    exact_backward<C, MULTI, kKeepMI>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move,
+                                      orow + 6 * (int64_t)(r.lr + 1), pl + 2 * (int64_t)(r.lr + 1) * r.width, T, sh);
   }
-}
-
-// backward_matrix: M/I planes for rows lr..1 and the raw special rows (row lr:
-// E and C; rows lr-1..1: N B E J C scale; row 0: the B sum in slot 1).
-template <int VC>
-__global__ void __launch_bounds__(32) env_backward_kernel(const EnvRec* __restrict__ recs, int n,
-                                                          const DevProfile* __restrict__ profs,
-                                                          const float* __restrict__ vfb,
-                                                          const uint8_t* __restrict__ res,
-                                                          const int64_t* __restrict__ toff, float* __restrict__ planes,
-                                                          float* __restrict__ rows) {
-  constexpr int RS = 32 * VC;
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += warps) {
-    const EnvRec r = recs[w];
-    const DevProfile P = profs[r.p];
-    const Img<VC> img{vfb + P.vfb_off};
-    const int M = P.m;
-    const int nl = (M + VC - 1) / VC;
-    const int lM = (M - 1) / VC;  // lane holding column M
-    const uint8_t* s = res + toff[r.t] + r.i0;
-    const int L = r.lr;
-    const float ploop = r.ploop, pmove = r.pmove, pe_loop = r.pe_loop, pe_move = r.pe_move;
-    float* BM = planes + r.plane_off + 2 * (int64_t)(L + 1) * RS;
-    float* BI = BM + (int64_t)(L + 1) * RS;
-    float* orow = rows + r.row_off + 6 * (int64_t)(L + 1);
-    float mn[VC], in_[VC], dn[VC];
-    // row L
-    float xc = pmove;
-    float xe = fmul(xc, pe_move);
-    float xj = 0.f, xn = 0.f;
-    {
-      float pmd0[VC], pdd0[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        pmd0[c] = img.at(kRowBwd + 2, c, lane);
-        pdd0[c] = img.at(kRowBwd + 6, c, lane);
-      }
-      float dcar = 0.f;
-      for (int sl = lM; sl >= 0; sl--) {
-        if (lane == sl) {
-#pragma unroll
-          for (int c = VC - 1; c >= 0; c--) {
-            const int k = lane * VC + c + 1;
-            if (k > M) {
-              mn[c] = dn[c] = 0.f;
-            } else if (k == M) {
-              mn[c] = dn[c] = xe;
-              dcar = xe;
-            } else {
-              mn[c] = fadd(xe, fmul(dcar, pmd0[c]));
-              dn[c] = fadd(xe, fmul(dcar, pdd0[c]));
-              dcar = dn[c];
-            }
-          }
-        }
-        dcar = __shfl_sync(kFull, dcar, sl);
-      }
-      if (lane > lM) {
-#pragma unroll
-        for (int c = 0; c < VC; c++) mn[c] = dn[c] = 0.f;
-      }
-#pragma unroll
-      for (int c = 0; c < VC; c++) in_[c] = 0.f;
-    }
-    if (L > 0) {
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        BM[(int64_t)L * RS + c * 32 + lane] = mn[c];
-        BI[(int64_t)L * RS + c * 32 + lane] = 0.f;
-      }
-    }
-    if (lane == 0 && L > 0) {
-      float* o = orow + 6 * L;
-      o[0] = 0.f; o[1] = 0.f; o[2] = xe; o[3] = 0.f; o[4] = xc; o[5] = 0.f;
-    }
-    for (int i = L - 1; i >= 1; i--) {
-      const int x = __ldg(s + i);
-      const float ins = x != 24 ? 1.f : 0.f;
-      float eo[VC], me[VC], bt[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        eo[c] = img.at(kRowMo + x, c, lane);
-        me[c] = fmul(mn[c], eo[c]);
-        bt[c] = fmul(fmul(mn[c], img.at(kRowBwd + 7, c, lane)), eo[c]);
-      }
-      // B sum, ascending k
-      float b = 0.f;
-      for (int sl = 0; sl < nl; sl++) {
-        if (lane == sl) {
-#pragma unroll
-          for (int c = 0; c < VC; c++) b = fadd(b, bt[c]);
-        }
-        b = __shfl_sync(kFull, b, sl);
-      }
-      const float xb = b;
-      xj = fadd(fmul(xj, ploop), fmul(xb, pmove));
-      xc = fmul(xc, ploop);
-      xe = fadd(fmul(xj, pe_loop), fmul(xc, pe_move));
-      xn = fadd(fmul(xn, ploop), fmul(xb, pmove));
-      float rowmax = fmaxf(fmaxf(fmaxf(fmaxf(xb, xe), xn), xj), xc);
-      const float me_up = __shfl_down_sync(kFull, me[0], 1);
-      float mnext[VC], iv[VC], mc[VC], ic[VC], dc[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        mnext[c] = c < VC - 1 ? me[c + 1] : (lane < 31 ? me_up : 0.f);
-        iv[c] = fmul(in_[c], ins);
-      }
-      float pdm[VC], pdd[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        pdm[c] = img.at(kRowBwd + 5, c, lane);
-        pdd[c] = img.at(kRowBwd + 6, c, lane);
-      }
-      // D chain, descending k
-      float dcar = 0.f;
-      for (int sl = lM; sl >= 0; sl--) {
-        if (lane == sl) {
-#pragma unroll
-          for (int c = VC - 1; c >= 0; c--) {
-            const int k = lane * VC + c + 1;
-            if (k > M) {
-              dc[c] = 0.f;
-            } else if (k == M) {
-              dc[c] = xe;
-              dcar = xe;
-            } else {
-              dc[c] = fadd(fadd(fmul(mnext[c], pdm[c]), fmul(dcar, pdd[c])), xe);
-              dcar = dc[c];
-            }
-          }
-        }
-        dcar = __shfl_sync(kFull, dcar, sl);
-      }
-      if (lane > lM) {
-#pragma unroll
-        for (int c = 0; c < VC; c++) dc[c] = 0.f;
-      }
-      const float dc_up = __shfl_down_sync(kFull, dc[0], 1);
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        const int k = lane * VC + c + 1;
-        const float dnext = c < VC - 1 ? dc[c + 1] : (lane < 31 ? dc_up : 0.f);
-        if (k < M) {
-          const float mv = fadd(fadd(fadd(fmul(mnext[c], img.at(kRowBwd + 0, c, lane)),
-                                          fmul(iv[c], img.at(kRowBwd + 1, c, lane))), xe),
-                                fmul(dnext, img.at(kRowBwd + 2, c, lane)));
-          mc[c] = mv;
-          ic[c] = fadd(fmul(mnext[c], img.at(kRowBwd + 3, c, lane)), fmul(iv[c], img.at(kRowBwd + 4, c, lane)));
-          rowmax = fmaxf(rowmax, mv);
-        } else if (k == M) {
-          mc[c] = xe;
-          ic[c] = 0.f;
-        } else {
-          mc[c] = 0.f;
-          ic[c] = 0.f;
-        }
-      }
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) rowmax = fmaxf(rowmax, __shfl_xor_sync(kFull, rowmax, o));
-      float scale = 0.f;
-      float xb_o = xb;
-      if (rowmax > 1.0e4f) {
-        const float inv = __fdiv_rn(1.0f, rowmax);
-#pragma unroll
-        for (int c = 0; c < VC; c++) {
-          mc[c] = fmul(mc[c], inv);
-          ic[c] = fmul(ic[c], inv);
-          dc[c] = fmul(dc[c], inv);
-        }
-        xb_o = fmul(xb, inv);
-        xe = fmul(xe, inv);
-        xn = fmul(xn, inv);
-        xj = fmul(xj, inv);
-        xc = fmul(xc, inv);
-        scale = rowmax;
-      }
-      if (lane == 0) {
-        float* o = orow + 6 * i;
-        o[0] = xn; o[1] = xb_o; o[2] = xe; o[3] = xj; o[4] = xc; o[5] = scale;
-      }
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        BM[(int64_t)i * RS + c * 32 + lane] = mc[c];
-        BI[(int64_t)i * RS + c * 32 + lane] = ic[c];
-        mn[c] = mc[c];
-        in_[c] = ic[c];
-        dn[c] = dc[c];
-      }
-    }
-    // row 0: B sum with residue 1
-    if (L > 0) {
-      const int x0 = __ldg(s);
-      float bt[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) bt[c] = fmul(fmul(mn[c], img.at(kRowBwd + 7, c, lane)), img.at(kRowMo + x0, c, lane));
-      float b = 0.f;
-      for (int sl = 0; sl < nl; sl++) {
-        if (lane == sl) {
-#pragma unroll
-          for (int c = 0; c < VC; c++) b = fadd(b, bt[c]);
-        }
-        b = __shfl_sync(kFull, b, sl);
-      }
-      if (lane == 0) {
-        float* o = orow;
-        o[0] = 0.f; o[1] = b; o[2] = 0.f; o[3] = 0.f; o[4] = 0.f; o[5] = 0.f;
-      }
-    }
-  }
-}
-
-// Per-lane column arrays of a warp-per-envelope kernel: registers for narrow
-// profiles, shared memory for wide ones (VC >= kPostSmemVC), where holding
-// the post kernel's 17 arrays of VC floats in registers spills to local memory.
-// In shared memory element c of a lane's array sits at s[32 * c]: a warp's
-// access to one c is one conflict-free wavefront.
-template <int VC, bool SH>
-struct Cols {
-  float r[SH ? 1 : VC];
-  float* s;
-  __device__ __forceinline__ float& operator[](int c) {
-    if constexpr (SH) return s[c * 32];
-    else return r[c];
-  }
-};
-constexpr int kPostSmemVC = 16;
-constexpr int kPostArrays = 17;  // tp[8], sm, omp, oip, odp, pm, pi, om, oi, od
-// Dynamic shared memory of env_post_kernel<VC> (one warp per CTA): the row
-// buffer of the insert-posterior sum, then the column arrays when they live
-// in shared memory.
-__host__ __device__ constexpr size_t env_post_smem(int vc) {
-  return ((vc >= kPostSmemVC ? (size_t)kPostArrays : 0) + 1) * 32 * vc * sizeof(float);
 }
 
 __device__ __forceinline__ float oa_gate(float t, float v) { return t > 0.0f ? v : 0.0f; }
 __device__ __forceinline__ float oa_dis(float t, float v) { return t == 0.0f ? SX_NEG_INF : v; }
 
+// Traceback decisions of a cell (i, k), four bits: 0-1 the predecessor of M (M,
+// I, D at (i-1, k-1), or B), bit 2 set if I comes from I, bit 3 set if the D
+// to the RIGHT of the cell, (i, k+1), comes from D.  A row's decisions are
+// packed, column k at nibble k - 1.
+enum : unsigned { kOaM = 0, kOaI = 1, kOaD = 2, kOaB = 3, kOaIfromI = 4, kOaDfromD = 8 };
+
+enum St { kSM, kSI, kSD };  // traceback states
+
+struct OaShared {  // exchange between the warps of a team
+  float val[kXMaxWarps];      // composite D map of the warp: v -> max(val, v), or the constant val
+  int cst[kXMaxWarps];
+  float prev[3][kXMaxWarps];  // OA M, I, D of the last column
+  float mx[kXMaxWarps];
+};
+
 // decode + null2 sums + optimal-accuracy DP and traceback.  Reads the forward
 // and backward M/I planes, the host's per-row factor exp(lnF + lnB - lnZ) and
-// N/J/C posteriors; overwrites the backward planes with the OA M/I matrices
-// (each backward row is read before its OA row is written) and fills the OD
-// plane and the OA special arrays, which the traceback (lane 0) reads.
-template <int VC>
-__global__ void __launch_bounds__(32) env_post_kernel(const EnvRec* __restrict__ recs, int n,
-                                                      const DevProfile* __restrict__ profs,
-                                                      const float* __restrict__ vfb, float* __restrict__ planes,
-                                                      float* __restrict__ aux, const double* __restrict__ facs,
-                                                      float* __restrict__ outs) {
-  constexpr int RS = 32 * VC;
+// N/J/C posteriors; overwrites the backward M plane with the OA M matrix (each
+// row is read before its OA row is written), fills the OD plane, the cells'
+// traceback decisions and the OA specials E and C.
+//
+// A row's latency: the D chain od[k+1] = max(gate(t_md, om[k]), gate(t_dd,
+// od[k])) only selects and takes maxima of non-negative values (or -inf),
+// exact in any order, so it runs as a scan.  The step out of column k maps the
+// chain value v to max(a_k, v) when t_dd > 0 and to the constant max(a_k, 0)
+// otherwise; lanes compose their columns' maps, a segmented max scan composes
+// them across the warp (a constant starts a segment) and the warps' composites
+// go through shared memory.  With the decisions noted while the row is in
+// registers the traceback loads half a byte a step, 32 steps of a run of
+// matches at a time, instead of following four chains of floats.
+template <int C, bool MULTI>
+__global__ void __launch_bounds__(256) env_oa_kernel(const EnvRec* __restrict__ recs, int n,
+                                                     const DevProfile* __restrict__ profs,
+                                                     const float* __restrict__ ximg, float* planes, float* aux,
+                                                     const double* __restrict__ facs, float* __restrict__ outs) {
+  extern __shared__ float4 sm_row[];
+  __shared__ OaShared sh;
+  const int w = MULTI ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (w >= n) return;  // uniform over the team
   const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += warps) {
-    const EnvRec r = recs[w];
-    const DevProfile P = profs[r.p];
-    const Img<VC> img{vfb + P.vfb_off};
-    const int M = P.m;
-    const int nl = (M + VC - 1) / VC;
-    const int L = r.lr;
-    const int64_t PL = (int64_t)(L + 1) * RS;
-    const float* FM = planes + r.plane_off;
-    const float* FI = FM + PL;
-    float* OM = planes + r.plane_off + 2 * PL;  // backward M, then OA M
-    float* OI = OM + PL;                        // backward I, then OA I
-    float* OD = OI + PL;
-    float* ab = aux + r.aux_off;
-    const float* pn = ab;
-    const float* pj = ab + (L + 1);
-    const float* pc = ab + 2 * (L + 1);
-    float* sxe = ab + 3 * (L + 1);
-    float* sxn = sxe + (L + 1);
-    float* sxj = sxn + (L + 1);
-    float* sxb = sxj + (L + 1);
-    float* sxc = sxb + (L + 1);
-    const double* fac = facs + r.fac_off;
-    float* out = outs + r.out_off;
-    const bool ploop0 = r.ploop == 0.0f, pe_loop0 = r.pe_loop == 0.0f, pe_move0 = r.pe_move == 0.0f,
-               pmove0 = r.pmove == 0.0f;
-    // probability transitions at column k: p_bm[k], p_mm[k-1], p_im[k-1], p_dm[k-1],
-    // p_mi[k], p_ii[k], p_md[k-1], p_dd[k-1]
-    constexpr bool SH = VC >= kPostSmemVC;
-    extern __shared__ float post_smem[];
-    Cols<VC, SH> tp[8], sm, omp, oip, odp, pm, pi, om, oi, od;
-    float* sirow = post_smem;  // the row's insert posteriors, element (c, lane) at c * 32 + lane
-    if constexpr (SH) {
-      float* b = post_smem + 32 * VC + lane;
+  const int warp = MULTI ? threadIdx.x >> 5 : 0;
+  const int nw = MULTI ? blockDim.x >> 5 : 1;
+  const int width = nw * 32 * C;
+  const int k0 = (MULTI ? threadIdx.x : lane) * C;
+  const bool lead = MULTI ? threadIdx.x == 0 : lane == 0;
+  float* T = reinterpret_cast<float*>(sm_row) + (MULTI ? 0 : (threadIdx.x >> 5) * 32 * C);
+  const EnvRec r = recs[w];
+  const float* img = ximg + profs[r.p].x_off;
+  const int M = profs[r.p].m;
+  const int L = r.lr;
+  const int64_t PL = (int64_t)(L + 1) * width;
+  const float* FM = planes + r.plane_off;
+  const float* FI = FM + PL;
+  float* OM = planes + r.plane_off + 2 * PL;  // backward M, then OA M
+  const float* BI = OM + PL;
+  float* OD = OM + 2 * PL;
+  uint8_t* dec = reinterpret_cast<uint8_t*>(OM + 3 * PL);
+  const int dec_row = width / 2;  // bytes
+  const float* pn = aux + r.aux_off;
+  const float* pj = pn + (L + 1);
+  const float* pc = pn + 2 * (L + 1);
+  float* sxe = aux + r.aux_off + 3 * (L + 1);
+  float* sxc = sxe + (L + 1);
+  const double* fac = facs + r.fac_off;
+  float* out = outs + r.out_off;
+  const bool ploop0 = r.ploop == 0.0f, pe_loop0 = r.pe_loop == 0.0f, pe_move0 = r.pe_move == 0.0f,
+             pmove0 = r.pmove == 0.0f;
+  float tr[6][C], md[C], dd[C];  // bm, mm im dm into the column, mi ii; md dd out of it
 #pragma unroll
-      for (int q = 0; q < 8; q++) tp[q].s = b + q * 32 * VC;
-      sm.s = b + 8 * 32 * VC;
-      omp.s = b + 9 * 32 * VC;
-      oip.s = b + 10 * 32 * VC;
-      odp.s = b + 11 * 32 * VC;
-      pm.s = b + 12 * 32 * VC;
-      pi.s = b + 13 * 32 * VC;
-      om.s = b + 14 * 32 * VC;
-      oi.s = b + 15 * 32 * VC;
-      od.s = b + 16 * 32 * VC;
+  for (int q = 0; q < 6; q++) load_cols<C>(img + (kXFwd + q) * width + k0, tr[q]);
+  load_cols<C>(img + (kXBwd + 2) * width + k0, md);
+  load_cols<C>(img + (kXBwd + 6) * width + k0, dd);
+  float sm[C], omp[C], oip[C], odp[C], fm[C], fi[C], bm[C], bi[C];
+#pragma unroll
+  for (int c = 0; c < C; c++) {
+    sm[c] = 0.f;
+    omp[c] = oip[c] = odp[c] = SX_NEG_INF;
+    fm[c] = fi[c] = bm[c] = bi[c] = 0.f;
+  }
+  // plane rows are read a row ahead, as plain loads (the OA M plane is written here)
+  auto load_row = [&](int i) {
+    const int64_t at = (int64_t)i * width + k0;
+#pragma unroll
+    for (int q = 0; q < C / 4; q++) {
+      const float4 a = reinterpret_cast<const float4*>(FM + at)[q], b = reinterpret_cast<const float4*>(OM + at)[q];
+      const float4 c = reinterpret_cast<const float4*>(FI + at)[q], d = reinterpret_cast<const float4*>(BI + at)[q];
+      fm[4 * q] = a.x; fm[4 * q + 1] = a.y; fm[4 * q + 2] = a.z; fm[4 * q + 3] = a.w;
+      bm[4 * q] = b.x; bm[4 * q + 1] = b.y; bm[4 * q + 2] = b.z; bm[4 * q + 3] = b.w;
+      fi[4 * q] = c.x; fi[4 * q + 1] = c.y; fi[4 * q + 2] = c.z; fi[4 * q + 3] = c.w;
+      bi[4 * q] = d.x; bi[4 * q + 1] = d.y; bi[4 * q + 2] = d.z; bi[4 * q + 3] = d.w;
     }
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-#pragma unroll
-      for (int c = 0; c < VC; c++) tp[q][c] = img.at(kRowFwd + q, c, lane);
-#pragma unroll
-    for (int c = 0; c < VC; c++) {
-      sm[c] = 0.f;
-      omp[c] = oip[c] = odp[c] = SX_NEG_INF;
-      OM[c * 32 + lane] = SX_NEG_INF;
-      OI[c * 32 + lane] = SX_NEG_INF;
-      OD[c * 32 + lane] = SX_NEG_INF;
-    }
-    float si = 0.f;
-    float xbp = 0.f, xnp = 0.f, xjp = SX_NEG_INF, xcp = SX_NEG_INF;
+  };
+  double f = 0.0;
+  float pnv = 0.f, pjv = 0.f, pcv = 0.f;
+  auto load_specials = [&](int i) {
+    f = fac[i];
+    pnv = pn[i];
+    pjv = pj[i];
+    pcv = pc[i];
+  };
+  if (L >= 1) {
+    load_row(1);
+    load_specials(1);
+  }
+  float lm = SX_NEG_INF, li = SX_NEG_INF, ld = SX_NEG_INF;  // the left warp's last column, previous row (lane 0)
+  float xb = 0.f, xn = 0.f, xj = SX_NEG_INF, xc = SX_NEG_INF;
+  if (lead) {
+    sxe[0] = SX_NEG_INF;
+    sxc[0] = SX_NEG_INF;
+  }
+  for (int i = 1; i <= L; i++) {
+    float om[C], oi[C], od[C];
+    float oml = __shfl_up_sync(kFull, omp[C - 1], 1), oil = __shfl_up_sync(kFull, oip[C - 1], 1);
+    float odl = __shfl_up_sync(kFull, odp[C - 1], 1);
     if (lane == 0) {
-      sxe[0] = SX_NEG_INF; sxn[0] = 0.f; sxj[0] = SX_NEG_INF; sxb[0] = 0.f; sxc[0] = SX_NEG_INF;
+      oml = lm;
+      oil = li;
+      odl = ld;
     }
-    for (int i = 1; i <= L; i++) {
-      const double f = fac[i];
+    unsigned bits = 0;
+    float emax = SX_NEG_INF;
 #pragma unroll
-      for (int c = 0; c < VC; c++) {
-        const int k = lane * VC + c + 1;
-        const int64_t e = (int64_t)i * RS + c * 32 + lane;
-        pm[c] = k <= M ? (float)__dmul_rn(__dmul_rn((double)FM[e], (double)OM[e]), f) : 0.f;
-        pi[c] = k < M ? (float)__dmul_rn(__dmul_rn((double)FI[e], (double)OI[e]), f) : 0.f;
-        if (k <= M) sm[c] = fadd(sm[c], pm[c]);
-      }
-      // si: every insert posterior, row-major in k.  The row's values go to
-      // shared memory and lane 0 adds them in column order (the same order
-      // and roundings as a lane-to-lane baton, without its 32 shuffle hops).
-#pragma unroll
-      for (int c = 0; c < VC; c++) sirow[c * 32 + lane] = pi[c];
-      __syncwarp();
-      if (lane == 0) {
-        int c = 0, l = 0;
-        for (int k = 1; k <= M; k++) {
-          si = fadd(si, sirow[c * 32 + l]);
-          if (++c == VC) {
-            c = 0;
-            l++;
-          }
-        }
-      }
-      __syncwarp();
-      // OA row: M and I from the previous row, then the D chain in order
-      const float oml0 = __shfl_up_sync(kFull, omp[VC - 1], 1);
-      const float oil0 = __shfl_up_sync(kFull, oip[VC - 1], 1);
-      const float odl0 = __shfl_up_sync(kFull, odp[VC - 1], 1);
-      float emax = SX_NEG_INF;
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        const int k = lane * VC + c + 1;
-        om[c] = oi[c] = SX_NEG_INF;
-        if (k <= M) {
-          float sv = oa_gate(tp[0][c], xbp);
-          if (k >= 2) {
-            const float omv = c ? omp[c - 1] : oml0, oiv = c ? oip[c - 1] : oil0, odv = c ? odp[c - 1] : odl0;
-            sv = fmaxf(sv, oa_gate(tp[1][c], omv));
-            sv = fmaxf(sv, oa_gate(tp[2][c], oiv));
-            sv = fmaxf(sv, oa_gate(tp[3][c], odv));
-          } else {
-            sv = fmaxf(sv, 0.0f);
-          }
-          om[c] = fadd(sv, pm[c]);
-          emax = fmaxf(emax, om[c]);
-          oi[c] = fadd(fmaxf(oa_gate(tp[4][c], omp[c]), oa_gate(tp[5][c], oip[c])), pi[c]);
-        }
-      }
-      const float omleft0 = __shfl_up_sync(kFull, om[VC - 1], 1);
-      // The D chain od[k] = max(gate(t_md, om[k-1]), gate(t_dd, od[k-1])) only
-      // selects and takes maxima of non-negative values (or -inf), exact in
-      // any order, so it runs as a scan.  Column k maps the chain value v to
-      // max(a_k, v) when t_dd > 0 and to the constant max(a_k, 0) otherwise
-      // (k = 1: the constant -inf; k > M: the identity).  Each lane composes
-      // its columns' maps, the composites are scanned across lanes (5 shuffle
-      // rounds), and each lane replays its columns from its carry.
-      bool lc = false;          // the lane's composite: constant (true) or v -> max(lv, v)
-      float lv = SX_NEG_INF;
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        const int k = lane * VC + c + 1;
-        if (k > M) continue;
-        if (k == 1) {
-          lc = true;
-          lv = SX_NEG_INF;
-          continue;
-        }
-        const float a = oa_gate(tp[6][c], c ? om[c - 1] : omleft0);
-        if (tp[7][c] > 0.0f) {
-          lv = fmaxf(lv, a);
+    for (int c = 0; c < C; c++) {
+      const int k = k0 + c + 1;
+      const float pm = k <= M ? (float)__dmul_rn(__dmul_rn((double)fm[c], (double)bm[c]), f) : 0.f;
+      const float pi = k < M ? (float)__dmul_rn(__dmul_rn((double)fi[c], (double)bi[c]), f) : 0.f;
+      sm[c] = fadd(sm[c], pm);
+      om[c] = oi[c] = SX_NEG_INF;
+      if (k <= M) {
+        const float omv = c ? omp[c - 1] : oml, oiv = c ? oip[c - 1] : oil, odv = c ? odp[c - 1] : odl;
+        float sv = oa_gate(tr[0][c], xb);
+        unsigned best = kOaB;
+        if (k >= 2) {
+          sv = fmaxf(sv, oa_gate(tr[1][c], omv));
+          sv = fmaxf(sv, oa_gate(tr[2][c], oiv));
+          sv = fmaxf(sv, oa_gate(tr[3][c], odv));
+          // the first of M, I, D, B with the largest value
+          float top = oa_dis(tr[1][c], omv);
+          best = kOaM;
+          float v = oa_dis(tr[2][c], oiv);
+          if (v > top) { top = v; best = kOaI; }
+          v = oa_dis(tr[3][c], odv);
+          if (v > top) { top = v; best = kOaD; }
+          v = oa_dis(tr[0][c], xb);
+          if (v > top) best = kOaB;
         } else {
-          lc = true;
-          lv = fmaxf(a, 0.0f);
+          sv = fmaxf(sv, 0.0f);
+          // M, I and D have no cell to the left: the first of (-inf, -inf, -inf, B)
+          best = oa_dis(tr[0][c], xb) > SX_NEG_INF ? kOaB : kOaM;
         }
+        om[c] = fadd(sv, pm);
+        emax = fmaxf(emax, om[c]);
+        oi[c] = fadd(fmaxf(oa_gate(tr[4][c], omp[c]), oa_gate(tr[5][c], oip[c])), pi);
+        const bool from_i = !(oa_dis(tr[4][c], omp[c]) >= oa_dis(tr[5][c], oip[c]));
+        bits |= (best | (from_i ? kOaIfromI : 0u)) << (4 * c);
       }
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {  // inclusive scan: earlier lanes' composite, then this lane's
-        const int pc = __shfl_up_sync(kFull, (int)lc, o);
-        const float pv = __shfl_up_sync(kFull, lv, o);
-        if (lane >= o && !lc) {
-          lv = fmaxf(pv, lv);
-          lc = pc != 0;
-        }
-      }
-      float dcar = __shfl_up_sync(kFull, lv, 1);  // chain value entering this lane's first column
-      if (lane == 0) dcar = SX_NEG_INF;
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        const int k = lane * VC + c + 1;
-        if (k > M) {
-          od[c] = SX_NEG_INF;
-        } else if (k == 1) {
-          od[c] = SX_NEG_INF;
-          dcar = SX_NEG_INF;
-        } else {
-          const float omk1 = c ? om[c - 1] : omleft0;
-          od[c] = fmaxf(oa_gate(tp[6][c], omk1), oa_gate(tp[7][c], dcar));
-          dcar = od[c];
-          emax = fmaxf(emax, od[c]);
-        }
-      }
-      if (lane >= nl) {
-#pragma unroll
-        for (int c = 0; c < VC; c++) od[c] = SX_NEG_INF;
-      }
-#pragma unroll
-      for (int o = 16; o >= 1; o >>= 1) emax = fmaxf(emax, __shfl_xor_sync(kFull, emax, o));
-      const float xe_i = emax;
-      float t1 = ploop0 ? 0.0f : fadd(xjp, pj[i]);
-      float t2 = pe_loop0 ? 0.0f : xe_i;
-      const float xj_i = fmaxf(t1, t2);
-      t1 = ploop0 ? 0.0f : fadd(xcp, pc[i]);
-      t2 = pe_move0 ? 0.0f : xe_i;
-      const float xc_i = fmaxf(t1, t2);
-      const float xn_i = ploop0 ? 0.0f : fadd(xnp, pn[i]);
-      t1 = pmove0 ? 0.0f : xn_i;
-      t2 = pmove0 ? 0.0f : xj_i;
-      const float xb_i = fmaxf(t1, t2);
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        const int64_t e = (int64_t)i * RS + c * 32 + lane;
-        OM[e] = om[c];
-        OI[e] = oi[c];
-        OD[e] = od[c];
-        omp[c] = om[c];
-        oip[c] = oi[c];
-        odp[c] = od[c];
-      }
-      if (lane == 0) {
-        sxe[i] = xe_i; sxn[i] = xn_i; sxj[i] = xj_i; sxb[i] = xb_i; sxc[i] = xc_i;
-      }
-      xbp = xb_i;
-      xnp = xn_i;
-      xjp = xj_i;
-      xcp = xc_i;
     }
-    // null2 column sums: v[x] = sum_k (sm[k] * norm) * mo[x][k], k ascending
-    const float norm = __fdiv_rn(1.0f, (float)max(L, 1));
-    for (int x = 0; x < 20; x++) {
-      float v = 0.f;
-      for (int sl = 0; sl < nl; sl++) {
-        if (lane == sl) {
+    if (i < L) load_row(i + 1);
+    // the lane's composite map of its columns' D steps
+    bool lc = false;
+    float lv = SX_NEG_INF, a[C];
 #pragma unroll
-          for (int c = 0; c < VC; c++)
-            if (lane * VC + c + 1 <= M) v = fadd(v, fmul(fmul(sm[c], norm), img.at(kRowMo + x, c, lane)));
-        }
-        v = __shfl_sync(kFull, v, sl);
+    for (int c = 0; c < C; c++) {
+      a[c] = oa_gate(md[c], om[c]);
+      if (dd[c] > 0.0f) {
+        lv = fmaxf(lv, a[c]);
+      } else {
+        lc = true;
+        lv = fmaxf(a[c], 0.0f);
       }
-      if (lane == 0) out[x] = v;
     }
-    __syncwarp();  // the OA planes written by every lane, read by lane 0 below
-    if (lane == 0) {
-      out[20] = si;
-      // traceback (optimal_accuracy_coords, dp.rs:1420-1564)
-      auto TP = [&](int q, int k) { return img.at(kRowFwd + q, (k - 1) % VC, (k - 1) / VC); };
-      auto at = [&](const float* pl, int row, int k) { return pl[plane_at<VC>(row, k)]; };
-      enum St { SC, SE, SM, SI, SD, SB, SJ, SN };
-      St s0 = SC;
-      const int q_stripes = max(2, (M - 1) / 4 + 1);
-      int i = L, k = 0;
-      bool got_first = false, got_last = false;
-      int ci0 = 0, ci1 = 0, ck0 = 0, ck1 = 0;
-      const int64_t limit = 8LL * (L + 2) * (M + 2) + 64;
-      for (int64_t guard = 1; guard <= limit; guard++) {
-        St s1;
-        if (s0 == SC) {
-          if (i == 0) break;
-          const float a = ploop0 ? SX_NEG_INF : fadd(sxc[i - 1], pc[i]);
-          const float b = pe_move0 ? SX_NEG_INF : sxe[i];
-          s1 = a > b ? SC : SE;
-        } else if (s0 == SE) {
-          float mx = SX_NEG_INF;
-          int pick = 0;
-          St pst = SM;
-          for (int q = 0; q < q_stripes; q++) {
-            for (int rr = 0; rr < 4; rr++) {
-              const int kk = rr * q_stripes + q + 1;
-              if (kk <= M && at(OM, i, kk) >= mx) { mx = at(OM, i, kk); pick = kk; pst = SM; }
-            }
-            for (int rr = 0; rr < 4; rr++) {
-              const int kk = rr * q_stripes + q + 1;
-              if (kk <= M && at(OD, i, kk) > mx) { mx = at(OD, i, kk); pick = kk; pst = SD; }
-            }
-          }
-          if (pick == 0) break;
-          k = pick;
-          s1 = pst;
-        } else if (s0 == SM) {
-          if (i < 1 || k < 1) break;  // no predecessor left (reachable only when every path is -inf)
-          if (!got_last) { got_last = true; ci1 = i; ck1 = k; }
-          got_first = true;
-          ci0 = i;
-          ck0 = k;
-          float path[4] = {SX_NEG_INF, SX_NEG_INF, SX_NEG_INF, oa_dis(TP(0, k), sxb[i - 1])};
-          if (k >= 2) {
-            path[0] = oa_dis(TP(1, k), at(OM, i - 1, k - 1));
-            path[1] = oa_dis(TP(2, k), at(OI, i - 1, k - 1));
-            path[2] = oa_dis(TP(3, k), at(OD, i - 1, k - 1));
-          }
-          int best = 0;
-          for (int t = 1; t < 4; t++)
-            if (path[t] > path[best]) best = t;
-          k -= 1;
-          i -= 1;
-          s1 = best == 0 ? SM : best == 1 ? SI : best == 2 ? SD : SB;
-        } else if (s0 == SD) {
-          if (k < 1) break;
-          float a = SX_NEG_INF, b = SX_NEG_INF;
-          if (k >= 2) {
-            a = oa_dis(TP(6, k), at(OM, i, k - 1));
-            b = oa_dis(TP(7, k), at(OD, i, k - 1));
-          }
-          k -= 1;
-          s1 = a >= b ? SM : SD;
-        } else if (s0 == SI) {
-          if (i < 1 || k < 1) break;
-          const float a = oa_dis(TP(4, k), at(OM, i - 1, k));
-          const float b = oa_dis(TP(5, k), at(OI, i - 1, k));
-          i -= 1;
-          s1 = a >= b ? SM : SI;
-        } else if (s0 == SB) {
-          const float a = pmove0 ? SX_NEG_INF : sxn[i];
-          const float b = pmove0 ? SX_NEG_INF : sxj[i];
-          if (a > b) s1 = SN;
-          else break;
-        } else {
-          break;
-        }
-        if ((s1 == SN || s1 == SJ || s1 == SC) && s1 == s0) i -= 1;
-        if (s1 == SN) break;
-        s0 = s1;
+    const unsigned cm = __ballot_sync(kFull, lc);
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned upto = cm & (below | (1u << lane));
+    const int head = upto ? 31 - __clz(upto) : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float pv = __shfl_up_sync(kFull, lv, o);
+      if (lane - o >= head) lv = fmaxf(lv, pv);
+    }
+    float in = SX_NEG_INF;  // D of the warp's first column
+    if constexpr (MULTI) {
+      if (lane == 31) {
+        sh.val[warp] = lv;
+        sh.cst[warp] = cm != 0;
       }
-      const bool found = got_first && got_last;
-      out[21] = found ? 1.f : 0.f;
-      out[22] = (float)ci0;
-      out[23] = (float)ci1;
-      out[24] = (float)ck0;
-      out[25] = (float)ck1;
+      __syncthreads();
+      for (int q = 0; q < warp; q++) in = sh.cst[q] ? sh.val[q] : fmaxf(in, sh.val[q]);
+    }
+    float v = __shfl_up_sync(kFull, lv, 1);
+    if (lane == 0) v = in;
+    else if (!(cm & below)) v = fmaxf(v, in);
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      const int k = k0 + c + 1;
+      od[c] = k <= M ? v : SX_NEG_INF;
+      if (k <= M) emax = fmaxf(emax, v);
+      if (!(oa_dis(md[c], om[c]) >= oa_dis(dd[c], od[c]))) bits |= kOaDfromD << (4 * c);
+      v = dd[c] > 0.0f ? fmaxf(a[c], v) : fmaxf(a[c], 0.0f);
+    }
+    emax = warp_max_f32(emax);
+    if constexpr (MULTI) {
+      if (lane == 31) {
+        sh.mx[warp] = emax;
+        sh.prev[0][warp] = om[C - 1];
+        sh.prev[1][warp] = oi[C - 1];
+        sh.prev[2][warp] = od[C - 1];
+      }
+      __syncthreads();
+      for (int q = 0; q < nw; q++) emax = fmaxf(emax, sh.mx[q]);
+      if (lane == 0 && warp) {
+        lm = sh.prev[0][warp - 1];
+        li = sh.prev[1][warp - 1];
+        ld = sh.prev[2][warp - 1];
+      }
+    }
+    float t1 = ploop0 ? 0.0f : fadd(xj, pjv), t2 = pe_loop0 ? 0.0f : emax;
+    xj = fmaxf(t1, t2);
+    t1 = ploop0 ? 0.0f : fadd(xc, pcv);
+    t2 = pe_move0 ? 0.0f : emax;
+    xc = fmaxf(t1, t2);
+    xn = ploop0 ? 0.0f : fadd(xn, pnv);
+    t1 = pmove0 ? 0.0f : xn;
+    t2 = pmove0 ? 0.0f : xj;
+    xb = fmaxf(t1, t2);
+    if (i < L) load_specials(i + 1);
+    const int64_t at = (int64_t)i * width + k0;
+    store_cols<C>(OM + at, om);
+    store_cols<C>(OD + at, od);
+    uint8_t* db = dec + (int64_t)i * dec_row + k0 / 2;
+    if constexpr (C == 8) *reinterpret_cast<uint32_t*>(db) = bits;
+    else *reinterpret_cast<uint16_t*>(db) = (uint16_t)bits;
+    if (lead) {
+      sxe[i] = emax;
+      sxc[i] = xc;
+    }
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      omp[c] = om[c];
+      oip[c] = oi[c];
+      odp[c] = od[c];
     }
   }
+  // null2 column sums: v[x] = sum_k (sm[k] * norm) * mo[x][k], k ascending, one
+  // residue a lane
+  const float norm = __fdiv_rn(1.0f, (float)max(L, 1));
+#pragma unroll
+  for (int c = 0; c < C; c++) sm[c] = fmul(sm[c], norm);
+  store_cols<C>(T + k0, sm);
+  team_sync<MULTI>();  // also makes the planes and decisions of every thread visible to the first warp
+  if (MULTI && warp) return;
+  if (lane < 20) {
+    const float4* s4 = reinterpret_cast<const float4*>(T);
+    const float4* m4 = reinterpret_cast<const float4*>(img + (kXMo + lane) * width);
+    float v = 0.f;
+#pragma unroll 4
+    for (int q = 0; q < (M + 3) / 4; q++) {
+      const float4 a = s4[q], b = __ldg(m4 + q);
+      v = fadd(fadd(fadd(fadd(v, fmul(a.x, b.x)), fmul(a.y, b.y)), fmul(a.z, b.z)), fmul(a.w, b.w));
+    }
+    out[lane] = v;
+  }
+  __syncwarp();
+  // traceback (optimal_accuracy_coords, dp.rs:1420-1564): every lane follows
+  // the same path.  C loops down to the last row whose E is not below it.
+  int i = L;
+  while (i >= 1) {
+    const int q = i - lane;
+    bool stop = q < 1;
+    if (!stop) {
+      const float a = ploop0 ? SX_NEG_INF : fadd(sxc[q - 1], pc[q]);
+      const float b = pe_move0 ? SX_NEG_INF : sxe[q];
+      stop = !(a > b);
+    }
+    const unsigned m = __ballot_sync(kFull, stop);
+    if (m) {
+      i -= __ffs(m) - 1;
+      break;
+    }
+    i -= 32;
+  }
+  int k = 0;
+  St s0 = kSM;
+  if (i >= 1) {
+    // E: among the cells equal to the row's maximum the last M in striped
+    // order, or else the first D
+    const int Q = max(2, (M - 1) / 4 + 1);
+    const float mx = sxe[i];
+    int mkey = -1, dkey = INT_MAX;
+    for (int kk = lane + 1; kk <= M; kk += 32) {
+      const int key = ((kk - 1) % Q) * 4 + (kk - 1) / Q;
+      if (OM[(int64_t)i * width + kk - 1] == mx) mkey = max(mkey, key);
+      if (OD[(int64_t)i * width + kk - 1] == mx) dkey = min(dkey, key);
+    }
+    mkey = __reduce_max_sync(kFull, mkey);
+    dkey = __reduce_min_sync(kFull, dkey);
+    if (mkey >= 0) {
+      k = (mkey & 3) * Q + (mkey >> 2) + 1;
+    } else if (dkey != INT_MAX) {
+      k = (dkey & 3) * Q + (dkey >> 2) + 1;
+      s0 = kSD;
+    }
+  }
+  bool found = false;
+  int ci0 = 0, ci1 = 0, ck0 = 0, ck1 = 0;
+  auto nibble = [&](int ii, int kk) -> unsigned {
+    return ii >= 1 && kk >= 1 ? (dec[(int64_t)ii * dec_row + (kk - 1) / 2] >> (4 * ((kk - 1) & 1))) & 15u : 0u;
+  };
+  while (i >= 1 && k >= 1) {  // every turn moves up or left
+    if (s0 == kSM) {
+      const unsigned mine = nibble(i - lane, k - lane);
+      const bool on = i - lane >= 1 && k - lane >= 1;
+      if (!found) {
+        found = true;
+        ci1 = i;
+        ck1 = k;
+      }
+      // the run of matches: lanes before the first whose predecessor is not M
+      const unsigned stop = __ballot_sync(kFull, !on || (mine & 3u) != kOaM);
+      const int run = stop ? __ffs(stop) - 1 : 32;
+      const bool inside = run < 32 && i - run >= 1 && k - run >= 1;  // lane `run` is a cell (a match) of the path
+      const int last = inside ? run : run - 1;  // run >= 1 here if not inside: lane 0 is a cell
+      ci0 = i - last;
+      ck0 = k - last;
+      if (run == 32) {
+        i -= 32;
+        k -= 32;
+        continue;
+      }
+      if (!inside) break;  // the path left the matrix
+      const unsigned p = __shfl_sync(kFull, mine, run) & 3u;
+      i -= run + 1;
+      k -= run + 1;
+      if (p == kOaB) break;
+      s0 = p == kOaI ? kSI : kSD;
+    } else if (s0 == kSI) {
+      const unsigned d = nibble(i, k);
+      i -= 1;
+      if (!(d & kOaIfromI)) s0 = kSM;
+    } else {
+      const unsigned d = nibble(i, k - 1);  // 0 for k = 1: no D there, the path ends at the left edge
+      k -= 1;
+      if (!(d & kOaDfromD)) s0 = kSM;
+    }
+  }
+  if (lane == 0) {
+    out[21] = found ? 1.f : 0.f;
+    out[22] = (float)ci0;
+    out[23] = (float)ci1;
+    out[24] = (float)ck0;
+    out[25] = (float)ck1;
+  }
+}
+
+// si: every insert posterior of the envelope added in row-major order (the
+// null2 length correction, dp.rs:1310-1350).  The sum is one chain of L * M
+// adds, but a term below half an ulp of the running sum leaves it unchanged,
+// and the sum never falls: kInsertRows warps compute one row each against the
+// sum as it stood a batch earlier and keep, in order, the groups of four
+// columns with a term that can still count; one warp adds those while the
+// others prepare the next rows.
+constexpr int kInsertRows = 8;
+static __global__ void __launch_bounds__(32 * (kInsertRows + 1)) env_insert_kernel(
+    const EnvRec* __restrict__ recs, int n, const DevProfile* __restrict__ profs, const float* __restrict__ planes,
+    const double* __restrict__ facs, float* __restrict__ outs, int max_width) {
+  extern __shared__ float4 sm_row[];  // 2 batches x kInsertRows lists of max_width / 4 groups
+  __shared__ int s_n[2][kInsertRows];
+  __shared__ float s_si;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const EnvRec r = recs[blockIdx.x];
+  const int M = profs[r.p].m, L = r.lr, width = r.width;
+  const int64_t PL = (int64_t)(L + 1) * width;
+  const float* FI = planes + r.plane_off + PL;
+  const float* BI = planes + r.plane_off + 3 * PL;
+  const double* fac = facs + r.fac_off;
+  const int cap = max_width / 4;
+  if (threadIdx.x == 0) s_si = 0.f;
+  __syncthreads();
+  const int batches = (L + kInsertRows - 1) / kInsertRows;
+  float si = 0.f;
+  for (int b = 0; b <= batches; b++) {  // batch b is prepared while batch b - 1 is added
+    if (warp == 0) {
+      if (b) {
+        for (int q = 0; q < kInsertRows; q++) {
+          const float4* t = sm_row + (((b - 1) & 1) * kInsertRows + q) * cap;
+          const int m = s_n[(b - 1) & 1][q];
+          float4 x = m ? t[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int e = 0; e < m; e++) {
+            const float4 nx = e + 1 < m ? t[e + 1] : x;
+            si = fadd(fadd(fadd(fadd(si, x.x), x.y), x.z), x.w);
+            x = nx;
+          }
+        }
+      }
+    } else {
+      const int q = warp - 1, i = b * kInsertRows + q + 1;
+      int m = 0;
+      if (i <= L) {
+        // half an ulp of the sum: 2^(exponent - 24), 0 for a sum below 2^-102
+        const int e = (__float_as_int(s_si) >> 23) - 24;
+        const float half = e > 0 ? __int_as_float(e << 23) : 0.f;
+        const double f = fac[i];
+        float4* list = sm_row + ((b & 1) * kInsertRows + q) * cap;
+        const float4* fi = reinterpret_cast<const float4*>(FI + (int64_t)i * width) + lane;
+        const float4* bi = reinterpret_cast<const float4*>(BI + (int64_t)i * width) + lane;
+        for (int base = 0; base < M; base += 512) {  // four loads of each plane in flight
+          float4 x[4], y[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (base + 128 * u < M) {  // width is a multiple of 128
+              x[u] = __ldg(fi + base / 4 + 32 * u);
+              y[u] = __ldg(bi + base / 4 + 32 * u);
+            }
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            if (base + 128 * u >= M) break;
+            const int k = base + 128 * u + 4 * lane;  // columns k+1 .. k+4
+            auto post = [&](float a, float c, int kk) {
+              return kk < M ? (float)__dmul_rn(__dmul_rn((double)a, (double)c), f) : 0.f;
+            };
+            const float4 p = make_float4(post(x[u].x, y[u].x, k + 1), post(x[u].y, y[u].y, k + 2),
+                                         post(x[u].z, y[u].z, k + 3), post(x[u].w, y[u].w, k + 4));
+            // counts unless zero or below half an ulp (NaN counts)
+            auto counts = [&](float t) { return t != 0.f && !(t < half); };
+            const bool any = counts(p.x) || counts(p.y) || counts(p.z) || counts(p.w);
+            const unsigned mask = __ballot_sync(kFull, any);
+            if (any) list[m + __popc(mask & ((1u << lane) - 1u))] = p;
+            m += __popc(mask);
+          }
+        }
+      }
+      if (lane == 0) s_n[b & 1][q] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_si = si;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) outs[r.out_off + 20] = si;
 }
 
 
 // ---- stochastic traceback ensembles of multi-domain regions ------------------
 // region_trace_ensemble (src/hmmer/pipeline.rs:360-477) up to the clustering:
 // kTraceSamples sampled traces (stochastic_trace, src/hmmer/dp.rs:1075-1258)
-// through the region's multihit Forward matrix (env_forward_kernel<VC, true>,
+// through the region's multihit Forward matrix (env_rows_kernel<C, MULTI, true>,
 // diagonal layout), one Easel LCG stream per region, the per-trace null2 of
 // every sampled domain and its per-position sums.  The host clusters the
 // samples and takes the logs.
@@ -766,7 +546,7 @@ struct TraceRec {
   int32_t i0, lr;      // region residues i0 .. i0+lr-1 (0-based)
   float ploop, pmove;  // multihit special transitions of the target's length
   float pe_loop, pe_move;
-  int64_t plane_off;   // diagonal M I D planes of env_forward_kernel<VC, true>
+  int64_t plane_off;   // diagonal M I D planes of env_rows_kernel<C, MULTI, true>
   int64_t row_off;     // its raw special rows, 6 (lr+1)
   int64_t n2_off;      // per-position null2 sums, lr+1 floats (slot 0 unused)
   int64_t col_off;     // the profile's column table (kTraceCol floats per column)

@@ -1,5 +1,7 @@
-// Forward and Backward in the reference's order of operations
-// (src/hmmer/dp.rs:229-392): the raw special rows of final pairs.
+// Forward and Backward in the reference's order of operations: the raw special
+// rows of final pairs (src/hmmer/dp.rs:229-392) and, with the M and I matrices
+// kept, the full-matrix passes of envelopes and multi-domain regions
+// (dp.rs:442-601).
 //
 // A team -- one warp up to 256 columns, a CTA of several warps above -- runs
 // one pair in one direction, thread t holding columns t*C+1 .. t*C+C.  What
@@ -19,6 +21,8 @@
 //     a scan of the lanes' transfers gives the first guess and two or three
 //     rounds repair its last bits;
 //   * the descending D chain of Backward, the same way from the other end.
+// A thread's Forward chain starts from the D of its first column and ends with
+// the D of its right neighbour's, so it needs no match value but its own.
 // Between warps the carry goes through shared memory: each warp runs its D
 // chain from carry 0, publishes its end, takes its neighbour's and repairs its
 // first lanes; a warp whose own end that changed (its 256 columns did not
@@ -55,7 +59,7 @@ struct RowRec {
 };
 
 struct XShared {  // exchange between the warps of a team
-  float mv[kXMaxWarps];       // last (Forward) or first (Backward) column's new match value
+  float mv[kXMaxWarps];       // Backward: the first column's match term
   float end[kXMaxWarps];      // D at the warp's end of the chain
   float prev[3][kXMaxWarps];  // M, I, D of the last column
   int mx[kXMaxWarps];
@@ -159,20 +163,26 @@ __device__ __forceinline__ float scan_guess(float a, int lane, const float (&bs)
   return UP ? __shfl_up_sync(kFull, a, 1) : __shfl_down_sync(kFull, a, 1);
 }
 
-// Ascending D chain of a warp from `in` at its first column: rounds from the
-// guessed carries `cin` until no carry changes.
+// Ascending D chain of a warp whose first column has D = `in`: rounds from the
+// guessed carries `cin` until no carry changes.  a and p are the terms and
+// factors out of each column; returns the D right of the lane's last column.
 template <int C>
-__device__ __forceinline__ void settle_up(float (&d)[C], const float (&a)[C], const float (&p)[C], float cin, float in,
-                                          int lane) {
+__device__ __forceinline__ float settle_up(float (&d)[C], const float (&a)[C], const float (&p)[C], float cin, float in,
+                                           int lane) {
+  float v = 0.f;
   for (int it = 0; it < 32; it++) {
-    float v = cin;
+    v = cin;
 #pragma unroll
-    for (int c = 0; c < C; c++) d[c] = v = fadd(a[c], fmul(v, p[c]));
+    for (int c = 0; c < C; c++) {
+      d[c] = v;
+      v = fadd(a[c], fmul(v, p[c]));
+    }
     const float up = __shfl_up_sync(kFull, v, 1);
     const float nc = lane ? up : in;
     if (__all_sync(kFull, same_bits(nc, cin))) break;
     cin = nc;
   }
+  return v;
 }
 // Descending: d[k] = ((a_k + p_k d[k+1]) + e) from `in` past its last column.
 template <int C>
@@ -189,11 +199,24 @@ __device__ __forceinline__ void settle_down(float (&d)[C], const float (&a)[C], 
   }
 }
 
-// Forward (dp.rs:229-298).
-template <int C, bool MULTI>
+// What a pass keeps of the matrices: nothing, the M and I planes (rows 0..L of
+// the team's width), or the M, I and D planes in the diagonal layout that the
+// stochastic traceback reads.
+enum Keep { kKeepNone, kKeepMI, kKeepDiag };
+
+// Diagonal layout of a region's M/I/D planes for the stochastic traceback:
+// cell (i, k), 1 <= i <= lr, 1 <= k <= M, at (i - k + M - 1) * M + (k - 1), so
+// the cells of a run of match states, (i, k) -> (i-1, k-1), are adjacent.
+__host__ __device__ __forceinline__ int64_t diag_at(int64_t i, int k, int M) {
+  return (i - k + M - 1) * (int64_t)M + (k - 1);
+}
+__host__ __device__ __forceinline__ int64_t diag_plane(int64_t lr, int M) { return (lr + M - 1) * (int64_t)M; }
+
+// Forward (dp.rs:229-298, 442-513).
+template <int C, bool MULTI, Keep KEEP>
 __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int M, const uint8_t* __restrict__ s, int L,
                                               float ploop, float pmove, float pe_loop, float pe_move, float* orow,
-                                              float* T, XShared& sh) {
+                                              float* planes, float* T, XShared& sh) {
   const int lane = threadIdx.x & 31;
   const int warp = MULTI ? threadIdx.x >> 5 : 0;
   const int width = (MULTI ? blockDim.x : 32) * C;
@@ -201,9 +224,14 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
   const bool lead = MULTI ? threadIdx.x == 0 : lane == 0;
   const int nsum = max(16, (M + 15) & ~15);
   const float* im = img + k0;
-  float tr[8][C];
+  float tr[8][C];  // bm, mm im dm into the column, mi ii, then md dd out of it
 #pragma unroll
-  for (int q = 0; q < 8; q++) load_cols<C>(im + (kXFwd + q) * width, tr[q]);
+  for (int q = 0; q < 6; q++) load_cols<C>(im + (kXFwd + q) * width, tr[q]);
+  load_cols<C>(im + (kXBwd + 2) * width, tr[6]);
+  load_cols<C>(im + (kXBwd + 6) * width, tr[7]);
+  float* FM = planes;
+  float* FI = KEEP == kKeepDiag ? FM + diag_plane(L, M) : FM + (int64_t)(L + 1) * width;
+  float* FD = FI + diag_plane(L, M);
   float bs[5], ball, b = 1.f;
 #pragma unroll
   for (int c = 0; c < C; c++) b = b * tr[7][c];
@@ -247,33 +275,24 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
       mv[c] = fmul(t, eo[c]);
       iv[c] = fmul(fadd(fmul(mp[c], tr[4][c]), fmul(ip[c], tr[5][c])), ins);
     }
-    float mcl = __shfl_up_sync(kFull, mv[C - 1], 1);
-    if constexpr (MULTI) {
-      if (lane == 31) sh.mv[warp] = mv[C - 1];
-      __syncthreads();
-      if (lane == 0) mcl = warp ? sh.mv[warp - 1] : 0.f;
-    } else {
-      if (lane == 0) mcl = 0.f;
-    }
     float end = 0.f;
 #pragma unroll
     for (int c = 0; c < C; c++) {
-      a[c] = fmul(c ? mv[c - 1] : mcl, tr[6][c]);
+      a[c] = fmul(mv[c], tr[6][c]);
       end = fadd(a[c], fmul(end, tr[7][c]));
     }
     float g = scan_guess<true>(end, lane, bs, steps);
     if (lane == 0) g = 0.f;
-    settle_up<C>(dv, a, tr[7], g, 0.f, lane);
+    end = settle_up<C>(dv, a, tr[7], g, 0.f, lane);
     if constexpr (MULTI) {
-      if (lane == 31) sh.end[warp] = dv[C - 1];
+      if (lane == 31) sh.end[warp] = end;
       __syncthreads();
       if (warp) {
-        const float in = sh.end[warp - 1];
-        const float own = dv[C - 1];
+        const float in = sh.end[warp - 1], own = end;
         float c0 = __shfl_up_sync(kFull, own, 1);
         c0 = lane ? fadd(c0, fmul(bpre, in)) : in;
-        settle_up<C>(dv, a, tr[7], c0, in, lane);
-        if (lane == 31 && !same_bits(dv[C - 1], own)) sh.flag = 1;
+        end = settle_up<C>(dv, a, tr[7], c0, in, lane);
+        if (lane == 31 && !same_bits(end, own)) sh.flag = 1;
       }
     }
     auto publish = [&]() {
@@ -292,13 +311,13 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
     if constexpr (MULTI) {
       if (sh.flag) {  // a warp's end changed: exchange the ends until none does
         for (int it = 0; it <= kXMaxWarps; it++) {
-          const float own = dv[C - 1];
+          const float own = end;
           if (lane == 31) sh.end[warp] = own;
           __syncthreads();
           const float in = warp ? sh.end[warp - 1] : 0.f;
           const float up = __shfl_up_sync(kFull, own, 1);
-          settle_up<C>(dv, a, tr[7], lane ? up : in, in, lane);
-          if (!__syncthreads_or(lane == 31 && !same_bits(dv[C - 1], own))) break;
+          end = settle_up<C>(dv, a, tr[7], lane ? up : in, in, lane);
+          if (!__syncthreads_or(lane == 31 && !same_bits(end, own))) break;
         }
         publish();
       }
@@ -337,6 +356,21 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
       float* o = orow + 6 * (int64_t)(i + 1);
       o[0] = xn; o[1] = xb; o[2] = xe; o[3] = xj; o[4] = xc; o[5] = scale;
     }
+    if constexpr (KEEP == kKeepMI) {
+      store_cols<C>(FM + (int64_t)(i + 1) * width + k0, mv);
+      store_cols<C>(FI + (int64_t)(i + 1) * width + k0, iv);
+    } else if constexpr (KEEP == kKeepDiag) {
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        const int k = k0 + c + 1;
+        if (k <= M) {
+          const int64_t at = diag_at(i + 1, k, M);
+          FM[at] = mv[c];
+          FI[at] = iv[c];
+          FD[at] = dv[c];
+        }
+      }
+    }
 #pragma unroll
     for (int c = 0; c < C; c++) {
       mp[c] = mv[c];
@@ -349,12 +383,13 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
   }
 }
 
-// Backward (dp.rs:301-392): row L (E, C), rows L-1..1 (N B E J C, rescale
-// factor) and the row-0 B sum in slot 1 of row 0.
-template <int C, bool MULTI>
+// Backward (dp.rs:301-392, 516-601): row L (E, C), rows L-1..1 (N B E J C,
+// rescale factor) and the row-0 B sum in slot 1 of row 0.
+template <int C, bool MULTI, Keep KEEP>
 __device__ __forceinline__ void exact_backward(const float* __restrict__ img, int M, const uint8_t* __restrict__ s,
                                                int L, float ploop, float pmove, float pe_loop, float pe_move,
-                                               float* orow, float* T, XShared& sh) {
+                                               float* orow, float* planes, float* T, XShared& sh) {
+  static_assert(KEEP != kKeepDiag, "only the Forward matrix is kept in the diagonal layout");
   const int lane = threadIdx.x & 31;
   const int warp = MULTI ? threadIdx.x >> 5 : 0;
   const int nw = MULTI ? blockDim.x >> 5 : 1;
@@ -436,6 +471,12 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
   }
 #pragma unroll
   for (int c = 0; c < C; c++) mn[c] = fadd(xe, fmul(c < C - 1 ? dc[c + 1] : dnr, tr[2][c]));
+  float* BM = planes;
+  float* BI = BM + (int64_t)(L + 1) * width;
+  if constexpr (KEEP == kKeepMI) {
+    store_cols<C>(BM + (int64_t)L * width + k0, mn);
+    store_cols<C>(BI + (int64_t)L * width + k0, in_);
+  }
   if (lead) {
     float* o = orow + 6 * (int64_t)L;
     o[0] = 0.f; o[1] = 0.f; o[2] = xe; o[3] = 0.f; o[4] = xc; o[5] = 0.f;
@@ -523,6 +564,10 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
       float* o = orow + 6 * (int64_t)i;
       o[0] = xn; o[1] = xb_o; o[2] = xe; o[3] = xj; o[4] = xc; o[5] = scale;
     }
+    if constexpr (KEEP == kKeepMI) {
+      store_cols<C>(BM + (int64_t)i * width + k0, mn);
+      store_cols<C>(BI + (int64_t)i * width + k0, in_);
+    }
 #pragma unroll
     for (int c = 0; c < C; c++) eo[c] = eon[c];
     x = x1;
@@ -556,9 +601,10 @@ __global__ void __launch_bounds__(256) exact_rows_kernel(const RowRec* __restric
   const uint8_t* s = res + toff[r.t];
   const float4 xs = xsc[r.t];
   if (blockIdx.y == 0)
-    exact_forward<C, MULTI>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off, T, sh);
+    exact_forward<C, MULTI, kKeepNone>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off, nullptr, T, sh);
   else
-    exact_backward<C, MULTI>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off + 6 * (int64_t)(L + 1), T, sh);
+    exact_backward<C, MULTI, kKeepNone>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off + 6 * (int64_t)(L + 1),
+                                        nullptr, T, sh);
 }
 
 }  // namespace sxk

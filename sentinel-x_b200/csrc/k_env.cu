@@ -1,25 +1,25 @@
 // Instantiations of the envelope-rescoring and region kernels, one per
-// column width.
+// kXShapes entry's kernel.
 #include "shapes.hpp"
 
 namespace sx {
-namespace {
-template <int I>
-struct EnvTable {
-  static void fill(KernelTables& t) {
-    t.envf[I] = sxk::env_forward_kernel<kVcBins[I]>;
-    t.envb[I] = sxk::env_backward_kernel<kVcBins[I]>;
-    t.envp[I] = sxk::env_post_kernel<kVcBins[I]>;
-    t.regf[I] = sxk::env_forward_kernel<kVcBins[I], true>;
-    EnvTable<I + 1>::fill(t);
-  }
-};
-template <>
-struct EnvTable<kNumVbins> {
-  static void fill(KernelTables&) {}
-};
-}  // namespace
 
-void fill_env_tables(KernelTables& t) { EnvTable<0>::fill(t); }
+void fill_env_tables(KernelTables& t) {
+  for (int s = 0; s < kNumXShapes; s++) {
+    if (kXShapes[s].warps > 1) {
+      t.envr[s] = sxk::env_rows_kernel<8, true, false>;
+      t.regf[s] = sxk::env_rows_kernel<8, true, true>;
+      t.envoa[s] = sxk::env_oa_kernel<8, true>;
+    } else if (kXShapes[s].c == 8) {
+      t.envr[s] = sxk::env_rows_kernel<8, false, false>;
+      t.regf[s] = sxk::env_rows_kernel<8, false, true>;
+      t.envoa[s] = sxk::env_oa_kernel<8, false>;
+    } else {
+      t.envr[s] = sxk::env_rows_kernel<4, false, false>;
+      t.regf[s] = sxk::env_rows_kernel<4, false, true>;
+      t.envoa[s] = sxk::env_oa_kernel<4, false>;
+    }
+  }
+}
 
 }  // namespace sx

@@ -120,8 +120,13 @@ void queue_rows(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T
   join_aux(S.hi);
 }
 
+// Floats of one chunk of rows: at most 128 MB, which fills the GPU many times
+// over with the shortest targets and keeps the page-locked copy in the pool
+// (one chunk of 485 MB, 100,000 pairs of 100 residues, spent 0.3 s locking
+// fresh pages on each call).
 int64_t rows_budget(const sx_engine* E) {
-  return std::max<int64_t>(scratch_budget(E, E->batch_bytes) / (int64_t)sizeof(float), 2 << 20);
+  return std::max<int64_t>(scratch_budget(E, std::min<int64_t>(E->batch_bytes, 128LL << 20)) / (int64_t)sizeof(float),
+                           2 << 20);
 }
 
 void rows_pass(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T, const std::vector<FinalPair>& pairs,
@@ -1035,23 +1040,24 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
   HostQueue hq(E->host_threads);  // declared after what its jobs use, so it is joined first
   // device rows of a block's final pairs; their domain definition is queued
   // and runs while the engine thread moves on to the next block
-  // Domain definition of a block runs on the host pool, hidden behind the
-  // device work of later blocks, while that host work stays well below the
-  // block's device time; past that (hit-heavy blocks) the envelopes' full-
-  // matrix passes go to the device.  Host: ~44 ns per DP cell of the final
-  // pairs per thread; device cascade ~4.4e12 cells/s (B200, Pfam-scale).
-  auto device_envelopes = [&](const BlockOut* B, double block_cells, bool last_of_several) {
+  // A block's decoding, regions and traces run on the host pool, beside the
+  // device work of later blocks; its envelopes' full-matrix passes go to the
+  // device after the cascade, all blocks' at once, unless the host would do
+  // them in less than a pass and its round trips cost (~0.5 ms).  Host: ~44 ns
+  // per DP cell of the final pairs per thread, the largest pair on one thread.
+  // Measured, device against host passes: one profile of M = 100 5.1 / 6.5 ms,
+  // 13 profiles 8.7 / 13.3, marker-set genome 92 / 695, 16 M short pairs 88 /
+  // 119, Pfam-scale 441 / 461.
+  auto device_envelopes = [&](const BlockOut* B) {
     if (E->flags & SX_FLAG_ENV_DEVICE) return true;
     if (E->flags & SX_FLAG_ENV_HOST) return false;
-    // the last block's host work is hidden behind nothing: its envelopes go
-    // to the device passes, which run them all at once (Pfam-scale search
-    // 461 -> 452 ms, the tail after the last device stage 49 -> 33 ms)
-    if (last_of_several) return true;
-    double fin = 0;
-    for (const auto& f : B->finals) fin += (double)P->h[f.p].m * (double)T->len[f.t];
-    const double host_ms = fin * 44e-9 * 1e3 / std::max(1, E->host_threads);
-    const double dev_ms = block_cells / 4.4e12 * 1e3;
-    return host_ms > 0.5 * dev_ms + 5.0;
+    double sum = 0, most = 0;
+    for (const auto& f : B->finals) {
+      const double cells = (double)P->h[f.p].m * (double)T->len[f.t];
+      sum += cells;
+      most = std::max(most, cells);
+    }
+    return std::max(most, sum / std::max(1, E->host_threads)) * 44e-6 > 0.5;
   };
   // Stochastic traces of a block's multi-domain regions: on the host pool at
   // once (hidden behind later device work) unless their estimated host time
@@ -1203,7 +1209,7 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
     while (!cascade_finish(E, S, P, T, th, o, runs[b], B->finals)) cascade_launch(E, S, P, T, th, runs[b]);
     timeline.add("b" + std::to_string(b) + "_cascade", t_start);
     nfinal += (int64_t)B->finals.size();
-    rows_and_queue(S, B, device_envelopes(B, runs[b].cells_total, b + 1 == runs.size() && runs.size() > 1));
+    rows_and_queue(S, B, device_envelopes(B));
   }
   if (!unfiltered.empty() && nt > 0) {
     outs.push_back(std::make_unique<BlockOut>());

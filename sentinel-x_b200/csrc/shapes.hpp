@@ -114,17 +114,17 @@ typedef void (*AdjFFn)(const sxk::AdjPair*, int, const DevProfile*, const float*
                        const int32_t*, const float4*, float*, double*, double*);
 typedef void (*AdjBFn)(const sxk::AdjPair*, int, const DevProfile*, const float*, const uint8_t*, const int64_t*,
                        const int32_t*, const float4*, float*, const double*, const double*, float*);
-typedef void (*EnvPassFn)(const sxk::EnvRec*, int, const DevProfile*, const float*, const uint8_t*, const int64_t*,
+typedef void (*EnvRowsFn)(const sxk::EnvRec*, int, const DevProfile*, const float*, const uint8_t*, const int64_t*,
                           float*, float*);
-typedef void (*EnvPostFn)(const sxk::EnvRec*, int, const DevProfile*, const float*, float*, float*, const double*,
-                          float*);
+typedef void (*EnvOaFn)(const sxk::EnvRec*, int, const DevProfile*, const float*, float*, float*, const double*,
+                        float*);
 
 struct KernelTables {
   MsvFn msv[kNumMsvShapes];
   Msv16Fn msv16[kNumMsvShapes];  // the packed pre-screen, same shapes
-  EnvPassFn envf[kNumVbins], envb[kNumVbins];
-  EnvPostFn envp[kNumVbins];
-  EnvPassFn regf[kNumVbins];
+  EnvRowsFn envr[kNumXShapes];  // envelopes: Forward and Backward matrices
+  EnvRowsFn regf[kNumXShapes];  // regions: Forward matrix in the diagonal layout
+  EnvOaFn envoa[kNumXShapes];   // envelopes: posteriors, null2, optimal accuracy
   VitFn vit[kNumVbins];
   FwdFn fwd_scan[kNumVbins];  // the F3 pre-screen
   XRowsFn xrows[kNumXShapes];  // exact Forward and Backward rows
