@@ -66,6 +66,85 @@ __device__ __forceinline__ int q32_up(float x) {
   return (int)ceilf(__fmul_rn(x, 1048576.0f)) + kQ32Rho;
 }
 
+// The recurrence cell = max(diagonal, B) + e and the row maximum cost three
+// packed ALU operations a column as they stand, and the ALU pipe (64 packed
+// operations per clock per SM, fused or not: add, max, max(a + b, c) and
+// max(a, b, c) all issue at that rate on B200) is the kernel's bound.  So a
+// lane holds w = max(cell, B) instead, the next row's input:
+//     w'[k] = max(w[k-1] + e[k], B')            one fused operation,
+//     E = max over w'                           half a three-input maximum,
+// 1.5 operations a column, with B' the B of the row being computed.  That
+// depends on the row's own E only when E raises base = max(N, J), which is rare
+// (a pair's few best rows): B' is predicted from base decayed by tloop, the
+// lanes vote on whether any E lies above the threshold at which it raises base,
+// and only then the group takes its maximum, updates base and raises w to the
+// row's B (w' = max(cell, B') and B >= B', so max(w', B) = max(cell, B)).
+// J itself matters only at the target's end: each lane keeps its own J from its
+// own columns' maximum and the group combines them once, which is exact, as
+// max and the common decay commute.
+// The two profiles' base and constants are int32 in units of 2^-25 nat here,
+// so the int16 value of a state is the upper half of its word.  J itself
+// matters only at the target's end: above N it is base; below N the pair's
+// bound is below N's, which fails F1 (where it might not, or where the bound
+// itself is asked for, the tile also tracks J).
+//   * E taken over w' is max(E, B').  That cannot raise base, as B' plus the
+//     E->J cost is below it.
+//   * rows past the target's end in its last block of four read '*' (-16 nats
+//     everywhere): they raise nothing and their decay is undone.
+//   * a target long enough to reach the entry floor or to have tloop rounded
+//     up to 0 (L > 390,000) is recomputed by the plain recurrence.
+//   * a tile that tracks J keeps it per lane, of the lane's own columns, and
+//     the group combines them once, which is exact, as max and the common decay commute;
+//     a final J at or below the final B's level may come from B' and is
+//     recomputed by the plain recurrence too (no row of the target scored above
+//     its entry: all '*', say).
+// Bound now: the ALU pipe, about 70 operations per row of 40 columns, and 2
+// bytes of shared memory per cell (64 cells per clock per SM).  The next row's
+// first scores are loaded before the vote, whose branch would otherwise keep
+// them behind it.  Measured on B200 (296 profiles of one length x 12,000
+// targets, useful cells per clock per SM, before -> now): M = 100 40.0 -> 46.1,
+// 160 42.9 -> 50.7, 208 44.4 -> 53.1, 300 40.1 -> 49.6, 600 39.6 -> 50.7, 1000
+// 45.3 -> 53.9; the Pfam-scale search's pre-screen 298 -> 255 ms, and 211 with
+// tiles of equal work.
+//
+// Plain recurrence of one target for the group (see above); w is scratch.
+// Returns J of both halves at row L (units of 2^-20 nat) and the caps' flags.
+template <int G, int C, int ROWP>
+__device__ __noinline__ int4 msv16_plain(const uint4* __restrict__ rows, const uint8_t* __restrict__ seq, int L, int j,
+                                         unsigned gmask, int tloop, int tmove, int tbm_a, int tbm_b, int cap_a,
+                                         int cap_b, int nln2) {
+  unsigned w[C];
+#pragma unroll
+  for (int c = 0; c < C; c++) w[c] = kQ16Neg2;
+  int xn = 0, xja = kQ32Neg, xjb = kQ32Neg;
+  bool biga = false, bigb = false;
+  auto entry = [&](int xb, int tbm) { return max((xb + tbm + 2047) >> (kQ32Shift - kQ16Shift), kQ16BeFloor); };
+  unsigned bew = __byte_perm((unsigned)entry(tmove, tbm_a), (unsigned)entry(tmove, tbm_b), 0x5410);
+  for (int i = 0; i < L; i++) {
+    const uint4* rowp = rows + (int)seq[i] * ROWP + j;
+    unsigned left = __shfl_up_sync(gmask, w[C - 1], 1, G);
+    if (j == 0) left = kQ16Neg2;
+    unsigned xe = kQ16Neg2;
+#pragma unroll
+    for (int c = C - 1; c >= 0; c--) {
+      const uint4 a4 = rowp[(c >> 2) * G];
+      const unsigned ra = (c & 3) == 0 ? a4.x : (c & 3) == 1 ? a4.y : (c & 3) == 2 ? a4.z : a4.w;
+      w[c] = add2s16(max2s16(c ? w[c - 1] : left, bew), ra);
+      xe = max2s16(xe, w[c]);
+    }
+#pragma unroll
+    for (int o = G / 2; o >= 1; o >>= 1) xe = max2s16(xe, __shfl_xor_sync(gmask, xe, o, G));
+    const int ea = (int)(short)(xe & 0xffffu), eb = (int)xe >> 16;
+    biga |= ea > cap_a;
+    bigb |= eb > cap_b;
+    xja = max(xja + tloop, ea * 2048 + nln2);
+    xjb = max(xjb + tloop, eb * 2048 + nln2);
+    xn += tloop;
+    bew = __byte_perm((unsigned)entry(max(xn, xja) + tmove, tbm_a), (unsigned)entry(max(xn, xjb) + tmove, tbm_b), 0x5410);
+  }
+  return make_int4(xja, xjb, biga, bigb);
+}
+
 // Bound of a profile pair against a slice of targets.  Each profile has its
 // own quantized image (25 rows of int16, the lane-major chunk layout of its
 // f32 MSV image, 4 columns per uint2); the CTA interleaves the two into words
@@ -90,9 +169,9 @@ __global__ void __launch_bounds__(256, 2) msv16_kernel(
   extern __shared__ uint4 sm_img[];
   __shared__ int s_next;
   const PackedTile tile = tiles[blockIdx.x];
-  const DevProfile PA = profs[tile.pa];
+  const DevProfile& PA = profs[tile.pa];
   const bool has_b = tile.pb >= 0;
-  const DevProfile PB = profs[has_b ? tile.pb : tile.pa];
+  const DevProfile& PB = profs[has_b ? tile.pb : tile.pa];
   {
     const uint2* sa = qimg + PA.q_off;
     const uint2* sb = qimg + PB.q_off;
@@ -114,47 +193,78 @@ __global__ void __launch_bounds__(256, 2) msv16_kernel(
   const uint4* my_rows = sm_img + (lane / G % NCOPY) * (COPY4 + G);
   const int gl = lane - j;
   const unsigned gmask = (G == 32) ? kFull : (((1u << G) - 1u) << gl);
-  const float s1a = thr[tile.pa].s1;
-  const float s1b = has_b ? thr[tile.pb].s1 : 0.f;
   const int cap_a = PA.q_cap, cap_b = has_b ? PB.q_cap : 32767;
   const int tbm_a = PA.q_tbm, tbm_b = PB.q_tbm;
   const int nln2 = (int)ceilf(-0.693147182464599609375f * 1048576.0f) + kQ32Rho;
+  const int nln2_25 = 32 * nln2;
+  constexpr int kJStart = -60 * (1 << 25);             // below every J a row can set
+  const int base_idle = 32767 * 65536 + nln2_25;       // a base no E raises
+  const float s1a = thr[tile.pa].s1, s1b = has_b ? thr[tile.pb].s1 : __int_as_float(0x7f800000);
+  // J below N matters where the bound is asked for and where a bound at N's
+  // level, -2.4 to -0.4 bits at any length, might pass
+  const bool track = bound_out != nullptr || !(s1a >= 0.5f) || !(s1b >= 0.5f);
 
-  unsigned prev[C];
+  unsigned w[C];
 #pragma unroll
-  for (int c = 0; c < C; c++) prev[c] = kQ16Neg2;
-  int xn = 0, xja = kQ32Neg, xjb = kQ32Neg, tloop = 0, tmove = 0;
-  unsigned bew = kQ16Neg2;
-  int fina = kQ32Neg, finb = kQ32Neg;
+  for (int c = 0; c < C; c++) w[c] = kQ16Neg2;
+  // of the current target, both halves, in 2^-25 nat: base at the block's start,
+  // the entry constant tmove + tbm + 2047 / 2^20, and J of this lane's columns
+  int base_a = base_idle, base_b = base_idle, ka = 0, kb = 0, ja = kJStart, jb = kJStart;
+  int tloop = 0;
+  unsigned bcur = kQ16Neg2;  // B of the last row computed
   bool biga = false, bigb = false;
-  float nullsc = 0.f;
-  int entry = -1, tgt = 0, L = 0, row = 0, boff = 0;
+  int entry = -1, L = 0, row = 0, boff = 0;
   const uint8_t* seq = res;
   uint4 rcur = make_uint4(0x18181818u, 0x18181818u, 0x18181818u, 0x18181818u), rnext = rcur;
   bool active = false, done = false;
+  auto upper = [](int a, int b) { return __byte_perm((unsigned)a, (unsigned)b, 0x7632); };  // int16 of two states
 
   for (;;) {
     if (!done && row >= L) {  // group-uniform: finish the current target, fetch the next
-      if (active && j == 0) {
-        const float uba = biga ? __int_as_float(0x7f800000) : __fmul_rn(__int2float_ru(fina + tmove), 9.5367431640625e-7f);
-        const float ubb = bigb ? __int_as_float(0x7f800000) : __fmul_rn(__int2float_ru(finb + tmove), 9.5367431640625e-7f);
-        const bool pa_ok = biga || bits_stat(uba, nullsc) >= s1a;
-        const bool pb_ok = has_b && (bigb || bits_stat(ubb, nullsc) >= s1b);
-        if (bound_out) {
-          const int64_t o = slot ? slot[entry] : entry;
-          bound_out[o] = uba;
-          if (has_b) bound_out[bound_stride + o] = ubb;
-        }
-        if (rlist) {
-          if (pa_ok) {
-            const unsigned pos = atomicAdd(&rcount[tile.pa - p0], 1u);
-            if (pos < rcap) rlist[(int64_t)(tile.pa - p0) * rcap + pos] = tgt;
-            else atomicOr(overflow, 1u);
+      if (active) {
+        const int tgt = list[entry];
+        const float4 tp = tpar[tgt];
+        const int tmove = q32_up(tp.y);
+        auto bound = [&](int xj) { return __fmul_rn(__int2float_ru(xj + tmove), 9.5367431640625e-7f); };
+        const int undo = (row - L) * tloop;
+        int xja = (base_a - undo) >> 5, xjb = (base_b - undo) >> 5;  // J where it is above N
+        bool plain = tloop >= 0 || row * tloop + min(ka, kb) < (kQ16BeFloor + 1) * 65536;
+        if (track) {
+#pragma unroll
+          for (int o = G / 2; o >= 1; o >>= 1) {
+            ja = max(ja, __shfl_xor_sync(gmask, ja, o, G));
+            jb = max(jb, __shfl_xor_sync(gmask, jb, o, G));
           }
-          if (pb_ok) {
-            const unsigned pos = atomicAdd(&rcount[tile.pb - p0], 1u);
-            if (pos < rcap) rlist[(int64_t)(tile.pb - p0) * rcap + pos] = tgt;
-            else atomicOr(overflow, 1u);
+          xja = ((ja - undo) >> 5) + nln2;
+          xjb = ((jb - undo) >> 5) + nln2;
+          plain |= ja <= base_a + ka || (has_b && jb <= base_b + kb);
+        }
+        if (plain) {
+          const int4 v = msv16_plain<G, C, ROWP>(my_rows, seq, L, j, gmask, tloop / 32, tmove, tbm_a, tbm_b, cap_a, cap_b, nln2);
+          xja = v.x;
+          xjb = v.y;
+          biga = v.z;
+          bigb = v.w;
+        }
+        if (j == 0) {
+          const float uba = biga ? __int_as_float(0x7f800000) : bound(xja);
+          const float ubb = bigb ? __int_as_float(0x7f800000) : bound(xjb);
+          if (bound_out) {
+            const int64_t o = slot ? slot[entry] : entry;
+            bound_out[o] = uba;
+            if (has_b) bound_out[bound_stride + o] = ubb;
+          }
+          if (rlist) {
+            if (biga || bits_stat(uba, tp.z) >= s1a) {
+              const unsigned pos = atomicAdd(&rcount[tile.pa - p0], 1u);
+              if (pos < rcap) rlist[(int64_t)(tile.pa - p0) * rcap + pos] = tgt;
+              else atomicOr(overflow, 1u);
+            }
+            if (has_b && (bigb || bits_stat(ubb, tp.z) >= s1b)) {
+              const unsigned pos = atomicAdd(&rcount[tile.pb - p0], 1u);
+              if (pos < rcap) rlist[(int64_t)(tile.pb - p0) * rcap + pos] = tgt;
+              else atomicOr(overflow, 1u);
+            }
           }
         }
       }
@@ -163,88 +273,99 @@ __global__ void __launch_bounds__(256, 2) msv16_kernel(
       e = __shfl_sync(gmask, e, gl);
       if (e < tile.end) {
         entry = e;
-        tgt = list[e];
+        const int tgt = list[e];
         L = tlen[tgt];
         seq = res + toff[tgt];
         const float4 tp = tpar[tgt];
-        tloop = q32_up(tp.x);
-        tmove = q32_up(tp.y);
-        nullsc = tp.z;
-        xn = 0;
-        xja = xjb = kQ32Neg;
-        fina = finb = kQ32Neg;
+        tloop = 32 * q32_up(tp.x);
+        const int tmove = q32_up(tp.y);
+        ka = 32 * (tmove + tbm_a + 2047);
+        kb = 32 * (tmove + tbm_b + 2047);
+        base_a = base_b = 0;  // N of row 0
+        ja = jb = kJStart;
         biga = bigb = false;
-        {  // entry score of row 1 from xB = tmove
-          const int bea = max((tmove + tbm_a + 2047) >> (kQ32Shift - kQ16Shift), kQ16BeFloor);
-          const int beb = max((tmove + tbm_b + 2047) >> (kQ32Shift - kQ16Shift), kQ16BeFloor);
-          bew = __byte_perm((unsigned)bea, (unsigned)beb, 0x5410);
-        }
-#pragma unroll
-        for (int c = 0; c < C; c++) prev[c] = kQ16Neg2;
-        row = 0;
-        boff = 0;
-        rcur = __ldg(reinterpret_cast<const uint4*>(seq));
-        rnext = __ldg(reinterpret_cast<const uint4*>(seq + 16));
+        bcur = upper(ka, kb);
         active = L > 0;
       } else {
         active = false;
         done = true;
         L = 0;
+        tloop = 0;
+        base_a = base_b = base_idle;
       }
+#pragma unroll
+      for (int c = 0; c < C; c++) w[c] = bcur;
+      row = 0;
+      boff = 0;
+      rcur = __ldg(reinterpret_cast<const uint4*>(seq));
+      rnext = __ldg(reinterpret_cast<const uint4*>(seq + 16));
     }
     if (__all_sync(kFull, done)) break;
 
     const int q = (row - boff) >> 2;
-    const int rem = L - row;
-    uint32_t w = q == 0 ? rcur.x : q == 1 ? rcur.y : q == 2 ? rcur.z : rcur.w;
-    if (done) w = 0x18181818u;
-    int xjra[4], xjrb[4];
+    uint32_t word = q == 0 ? rcur.x : q == 1 ? rcur.y : q == 2 ? rcur.z : rcur.w;
+    if (done) word = 0x18181818u;
+    // the E (both halves) above which a row of the block can raise base: the
+    // lowest of its rows, floor((base - nln2) / 2^-9 nat)
+    unsigned limit = upper(base_a + 4 * tloop - nln2_25, base_b + 4 * tloop - nln2_25);
+    auto row_of = [&](int r) { return my_rows + (int)((word >> (8 * r)) & 0xff) * ROWP + j; };
+    constexpr int NPF = NC4 < 6 ? NC4 : 6;  // score chunks of a row loaded ahead, the highest columns (used first)
+    uint4 ahead[NPF];
+    const uint4* rowp = row_of(0);
+#pragma unroll
+    for (int u = 0; u < NPF; u++) ahead[u] = rowp[(NC4 - 1 - u) * G];
 #pragma unroll
     for (int r = 0; r < 4; r++) {
-      const int x = (w >> (8 * r)) & 0xff;
-      const uint4* rowp = my_rows + x * ROWP + j;
+      // B of the row unless its E raises base
+      const unsigned bp = upper(base_a + ka + (r + 1) * tloop, base_b + kb + (r + 1) * tloop);
       uint4 rv[NC4];
 #pragma unroll
-      for (int c4 = 0; c4 < NC4; c4++) rv[c4] = rowp[c4 * G];
-      unsigned left = __shfl_up_sync(kFull, prev[C - 1], 1, G);
-      if (j == 0) left = kQ16Neg2;
+      for (int c4 = 0; c4 < NC4; c4++) rv[c4] = c4 >= NC4 - NPF ? ahead[NC4 - 1 - c4] : rowp[c4 * G];
+      unsigned left = __shfl_up_sync(kFull, w[C - 1], 1, G);
+      if (j == 0) left = bcur;
+      unsigned acc[4];
 #pragma unroll
-      for (int c = C - 1; c >= 1; c--) {
+      for (int c = C - 1; c >= 0; c--) {
         const uint4& a4 = rv[c >> 2];
         const unsigned ra = (c & 3) == 0 ? a4.x : (c & 3) == 1 ? a4.y : (c & 3) == 2 ? a4.z : a4.w;
-        prev[c] = add2s16(max2s16(prev[c - 1], bew), ra);
+        w[c] = __viaddmax_s16x2(c ? w[c - 1] : left, ra, bp);
+        if ((c & 1) == 0) {
+          const int p = c / 2, a = p & 3;
+          acc[a] = p + 4 < C / 2 ? __vimax3_s16x2(acc[a], w[c], w[c + 1]) : max2s16(w[c], w[c + 1]);
+        }
       }
-      prev[0] = add2s16(max2s16(left, bew), rv[0].x);
-      // row maximum: a tree of packed maxes, then a butterfly over the group
-      unsigned tv[C];
+      if (r < 3) {
+        rowp = row_of(r + 1);
 #pragma unroll
-      for (int c = 0; c < C; c++) tv[c] = prev[c];
+        for (int u = 0; u < NPF; u++) ahead[u] = rowp[(NC4 - 1 - u) * G];
+      }
+      unsigned xe = __vimax3_s16x2(acc[0], acc[1], acc[2]);
+      if (track) {
+        const unsigned e = max2s16(xe, acc[3]);
+        ja = __viaddmax_s32(ja, tloop, (int)(e << 16));
+        jb = __viaddmax_s32(jb, tloop, (int)(e & 0xffff0000u));
+      }
+      xe = __vimax3_s16x2(xe, acc[3], limit);
+      bcur = bp;
+      if (__any_sync(kFull, xe != limit)) {
+        // a row of some group may raise its base: every group takes its row
+        // maximum (an E at the limit raises nothing), and w the B that follows
 #pragma unroll
-      for (int span = 1; span < C; span <<= 1)
+        for (int o = G / 2; o >= 1; o >>= 1) xe = max2s16(xe, __shfl_xor_sync(kFull, xe, o, G));
+        biga |= (int)(short)(xe & 0xffffu) > cap_a;
+        bigb |= ((int)xe >> 16) > cap_b;
+        const int decay = (r + 1) * tloop;
+        const int na = max(base_a + decay, (int)(xe << 16) + nln2_25), nb = max(base_b + decay, (int)(xe & 0xffff0000u) + nln2_25);
+        base_a = na - decay;
+        base_b = nb - decay;
+        bcur = upper(na + ka, nb + kb);
+        limit = upper(base_a + 4 * tloop - nln2_25, base_b + 4 * tloop - nln2_25);
 #pragma unroll
-        for (int c = 0; c + span < C; c += 2 * span) tv[c] = max2s16(tv[c], tv[c + span]);
-      unsigned xe = tv[0];
-#pragma unroll
-      for (int o = G / 2; o >= 1; o >>= 1) xe = max2s16(xe, __shfl_xor_sync(kFull, xe, o, G));
-      const int ea = (int)(short)(xe & 0xffffu), eb = (int)xe >> 16;
-      biga |= ea > cap_a;
-      bigb |= eb > cap_b;
-      // special states, int32 upper bounds of the reference's f32 N/J/C/B
-      // (J and C follow the same recurrence, as in msv_kernel)
-      xja = max(xja + tloop, ea * 2048 + nln2);
-      xjb = max(xjb + tloop, eb * 2048 + nln2);
-      xn += tloop;
-      const int xba = max(xn, xja) + tmove, xbb = max(xn, xjb) + tmove;
-      const int bea = max((xba + tbm_a + 2047) >> (kQ32Shift - kQ16Shift), kQ16BeFloor);
-      const int beb = max((xbb + tbm_b + 2047) >> (kQ32Shift - kQ16Shift), kQ16BeFloor);
-      bew = __byte_perm((unsigned)bea, (unsigned)beb, 0x5410);
-      xjra[r] = xja;
-      xjrb[r] = xjb;
+        for (int c = 0; c < C; c++) w[c] = max2s16(w[c], bcur);
+      }
     }
-    if (rem >= 1 && rem <= 4) {
-      fina = rem == 1 ? xjra[0] : rem == 2 ? xjra[1] : rem == 3 ? xjra[2] : xjra[3];
-      finb = rem == 1 ? xjrb[0] : rem == 2 ? xjrb[1] : rem == 3 ? xjrb[2] : xjrb[3];
-    }
+    base_a += 4 * tloop;
+    base_b += 4 * tloop;
     row += 4;
     if (row - boff == 16) {
       boff += 16;

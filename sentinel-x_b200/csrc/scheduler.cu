@@ -394,6 +394,10 @@ void launch_msv(sx_engine* E, Slot& S, Streams& X, const sx_profiles* P, const s
 
 // The block's pre-screened profiles: pairs of one MSV shape (similar M
 // adjacent) as tiles over slices of the length-sorted targets, grouped by shape.
+// 40 tiles per resident CTA (two per SM): at 16 the last wave of the Pfam-scale
+// search costs 13 ms more, at 128 the ends of the tiles do (224, 211, 212 ms at
+// 16, 64, 128; a marker-set genome's 26 ms grow by 1 ms from 16 to 64).
+constexpr double kPackedWaves = 40;
 std::vector<std::vector<sxk::PackedTile>> make_packed_tiles(const sx_engine* E, const sx_profiles* P,
                                                             const sx_targets* T, const std::vector<int>& prof) {
   std::vector<std::vector<sxk::PackedTile>> by_shape(kNumMsvShapes);
@@ -406,22 +410,38 @@ std::vector<std::vector<sxk::PackedTile>> make_packed_tiles(const sx_engine* E, 
     std::stable_sort(g.begin(), g.end(), [&](int a, int b) { return P->h[a].m > P->h[b].m; });
     for (size_t q = 0; q < g.size(); q += 2) pairs.emplace_back(g[q], q + 1 < g.size() ? g[q + 1] : -1);
   }
-  const int np = (int)pairs.size();
-  int nslices = (int)std::ceil(16.0 * E->num_sms * 2 / std::max(1, np));
-  nslices = std::max(1, std::min(nslices, std::max(1, nt / 32)));
-  std::vector<int> cut(nslices + 1, nt);
-  cut[0] = 0;
-  {
-    double acc = 0, per = T->residues / nslices;
-    int s = 1;
-    for (int q = 0; q < nt && s < nslices; q++) {
-      acc += T->len[T->order[q]];
-      if (acc >= per * s) cut[s++] = q + 1;
+  // Slices of equal work over all pairs: a pair's share grows with its padded
+  // width, so no tile of a wide pair outlasts the others by several times (with
+  // one slice count for all pairs, the widest tile of the Pfam-scale search ran
+  // 100 ms of its 255)
+  double total = 0;
+  auto width = [&](const std::pair<int, int>& pr) {
+    const MsvShape& v = kMsvShapes[P->msv_shape[pr.first]];
+    return (double)v.g * v.c;
+  };
+  for (const auto& pr : pairs) total += width(pr);
+  const double share = total / (kPackedWaves * 2.0 * E->num_sms);  // width x targets' share of one tile
+  std::unordered_map<int, std::vector<int>> cuts;  // by slice count: boundaries with about equal residues
+  auto cuts_for = [&](int n) -> const std::vector<int>& {
+    std::vector<int>& cut = cuts[n];
+    if (cut.empty()) {
+      cut.assign(n + 1, nt);
+      cut[0] = 0;
+      double acc = 0;
+      int s = 1;
+      for (int q = 0; q < nt && s < n; q++) {
+        acc += T->len[T->order[q]];
+        if (acc >= T->residues / n * s) cut[s++] = q + 1;
+      }
     }
-  }
-  for (const auto& pr : pairs)
-    for (int s = 0; s < nslices; s++)
+    return cut;
+  };
+  for (const auto& pr : pairs) {
+    const int n = std::max(1, std::min((int)std::ceil(width(pr) / share), std::max(1, nt / 32)));
+    const std::vector<int>& cut = cuts_for(n);
+    for (int s = 0; s < n; s++)
       if (cut[s + 1] > cut[s]) by_shape[P->msv_shape[pr.first]].push_back({pr.first, pr.second, cut[s], cut[s + 1]});
+  }
   return by_shape;
 }
 
@@ -463,15 +483,25 @@ void launch_prescreen(sx_engine* E, Slot& S, Streams& X, const sx_profiles* P, c
   join_aux(X);
 }
 
+// Tiles per resident CTA (two per SM), at least two a profile: with two tiles
+// for every profile the widest set the pace (Pfam-scale 19.5 -> 12.5 ms); more
+// than ten stage the images more often than they even out (17 ms at 32).
+constexpr double kRescoreWaves = 5;
 // Exact MSV of the pre-screen's survivors: per profile `nsub` strided
 // sub-tiles over its rescoring list; scores and F1 decisions as in a full
 // MSV pass (survivors appended to the stage-0 lists).
 void launch_rescore(sx_engine* E, Slot& S, Streams& X, const sx_profiles* P, const sx_targets* T,
                     const std::vector<int>& prof, unsigned rcap, int p0) {
   std::vector<std::vector<MsvTile>> tiles(kNumMsvShapes);
-  const int nsub = std::max(2, std::min(32, (int)std::ceil(4.0 * E->num_sms / std::max<size_t>(1, prof.size()))));
-  for (int pi : prof)
+  // sub-tiles of equal expected work: a profile's share grows with its width
+  double total = 0;
+  auto width = [&](int pi) { return (double)kMsvShapes[P->msv_shape[pi]].g * kMsvShapes[P->msv_shape[pi]].c; };
+  for (int pi : prof) total += width(pi);
+  const double share = std::max(1.0, total / (kRescoreWaves * 2.0 * E->num_sms));
+  for (int pi : prof) {
+    const int nsub = std::max(2, std::min(64, (int)std::ceil(width(pi) / share)));
     for (int q = 0; q < nsub; q++) tiles[P->msv_shape[pi]].push_back({pi, q, nsub, 0});
+  }
   launch_msv(E, S, X, P, T, tiles, S.rlist.p, nullptr, nullptr, S.lists[0].p, S.bins[0].p, S.counts.p, S.rcount.p,
              rcap, p0);
 }
@@ -685,8 +715,13 @@ void long_rows(sx_engine* E, const sx_profiles* P, const sx_targets* T, const st
 // definition of a block overlaps the device work of the blocks after it.
 std::vector<std::pair<int, int>> profile_blocks(const sx_engine* E, const sx_profiles* P, const sx_targets* T,
                                                 const std::vector<Thresholds>& th) {
-  constexpr double kCellsPerBlock = 2.5e11;  // ~80 ms of B200 cascade
-  constexpr int kMaxBlocks = 5;  // more blocks cost more than their shorter tail saves
+  // With the envelopes on the device little host work is left to hide behind a
+  // later block, and each block adds its own last waves: Pfam-scale (3e12
+  // cells) 342 ms in one block, 351 in two, 367 in three, 395 in five; 800
+  // viral profiles 80 / 82 / 86 / 93.  Larger searches are split to bound the
+  // survivor lists.
+  constexpr double kCellsPerBlock = 6e12;
+  constexpr int kMaxBlocks = 5;
   const int np = (int)P->h.size();
   std::vector<double> w(np, 0.0);
   double total = 0;
@@ -704,9 +739,7 @@ std::vector<std::pair<int, int>> profile_blocks(const sx_engine* E, const sx_pro
   nb = std::max(1, std::min(nb, nfilt));
   // relative block sizes: the last two blocks of an automatic partition of
   // four or more are smaller (0.7 and 0.4 of the others), so the work left
-  // after the last MSV stage -- that block's later device stages and its
-  // domain definition -- is short (Pfam-scale: 1,1,1,0.7,0.4 449 ms per
-  // search; 0.6,0.3 454; 1,0.5 461; five equal blocks 487)
+  // after the last MSV stage is short
   std::vector<double> rel(nb, 1.0);
   if (E->pipeline_blocks <= 0 && nb >= 4) {
     rel[nb - 2] = 0.7;
