@@ -659,6 +659,7 @@ void pack_profiles(sx_profiles* P);
 void pack_targets(sx_targets* T);
 void append_target(sx_targets* T, const uint8_t* dig, size_t l);
 std::vector<Thresholds> make_thresholds(const std::vector<ProfileHost>& H, const SearchOpts& o);
+void allow_smem(const void* kernel, size_t bytes);
 void fork_aux(Streams& X);
 void join_aux(Streams& X);
 void note_free_memory(sx_engine* E);
@@ -674,7 +675,7 @@ double elapsed_ms(cudaEvent_t a, cudaEvent_t b);
 int long_grid(const sx_engine* E, size_t n);
 int64_t long_stride(const sx_profiles* P, const std::vector<sxk::LongPair>& v, size_t a, size_t b);
 void long_scores(sx_engine* E, const sx_profiles* P, const sx_targets* T, const std::vector<sxk::LongPair>& v,
-                 bool viterbi, std::vector<float>& out);
+                 bool viterbi, std::vector<float>& out);  // v: any profiles of M > kMaxM
 int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx_search_cfg* cfg, sx_hits* out);
 int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T, std::vector<EnvSource>& srcs,
                         int nthr, PhaseLog* plog = nullptr);
@@ -697,9 +698,9 @@ void rows_pass_sync(sx_engine* E, const sx_profiles* P, const sx_targets* T, con
   });
 }
 
-// Raw Forward/Backward special rows of long-profile pairs, in chunks bounded
-// by the scratch budget; consume(first, n, fwd, bwd, off) per chunk, pair
-// first + q having its rows at fwd + off[q] and bwd + off[q].
+// Raw Forward/Backward special rows of pairs of profiles past the exact row
+// shapes, in chunks bounded by the scratch budget; consume(first, n, fwd, bwd,
+// off) per chunk, pair first + q having its rows at fwd + off[q] and bwd + off[q].
 using LongRowsSink = std::function<void(size_t, size_t, const float*, const float*, const std::vector<int64_t>&)>;
 void long_rows(sx_engine* E, const sx_profiles* P, const sx_targets* T, const std::vector<sxk::LongPair>& v,
                const LongRowsSink& consume);

@@ -24,6 +24,7 @@
 // 5.9 -> 1.0; 64 profiles of M 60-700 (61) 10.4 -> 2.4 and 13.0 -> 1.4.
 #pragma once
 #include <climits>
+#include <type_traits>
 
 #include "exact_rows.cuh"
 
@@ -52,8 +53,8 @@ constexpr int kEnvOut = 32;
 
 // Forward (blockIdx.y = 0) and Backward (1) matrices and raw rows of n
 // envelopes; DIAG: the Forward matrices of regions in the diagonal layout.
-template <int C, bool MULTI, bool DIAG>
-__global__ void __launch_bounds__(256) env_rows_kernel(const EnvRec* __restrict__ recs, int n,
+template <int C, bool MULTI, TransIn IN, bool DIAG>
+__global__ void __launch_bounds__(team_threads(IN)) env_rows_kernel(const EnvRec* __restrict__ recs, int n,
                                                        const DevProfile* __restrict__ profs,
                                                        const float* __restrict__ ximg,
                                                        const uint8_t* __restrict__ res,
@@ -71,11 +72,11 @@ __global__ void __launch_bounds__(256) env_rows_kernel(const EnvRec* __restrict_
   float* pl = planes + r.plane_off;
   float* orow = rows + r.row_off;
   if constexpr (DIAG) {
-    exact_forward<C, MULTI, kKeepDiag>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move, orow, pl, T, sh);
+    exact_forward<C, MULTI, IN, kKeepDiag>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move, orow, pl, T, sh);
   } else if (blockIdx.y == 0) {
-    exact_forward<C, MULTI, kKeepMI>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move, orow, pl, T, sh);
+    exact_forward<C, MULTI, IN, kKeepMI>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move, orow, pl, T, sh);
   } else {
-    exact_backward<C, MULTI, kKeepMI>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move,
+    exact_backward<C, MULTI, IN, kKeepMI>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move,
                                       orow + 6 * (int64_t)(r.lr + 1), pl + 2 * (int64_t)(r.lr + 1) * r.width, T, sh);
   }
 }
@@ -113,8 +114,8 @@ struct OaShared {  // exchange between the warps of a team
 // go through shared memory.  With the decisions noted while the row is in
 // registers the traceback loads half a byte a step, 32 steps of a run of
 // matches at a time, instead of following four chains of floats.
-template <int C, bool MULTI>
-__global__ void __launch_bounds__(256) env_oa_kernel(const EnvRec* __restrict__ recs, int n,
+template <int C, bool MULTI, TransIn IN>
+__global__ void __launch_bounds__(team_threads(IN)) env_oa_kernel(const EnvRec* __restrict__ recs, int n,
                                                      const DevProfile* __restrict__ profs,
                                                      const float* __restrict__ ximg, float* planes, float* aux,
                                                      const double* __restrict__ facs, float* __restrict__ outs) {
@@ -150,11 +151,8 @@ __global__ void __launch_bounds__(256) env_oa_kernel(const EnvRec* __restrict__ 
   float* out = outs + r.out_off;
   const bool ploop0 = r.ploop == 0.0f, pe_loop0 = r.pe_loop == 0.0f, pe_move0 = r.pe_move == 0.0f,
              pmove0 = r.pmove == 0.0f;
-  float tr[6][C], md[C], dd[C];  // bm, mm im dm into the column, mi ii; md dd out of it
-#pragma unroll
-  for (int q = 0; q < 6; q++) load_cols<C>(img + (kXFwd + q) * width + k0, tr[q]);
-  load_cols<C>(img + (kXBwd + 2) * width + k0, md);
-  load_cols<C>(img + (kXBwd + 6) * width + k0, dd);
+  TeamTrans<C, IN, false> tr;
+  tr.init(img, width, k0, T + width);
   float sm[C], omp[C], oip[C], odp[C], fm[C], fi[C], bm[C], bi[C];
 #pragma unroll
   for (int c = 0; c < C; c++) {
@@ -202,8 +200,9 @@ __global__ void __launch_bounds__(256) env_oa_kernel(const EnvRec* __restrict__ 
       oil = li;
       odl = ld;
     }
-    unsigned bits = 0;
+    std::conditional_t<(C > 8), uint64_t, unsigned> bits = 0;  // four a column
     float emax = SX_NEG_INF;
+    const auto tbm = tr.row(0), tmm = tr.row(1), tim = tr.row(2), tdm = tr.row(3), tmi = tr.row(4), tii = tr.row(5);
 #pragma unroll
     for (int c = 0; c < C; c++) {
       const int k = k0 + c + 1;
@@ -213,37 +212,38 @@ __global__ void __launch_bounds__(256) env_oa_kernel(const EnvRec* __restrict__ 
       om[c] = oi[c] = SX_NEG_INF;
       if (k <= M) {
         const float omv = c ? omp[c - 1] : oml, oiv = c ? oip[c - 1] : oil, odv = c ? odp[c - 1] : odl;
-        float sv = oa_gate(tr[0][c], xb);
+        float sv = oa_gate(tbm[c], xb);
         unsigned best = kOaB;
         if (k >= 2) {
-          sv = fmaxf(sv, oa_gate(tr[1][c], omv));
-          sv = fmaxf(sv, oa_gate(tr[2][c], oiv));
-          sv = fmaxf(sv, oa_gate(tr[3][c], odv));
+          sv = fmaxf(sv, oa_gate(tmm[c], omv));
+          sv = fmaxf(sv, oa_gate(tim[c], oiv));
+          sv = fmaxf(sv, oa_gate(tdm[c], odv));
           // the first of M, I, D, B with the largest value
-          float top = oa_dis(tr[1][c], omv);
+          float top = oa_dis(tmm[c], omv);
           best = kOaM;
-          float v = oa_dis(tr[2][c], oiv);
+          float v = oa_dis(tim[c], oiv);
           if (v > top) { top = v; best = kOaI; }
-          v = oa_dis(tr[3][c], odv);
+          v = oa_dis(tdm[c], odv);
           if (v > top) { top = v; best = kOaD; }
-          v = oa_dis(tr[0][c], xb);
+          v = oa_dis(tbm[c], xb);
           if (v > top) best = kOaB;
         } else {
           sv = fmaxf(sv, 0.0f);
           // M, I and D have no cell to the left: the first of (-inf, -inf, -inf, B)
-          best = oa_dis(tr[0][c], xb) > SX_NEG_INF ? kOaB : kOaM;
+          best = oa_dis(tbm[c], xb) > SX_NEG_INF ? kOaB : kOaM;
         }
         om[c] = fadd(sv, pm);
         emax = fmaxf(emax, om[c]);
-        oi[c] = fadd(fmaxf(oa_gate(tr[4][c], omp[c]), oa_gate(tr[5][c], oip[c])), pi);
-        const bool from_i = !(oa_dis(tr[4][c], omp[c]) >= oa_dis(tr[5][c], oip[c]));
-        bits |= (best | (from_i ? kOaIfromI : 0u)) << (4 * c);
+        oi[c] = fadd(fmaxf(oa_gate(tmi[c], omp[c]), oa_gate(tii[c], oip[c])), pi);
+        const bool from_i = !(oa_dis(tmi[c], omp[c]) >= oa_dis(tii[c], oip[c]));
+        bits |= (decltype(bits))(best | (from_i ? kOaIfromI : 0u)) << (4 * c);
       }
     }
     if (i < L) load_row(i + 1);
     // the lane's composite map of its columns' D steps
     bool lc = false;
     float lv = SX_NEG_INF, a[C];
+    const auto md = tr.row(6), dd = tr.row(7);
 #pragma unroll
     for (int c = 0; c < C; c++) {
       a[c] = oa_gate(md[c], om[c]);
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(256) env_oa_kernel(const EnvRec* __restrict__ 
       const int k = k0 + c + 1;
       od[c] = k <= M ? v : SX_NEG_INF;
       if (k <= M) emax = fmaxf(emax, v);
-      if (!(oa_dis(md[c], om[c]) >= oa_dis(dd[c], od[c]))) bits |= kOaDfromD << (4 * c);
+      if (!(oa_dis(md[c], om[c]) >= oa_dis(dd[c], od[c]))) bits |= (decltype(bits))kOaDfromD << (4 * c);
       v = dd[c] > 0.0f ? fmaxf(a[c], v) : fmaxf(a[c], 0.0f);
     }
     emax = warp_max_f32(emax);
@@ -313,7 +313,8 @@ __global__ void __launch_bounds__(256) env_oa_kernel(const EnvRec* __restrict__ 
     store_cols<C>(OM + at, om);
     store_cols<C>(OD + at, od);
     uint8_t* db = dec + (int64_t)i * dec_row + k0 / 2;
-    if constexpr (C == 8) *reinterpret_cast<uint32_t*>(db) = bits;
+    if constexpr (C == 16) *reinterpret_cast<uint64_t*>(db) = bits;
+    else if constexpr (C == 8) *reinterpret_cast<uint32_t*>(db) = (uint32_t)bits;
     else *reinterpret_cast<uint16_t*>(db) = (uint16_t)bits;
     if (lead) {
       sxe[i] = emax;
@@ -440,18 +441,18 @@ __global__ void __launch_bounds__(256) env_oa_kernel(const EnvRec* __restrict__ 
 // si: every insert posterior of the envelope added in row-major order (the
 // null2 length correction, dp.rs:1310-1350).  The sum is one chain of L * M
 // adds, but a term below half an ulp of the running sum leaves it unchanged,
-// and the sum never falls: kInsertRows warps compute one row each against the
+// and the sum never falls: up to kInsertRows warps compute one row each against the
 // sum as it stood a batch earlier and keep, in order, the groups of four
 // columns with a term that can still count; one warp adds those while the
 // others prepare the next rows.
-constexpr int kInsertRows = 8;
+constexpr int kInsertRows = 8;  // at most: blockDim.x / 32 - 1 rows a batch
 static __global__ void __launch_bounds__(32 * (kInsertRows + 1)) env_insert_kernel(
     const EnvRec* __restrict__ recs, int n, const DevProfile* __restrict__ profs, const float* __restrict__ planes,
     const double* __restrict__ facs, float* __restrict__ outs, int max_width) {
-  extern __shared__ float4 sm_row[];  // 2 batches x kInsertRows lists of max_width / 4 groups
+  extern __shared__ float4 sm_row[];  // 2 batches x `rows` lists of max_width / 4 groups
   __shared__ int s_n[2][kInsertRows];
   __shared__ float s_si;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rows = (blockDim.x >> 5) - 1;
   const EnvRec r = recs[blockIdx.x];
   const int M = profs[r.p].m, L = r.lr, width = r.width;
   const int64_t PL = (int64_t)(L + 1) * width;
@@ -461,13 +462,13 @@ static __global__ void __launch_bounds__(32 * (kInsertRows + 1)) env_insert_kern
   const int cap = max_width / 4;
   if (threadIdx.x == 0) s_si = 0.f;
   __syncthreads();
-  const int batches = (L + kInsertRows - 1) / kInsertRows;
+  const int batches = (L + rows - 1) / rows;
   float si = 0.f;
   for (int b = 0; b <= batches; b++) {  // batch b is prepared while batch b - 1 is added
     if (warp == 0) {
       if (b) {
-        for (int q = 0; q < kInsertRows; q++) {
-          const float4* t = sm_row + (((b - 1) & 1) * kInsertRows + q) * cap;
+        for (int q = 0; q < rows; q++) {
+          const float4* t = sm_row + (((b - 1) & 1) * rows + q) * cap;
           const int m = s_n[(b - 1) & 1][q];
           float4 x = m ? t[0] : make_float4(0.f, 0.f, 0.f, 0.f);
           for (int e = 0; e < m; e++) {
@@ -478,14 +479,14 @@ static __global__ void __launch_bounds__(32 * (kInsertRows + 1)) env_insert_kern
         }
       }
     } else {
-      const int q = warp - 1, i = b * kInsertRows + q + 1;
+      const int q = warp - 1, i = b * rows + q + 1;
       int m = 0;
       if (i <= L) {
         // half an ulp of the sum: 2^(exponent - 24), 0 for a sum below 2^-102
         const int e = (__float_as_int(s_si) >> 23) - 24;
         const float half = e > 0 ? __int_as_float(e << 23) : 0.f;
         const double f = fac[i];
-        float4* list = sm_row + ((b & 1) * kInsertRows + q) * cap;
+        float4* list = sm_row + ((b & 1) * rows + q) * cap;
         const float4* fi = reinterpret_cast<const float4*>(FI + (int64_t)i * width) + lane;
         const float4* bi = reinterpret_cast<const float4*>(BI + (int64_t)i * width) + lane;
         for (int base = 0; base < M; base += 512) {  // four loads of each plane in flight
@@ -527,7 +528,7 @@ static __global__ void __launch_bounds__(32 * (kInsertRows + 1)) env_insert_kern
 // ---- stochastic traceback ensembles of multi-domain regions ------------------
 // region_trace_ensemble (src/hmmer/pipeline.rs:360-477) up to the clustering:
 // kTraceSamples sampled traces (stochastic_trace, src/hmmer/dp.rs:1075-1258)
-// through the region's multihit Forward matrix (env_rows_kernel<C, MULTI, true>,
+// through the region's multihit Forward matrix (env_rows_kernel<..., DIAG>,
 // diagonal layout), one Easel LCG stream per region, the per-trace null2 of
 // every sampled domain and its per-position sums.  The host clusters the
 // samples and takes the logs.
@@ -546,7 +547,7 @@ struct TraceRec {
   int32_t i0, lr;      // region residues i0 .. i0+lr-1 (0-based)
   float ploop, pmove;  // multihit special transitions of the target's length
   float pe_loop, pe_move;
-  int64_t plane_off;   // diagonal M I D planes of env_rows_kernel<C, MULTI, true>
+  int64_t plane_off;   // diagonal M I D planes of env_rows_kernel<..., DIAG>
   int64_t row_off;     // its raw special rows, 6 (lr+1)
   int64_t n2_off;      // per-position null2 sums, lr+1 floats (slot 0 unused)
   int64_t col_off;     // the profile's column table (kTraceCol floats per column)

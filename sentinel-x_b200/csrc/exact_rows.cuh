@@ -91,6 +91,57 @@ __device__ __forceinline__ void store_cols(float* p, const float (&v)[C]) {
     reinterpret_cast<float4*>(p)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
 }
 
+// Where a thread keeps its columns of the eight transition rows: registers, or
+// (teams of more than eight warps have 128 registers a thread) shared memory,
+// or the image itself when 8 rows of the team's width do not fit there.
+enum TransIn { kTrReg, kTrShared, kTrGlobal };
+template <int C>
+struct ColVec {
+  float v[C];
+  __device__ __forceinline__ float operator[](int c) const { return v[c]; }
+};
+template <int C, TransIn IN, bool BWD>
+struct TeamTrans {
+  float r[IN == kTrReg ? 8 : 1][C];
+  const float* p;
+  int width;
+  // Forward and optimal accuracy: bm, mm im dm into the column, mi ii, then md
+  // dd out of it; Backward: mm mi md im ii dm dd bm
+  static __device__ __forceinline__ int image_row(int q) { return BWD ? kXBwd + q : q < 6 ? kXFwd + q : q == 6 ? kXBwd + 2 : kXBwd + 6; }
+  __device__ __forceinline__ void init(const float* __restrict__ img, int w, int k0, float* shared) {
+    width = w;
+    p = IN == kTrShared ? shared + k0 : img + k0;
+    if constexpr (IN != kTrGlobal) {
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        if constexpr (IN == kTrReg) {
+          load_cols<C>(img + image_row(q) * w + k0, r[q]);
+        } else {  // every thread reads back its own columns only
+          float v[C];
+          load_cols<C>(img + image_row(q) * w + k0, v);
+          store_cols<C>(shared + q * w + k0, v);
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ ColVec<C> row(int q) const {
+    ColVec<C> o;
+    if constexpr (IN == kTrReg) {
+#pragma unroll
+      for (int c = 0; c < C; c++) o.v[c] = r[q][c];
+    } else if constexpr (IN == kTrShared) {
+#pragma unroll
+      for (int u = 0; u < C / 4; u++) {
+        const float4 x = reinterpret_cast<const float4*>(p + q * width)[u];
+        o.v[4 * u] = x.x; o.v[4 * u + 1] = x.y; o.v[4 * u + 2] = x.z; o.v[4 * u + 3] = x.w;
+      }
+    } else {
+      load_cols<C>(p + image_row(q) * width, o.v);
+    }
+    return o;
+  }
+};
+
 __device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_int(a) == __float_as_int(b); }
 
 // t[0] + t[1] + ... + t[n-1] in that order from 0 (n a positive multiple of
@@ -167,7 +218,7 @@ __device__ __forceinline__ float scan_guess(float a, int lane, const float (&bs)
 // guessed carries `cin` until no carry changes.  a and p are the terms and
 // factors out of each column; returns the D right of the lane's last column.
 template <int C>
-__device__ __forceinline__ float settle_up(float (&d)[C], const float (&a)[C], const float (&p)[C], float cin, float in,
+__device__ __forceinline__ float settle_up(float (&d)[C], const float (&a)[C], const ColVec<C>& p, float cin, float in,
                                            int lane) {
   float v = 0.f;
   for (int it = 0; it < 32; it++) {
@@ -186,7 +237,7 @@ __device__ __forceinline__ float settle_up(float (&d)[C], const float (&a)[C], c
 }
 // Descending: d[k] = ((a_k + p_k d[k+1]) + e) from `in` past its last column.
 template <int C>
-__device__ __forceinline__ void settle_down(float (&d)[C], const float (&a)[C], const float (&p)[C], float e, float cin,
+__device__ __forceinline__ void settle_down(float (&d)[C], const float (&a)[C], const ColVec<C>& p, float e, float cin,
                                             float in, int lane) {
   for (int it = 0; it < 32; it++) {
     float v = cin;
@@ -213,7 +264,7 @@ __host__ __device__ __forceinline__ int64_t diag_at(int64_t i, int k, int M) {
 __host__ __device__ __forceinline__ int64_t diag_plane(int64_t lr, int M) { return (lr + M - 1) * (int64_t)M; }
 
 // Forward (dp.rs:229-298, 442-513).
-template <int C, bool MULTI, Keep KEEP>
+template <int C, bool MULTI, TransIn IN, Keep KEEP>
 __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int M, const uint8_t* __restrict__ s, int L,
                                               float ploop, float pmove, float pe_loop, float pe_move, float* orow,
                                               float* planes, float* T, XShared& sh) {
@@ -224,17 +275,17 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
   const bool lead = MULTI ? threadIdx.x == 0 : lane == 0;
   const int nsum = max(16, (M + 15) & ~15);
   const float* im = img + k0;
-  float tr[8][C];  // bm, mm im dm into the column, mi ii, then md dd out of it
-#pragma unroll
-  for (int q = 0; q < 6; q++) load_cols<C>(im + (kXFwd + q) * width, tr[q]);
-  load_cols<C>(im + (kXBwd + 2) * width, tr[6]);
-  load_cols<C>(im + (kXBwd + 6) * width, tr[7]);
+  TeamTrans<C, IN, false> tr;
+  tr.init(img, width, k0, T + width);
   float* FM = planes;
   float* FI = KEEP == kKeepDiag ? FM + diag_plane(L, M) : FM + (int64_t)(L + 1) * width;
   float* FD = FI + diag_plane(L, M);
   float bs[5], ball, b = 1.f;
+  {
+    const auto dd = tr.row(7);
 #pragma unroll
-  for (int c = 0; c < C; c++) b = b * tr[7][c];
+    for (int c = 0; c < C; c++) b = b * dd[c];
+  }
   const int steps = scan_factors<true>(b, lane, bs, ball);
   float bpre = __shfl_up_sync(kFull, ball, 1);
   if (lane == 0) bpre = 1.f;
@@ -266,24 +317,28 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
       dpl = ld;
     }
     float mv[C], iv[C], a[C], dv[C];
+    {
+      const auto bm = tr.row(0), mm = tr.row(1), im = tr.row(2), dm = tr.row(3), mi = tr.row(4), ii = tr.row(5);
 #pragma unroll
-    for (int c = 0; c < C; c++) {
-      float t = fmul(xb, tr[0][c]);
-      t = fadd(t, fmul(c ? mp[c - 1] : mpl, tr[1][c]));
-      t = fadd(t, fmul(c ? ip[c - 1] : ipl, tr[2][c]));
-      t = fadd(t, fmul(c ? dp[c - 1] : dpl, tr[3][c]));
-      mv[c] = fmul(t, eo[c]);
-      iv[c] = fmul(fadd(fmul(mp[c], tr[4][c]), fmul(ip[c], tr[5][c])), ins);
+      for (int c = 0; c < C; c++) {
+        float t = fmul(xb, bm[c]);
+        t = fadd(t, fmul(c ? mp[c - 1] : mpl, mm[c]));
+        t = fadd(t, fmul(c ? ip[c - 1] : ipl, im[c]));
+        t = fadd(t, fmul(c ? dp[c - 1] : dpl, dm[c]));
+        mv[c] = fmul(t, eo[c]);
+        iv[c] = fmul(fadd(fmul(mp[c], mi[c]), fmul(ip[c], ii[c])), ins);
+      }
     }
     float end = 0.f;
+    const auto md = tr.row(6), dd = tr.row(7);
 #pragma unroll
     for (int c = 0; c < C; c++) {
-      a[c] = fmul(mv[c], tr[6][c]);
-      end = fadd(a[c], fmul(end, tr[7][c]));
+      a[c] = fmul(mv[c], md[c]);
+      end = fadd(a[c], fmul(end, dd[c]));
     }
     float g = scan_guess<true>(end, lane, bs, steps);
     if (lane == 0) g = 0.f;
-    end = settle_up<C>(dv, a, tr[7], g, 0.f, lane);
+    end = settle_up<C>(dv, a, dd, g, 0.f, lane);
     if constexpr (MULTI) {
       if (lane == 31) sh.end[warp] = end;
       __syncthreads();
@@ -291,7 +346,7 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
         const float in = sh.end[warp - 1], own = end;
         float c0 = __shfl_up_sync(kFull, own, 1);
         c0 = lane ? fadd(c0, fmul(bpre, in)) : in;
-        end = settle_up<C>(dv, a, tr[7], c0, in, lane);
+        end = settle_up<C>(dv, a, dd, c0, in, lane);
         if (lane == 31 && !same_bits(end, own)) sh.flag = 1;
       }
     }
@@ -316,7 +371,7 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
           __syncthreads();
           const float in = warp ? sh.end[warp - 1] : 0.f;
           const float up = __shfl_up_sync(kFull, own, 1);
-          end = settle_up<C>(dv, a, tr[7], lane ? up : in, in, lane);
+          end = settle_up<C>(dv, a, dd, lane ? up : in, in, lane);
           if (!__syncthreads_or(lane == 31 && !same_bits(end, own))) break;
         }
         publish();
@@ -385,7 +440,7 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
 
 // Backward (dp.rs:301-392, 516-601): row L (E, C), rows L-1..1 (N B E J C,
 // rescale factor) and the row-0 B sum in slot 1 of row 0.
-template <int C, bool MULTI, Keep KEEP>
+template <int C, bool MULTI, TransIn IN, Keep KEEP>
 __device__ __forceinline__ void exact_backward(const float* __restrict__ img, int M, const uint8_t* __restrict__ s,
                                                int L, float ploop, float pmove, float pe_loop, float pe_move,
                                                float* orow, float* planes, float* T, XShared& sh) {
@@ -398,12 +453,14 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
   const bool lead = MULTI ? threadIdx.x == 0 : lane == 0;
   const int nsum = max(16, (M + 15) & ~15);
   const float* im = img + k0;
-  float tr[8][C];  // mm mi md im ii dm dd bm
-#pragma unroll
-  for (int q = 0; q < 8; q++) load_cols<C>(im + (kXBwd + q) * width, tr[q]);
+  TeamTrans<C, IN, true> tr;
+  tr.init(img, width, k0, T + width);
   float bs[5], ball, b = 1.f;
+  {
+    const auto dd = tr.row(6);
 #pragma unroll
-  for (int c = 0; c < C; c++) b = b * tr[6][c];
+    for (int c = 0; c < C; c++) b = b * dd[c];
+  }
   const int steps = scan_factors<false>(b, lane, bs, ball);
   float bpre = __shfl_down_sync(kFull, ball, 1);  // product over the lanes right of this one
   if (lane == 31) bpre = 1.f;
@@ -421,11 +478,12 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
   // the D right of its last column; true if the ends must be exchanged again
   auto d_chain = [&](float e) -> float {
     float end = 0.f;
+    const auto dd = tr.row(6);
 #pragma unroll
-    for (int c = C - 1; c >= 0; c--) end = fadd(fadd(al[c], fmul(end, tr[6][c])), e);
+    for (int c = C - 1; c >= 0; c--) end = fadd(fadd(al[c], fmul(end, dd[c])), e);
     float g = scan_guess<false>(end, lane, bs, steps);
     if (lane == 31) g = 0.f;
-    settle_down<C>(dc, al, tr[6], e, g, 0.f, lane);
+    settle_down<C>(dc, al, dd, e, g, 0.f, lane);
     float in = 0.f;
     if constexpr (MULTI) {
       if (lane == 0) sh.end[warp] = dc[0];
@@ -435,7 +493,7 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
         const float own = dc[0];
         float c0 = __shfl_down_sync(kFull, own, 1);
         c0 = lane < 31 ? fadd(c0, fmul(bpre, in)) : in;
-        settle_down<C>(dc, al, tr[6], e, c0, in, lane);
+        settle_down<C>(dc, al, dd, e, c0, in, lane);
         if (lane == 0 && !same_bits(dc[0], own)) sh.flag = 1;
       }
     }
@@ -444,13 +502,14 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
   };
   auto d_again = [&](float e) -> float {  // a warp's end changed
     float in = 0.f;
+    const auto dd = tr.row(6);
     for (int it = 0; it <= kXMaxWarps; it++) {
       const float own = dc[0];
       if (lane == 0) sh.end[warp] = own;
       __syncthreads();
       in = warp + 1 < nw ? sh.end[warp + 1] : 0.f;
       const float dn = __shfl_down_sync(kFull, own, 1);
-      settle_down<C>(dc, al, tr[6], e, lane < 31 ? dn : in, in, lane);
+      settle_down<C>(dc, al, dd, e, lane < 31 ? dn : in, in, lane);
       if (!__syncthreads_or(lane == 0 && !same_bits(dc[0], own))) break;
     }
     const float dn = __shfl_down_sync(kFull, dc[0], 1);
@@ -469,8 +528,11 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
     __syncthreads();
     if (lead) sh.flag = 0;
   }
+  {
+    const auto md = tr.row(2);
 #pragma unroll
-  for (int c = 0; c < C; c++) mn[c] = fadd(xe, fmul(c < C - 1 ? dc[c + 1] : dnr, tr[2][c]));
+    for (int c = 0; c < C; c++) mn[c] = fadd(xe, fmul(c < C - 1 ? dc[c + 1] : dnr, md[c]));
+  }
   float* BM = planes;
   float* BI = BM + (int64_t)(L + 1) * width;
   if constexpr (KEEP == kKeepMI) {
@@ -485,10 +547,11 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
   float me[C];
   auto b_terms = [&](const float (&eo)[C]) {
     float bt[C];
+    const auto bm = tr.row(7);
 #pragma unroll
     for (int c = 0; c < C; c++) {
       me[c] = fmul(mn[c], eo[c]);
-      bt[c] = fmul(fmul(mn[c], tr[7][c]), eo[c]);
+      bt[c] = fmul(fmul(mn[c], bm[c]), eo[c]);
     }
     store_cols<C>(T + k0, bt);
     if (MULTI && lane == 0) sh.mv[warp] = me[0];
@@ -511,20 +574,24 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
     xe = fadd(fmul(xj, pe_loop), fmul(xc, pe_move));
     xn = fadd(fmul(xn, ploop), fmul(xb, pmove));
     float iv[C];
+    {
+      const auto dm = tr.row(5);
 #pragma unroll
-    for (int c = 0; c < C; c++) {
-      iv[c] = fmul(in_[c], ins);
-      al[c] = fmul(c < C - 1 ? me[c + 1] : me_up, tr[5][c]);
+      for (int c = 0; c < C; c++) {
+        iv[c] = fmul(in_[c], ins);
+        al[c] = fmul(c < C - 1 ? me[c + 1] : me_up, dm[c]);
+      }
     }
     dnr = d_chain(xe);
     float rowmax = 0.f;
     auto cells = [&]() {
       rowmax = fmaxf(fmaxf(fmaxf(fmaxf(xb, xe), xn), xj), xc);
+      const auto mm = tr.row(0), mi = tr.row(1), md = tr.row(2), im = tr.row(3), ii = tr.row(4);
 #pragma unroll
       for (int c = 0; c < C; c++) {
         const float mnext = c < C - 1 ? me[c + 1] : me_up, dnext = c < C - 1 ? dc[c + 1] : dnr;
-        mn[c] = fadd(fadd(fadd(fmul(mnext, tr[0][c]), fmul(iv[c], tr[1][c])), xe), fmul(dnext, tr[2][c]));
-        in_[c] = fadd(fmul(mnext, tr[3][c]), fmul(iv[c], tr[4][c]));
+        mn[c] = fadd(fadd(fadd(fmul(mnext, mm[c]), fmul(iv[c], mi[c])), xe), fmul(dnext, md[c]));
+        in_[c] = fadd(fmul(mnext, im[c]), fmul(iv[c], ii[c]));
         rowmax = fmaxf(rowmax, mn[c]);
       }
       // values are never negative, so their bit patterns order as integers
@@ -579,10 +646,14 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
   if (lead) orow[1] = b0;
 }
 
+// Threads of the largest CTA of a kernel variant.
+constexpr int team_threads(TransIn in) { return in == kTrReg ? 256 : 32 * kXMaxWarps; }
+
 // Forward (blockIdx.y = 0) and Backward (1) rows of n pairs.  MULTI: a CTA per
-// pair; otherwise a warp per pair.  Dynamic shared memory: one row per team.
-template <int C, bool MULTI>
-__global__ void __launch_bounds__(256) exact_rows_kernel(const RowRec* __restrict__ recs, int n,
+// pair; otherwise a warp per pair.  Dynamic shared memory: one row per team,
+// and the transition rows where they are kept there.
+template <int C, bool MULTI, TransIn IN>
+__global__ void __launch_bounds__(team_threads(IN)) exact_rows_kernel(const RowRec* __restrict__ recs, int n,
                                                          const DevProfile* __restrict__ profs,
                                                          const float* __restrict__ ximg,
                                                          const uint8_t* __restrict__ res,
@@ -601,9 +672,9 @@ __global__ void __launch_bounds__(256) exact_rows_kernel(const RowRec* __restric
   const uint8_t* s = res + toff[r.t];
   const float4 xs = xsc[r.t];
   if (blockIdx.y == 0)
-    exact_forward<C, MULTI, kKeepNone>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off, nullptr, T, sh);
+    exact_forward<C, MULTI, IN, kKeepNone>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off, nullptr, T, sh);
   else
-    exact_backward<C, MULTI, kKeepNone>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off + 6 * (int64_t)(L + 1),
+    exact_backward<C, MULTI, IN, kKeepNone>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off + 6 * (int64_t)(L + 1),
                                         nullptr, T, sh);
 }
 

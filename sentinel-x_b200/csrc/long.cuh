@@ -1,17 +1,18 @@
-// Profiles longer than the warp-chunked kernels' 32 x 64 = 2048 columns
-// (marker models of long proteins).  One CTA of kPlainThreads threads per
-// (profile, target) pair; thread t owns columns k = t+1, t+1+kPlainThreads, ...;
-// the rows live in a per-CTA slice of global scratch (L1/L2 resident), and the
-// sequential parts of a row (the Viterbi and Forward/Backward D chains, the
-// Forward row sum and the Backward B sum) are run in order by thread 0.  The
-// arithmetic is the reference's, operation for operation, as in the
-// warp-chunked kernels, so the scores and raw rows are identical.
+// Profiles longer than the exact row shapes take (M > 8192; between 2048 and
+// that, wide.cuh).  One CTA of kPlainThreads threads per (profile, target)
+// pair; thread t owns columns k = t+1, t+1+kPlainThreads, ...; the rows live in
+// a per-CTA slice of global scratch (L1/L2 resident), and the sequential parts
+// of a row (the Viterbi and Forward/Backward D chains, the Forward row sum and
+// the Backward B sum) are run in order by thread 0.  The arithmetic is the
+// reference's, operation for operation, so the scores and raw rows are
+// identical.
 //
 // Profile image (the plain layout extended): rows of M+1 floats indexed by k,
 //   0..24  msc[x][k]       25..32 log transitions  mm mi md im ii dm dd bm
 //   33..57 mo[x][k]        58..65 probabilities    mm mi md im ii dm dd bm
 #pragma once
 #include "plain.cuh"
+#include "wide.cuh"
 
 namespace sxk {
 
@@ -19,10 +20,6 @@ constexpr int kLongRows = 66;
 enum { kLT = 25, kLMo = 33, kLP = 58 };  // first rows of log transitions, odds, probabilities
 enum { kQMM = 0, kQMI, kQMD, kQIM, kQII, kQDM, kQDD, kQBM };
 constexpr int kLongArrays = 6;  // scratch rows of M+1 floats per CTA
-
-struct LongPair {
-  int32_t p, t;
-};
 
 // MSV (src/hmmer/dp.rs:92-145): score of every pair.
 static __global__ void __launch_bounds__(kPlainThreads) long_msv_kernel(

@@ -206,14 +206,16 @@ void pack_images(const ProfileHost& h, const DevProfile& d, float4* msv, float4*
 
 // Row image of the exact row passes (exact_rows.cuh): kXRows rows of the
 // shape's width, column k at k - 1, zero past column M and for the transitions
-// node M does not have.
+// node M does not have.  Wide profiles (M > kMaxM) add the log-space rows of
+// wide.cuh, -inf there.
+int ximage_rows(int m) { return is_long(m) ? (int)sxk::kXWideRows : (int)sxk::kXRows; }
 void pack_ximage(const ProfileHost& h, const DevProfile& d, float* out) {
   const int m = h.m, w = xwidth(d.xshape);
   float* base = out + d.x_off;
-  auto put = [&](int r, const float* src, int n) {  // columns 1..n from src[0..n)
+  auto put = [&](int r, const float* src, int n, float pad = 0.0f) {  // columns 1..n from src[0..n)
     float* o = base + (size_t)r * w;
     std::copy(src, src + n, o);
-    std::fill(o + n, o + w, 0.0f);
+    std::fill(o + n, o + w, pad);
   };
   for (int x = 0; x < 25; x++) put(sxk::kXMo + x, h.mo_row(x) + 1, m);
   const auto& p = h.p;
@@ -223,6 +225,11 @@ void pack_ximage(const ProfileHost& h, const DevProfile& d, float* out) {
     put(sxk::kXFwd + q, p[fwd[q]].data() + (at_k[q] ? 1 : 0), q == 4 || q == 5 ? std::max(m - 1, 0) : m);
   const int bwd[8] = {TMM, TMI, TMD, TIM, TII, TDM, TDD, TBM};
   for (int q = 0; q < 8; q++) put(sxk::kXBwd + q, p[bwd[q]].data() + 1, q < 7 ? std::max(m - 1, 0) : m);
+  if (!is_long(m)) return;
+  for (int x = 0; x < 25; x++) put(sxk::kXMsc + x, h.msc_row(x) + 1, m, kNegInf);
+  const bool into[8] = {false, true, true, true, false, false, false, false};  // transitions out of k - 1
+  for (int q = 0; q < 8; q++)
+    put(sxk::kXVit + q, h.t[fwd[q]].data() + (into[q] ? 0 : 1), q >= 4 ? m - 1 : m, kNegInf);
 }
 
 // Quantized MSV image of the packed pre-screen (prescreen.cuh): the match
@@ -357,10 +364,12 @@ void pack_profiles(sx_profiles* P) {
     memset(&d, 0, sizeof d);
     d.m = h.m;
     d.msv_tbm = h.msv_tbm;
-    if (is_long(h.m)) {  // no warp-chunked, MSV or Viterbi images: the long kernels read the plain image
+    if (is_long(h.m)) {  // no warp-chunked, MSV or Viterbi images: the row image, or the plain one past its widths
       P->msv_shape[i] = -1;
-      d.vbin = d.vshape = d.xshape = -1;
+      d.vbin = d.vshape = -1;
+      d.xshape = choose_xshape(h.m);
       d.x_off = x_total;
+      if (d.xshape >= 0) x_total += (int64_t)ximage_rows(h.m) * xwidth(d.xshape);
       d.msv_off = msv_total;
       d.vfb_off = vfb_total;
       d.vit_off = vit_total;
@@ -386,7 +395,7 @@ void pack_profiles(sx_profiles* P) {
     vfb_total += (int64_t)sxk::kImgRows * 32 * d.vc;
     d.xshape = choose_xshape(h.m);
     d.x_off = x_total;
-    x_total += (int64_t)sxk::kXRows * xwidth(d.xshape);
+    x_total += (int64_t)ximage_rows(h.m) * xwidth(d.xshape);
     d.vshape = shape_for(P->eng, 1, h.m);
     if (d.vshape < 0) throw CudaError{SX_EINVAL, "profile '" + h.name + "' too long for the Viterbi shapes"};
     d.vit_off = vit_total;
@@ -405,9 +414,9 @@ void pack_profiles(sx_profiles* P) {
   std::vector<uint2> qimg((size_t)std::max<int64_t>(q_total, 1));
   std::vector<uint4> qvimg((size_t)std::max<int64_t>(qv_total, 1));
   for (size_t i = 0; i < np; i++) {
+    if (P->dp[i].xshape >= 0) pack_ximage(P->h[i], P->dp[i], ximg.data());
     if (P->dp[i].vbin >= 0) {
       pack_images(P->h[i], P->dp[i], msv.data(), vit.data(), vfb.data());
-      pack_ximage(P->h[i], P->dp[i], ximg.data());
       // a profile whose rounded scores leave less than half of the int16
       // range as headroom (scores above +16 nats) stays on the exact kernel
       const int emax = pack_qimage(P->h[i], P->dp[i], qimg.data());
@@ -428,15 +437,16 @@ void pack_profiles(sx_profiles* P) {
     pack_bias(P->h[i], bias.data() + i * 54);
   }
   // plain layout: 25 msc rows then mm mi md im ii dm dd bm, each M+1 long;
-  // long profiles add the 25 odds rows and the 8 probability rows (same order),
-  // the image of the long kernels
+  // profiles past the exact row shapes add the 25 odds rows and the 8
+  // probability rows (same order), the image of the long kernels
+  auto huge = [&](size_t i) { return P->dp[i].xshape < 0; };
   std::vector<sxk::PlainProfile> pprof(np);
   int64_t plain_total = 0;
   for (size_t i = 0; i < np; i++) {
     pprof[i].off = plain_total;
     pprof[i].m = P->h[i].m;
     pprof[i].pad = 0;
-    plain_total += (is_long(P->h[i].m) ? (int64_t)sxk::kLongRows : 33LL) * (P->h[i].m + 1);
+    plain_total += (huge(i) ? (int64_t)sxk::kLongRows : 33LL) * (P->h[i].m + 1);
   }
   std::vector<float> plain((size_t)std::max<int64_t>(plain_total, 1));
   for (size_t i = 0; i < np; i++) {
@@ -446,7 +456,7 @@ void pack_profiles(sx_profiles* P) {
     memcpy(b, h.msc.data(), sizeof(float) * 25 * w);
     const int order[8] = {TMM, TMI, TMD, TIM, TII, TDM, TDD, TBM};
     for (int q = 0; q < 8; q++) memcpy(b + (25 + q) * w, h.t[order[q]].data(), sizeof(float) * w);
-    if (is_long(h.m)) {
+    if (huge(i)) {
       memcpy(b + sxk::kLMo * w, h.mo.data(), sizeof(float) * 25 * w);
       for (int q = 0; q < 8; q++) memcpy(b + (sxk::kLP + q) * w, h.p[order[q]].data(), sizeof(float) * w);
     }

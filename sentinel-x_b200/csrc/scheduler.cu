@@ -9,6 +9,12 @@
 namespace sxe {
 
 
+// Lets a kernel take more shared memory than the default 48 KB (which the
+// dynamic part shares with the kernel's static arrays).
+void allow_smem(const void* kernel, size_t bytes) {
+  if (bytes > (32u << 10)) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 // Fan independent launches out over the auxiliary streams and join them back
 // into the engine stream.
 void fork_aux(Streams& X) {
@@ -112,7 +118,8 @@ void queue_rows(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T
     load[a] += o.first;
     const int teams = sh.warps > 1 ? 1 : kRowsWarps;  // per CTA
     const dim3 grid((unsigned)((n + teams - 1) / teams), 2);
-    K.xrows[x]<<<grid, 32 * teams * sh.warps, sizeof(float) * (size_t)teams * xwidth(x), S.hi.aux[a]>>>(
+    allow_smem((const void*)K.xrows[x], xsmem(x, teams));
+    K.xrows[x]<<<grid, 32 * teams * sh.warps, xsmem(x, teams), S.hi.aux[a]>>>(
         S.rrecs.p + c.first[x], n, P->d_prof.p, P->d_x.p, T->d_res.p, T->d_off.p, T->d_len.p, T->d_xsc.p, S.rows.p);
     E->stats.kernel_launches++;
   }
@@ -642,35 +649,63 @@ int64_t long_stride(const sx_profiles* P, const std::vector<sxk::LongPair>& v, s
   return (int64_t)sxk::kLongArrays * (m + 1);
 }
 
-// MSV (viterbi = false) or Viterbi scores of long-profile pairs.
+// MSV (viterbi = false) or Viterbi scores of long-profile pairs: a launch per
+// row shape, longest targets first, and one of the long kernels for the rest.
 void long_scores(sx_engine* E, const sx_profiles* P, const sx_targets* T, const std::vector<sxk::LongPair>& v,
                  bool viterbi, std::vector<float>& out) {
   out.assign(v.size(), kNegInf);
   if (v.empty()) return;
+  const auto& K = kernels();
   cudaStream_t s = E->stream;
-  const int grid = long_grid(E, v.size());
-  const int64_t stride = long_stride(P, v, 0, v.size());
-  E->long_pairs.upload(v.data(), v.size(), s);
-  E->long_scratch.alloc((size_t)grid * (size_t)stride);
+  std::vector<size_t> order(v.size());
+  std::iota(order.begin(), order.end(), (size_t)0);
+  std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) {
+    const int sa = P->dp[v[a].p].xshape, sb = P->dp[v[b].p].xshape;
+    return sa != sb ? sa > sb : T->len[v[a].t] > T->len[v[b].t];
+  });
+  std::vector<sxk::LongPair> lst(v.size());
+  for (size_t i = 0; i < v.size(); i++) lst[i] = v[order[i]];
+  E->long_pairs.upload(lst.data(), lst.size(), s);
   E->long_out.alloc(v.size());
-  if (viterbi)
-    sxk::long_viterbi_kernel<<<grid, sxk::kPlainThreads, 0, s>>>(E->long_pairs.p, (int)v.size(), P->d_pprof.p,
-                                                                P->d_plain.p, T->d_res.p, T->d_off.p, T->d_len.p,
-                                                                T->d_xsc.p, E->long_scratch.p, stride, E->long_out.p);
-  else
-    sxk::long_msv_kernel<<<grid, sxk::kPlainThreads, 0, s>>>(E->long_pairs.p, (int)v.size(), P->d_pprof.p,
-                                                            P->d_plain.p, P->d_prof.p, T->d_res.p, T->d_off.p,
-                                                            T->d_len.p, T->d_tpar.p, E->long_scratch.p, stride,
-                                                            E->long_out.p);
-  CK(cudaGetLastError());
-  E->stats.kernel_launches++;
-  CK(cudaMemcpyAsync(out.data(), E->long_out.p, sizeof(float) * v.size(), cudaMemcpyDeviceToHost, s));
+  for (size_t a = 0, b = 0; a < lst.size(); a = b) {
+    const int x = P->dp[lst[a].p].xshape;
+    while (b < lst.size() && P->dp[lst[b].p].xshape == x) b++;
+    const int n = (int)(b - a);
+    const sxk::LongPair* pairs = E->long_pairs.p + a;
+    float* to = E->long_out.p + a;
+    if (x >= 0) {
+      const int threads = 32 * kXShapes[x].warps;
+      const size_t smem = xtrans(x) == sxk::kTrShared ? 8 * sizeof(float) * (size_t)xwidth(x) : 0;
+      allow_smem((const void*)K.wvit[x], smem);
+      if (viterbi)
+        K.wvit[x]<<<n, threads, smem, s>>>(pairs, P->d_prof.p, P->d_x.p, T->d_res.p, T->d_off.p, T->d_len.p, T->d_xsc.p, to);
+      else
+        K.wmsv[x]<<<n, threads, 0, s>>>(pairs, P->d_prof.p, P->d_x.p, T->d_res.p, T->d_off.p, T->d_len.p, T->d_tpar.p, to);
+    } else {
+      const int grid = long_grid(E, (size_t)n);
+      const int64_t stride = long_stride(P, lst, a, b);
+      E->long_scratch.alloc((size_t)grid * (size_t)stride);
+      if (viterbi)
+        sxk::long_viterbi_kernel<<<grid, sxk::kPlainThreads, 0, s>>>(pairs, n, P->d_pprof.p, P->d_plain.p, T->d_res.p,
+                                                                    T->d_off.p, T->d_len.p, T->d_xsc.p,
+                                                                    E->long_scratch.p, stride, to);
+      else
+        sxk::long_msv_kernel<<<grid, sxk::kPlainThreads, 0, s>>>(pairs, n, P->d_pprof.p, P->d_plain.p, P->d_prof.p,
+                                                                T->d_res.p, T->d_off.p, T->d_len.p, T->d_tpar.p,
+                                                                E->long_scratch.p, stride, to);
+    }
+    CK(cudaGetLastError());
+    E->stats.kernel_launches++;
+  }
+  std::vector<float> got(v.size());
+  CK(cudaMemcpyAsync(got.data(), E->long_out.p, sizeof(float) * v.size(), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
+  for (size_t i = 0; i < v.size(); i++) out[order[i]] = got[i];
 }
 
-// Raw Forward/Backward special rows of long-profile pairs, in chunks bounded
-// by the scratch budget; consume(first, n, fwd, bwd, off) per chunk, pair
-// first + q having its rows at fwd + off[q] and bwd + off[q].
+// Raw Forward/Backward special rows of pairs of profiles past the exact row
+// shapes, in chunks bounded by the scratch budget; consume(first, n, fwd, bwd,
+// off) per chunk, pair first + q having its rows at fwd + off[q] and bwd + off[q].
 void long_rows(sx_engine* E, const sx_profiles* P, const sx_targets* T, const std::vector<sxk::LongPair>& v,
                const LongRowsSink& consume) {
   cudaStream_t s = E->stream;
@@ -1034,6 +1069,12 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
       long_exact[pi] = (char)th[pi].exact;
       th[pi].exact = 0;
     }
+  // the exact F3 check of a final pair (pipeline.rs:179-183)
+  auto f3_fails = [&](const FinalPair& f, float fwdsc) {
+    const ProfileHost& h = P->h[f.p];
+    return (th[f.p].exact || long_exact[f.p]) &&
+           std::exp(exp_tail_logsurv((double)((fwdsc - f.filtersc) / kLn2f), h.fwd[0], h.fwd[1])) > o.f3;
+  };
   E->thr.upload(th.data(), th.size(), s);
   for (Slot& S : E->sl) {
     S.overflow.alloc(1);
@@ -1147,9 +1188,7 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
               const float* fr = ch->fwd(q);
               const float* br = ch->bwd(q);
               const float fwdsc = forward_score_from_rows(h, l, fr);
-              if (th[f.p].exact &&
-                  std::exp(exp_tail_logsurv((double)((fwdsc - f.filtersc) / kLn2f), h.fwd[0], h.fwd[1])) > o.f3)
-                return;
+              if (f3_fails(f, fwdsc)) return;
               n_domain++;
               B->res[i].hit = define_domains(h, T->dsq.data() + T->off[f.t], l, RawRows{fr, br}, fwdsc, o, B->res[i].h);
             });
@@ -1173,9 +1212,7 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
             const float* fr = ch->fwd(q);
             const float* br = ch->bwd(q);
             const float fwdsc = forward_score_from_rows(h, l, fr);
-            if (th[f.p].exact &&
-                std::exp(exp_tail_logsurv((double)((fwdsc - f.filtersc) / kLn2f), h.fwd[0], h.fwd[1])) > o.f3)
-              return;
+            if (f3_fails(f, fwdsc)) return;
             n_domain++;
             db.begin(q, h, f.p, T->dsq.data() + T->off[f.t], l, f.t, RawRows{fr, br}, fwdsc, true);
             begun[q] = 1;
@@ -1252,6 +1289,78 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
     nfinal += (int64_t)B->finals.size();
     rows_and_queue(E->sl[0], B, !(E->flags & SX_FLAG_ENV_HOST));  // every pair reaches domain definition
   }
+  // profiles longer than kMaxM: MSV on the device, the exact host checks of the
+  // F1 / bias / F2 filters on its scores (those cascade_finish re-runs), the
+  // Viterbi scores of the survivors; then rows and domain definition as for
+  // every other block, or, past the exact row shapes, the long kernels' rows and
+  // the host
+  if (!longs.empty() && nt > 0) {
+    outs.push_back(std::make_unique<BlockOut>());
+    BlockOut* B = outs.back().get();
+    std::vector<sxk::LongPair> filt;
+    std::vector<FinalPair> fin;
+    for (int pi : longs)
+      for (size_t t = 0; t < nt; t++) {
+        if (long_exact[pi]) filt.push_back({pi, (int32_t)t});
+        else fin.push_back({pi, (int32_t)t, 0.f, 0.f, 0.f, -1});
+      }
+    std::vector<float> usc, vsc, fsc(filt.size(), 0.f);
+    long_scores(E, P, T, filt, false, usc);
+    std::vector<char> pass1(filt.size(), 0);
+    parallel_for(filt.size(), E->host_threads, [&](size_t i) {
+      const ProfileHost& h = P->h[filt[i].p];
+      const int64_t l = T->len[filt[i].t];
+      const float nullsc = null1_score(l);
+      if (gumbel_survival((double)((usc[i] - nullsc) / kLn2f), h.msv[0], h.msv[1]) > o.f1) return;
+      fsc[i] = composition_bias_score(h, T->dsq.data() + T->off[filt[i].t], l);
+      if (gumbel_survival((double)((usc[i] - fsc[i]) / kLn2f), h.msv[0], h.msv[1]) > o.f1) return;
+      pass1[i] = 1;
+    });
+    std::vector<sxk::LongPair> surv;
+    std::vector<size_t> from;
+    for (size_t i = 0; i < filt.size(); i++)
+      if (pass1[i]) {
+        surv.push_back(filt[i]);
+        from.push_back(i);
+      }
+    long_scores(E, P, T, surv, true, vsc);
+    for (size_t q = 0; q < surv.size(); q++) {
+      const size_t i = from[q];
+      const ProfileHost& h = P->h[surv[q].p];
+      if (gumbel_survival((double)((vsc[q] - fsc[i]) / kLn2f), h.vit[0], h.vit[1]) > o.f2) continue;
+      fin.push_back({surv[q].p, surv[q].t, usc[i], fsc[i], vsc[q], -1});
+    }
+    for (const sxk::LongPair& q : filt) {
+      E->stats.pairs_in[0]++;
+      E->stats.cells[0] += (double)P->h[q.p].m * (double)T->len[q.t];
+    }
+    nfinal += (int64_t)fin.size();
+    std::vector<FinalPair> huge;
+    for (const FinalPair& f : fin) (P->dp[f.p].xshape >= 0 ? B->finals : huge).push_back(f);
+    if (!B->finals.empty()) rows_and_queue(E->sl[0], B, device_envelopes(B));
+    if (!huge.empty()) {
+      outs.push_back(std::make_unique<BlockOut>());
+      BlockOut* H = outs.back().get();
+      H->finals = std::move(huge);
+      H->res.resize(H->finals.size());
+      std::vector<sxk::LongPair> lp;
+      for (const FinalPair& f : H->finals) lp.push_back({f.p, f.t});
+      long_rows(E, P, T, lp, [&](size_t first, size_t n, const float* f, const float* b, const std::vector<int64_t>& off) {
+        parallel_for(n, E->host_threads, [&](size_t q) {
+          const size_t i = first + q;
+          const FinalPair& fp = H->finals[i];
+          const ProfileHost& h = P->h[fp.p];
+          const int64_t l = T->len[fp.t];
+          const float* fr = f + off[q];
+          const float* br = b + off[q];
+          const float fwdsc = forward_score_from_rows(h, l, fr);
+          if (f3_fails(fp, fwdsc)) return;
+          n_domain++;
+          H->res[i].hit = define_domains(h, T->dsq.data() + T->off[fp.t], l, RawRows{fr, br}, fwdsc, o, H->res[i].h);
+        });
+      });
+    }
+  }
   const auto t_dev = std::chrono::steady_clock::now();
   PhaseLog plog;
   plog.add("cascade_and_rows", t_start);
@@ -1292,70 +1401,6 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
     });
     plog.add("finish", t_fin);
     E->stats.ms[5] += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_env).count();
-  }
-  // profiles longer than kMaxM: MSV on the device, the exact host checks of the
-  // F1 / bias / F2 filters on its scores (those cascade_finish re-runs), the
-  // Viterbi scores of the survivors, then the rows of the final pairs, F3 and
-  // domain definition on the host pool
-  if (!longs.empty() && nt > 0) {
-    outs.push_back(std::make_unique<BlockOut>());
-    BlockOut* B = outs.back().get();
-    std::vector<sxk::LongPair> filt;
-    for (int pi : longs)
-      for (size_t t = 0; t < nt; t++) {
-        if (long_exact[pi]) filt.push_back({pi, (int32_t)t});
-        else B->finals.push_back({pi, (int32_t)t, 0.f, 0.f, 0.f, -1});
-      }
-    std::vector<float> usc, vsc, fsc(filt.size(), 0.f);
-    long_scores(E, P, T, filt, false, usc);
-    std::vector<char> pass1(filt.size(), 0);
-    parallel_for(filt.size(), E->host_threads, [&](size_t i) {
-      const ProfileHost& h = P->h[filt[i].p];
-      const int64_t l = T->len[filt[i].t];
-      const float nullsc = null1_score(l);
-      if (gumbel_survival((double)((usc[i] - nullsc) / kLn2f), h.msv[0], h.msv[1]) > o.f1) return;
-      fsc[i] = composition_bias_score(h, T->dsq.data() + T->off[filt[i].t], l);
-      if (gumbel_survival((double)((usc[i] - fsc[i]) / kLn2f), h.msv[0], h.msv[1]) > o.f1) return;
-      pass1[i] = 1;
-    });
-    std::vector<sxk::LongPair> surv;
-    std::vector<size_t> from;
-    for (size_t i = 0; i < filt.size(); i++)
-      if (pass1[i]) {
-        surv.push_back(filt[i]);
-        from.push_back(i);
-      }
-    long_scores(E, P, T, surv, true, vsc);
-    for (size_t q = 0; q < surv.size(); q++) {
-      const size_t i = from[q];
-      const ProfileHost& h = P->h[surv[q].p];
-      if (gumbel_survival((double)((vsc[q] - fsc[i]) / kLn2f), h.vit[0], h.vit[1]) > o.f2) continue;
-      B->finals.push_back({surv[q].p, surv[q].t, usc[i], fsc[i], vsc[q], -1});
-    }
-    for (const sxk::LongPair& q : filt) {
-      E->stats.pairs_in[0]++;
-      E->stats.cells[0] += (double)P->h[q.p].m * (double)T->len[q.t];
-    }
-    B->res.resize(B->finals.size());
-    std::vector<sxk::LongPair> fin(B->finals.size());
-    for (size_t i = 0; i < fin.size(); i++) fin[i] = {B->finals[i].p, B->finals[i].t};
-    nfinal += (int64_t)fin.size();
-    long_rows(E, P, T, fin, [&](size_t first, size_t n, const float* f, const float* b, const std::vector<int64_t>& off) {
-      parallel_for(n, E->host_threads, [&](size_t q) {
-        const size_t i = first + q;
-        const FinalPair& fp = B->finals[i];
-        const ProfileHost& h = P->h[fp.p];
-        const int64_t l = T->len[fp.t];
-        const float* fr = f + off[q];
-        const float* br = b + off[q];
-        const float fwdsc = forward_score_from_rows(h, l, fr);
-        if (long_exact[fp.p] &&
-            std::exp(exp_tail_logsurv((double)((fwdsc - fp.filtersc) / kLn2f), h.fwd[0], h.fwd[1])) > o.f3)
-          return;
-        n_domain++;
-        B->res[i].hit = define_domains(h, T->dsq.data() + T->off[fp.t], l, RawRows{fr, br}, fwdsc, o, B->res[i].h);
-      });
-    });
   }
   E->stats.kernel_launches += env_launches.load();
   E->stats.pairs_out[5] = n_env.load();

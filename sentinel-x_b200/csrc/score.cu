@@ -141,10 +141,17 @@ int sx_score_pairs(sx_engine* e, const sx_profiles* p, const sx_targets* t, cons
       };
       std::vector<FinalPair> fp;
       for (size_t i = 0; i < npairs; i++)
-        if (!is_long(p->h[pair_profile[i]].m)) fp.push_back({pair_profile[i], pair_target[i], 0.f, 0.f, 0.f, (int32_t)i});
+        if (p->dp[pair_profile[i]].xshape >= 0) fp.push_back({pair_profile[i], pair_target[i], 0.f, 0.f, 0.f, (int32_t)i});
       rows_pass_sync(e, p, t, fp, [&](size_t q, const float* fr, const float* br) { put((size_t)fp[q].slot, fr, br); });
-      long_rows(e, p, t, lpairs, [&](size_t first, size_t n, const float* f, const float* b, const std::vector<int64_t>& off) {
-        for (size_t q = 0; q < n; q++) put(lng[first + q], f + off[q], b + off[q]);
+      std::vector<size_t> huge;  // past the exact row shapes
+      std::vector<sxk::LongPair> hpairs;
+      for (size_t q = 0; q < lng.size(); q++)
+        if (p->dp[lpairs[q].p].xshape < 0) {
+          huge.push_back(lng[q]);
+          hpairs.push_back(lpairs[q]);
+        }
+      long_rows(e, p, t, hpairs, [&](size_t first, size_t n, const float* f, const float* b, const std::vector<int64_t>& off) {
+        for (size_t q = 0; q < n; q++) put(huge[first + q], f + off[q], b + off[q]);
       });
     }
   } catch (const CudaError& ce) {

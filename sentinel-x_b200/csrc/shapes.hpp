@@ -11,6 +11,7 @@
 #include "adjoint.cuh"
 #include "envelope.cuh"
 #include "exact_rows.cuh"
+#include "wide.cuh"
 #include "prescreen.cuh"
 
 namespace sx {
@@ -37,7 +38,8 @@ constexpr MsvShape kMsvShapes[] = {
     {8, 36}, {8, 44}, {8, 52}, {8, 60}};
 constexpr int kNumMsvShapes = sizeof(kMsvShapes) / sizeof(kMsvShapes[0]);
 constexpr int kMaxM = 2048;  // columns of the warp-chunked and lane-group kernels
-// Longer profiles (marker models of long proteins) run through the long kernels.
+// Longer profiles (models of long proteins) take a pass of their own: wide.cuh
+// and the exact row shapes up to their width, long.cuh beyond it.
 inline bool is_long(int m) { return m > kMaxM; }
 // Viterbi lane-group shapes: G lanes per pair, C columns per lane, rt = the
 // transition rows held in registers for the whole pair (C <= 16).
@@ -85,10 +87,18 @@ constexpr int kNumVbins = sizeof(kVcBins) / sizeof(kVcBins[0]);
 struct XShape {
   int c, warps;
 };
-constexpr XShape kXShapes[] = {{4, 1}, {8, 1}, {8, 2}, {8, 3}, {8, 4}, {8, 6}, {8, 8}};
+constexpr XShape kXShapes[] = {{4, 1}, {8, 1}, {8, 2}, {8, 3}, {8, 4}, {8, 6}, {8, 8}, {8, 12}, {8, 16}, {16, 16}};
 constexpr int kNumXShapes = sizeof(kXShapes) / sizeof(kXShapes[0]);
 constexpr int xwidth(int s) { return 32 * kXShapes[s].c * kXShapes[s].warps; }
-static_assert(xwidth(kNumXShapes - 1) == kMaxM, "the exact row passes cover every warp-chunked profile");
+static_assert(xwidth(kNumXShapes - 1) >= kMaxM, "the exact row passes cover every warp-chunked profile");
+// where a shape's threads keep their transition rows, and the dynamic shared
+// memory of a CTA of `teams` teams: a row each, and those transitions
+constexpr sxk::TransIn xtrans(int s) {
+  return kXShapes[s].warps <= 8 ? sxk::kTrReg : kXShapes[s].c <= 8 ? sxk::kTrShared : sxk::kTrGlobal;
+}
+constexpr size_t xsmem(int s, int teams) {
+  return sizeof(float) * (size_t)xwidth(s) * (size_t)(teams + (xtrans(s) == sxk::kTrShared ? 8 : 0));
+}
 
 typedef void (*MsvFn)(const MsvTile*, const DevProfile*, const Thresholds*, const float4*, const uint8_t*,
                       const int64_t*, const int32_t*, const float4*, const int32_t*, float*, const int32_t*, PairRec*,
@@ -119,6 +129,9 @@ typedef void (*EnvRowsFn)(const sxk::EnvRec*, int, const DevProfile*, const floa
 typedef void (*EnvOaFn)(const sxk::EnvRec*, int, const DevProfile*, const float*, float*, float*, const double*,
                         float*);
 
+typedef void (*WideFn)(const sxk::LongPair*, const DevProfile*, const float*, const uint8_t*, const int64_t*,
+                       const int32_t*, const float4*, float*);
+
 struct KernelTables {
   MsvFn msv[kNumMsvShapes];
   Msv16Fn msv16[kNumMsvShapes];  // the packed pre-screen, same shapes
@@ -128,6 +141,7 @@ struct KernelTables {
   VitFn vit[kNumVbins];
   FwdFn fwd_scan[kNumVbins];  // the F3 pre-screen
   XRowsFn xrows[kNumXShapes];  // exact Forward and Backward rows
+  WideFn wmsv[kNumXShapes], wvit[kNumXShapes];  // M > kMaxM: MSV and Viterbi scores (nullptr for narrow shapes)
   AdjFFn adjf[kNumVbins];
   AdjBFn adjb[kNumVbins];
   VitGFn vitg[kNumVitShapes];

@@ -50,6 +50,28 @@ def test_scores_equal_the_oracle(engine, m, dd):
         assert got["backward"][i] == np.float32(o.backward(0, t)), (m, i)
 
 
+@pytest.mark.parametrize("dd", [None, 0.9995])
+@pytest.mark.parametrize("m", [2049, 3072, 3073, 4096, 4097, 8192, 8193])
+def test_wide_scores_equal_the_oracle(engine, m, dd):
+    """M above the lane-group kernels' columns (csrc/wide.cuh and the widest
+    row shapes), and the first M past those (csrc/long.cuh)."""
+    text, p = _text(m, dd, 40 + m)
+    rng = np.random.default_rng(m)
+    hom = synth.emit_homolog(rng, p)[:150]
+    targets = [synth.background_seq(rng, n) for n in (1, 2, 33)]
+    targets.append(synth.plant(rng, len(hom) + 20, [hom]))
+    targets.append(np.array([24, 3, 24, 24, 20, 21, 22, 23, 5, 24], np.uint8))
+    lens = np.array([len(t) for t in targets])
+    ps = engine.load_text(text)
+    ts = engine.targets_digital(np.concatenate(targets), np.concatenate([[0], np.cumsum(lens)[:-1]]), lens)
+    got = engine.score_pairs(ps, ts, np.zeros(len(targets), np.int32), np.arange(len(targets)),
+                             stages=("msv", "viterbi", "forward", "backward"))
+    o = O.Oracle(text=text)
+    for i, t in enumerate(targets):
+        for stage in got:
+            assert got[stage][i] == np.float32(getattr(o, stage)(0, t)), (m, i, stage)
+
+
 def _hits(hits, doms):
     """Hits with their domains, from either side's records."""
     out = []
@@ -70,10 +92,10 @@ def device_engine():
 
 
 @pytest.mark.parametrize("gappy", [False, True])
-@pytest.mark.parametrize("m", [3, 5, 127, 128, 129, 256, 257, 513, 1025, 1537, 2048])
+@pytest.mark.parametrize("m", [3, 5, 127, 128, 129, 256, 257, 513, 1025, 1537, 2048, 2049, 3073, 4100])
 def test_device_envelopes_equal_the_oracle(device_engine, m, gappy):
     """Envelope matrices, null2 and insert sums, optimal accuracy and its
-    traceback (runs of matches, inserts, deletes) on every team width, for
+    traceback (runs of matches, inserts, deletes) on the team widths, for
     homologs of well-behaved and of gap-rich models, alone and twice."""
     rng = np.random.default_rng(900 + m)
     p = synth.sample_profile(rng, m, f"env{m}")
