@@ -6,7 +6,7 @@ namespace {
 template <int I>
 struct Vit16Table {
   static void fill(Vit16Fn* t) {
-    t[I] = sxk::vit16_kernel<kVit16Shapes[I].g, kVit16Shapes[I].c>;
+    t[I] = sxk::vit16_kernel<kVit16Shapes[I].g, kVit16Shapes[I].c, kVit16Shapes[I].w>;
     Vit16Table<I + 1>::fill(t);
   }
 };

@@ -268,8 +268,8 @@ int pack_qimage(const ProfileHost& h, const DevProfile& d, uint2* out) {
 // 2^-12 nat; match scores clamped up to -8 nats, transitions clamped to
 // [-8 nats, 0] (t_bm to [-16 nats, 0]); -inf scores and columns past M take
 // the floor.  8 transition rows (each column's score in both int16 halves of
-// a word, 4 columns per uint4), then 25 match-score rows (4 columns per
-// uint2), lane-major like the f32 Viterbi image, at width G*C of the
+// a word, 4 columns per uint4), then 25 match-score rows and the row past a
+// target's end (4 columns per uint2), lane-major like the f32 Viterbi image, at width G*C of the
 // profile's pre-screen shape.  Returns the largest rounded match score.
 int pack_qvimage(const ProfileHost& h, const DevProfile& d, uint4* out) {
   const int m = h.m, G = kVit16Shapes[d.qv_shape].g, C = kVit16Shapes[d.qv_shape].c, NC4 = C / 4;
@@ -312,11 +312,11 @@ int pack_qvimage(const ProfileHost& h, const DevProfile& d, uint4* out) {
         base[(q * NC4 + c4) * G + j] = make_uint4(dup(tr(q, k)), dup(tr(q, k + 1)), dup(tr(q, k + 2)), dup(tr(q, k + 3)));
       }
   uint2* es = reinterpret_cast<uint2*>(base + 8 * row4);
-  for (int x = 0; x < 25; x++)
+  for (int x = 0; x < sxk::kV16Rows; x++)  // row 25: past a target's end
     for (int j = 0; j < G; j++)
       for (int c4 = 0; c4 < NC4; c4++) {
         int v[4];
-        for (int e = 0; e < 4; e++) v[e] = em(x, j * C + c4 * 4 + e + 1);
+        for (int e = 0; e < 4; e++) v[e] = x < 25 ? em(x, j * C + c4 * 4 + e + 1) : sxk::kV16EPast;
         uint2 w;
         w.x = (uint32_t)(v[0] & 0xffff) | ((uint32_t)(v[1] & 0xffff) << 16);
         w.y = (uint32_t)(v[2] & 0xffff) | ((uint32_t)(v[3] & 0xffff) << 16);
@@ -327,7 +327,7 @@ int pack_qvimage(const ProfileHost& h, const DevProfile& d, uint4* out) {
 // uint4 entries of a quantized Viterbi image of shape s
 int64_t qvimage_size(int s) {
   const int64_t row4 = (int64_t)(kVit16Shapes[s].c / 4) * kVit16Shapes[s].g;
-  return 8 * row4 + 25 * row4 / 2;
+  return 8 * row4 + sxk::kV16Rows * row4 / 2;
 }
 
 // Composition-bias filter table (src/hmmer/pipeline.rs:110-131): 54 doubles.

@@ -103,7 +103,7 @@ __device__ __forceinline__ int q32_up(float x) {
 // first scores are loaded before the vote, whose branch would otherwise keep
 // them behind it.  Measured on B200 (296 profiles of one length x 12,000
 // targets, useful cells per clock per SM, before -> now): M = 100 40.0 -> 46.1,
-// 160 42.9 -> 50.7, 208 44.4 -> 53.1, 300 40.1 -> 49.6, 600 39.6 -> 50.7, 1000
+// 160 42.9 -> 50.7, 208 44.4 -> 54.2, 300 40.1 -> 49.6, 600 39.6 -> 50.7, 1000
 // 45.3 -> 53.9; the Pfam-scale search's pre-screen 298 -> 255 ms, and 211 with
 // tiles of equal work.
 //
@@ -381,16 +381,35 @@ namespace sxk {
 
 // ---------------------------------------------------------------------------
 // Packed-integer Viterbi pre-screen: an upper bound of the reference's f32
-// Viterbi score (src/hmmer/dp.rs:152-189) for two targets of one profile at
-// once, in int16x2 lanes (target a in the low half, b in the high half).
+// Viterbi score (src/hmmer/dp.rs:152-189) for 2 W targets of one profile at
+// once, in W words of int16x2 (one target per half).
 //
 // Why: the exact lane-group kernel (viterbi_g_kernel) is bound by the
 // latency of each row's sequential parts -- the D chain, the carry vote, the
-// row-maximum butterfly, the special states -- and by the per-row control
-// around them, which a lane group pays once per pair.  Here one pass of all
-// of that serves two pairs: every 32-bit word holds the same column of two
-// DP rows, one max.s16x2 / add.s16x2 updates both, and the carry vote, the
-// butterfly and the loop control are shared.
+// row-maximum butterfly, the special states -- by the per-row control around
+// them, and by the 32 bytes of transitions it reads for every cell.  Here one
+// pass of all of that serves 2 W pairs: every max(a + b, c) is one fused
+// operation on two cells, W words share the transitions read from shared
+// memory and fill each other's latency, and rows run in blocks of four without
+// control flow:
+//   * the D chain runs in every lane at once, first without a carry, then from
+//     the carry its left neighbour ended with, until no lane's carry changes
+//     (integers: the fixed point is the sequential chain);
+//   * N, J and B as in the MSV pre-screen: base = max(N, J) decays, a vote finds
+//     the rows whose E raises it, J is kept per lane and combined at the end;
+//   * rows past a target's end in its last block read a score row of -24 nats
+//     (row 25 of the image), which raises nothing, and J's decay is undone.
+// Bound: shared memory (8 transition words and 2 W score halves per W words of
+// cells, 10 bytes a cell at W = 2 and 18 at W = 1) and the ALU pipe, about 11
+// operations a word; short of either, the latency of a row at 8 to 12 warps
+// per SM.  Measured on B200 (296 profiles of one length, their ~67,000 bias
+// survivors of 12,000 targets; before: one word, carries pushed column by
+// column, specials and a butterfly every row, list order): M = 60 4.3 -> 1.5
+// ms, 100 5.2 -> 2.4, 208 7.5 -> 3.7, 300 14.2 -> 5.5, and the Pfam-scale
+// search's 61 -> 34 ms.  M = 513 to 1536, exact before (600: 35 ms, 1000: 44),
+// is pre-screened with one word: 1000 11.7 + 6.0 ms exact; 48 columns a lane
+// spill, but still run 1.8 times the exact kernel's cells (a marker-set
+// genome's Viterbi stage 18.3 -> 10.5 ms).
 //
 // Exactness.  As for the MSV pre-screen, the bound never decides a pair: a
 // pair passes when its bound passes F2 (with the exact kernel's slack), and
@@ -426,14 +445,20 @@ constexpr int kV16BmFloor = -8192;   // -16 nats: lowest t_bm
 constexpr int kV16EFloor = -4096;    // -8 nats: lowest match score, and columns past M
 constexpr int kV16BFloor = -4096;    // -8 nats: lowest B state
 constexpr unsigned kV16Init2 = 0xc000c000u;  // (-16384, -16384): -inf before row 1 / left of column 1
-constexpr unsigned kV16Low2 = 0xa000a000u;   // (-24576, -24576): provisional D carry into a lane
+constexpr unsigned kV16Low2 = 0xa000a000u;   // (-24576, -24576): no D carry into a lane
+constexpr int kV16EPast = -12288;    // -24 nats: scores of the rows past a target's end
+constexpr unsigned kV16BFloor2 = 0xf000f000u;
+constexpr int kV16Rows = 26;         // score rows of an image: 25 residue codes and the row past the end
+
+constexpr int kV16Tile = 1024;       // entries of a tile that are ordered by length
+constexpr int kV16Buckets = 64;      // of 32 residues
 
 // One profile x every nsub-th entry (from sub) of its Viterbi pre-screen list.
 struct VitTile {
   int32_t p, sub, nsub, pad;
 };
 
-// int16x2 helpers: replace one half of a word by the same half of v.
+// int16x2 helper: replace one half of a word by the same half of v.
 __device__ __forceinline__ unsigned set_half(unsigned w, int h, unsigned v) {
   return h ? __byte_perm(w, v, 0x7610) : __byte_perm(w, v, 0x3254);
 }
@@ -442,269 +467,310 @@ __device__ __forceinline__ unsigned set_half(unsigned w, int h, unsigned v) {
 // (region (p - p0) * vcap of `vlist`, vcount[p - p0] entries).  The profile's
 // quantized image (qv_off, uint4 units): 8 transition rows of W/4 uint4 (each
 // column's score in both halves: t_mm t_im t_dm at k-1, t_bm t_mi t_ii at k,
-// t_md t_dd at k-1), then 25 match-score rows of W/4 uint2 (4 columns of
+// t_md t_dd at k-1), then kV16Rows match-score rows of W/4 uint2 (4 columns of
 // int16), both in the lane-major chunk layout of the f32 Viterbi image.
 // Per pair: with `score_out`, the bound (f32 nats; +inf when capped, NaN for
 // an empty target) goes to score_out[slot]; otherwise a pair whose bound
 // passes F2 is appended to the exact Viterbi's list (bin vshape).  stats[0..2]
 // accumulate the DP cells bounded, the cells of the passing pairs and the
 // passing pairs.
-template <int G, int C>
-__global__ void __launch_bounds__(128, (C <= 8 ? 4 : 3)) vit16_kernel(
+template <int G, int C, int W>
+__global__ void __launch_bounds__(128, (C * W <= 16 ? 3 : 2)) vit16_kernel(
     const VitTile* __restrict__ tiles, const DevProfile* __restrict__ profs, const Thresholds* __restrict__ thr,
     const uint4* __restrict__ qvimg, const uint8_t* __restrict__ res, const int64_t* __restrict__ toff,
     const int32_t* __restrict__ tlen, const float4* __restrict__ xsc, const PairRec* __restrict__ vlist,
     unsigned vcap, const unsigned* __restrict__ vcount, int p0, PairRec* __restrict__ out,
     const BinRegion* __restrict__ out_bins, unsigned* __restrict__ out_counts, unsigned* __restrict__ overflow,
     float slack, float* __restrict__ score_out, double* __restrict__ stats) {
-  static_assert(C % 4 == 0 && (G & (G - 1)) == 0 && G <= 32, "bad packed Viterbi shape");
+  static_assert(C % 8 == 0 && (G & (G - 1)) == 0 && G <= 32, "bad packed Viterbi shape");
   constexpr int NC4 = C / 4;
   constexpr int ROW4 = NC4 * G;  // uint4 per transition row, uint2 per score row
-  static_assert(ROW4 % 2 == 0, "score rows must fill whole uint4");
-  constexpr int NIMG4 = 8 * ROW4 + 25 * ROW4 / 2;
+  constexpr int H = 2 * W;       // targets of a group
+  constexpr int NIMG4 = 8 * ROW4 + kV16Rows * ROW4 / 2;
   extern __shared__ uint4 sm_v[];
   __shared__ unsigned s_next;
+  __shared__ unsigned s_at[kV16Buckets];
+  __shared__ uint16_t s_order[kV16Tile];
   const VitTile tile = tiles[blockIdx.x];
-  const DevProfile P = profs[tile.p];
+  const DevProfile& P = profs[tile.p];
   {
     const uint4* src = qvimg + P.qv_off;
     for (int q = threadIdx.x; q < NIMG4; q += blockDim.x) sm_v[q] = src[q];
   }
+  const unsigned n = min(vcount[tile.p - p0], vcap);
+  const PairRec* lst = vlist + (int64_t)(tile.p - p0) * vcap;
+  // the tile's entries, longest targets first, so that no long target starts
+  // when the others are about to end (a tile past the order's room keeps the
+  // list's)
+  const unsigned mine = n > (unsigned)tile.sub ? (n - tile.sub + tile.nsub - 1) / tile.nsub : 0;
+  const bool ordered = mine <= kV16Tile;
   if (threadIdx.x == 0) s_next = 0;
+  for (int q = threadIdx.x; q < kV16Buckets; q += blockDim.x) s_at[q] = 0;
   __syncthreads();
-  const uint4* Ts = sm_v;
-  const uint2* Es = reinterpret_cast<const uint2*>(sm_v + 8 * ROW4);
+  if (ordered) {
+    auto bucket = [&](unsigned k) {
+      return kV16Buckets - 1 - min(kV16Buckets - 1, tlen[lst[tile.sub + k * tile.nsub].t] >> 5);
+    };
+    for (unsigned k = threadIdx.x; k < mine; k += blockDim.x) atomicAdd(&s_at[bucket(k)], 1u);
+    __syncthreads();
+    if (threadIdx.x < 32) {  // exclusive prefix sums
+      unsigned before = 0;
+      for (int q = 0; q < kV16Buckets; q += 32) {
+        const unsigned v = s_at[q + threadIdx.x];
+        unsigned inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned up = __shfl_up_sync(kFull, inc, o);
+          if ((int)threadIdx.x >= o) inc += up;
+        }
+        s_at[q + threadIdx.x] = before + inc - v;
+        before += __shfl_sync(kFull, inc, 31);
+      }
+    }
+    __syncthreads();
+    for (unsigned k = threadIdx.x; k < mine; k += blockDim.x) s_order[atomicAdd(&s_at[bucket(k)], 1u)] = (uint16_t)k;
+  }
+  __syncthreads();
 
   const int lane = threadIdx.x & 31;
   const int j = lane & (G - 1);
   const int gl = lane - j;
   const unsigned gmask = (G == 32) ? kFull : (((1u << G) - 1u) << gl);
-  const int pl = tile.p - p0;
-  const unsigned n = min(vcount[pl], vcap);
-  const PairRec* lst = vlist + (int64_t)pl * vcap;
   const int cap = P.qv_cap;
-  const float s2 = thr[tile.p].s2;
   const int nln2 = (int)ceilf(-0.693147182464599609375f * 1048576.0f) + kQ32Rho;
-  const uint4* tr = Ts + j;
+  const int nln2_25 = 32 * nln2;
+  constexpr int kJStart = -60 * (1 << 25);
+  const int base_idle = 32767 * 65536 + nln2_25;  // a base no E raises
+  const uint4* tr = sm_v + j;
+  const uint2* es = reinterpret_cast<const uint2*>(sm_v + 8 * ROW4) + j;
+  const uint32_t* words = reinterpret_cast<const uint32_t*>(res);  // targets start on 16-byte boundaries
   auto T = [&](int q, int c4) -> uint4 { return tr[(q * NC4 + c4) * G]; };
   auto pick = [](const uint4& v, int e) -> unsigned { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; };
+  auto upper = [](int a, int b) { return __byte_perm((unsigned)a, (unsigned)b, 0x7632); };  // int16 of two states
 
-  unsigned mp[C], ip[C], dp[C], pre[C];
+  // rows carried on: I, D and pre = max(M + t_mm, I + t_im) of the next row
+  unsigned ip[W][C], dp[W][C], pre[W][C];
+  unsigned dpl[W], bw[W];  // D left of the lane's first column; B of the row being computed
 #pragma unroll
-  for (int c = 0; c < C; c++) mp[c] = ip[c] = dp[c] = pre[c] = kV16Init2;
-  unsigned bw = kV16Init2;   // B of both halves for the row being computed
-  unsigned dpl = kV16Init2;  // left lane's D at its last column, previous row
-  // per half: pair state
-  int L[2] = {0, 0}, row[2] = {0, 0}, boff[2] = {0, 0}, idx[2] = {0, 0};
-  int xn[2] = {0, 0}, xj[2] = {kQ32Neg, kQ32Neg}, fin[2] = {kQ32Neg, kQ32Neg}, tl[2] = {0, 0}, tm[2] = {0, 0};
-  bool act[2] = {false, false}, big[2] = {false, false}, dn[2] = {false, false};
-  const uint8_t* seq[2] = {res, res};
-  // residues: 16-byte words, the next one prefetched; wc = the current 4
-  // bytes, consumed from the low byte up (targets are padded with '*' to a
-  // 16-byte boundary and followed by 64 bytes of slack, so every byte read is
-  // a valid residue code)
-  uint4 rc[2], rn[2];
-  uint32_t wc[2] = {0x18181818u, 0x18181818u};
+  for (int w = 0; w < W; w++) {
 #pragma unroll
-  for (int h = 0; h < 2; h++) rc[h] = rn[h] = make_uint4(0x18181818u, 0x18181818u, 0x18181818u, 0x18181818u);
+    for (int c = 0; c < C; c++) ip[w][c] = dp[w][c] = pre[w][c] = kV16Init2;
+    dpl[w] = kV16Init2;
+    bw[w] = kV16BFloor2;
+  }
+  // per target, in 2^-25 nat: base, tloop, the constant of B (tmove + 2047 /
+  // 2^20) and J of this lane's columns; rows left, its list entry, the index of
+  // the residue word after the fetched ones, this block's word and the next
+  int base[H], tl[H], tk[H], jj[H], rem[H];
+  unsigned idx[H], wi[H], cur[H], nxt[H];
+#pragma unroll
+  for (int h = 0; h < H; h++) {
+    base[h] = base_idle;
+    tl[h] = tk[h] = rem[h] = 0;
+    jj[h] = kJStart;
+    idx[h] = wi[h] = 0;
+    cur[h] = nxt[h] = 0;
+  }
+  unsigned active = 0, done = 0, big = 0;  // by target
   double cells_in = 0.0, cells_pass = 0.0, npass = 0.0;
 
   for (;;) {
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      if (!dn[h] && row[h] >= L[h]) {  // group-uniform: finish this half's pair, take the next one
-        if (act[h] && j == 0) {
-          const PairRec r = lst[idx[h]];
-          const float ub = L[h] == 0 ? __int_as_float(0x7fc00000)
-                           : big[h]  ? __int_as_float(0x7f800000)
-                                     : __fmul_rn(__int2float_ru(fin[h]), 9.5367431640625e-7f);
-          if (score_out) {
-            score_out[r.slot] = ub;
-          } else if (L[h] > 0) {
-            const double cells = (double)P.m * (double)L[h];
-            cells_in += cells;
-            if (big[h] || bits_stat(ub, r.filtersc) >= s2 - slack) {
-              push_pair(r, P.vshape, out, out_bins, out_counts, overflow);
-              cells_pass += cells;
-              npass += 1.0;
+    for (int h = 0; h < H; h++) {
+      if (!(done >> h & 1) && rem[h] <= 0) {  // group-uniform: finish this target, take the next one
+        if (active >> h & 1) {
+          int jm = jj[h];
+#pragma unroll
+          for (int o = G / 2; o >= 1; o >>= 1) jm = max(jm, __shfl_xor_sync(gmask, jm, o, G));
+          if (j == 0) {
+            const PairRec r = lst[idx[h]];
+            const int L = tlen[r.t];
+            const int xj = ((jm + rem[h] * tl[h]) >> 5) + nln2;  // at row L: rem is minus the rows past it
+            const float ub = L == 0              ? __int_as_float(0x7fc00000)
+                             : (big >> h & 1)    ? __int_as_float(0x7f800000)
+                                                 : __fmul_rn(__int2float_ru(xj + q32_up(xsc[r.t].y)), 9.5367431640625e-7f);
+            if (score_out) {
+              score_out[r.slot] = ub;
+            } else if (L > 0) {
+              const double cells = (double)P.m * (double)L;
+              cells_in += cells;
+              if ((big >> h & 1) || bits_stat(ub, r.filtersc) >= thr[tile.p].s2 - slack) {
+                push_pair(r, P.vshape, out, out_bins, out_counts, overflow);
+                cells_pass += cells;
+                npass += 1.0;
+              }
             }
           }
         }
         unsigned k = 0;
         if (j == 0) k = atomicAdd(&s_next, 1u);
         k = __shfl_sync(gmask, k, gl);
-        const unsigned e = (unsigned)tile.sub + k * (unsigned)tile.nsub;
-        if (k < n && e < n) {
-          idx[h] = (int)e;
+        big &= ~(1u << h);
+        jj[h] = kJStart;
+        if (k < mine) {
+          const unsigned e = (unsigned)tile.sub + (ordered ? s_order[k] : k) * (unsigned)tile.nsub;
+          idx[h] = e;
           const int t = lst[e].t;
-          L[h] = tlen[t];
-          seq[h] = res + toff[t];
+          rem[h] = tlen[t];
+          wi[h] = (unsigned)(toff[t] >> 2);
+          cur[h] = __ldg(words + wi[h]);
+          nxt[h] = __ldg(words + wi[h] + 1);
+          wi[h] += 2;
           const float4 xs = xsc[t];
-          tl[h] = q32_up(xs.x);
-          tm[h] = q32_up(xs.y);
-          xn[h] = 0;
-          xj[h] = kQ32Neg;
-          fin[h] = kQ32Neg;
-          big[h] = false;
-          row[h] = 0;
-          boff[h] = 0;
-          rc[h] = __ldg(reinterpret_cast<const uint4*>(seq[h]));
-          rn[h] = __ldg(reinterpret_cast<const uint4*>(seq[h] + 16));
-          wc[h] = rc[h].x;
-          act[h] = true;
+          tl[h] = 32 * q32_up(xs.x);
+          tk[h] = 32 * (q32_up(xs.y) + 2047);
+          base[h] = 0;  // N of row 0
+          active |= 1u << h;
+          const int w = h >> 1;
 #pragma unroll
           for (int c = 0; c < C; c++) {
-            mp[c] = set_half(mp[c], h, kV16Init2);
-            ip[c] = set_half(ip[c], h, kV16Init2);
-            dp[c] = set_half(dp[c], h, kV16Init2);
-            pre[c] = set_half(pre[c], h, kV16Init2);
+            ip[w][c] = set_half(ip[w][c], h & 1, kV16Init2);
+            dp[w][c] = set_half(dp[w][c], h & 1, kV16Init2);
+            pre[w][c] = set_half(pre[w][c], h & 1, kV16Init2);
           }
-          dpl = set_half(dpl, h, kV16Init2);
-          // B of row 1: xB = tmove
-          const int b16 = max((tm[h] + 2047) >> (kQ32Shift - kQ16Shift), kV16BFloor);
-          bw = set_half(bw, h, ((unsigned)b16 & 0xffffu) * 0x10001u);
+          dpl[w] = set_half(dpl[w], h & 1, kV16Init2);
+          bw[w] = set_half(bw[w], h & 1, max2s16(upper(tk[h], tk[h]), kV16BFloor2));
         } else {
-          act[h] = false;
-          dn[h] = true;
-          L[h] = 0;
+          active &= ~(1u << h);
+          done |= 1u << h;
+          rem[h] = 0;
+          tl[h] = 0;
+          base[h] = base_idle;
         }
       }
     }
-    if (__all_sync(kFull, dn[0] && dn[1])) break;
+    if (__all_sync(kFull, done == (1u << H) - 1u)) break;
 
-    // this row's residue of each half (idle halves compute on stale ones)
-    int x[2];
+    // the block's residues; 25 from the target's end on
+    unsigned rw[H];
 #pragma unroll
-    for (int h = 0; h < 2; h++) x[h] = (int)(wc[h] & 0xffu);
-    // match scores of both halves, interleaved into words
-    unsigned ew[C];
-    {
-      const uint2* ea = Es + x[0] * ROW4 + j;
-      const uint2* eb = Es + x[1] * ROW4 + j;
+    for (int h = 0; h < H; h++) {
+      const unsigned past = rem[h] >= 4 ? 0u : 0xffffffffu << (8 * max(rem[h], 0));
+      rw[h] = (cur[h] & ~past) | (0x19191919u & past);
+      cur[h] = nxt[h];
+      if (active >> h & 1) nxt[h] = __ldg(words + wi[h]);
+      wi[h]++;
+    }
+#pragma unroll 1
+    for (int r = 0; r < 4; r++) {
+      unsigned m[W][C];
+      // match scores of both halves, interleaved into words
+#pragma unroll
+      for (int w = 0; w < W; w++) {
+        const uint2* ea = es + (int)(rw[2 * w] & 0xffu) * ROW4;
+        const uint2* eb = es + (int)(rw[2 * w + 1] & 0xffu) * ROW4;
+        rw[2 * w] >>= 8;
+        rw[2 * w + 1] >>= 8;
+#pragma unroll
+        for (int c4 = 0; c4 < NC4; c4++) {
+          const uint2 a = ea[c4 * G], b = eb[c4 * G];
+          m[w][4 * c4 + 0] = __byte_perm(a.x, b.x, 0x5410);
+          m[w][4 * c4 + 1] = __byte_perm(a.x, b.x, 0x7632);
+          m[w][4 * c4 + 2] = __byte_perm(a.y, b.y, 0x5410);
+          m[w][4 * c4 + 3] = __byte_perm(a.y, b.y, 0x7632);
+        }
+      }
+      // ---- M: max(pre, D[k-1] + t_dm, B + t_bm) + msc (dp.rs:167-169) ----
 #pragma unroll
       for (int c4 = 0; c4 < NC4; c4++) {
-        const uint2 a = ea[c4 * G], b = eb[c4 * G];
-        ew[4 * c4 + 0] = __byte_perm(a.x, b.x, 0x5410);
-        ew[4 * c4 + 1] = __byte_perm(a.x, b.x, 0x7632);
-        ew[4 * c4 + 2] = __byte_perm(a.y, b.y, 0x5410);
-        ew[4 * c4 + 3] = __byte_perm(a.y, b.y, 0x7632);
-      }
-    }
-    // ---- M: max(pre, D[k-1] + t_dm, B + t_bm) + msc (dp.rs:167-169) ----
-#pragma unroll
-    for (int c4 = 0; c4 < NC4; c4++) {
-      const uint4 tdm = T(2, c4), tbm = T(3, c4);
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const int c = 4 * c4 + e;
-        const unsigned dpv = c ? dp[c - 1] : dpl;
-        mp[c] = add2s16(max2s16(max2s16(pre[c], add2s16(dpv, pick(tdm, e))), add2s16(bw, pick(tbm, e))), ew[c]);
-      }
-    }
-    // ---- D chain (ascending; provisional carry into lanes other than the
-    // first), then the next row's pre and I (descending, in place) ----
-    const unsigned mcl0 = __shfl_up_sync(kFull, mp[C - 1], 1, G);
-    const unsigned ipl0 = __shfl_up_sync(kFull, ip[C - 1], 1, G);
-    const unsigned mcl = j ? mcl0 : kV16Init2, ipl = j ? ipl0 : kV16Init2;
-    {
-      unsigned d = j ? kV16Low2 : kV16Init2;
-#pragma unroll
-      for (int c4 = 0; c4 < NC4; c4++) {
-        const uint4 tmd = T(6, c4), tdd = T(7, c4);
+        const uint4 tdm = T(2, c4), tbm = T(3, c4);
 #pragma unroll
         for (int e = 0; e < 4; e++) {
           const int c = 4 * c4 + e;
-          const unsigned mcv = c ? mp[c - 1] : mcl;
-          d = max2s16(add2s16(mcv, pick(tmd, e)), add2s16(d, pick(tdd, e)));
-          dp[c] = d;
-        }
-      }
-    }
 #pragma unroll
-    for (int c4 = NC4 - 1; c4 >= 0; c4--) {
-      const uint4 tmm = T(0, c4), tim = T(1, c4), tmi = T(4, c4), tii = T(5, c4);
-#pragma unroll
-      for (int e = 3; e >= 0; e--) {
-        const int c = 4 * c4 + e;
-        const unsigned mpv = c ? mp[c - 1] : mcl, ipv = c ? ip[c - 1] : ipl;
-        pre[c] = max2s16(add2s16(mpv, pick(tmm, e)), add2s16(ipv, pick(tim, e)));
-        ip[c] = max2s16(add2s16(mp[c], pick(tmi, e)), add2s16(ip[c], pick(tii, e)));
-      }
-    }
-    // ---- carries across the group's lanes until nothing changes (exact:
-    // max-plus is monotone and the provisional carry is below every D) ----
-    bool settled = false;
-    for (int it = 0; it < G; it++) {
-      const unsigned c0 = __shfl_up_sync(kFull, dp[C - 1], 1, G);
-      unsigned cin = j ? c0 : kV16Init2;
-      const unsigned tdd0 = T(7, 0).x;
-      const bool need = max2s16(add2s16(cin, tdd0), dp[0]) != dp[0];
-      if (!__any_sync(kFull, need)) {
-        dpl = cin;
-        settled = true;
-        break;
-      }
-      bool go = true;
-#pragma unroll
-      for (int c4 = 0; c4 < NC4; c4++) {
-        if (go) {
-          const uint4 tdd = T(7, c4);
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const int c = 4 * c4 + e;
-            if (go) {
-              const unsigned nd = max2s16(dp[c], add2s16(cin, pick(tdd, e)));
-              if (nd == dp[c]) {
-                go = false;
-              } else {
-                dp[c] = nd;
-                cin = nd;
-              }
-            }
+          for (int w = 0; w < W; w++) {
+            const unsigned v = __viaddmax_s16x2(c ? dp[w][c - 1] : dpl[w], pick(tdm, e), pre[w][c]);
+            m[w][c] = add2s16(__viaddmax_s16x2(bw[w], pick(tbm, e), v), m[w][c]);
           }
         }
       }
-    }
-    if (!settled) {
-      const unsigned d0 = __shfl_up_sync(kFull, dp[C - 1], 1, G);
-      dpl = j ? d0 : kV16Init2;
-    }
-    // ---- row maximum over M (D never exceeds it), per half ----
-    unsigned tv[C];
+      // ---- D: every lane's chain without a carry, then from its neighbour's end ----
+      unsigned ml[W], il[W], cin[W];
 #pragma unroll
-    for (int c = 0; c < C; c++) tv[c] = mp[c];
-#pragma unroll
-    for (int span = 1; span < C; span <<= 1)
-#pragma unroll
-      for (int c = 0; c + span < C; c += 2 * span) tv[c] = max2s16(tv[c], tv[c + span]);
-    unsigned xe = tv[0];
-#pragma unroll
-    for (int o = G / 2; o >= 1; o >>= 1) xe = max2s16(xe, __shfl_xor_sync(kFull, xe, o, G));
-    // ---- special states per half (xC == xJ, as in the exact kernel) ----
-    int b16[2];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int eh = h ? ((int)xe >> 16) : (int)(short)(xe & 0xffffu);
-      big[h] |= eh > cap;
-      xj[h] = max(xj[h] + tl[h], eh * 2048 + nln2);
-      xn[h] += tl[h];
-      const int xb = max(xn[h], xj[h]) + tm[h];
-      b16[h] = max((xb + 2047) >> (kQ32Shift - kQ16Shift), kV16BFloor);
-      row[h]++;
-      if (row[h] == L[h]) fin[h] = xj[h] + tm[h];
-      if ((row[h] & 3) == 0) {
-        if (row[h] - boff[h] == 16) {
-          boff[h] += 16;
-          rc[h] = rn[h];
-          if (act[h]) rn[h] = __ldg(reinterpret_cast<const uint4*>(seq[h] + boff[h] + 16));
-        }
-        const int q = (row[h] - boff[h]) >> 2;
-        wc[h] = q == 0 ? rc[h].x : q == 1 ? rc[h].y : q == 2 ? rc[h].z : rc[h].w;
-      } else {
-        wc[h] >>= 8;
+      for (int w = 0; w < W; w++) {
+        ml[w] = __shfl_up_sync(kFull, m[w][C - 1], 1, G);
+        il[w] = __shfl_up_sync(kFull, ip[w][C - 1], 1, G);
+        if (j == 0) ml[w] = il[w] = kV16Init2;
+        cin[w] = j ? kV16Low2 : kV16Init2;
       }
+      bool again;
+      int it = 0;
+      do {
+        unsigned d[W];
+#pragma unroll
+        for (int w = 0; w < W; w++) d[w] = cin[w];
+#pragma unroll
+        for (int c4 = 0; c4 < NC4; c4++) {
+          const uint4 tmd = T(6, c4), tdd = T(7, c4);
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const int c = 4 * c4 + e;
+#pragma unroll
+            for (int w = 0; w < W; w++)
+              dp[w][c] = d[w] = __viaddmax_s16x2(d[w], pick(tdd, e), add2s16(c ? m[w][c - 1] : ml[w], pick(tmd, e)));
+          }
+        }
+        again = false;
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+          const unsigned up = __shfl_up_sync(kFull, d[w], 1, G);
+          const unsigned nc = j ? up : kV16Init2;
+          again |= nc != cin[w];
+          cin[w] = nc;
+        }
+      } while (__any_sync(kFull, again) && ++it < G);
+#pragma unroll
+      for (int w = 0; w < W; w++) dpl[w] = cin[w];
+      // ---- the next row's pre and I, in place ----
+#pragma unroll
+      for (int c4 = NC4 - 1; c4 >= 0; c4--) {
+        const uint4 tmm = T(0, c4), tim = T(1, c4), tmi = T(4, c4), tii = T(5, c4);
+#pragma unroll
+        for (int e = 3; e >= 0; e--) {
+          const int c = 4 * c4 + e;
+#pragma unroll
+          for (int w = 0; w < W; w++) {
+            pre[w][c] = __viaddmax_s16x2(c ? m[w][c - 1] : ml[w], pick(tmm, e), add2s16(c ? ip[w][c - 1] : il[w], pick(tim, e)));
+            ip[w][c] = __viaddmax_s16x2(m[w][c], pick(tmi, e), add2s16(ip[w][c], pick(tii, e)));
+          }
+        }
+      }
+      // ---- row maximum over M (D never exceeds it) of the lane's columns, J, base and B ----
+      bool raise = false;
+      unsigned xe[W];
+#pragma unroll
+      for (int w = 0; w < W; w++) {
+        unsigned a = max2s16(m[w][0], m[w][1]), b = max2s16(m[w][2], m[w][3]);
+#pragma unroll
+        for (int c = 4; c < C; c += 4) {
+          a = __vimax3_s16x2(a, m[w][c], m[w][c + 1]);
+          b = __vimax3_s16x2(b, m[w][c + 2], m[w][c + 3]);
+        }
+        xe[w] = max2s16(a, b);
+        jj[2 * w] = __viaddmax_s32(jj[2 * w], tl[2 * w], (int)(xe[w] << 16));
+        jj[2 * w + 1] = __viaddmax_s32(jj[2 * w + 1], tl[2 * w + 1], (int)(xe[w] & 0xffff0000u));
+        base[2 * w] += tl[2 * w];
+        base[2 * w + 1] += tl[2 * w + 1];
+        const unsigned limit = upper(base[2 * w] - nln2_25, base[2 * w + 1] - nln2_25);
+        raise |= max2s16(xe[w], limit) != limit;
+      }
+      if (__any_sync(kFull, raise)) {
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+          unsigned x = xe[w];
+#pragma unroll
+          for (int o = G / 2; o >= 1; o >>= 1) x = max2s16(x, __shfl_xor_sync(kFull, x, o, G));
+          if ((int)(short)(x & 0xffffu) > cap) big |= 1u << (2 * w);
+          if (((int)x >> 16) > cap) big |= 2u << (2 * w);
+          base[2 * w] = max(base[2 * w], (int)(x << 16) + nln2_25);
+          base[2 * w + 1] = max(base[2 * w + 1], (int)(x & 0xffff0000u) + nln2_25);
+        }
+      }
+#pragma unroll
+      for (int w = 0; w < W; w++) bw[w] = max2s16(upper(base[2 * w] + tk[2 * w], base[2 * w + 1] + tk[2 * w + 1]), kV16BFloor2);
     }
-    bw = __byte_perm((unsigned)b16[0], (unsigned)b16[1], 0x5410);
+#pragma unroll
+    for (int h = 0; h < H; h++) rem[h] -= done >> h & 1 ? 0 : 4;
   }
   // stats: one atomic per warp
   if (stats) {

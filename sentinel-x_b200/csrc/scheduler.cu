@@ -405,6 +405,10 @@ void launch_msv(sx_engine* E, Slot& S, Streams& X, const sx_profiles* P, const s
 // search costs 13 ms more, at 128 the ends of the tiles do (224, 211, 212 ms at
 // 16, 64, 128; a marker-set genome's 26 ms grow by 1 ms from 16 to 64).
 constexpr double kPackedWaves = 40;
+// Targets per lane group of a tile, at least (800 viral profiles 40.2 ms at 12,
+// 41.9 at 24; 296 profiles of M = 60 x 12,000 targets 9.3 without the limit,
+// 5.9 with it).
+constexpr int kGroupTargets = 12;
 std::vector<std::vector<sxk::PackedTile>> make_packed_tiles(const sx_engine* E, const sx_profiles* P,
                                                             const sx_targets* T, const std::vector<int>& prof) {
   std::vector<std::vector<sxk::PackedTile>> by_shape(kNumMsvShapes);
@@ -428,6 +432,7 @@ std::vector<std::vector<sxk::PackedTile>> make_packed_tiles(const sx_engine* E, 
   };
   for (const auto& pr : pairs) total += width(pr);
   const double share = total / (kPackedWaves * 2.0 * E->num_sms);  // width x targets' share of one tile
+  const int fill = (int)std::ceil(2.0 * E->num_sms / (double)std::max<size_t>(1, pairs.size()));
   std::unordered_map<int, std::vector<int>> cuts;  // by slice count: boundaries with about equal residues
   auto cuts_for = [&](int n) -> const std::vector<int>& {
     std::vector<int>& cut = cuts[n];
@@ -444,7 +449,12 @@ std::vector<std::vector<sxk::PackedTile>> make_packed_tiles(const sx_engine* E, 
     return cut;
   };
   for (const auto& pr : pairs) {
-    const int n = std::max(1, std::min((int)std::ceil(width(pr) / share), std::max(1, nt / 32)));
+    // a tile gives each of its lane groups kGroupTargets or more, or its end
+    // would be mostly idle groups; few pairs are cut finer, down to 32 targets,
+    // until they fill the GPU
+    const int groups = 256 / kMsvShapes[P->msv_shape[pr.first]].g;
+    const int most = std::max({1, nt / (kGroupTargets * groups), std::min(nt / 32, fill)});
+    const int n = std::max(1, std::min((int)std::ceil(width(pr) / share), most));
     const std::vector<int>& cut = cuts_for(n);
     for (int s = 0; s < n; s++)
       if (cut[s + 1] > cut[s]) by_shape[P->msv_shape[pr.first]].push_back({pr.first, pr.second, cut[s], cut[s + 1]});
@@ -585,11 +595,12 @@ void launch_stage(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets*
 
 // Packed Viterbi pre-screen of a block's bias-filter survivors (profiles
 // `prof`, per-profile lists in `vs`, `count[p - p0]` pairs in each): a
-// profile's list is cut into strided sub-tiles of about 24 rounds of the
-// pairs a CTA holds at once (with 6 a CTA's slot idles behind its longest
-// target too often: 69 ms against 59), larger M first, one launch per shape on the
-// slot's high-priority auxiliary streams; pairs whose bound passes F2 go to
-// the Viterbi lists (lists[1]), S.vstats collects cells and passes.
+// profile's list is cut into strided sub-tiles of about 8 rounds of the pairs a
+// CTA holds at once (with the longest targets of a tile first, 4 to 24 rounds
+// differ by 3% on the Pfam-scale search; a marker-set genome, whose lists are
+// short, takes 6.1 ms at 8 and 7.2 at 24), larger M first, one launch per shape
+// on the slot's high-priority auxiliary streams; pairs whose bound passes F2 go
+// to the Viterbi lists (lists[1]), S.vstats collects cells and passes.
 void launch_vprescreen(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T, const std::vector<int>& prof,
                        const VitScreen& vs, const std::vector<unsigned>& count) {
   const auto& K = kernels();
@@ -600,7 +611,7 @@ void launch_vprescreen(sx_engine* E, Slot& S, const sx_profiles* P, const sx_tar
     const unsigned n = std::min(count[pi - vs.p0], vs.cap);
     if (!n) continue;
     const Vit16Shape& v = kVit16Shapes[P->dp[pi].qv_shape];
-    const unsigned per = 24u * (unsigned)(vit16_threads(v) / 32) * (unsigned)(32 / v.g) * 2u;  // pairs per sub-tile
+    const unsigned per = 8u * (unsigned)(vit16_threads(v) / 32) * (unsigned)(32 / v.g) * 2u * (unsigned)v.w;  // pairs per sub-tile
     const int nsub = (int)std::min<unsigned>(256u, (n + per - 1) / per);
     for (int q = 0; q < nsub; q++) by_shape[P->dp[pi].qv_shape].push_back({pi, q, nsub, 0});
   }

@@ -239,7 +239,8 @@ int sx_score_prescreens(sx_engine* e, const sx_profiles* p, const sx_targets* t,
       // launch per profile (its list at p0 = the profile, count at index 0)
       std::vector<std::vector<int32_t>> byp(np);
       for (size_t i = 0; i < npairs; i++)
-        if (p->dp[pair_profile[i]].qv_shape >= 0) byp[pair_profile[i]].push_back((int32_t)i);
+        if (p->dp[pair_profile[i]].qv_shape >= 0 && p->h[pair_profile[i]].m <= kVit16BoundM)
+          byp[pair_profile[i]].push_back((int32_t)i);
       std::vector<PairRec> recs;
       std::vector<int64_t> seg;
       std::vector<int> profs;

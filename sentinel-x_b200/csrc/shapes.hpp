@@ -57,22 +57,20 @@ constexpr int kNumVitShapes = sizeof(kVitShapes) / sizeof(kVitShapes[0]);
 constexpr int kMaxBins = 32;  // survivor lists per stage (vbins or Viterbi shapes)
 static_assert(kNumVitShapes <= kMaxBins, "too many Viterbi shapes");
 
-// Packed Viterbi pre-screen shapes (prescreen.cuh vit16_kernel): G lanes per
-// pair of targets, C columns per lane; a profile takes the narrowest that
-// covers M, profiles wider than the last one are not pre-screened.  Above 64
-// columns 16 columns a lane beat 8 (Viterbi pre-screen of the Pfam-scale
-// search 65 -> 59 ms): the row's per-lane overhead is shared by twice the
-// cells, at 163 registers and three 128-thread CTAs per SM.
+// Packed Viterbi pre-screen shapes (prescreen.cuh vit16_kernel): G lanes hold C
+// columns each of 2 W targets; a profile takes the narrowest that covers M,
+// profiles wider than the last one are not pre-screened.
 struct Vit16Shape {
-  int g, c;
+  int g, c, w;
 };
-constexpr Vit16Shape kVit16Shapes[] = {{4, 8}, {8, 8}, {8, 16}, {16, 16}, {32, 16}};
+constexpr Vit16Shape kVit16Shapes[] = {{4, 8, 2}, {8, 8, 2}, {16, 8, 2}, {32, 8, 2}, {32, 16, 2}, {32, 32, 1}, {32, 48, 1}};
 constexpr int kNumVit16Shapes = sizeof(kVit16Shapes) / sizeof(kVit16Shapes[0]);
+constexpr int kVit16BoundM = 512;  // sx_score_prescreens reports bounds up to here
 // dynamic shared memory of one tile: 8 transition rows of 4 bytes per column
-// and 25 score rows of 2 bytes per column
-constexpr int vit16_smem(const Vit16Shape& v) { return 82 * v.g * v.c; }
-// threads per CTA: the kernel's launch bounds give 128 registers a thread
-// for C <= 8 (four 128-thread CTAs per SM), 168 for C = 16 (three)
+// and kV16Rows score rows of 2 bytes per column
+constexpr int vit16_smem(const Vit16Shape& v) { return (32 + 2 * sxk::kV16Rows) * v.g * v.c; }
+// threads per CTA: the kernel's launch bounds give 168 registers a thread for
+// up to 16 words of columns (three CTAs per SM), 255 above (two)
 constexpr int vit16_threads(const Vit16Shape&) { return 128; }
 
 // Warp-chunked column counts (columns per lane, 32 lanes per pair).

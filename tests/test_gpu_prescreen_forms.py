@@ -1,4 +1,4 @@
-"""The packed MSV pre-screen's decisions over the forms it has: tiles that
+"""The packed pre-screens' decisions over the forms they have: tiles that
 follow J and tiles that do not (F1 up to 1), lane widths at their edges,
 profile pairs with and without a second profile, targets of every length
 modulo the block of four, without any scoring residue, and repeated homologs
@@ -12,7 +12,7 @@ from sxhmm import synth
 
 pytestmark = pytest.mark.gpu
 
-MS = (1, 5, 32, 33, 64, 100, 129, 208, 256, 300, 513, 1025, 1601)
+MS = (1, 5, 32, 33, 64, 100, 129, 208, 256, 300, 513, 1024, 1025, 1536, 1601)
 
 
 def _workload():
