@@ -42,6 +42,7 @@ using sxk::Thresholds;
 namespace sxk {
 struct LongPair;
 struct PlainProfile;
+struct AdjPair;
 }  // namespace sxk
 
 namespace sxe {
@@ -534,8 +535,9 @@ struct sx_engine {
   DevBuf<float> scores;
   DevBuf<int32_t> slots, plist;
   DevBuf<sxk::AdjPair> adj_pairs;
-  DevBuf<float> adj_f, adj_out;
+  DevBuf<float> adj_f, adj_acc, adj_out;
   PinnedBuf<float> adj_host;  // staging of the adjoint's counts on their way to the caller
+  PinnedBuf<double> adj_lnz_host;
   DevBuf<double> adj_d, adj_lnz;
 };
 

@@ -1,5 +1,5 @@
 // Instantiations of the warp-chunked kernels (warp-per-pair Viterbi, the
-// Forward pre-screen, the adjoint passes), one per column width.
+// Forward pre-screen), one per column width.
 #include "shapes.hpp"
 
 namespace sx {
@@ -9,8 +9,6 @@ struct VbinTable {
   static void fill(KernelTables& t) {
     t.vit[I] = sxk::viterbi_kernel<kVcBins[I]>;
     t.fwd_scan[I] = sxk::forward_scan_kernel<kVcBins[I]>;
-    t.adjf[I] = sxk::adjoint_forward_kernel<kVcBins[I]>;
-    t.adjb[I] = sxk::adjoint_backward_kernel<kVcBins[I]>;
     VbinTable<I + 1>::fill(t);
   }
 };

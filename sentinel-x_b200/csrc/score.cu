@@ -1,5 +1,6 @@
 // C ABI: stage scores, pre-screen bounds and the adjoint for explicit pairs.
 #include "engine.hpp"
+#include "adjoint.cuh"
 #include "long.cuh"
 
 extern "C" {
@@ -329,6 +330,14 @@ int sx_score_prescreens(sx_engine* e, const sx_profiles* p, const sx_targets* t,
   return SX_OK;
 }
 
+// Parts of one adjoint call: at least kAdjPart pairs (fewer do not fill the
+// GPU), at most kAdjMaxParts (one event each), their kernels on kAdjStreams
+// streams -- on one the parts' last warps run alone, on many all parts end late
+// and no copy starts early.  4,096 pairs of M = 300, by streams 1, 2, 4, 8: 28,
+// 20, 17, 21 ms in eight parts; 26 ms in one part.
+static constexpr int kAdjPart = 512, kAdjMaxParts = 8, kAdjStreams = 4;
+static_assert(kAdjMaxParts <= 8 && kAdjStreams <= Streams::kAux, "events and streams of the engine's first slot");
+
 int sx_posterior_grad(sx_engine* e, const sx_profiles* p, const sx_targets* t, const int32_t* pair_profile,
                       const int32_t* pair_target, size_t npairs, int32_t m, float* d_msc, float* d_isc,
                       float* d_trans, double* lnz) {
@@ -352,21 +361,25 @@ int sx_posterior_grad(sx_engine* e, const sx_profiles* p, const sx_targets* t, c
   try {
     CK(cudaSetDevice(e->device));
     cudaStream_t s = e->stream;
-    const int vb = p->dp[pair_profile[0]].vbin, VC = kVcBins[vb];
-    const auto& K = kernels();
+    const int nw = sxk::adj_warps(m), tw = 32 * sxk::kAdjC * nw, width = xwidth(p->dp[pair_profile[0]].xshape);
     const int64_t budget = scratch_budget(e, std::max<int64_t>(e->batch_bytes, 64LL << 20));
+    const int64_t rowf = 3LL * tw, accf = (int64_t)sxk::kAdjEmRows * tw;
+    // a CTA per pair, or four one-warp teams to one
+    const int threads = nw > 1 ? 32 * nw : 128, per_cta = nw > 1 ? 1 : 4;
+    const auto fwd = nw > 1 ? sxk::adjoint_forward_kernel<true> : sxk::adjoint_forward_kernel<false>;
+    const auto bwd = nw > 1 ? sxk::adjoint_backward_kernel<true> : sxk::adjoint_backward_kernel<false>;
     size_t i0 = 0;
     while (i0 < npairs) {
-      // chunk: scratch floats per pair ~ (L/S + S + 2) * 3 * 32 * VC + 6 (L+1) + out, doubles (L+1)
+      // chunk: scratch floats per pair ~ (L/S + S + 2) * 3 * tw + 6 (L+1) + accumulators + out, doubles (L+1)
       std::vector<sxk::AdjPair> ap;
       int64_t fo = 0, dd = 0;
       size_t i1 = i0;
       while (i1 < npairs) {
         const int64_t L = t->len[pair_target[i1]];
         const int S = std::max<int>(1, (int)std::ceil(std::sqrt((double)std::max<int64_t>(L, 1))));
-        const int64_t rowf = 3LL * 32 * VC;
-        const int64_t need_f = (L / S + 1) * rowf + (S + 1) * rowf + 6 * (L + 1);
-        if (i1 > i0 && (fo + need_f + (int64_t)(i1 - i0 + 1) * (int64_t)out_per) * 4 + (dd + L + 1) * 8 > budget)
+        // a multiple of 4: the rows are read and written as float4
+        const int64_t need_f = (L / S + 1) * rowf + (S + 1) * rowf + ((6 * (L + 1) + 3) & ~(int64_t)3);
+        if (i1 > i0 && (fo + need_f + (int64_t)(i1 - i0 + 1) * ((int64_t)out_per + accf)) * 4 + (dd + L + 1) * 8 > budget)
           break;
         sxk::AdjPair a{};
         a.p = pair_profile[i1];
@@ -375,9 +388,10 @@ int sx_posterior_grad(sx_engine* e, const sx_profiles* p, const sx_targets* t, c
         a.ck_off = fo;
         a.seg_off = a.ck_off + (L / S + 1) * rowf;
         a.sp_off = a.seg_off + (S + 1) * rowf;
+        a.acc_off = (int64_t)(i1 - i0) * accf;
         a.out_off = (int64_t)(i1 - i0) * (int64_t)out_per;  // outputs packed per pair in their own buffer
         a.ls_off = dd;
-        fo = a.sp_off + 6 * (L + 1);
+        fo = a.ck_off + need_f;
         dd += L + 1;
         ap.push_back(a);
         i1++;
@@ -385,30 +399,58 @@ int sx_posterior_grad(sx_engine* e, const sx_profiles* p, const sx_targets* t, c
       const int n = (int)ap.size();
       e->adj_pairs.upload(ap.data(), ap.size(), s);
       e->adj_f.alloc((size_t)fo);
+      e->adj_acc.alloc((size_t)(n * accf));
       e->adj_out.alloc((size_t)n * out_per);
       e->adj_d.alloc((size_t)std::max<int64_t>(dd, 1));
       e->adj_lnz.alloc((size_t)n);
-      CK(cudaMemsetAsync(e->adj_out.p, 0, sizeof(float) * out_per * (size_t)n, s));
-      const int blocks = std::max(1, std::min((n + 3) / 4, e->num_sms * 32));
-      K.adjf[vb]<<<blocks, 128, 0, s>>>(e->adj_pairs.p, n, p->d_prof.p, p->d_vfb.p, t->d_res.p, t->d_off.p,
-                                        t->d_len.p, t->d_xsc.p, e->adj_f.p, e->adj_d.p, e->adj_lnz.p);
-      K.adjb[vb]<<<blocks, 128, 0, s>>>(e->adj_pairs.p, n, p->d_prof.p, p->d_vfb.p, t->d_res.p, t->d_off.p,
-                                        t->d_len.p, t->d_xsc.p, e->adj_f.p, e->adj_d.p, e->adj_lnz.p, e->adj_out.p);
-      CK(cudaGetLastError());
-      // scatter the packed [25W | 25W | 8W] outputs straight into the caller's three arrays
-      // one copy into page-locked staging, then the host threads split the
-      // counts into the caller's three arrays (and fault in their pages)
       e->adj_host.alloc(out_per * (size_t)n);
-      CK(cudaMemcpyAsync(e->adj_host.p, e->adj_out.p, sizeof(float) * out_per * (size_t)n, cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(lnz + i0, e->adj_lnz.p, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, s));
+      // Parts of the chunk: a part's kernels run while the part before it is
+      // copied into page-locked staging and the host threads split the one
+      // before that into the caller's three arrays (and fault in their pages).
+      const int parts = std::max(1, std::min(n / kAdjPart, kAdjMaxParts));
+      std::vector<int> at(parts + 1);
+      for (int q = 0; q <= parts; q++) at[q] = (int)((int64_t)n * q / parts);
+      fork_aux(e->sl[0].hi);
+      for (int q = 0; q < parts; q++) {
+        const int a = at[q], m2 = at[q + 1] - a;
+        cudaStream_t x = e->aux[q % kAdjStreams];
+        const sxk::AdjPair* pr = e->adj_pairs.p + a;
+        CK(cudaMemsetAsync(e->adj_acc.p + a * accf, 0, sizeof(float) * (size_t)(m2 * accf), x));
+        const int blocks = (m2 + per_cta - 1) / per_cta;
+        fwd<<<blocks, threads, 0, x>>>(pr, m2, p->d_prof.p, p->d_x.p, width, t->d_res.p, t->d_off.p, t->d_len.p,
+                                       t->d_xsc.p, e->adj_f.p, e->adj_d.p, e->adj_lnz.p + a);
+        bwd<<<blocks, threads, 0, x>>>(pr, m2, p->d_prof.p, p->d_x.p, width, t->d_res.p, t->d_off.p, t->d_len.p,
+                                       t->d_xsc.p, e->adj_f.p, e->adj_d.p, e->adj_lnz.p + a, e->adj_acc.p, e->adj_out.p);
+        for (int b = 0; b < m2; b += 32768) {  // grid.y limit
+          const int nb = std::min(32768, m2 - b);
+          sxk::adjoint_out_kernel<<<dim3((unsigned)std::max(1, (sxk::kAdjEmRows * W + 2047) / 2048), (unsigned)nb), 256, 0, x>>>(
+              pr + b, m, tw, e->adj_acc.p, e->adj_out.p);
+        }
+        CK(cudaGetLastError());
+        // copies one after another on the main stream, in part order
+        CK(cudaEventRecord(e->join_ev[q % kAdjStreams], x));
+        CK(cudaStreamWaitEvent(s, e->join_ev[q % kAdjStreams], 0));
+        CK(cudaMemcpyAsync(e->adj_host.p + a * out_per, e->adj_out.p + a * out_per, sizeof(float) * out_per * (size_t)m2,
+                           cudaMemcpyDeviceToHost, s));
+        CK(cudaEventRecord(e->ev[q], s));
+      }
+      // lnZ too through page-locked memory: a copy into the caller's pageable
+      // array would hold this thread until every part is done
+      e->adj_lnz_host.alloc((size_t)n);
+      CK(cudaMemcpyAsync(e->adj_lnz_host.p, e->adj_lnz.p, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost, s));
+      for (int q = 0; q < parts; q++) {
+        CK(cudaEventSynchronize(e->ev[q]));
+        const float* hs = e->adj_host.p + at[q] * out_per;
+        parallel_for((size_t)(at[q + 1] - at[q]), e->host_threads, [&](size_t y) {
+          const size_t z = i0 + (size_t)at[q] + y;
+          const float* src = hs + y * out_per;
+          memcpy(d_msc + z * 25 * W, src, sizeof(float) * 25 * W);
+          memcpy(d_isc + z * 25 * W, src + 25 * W, sizeof(float) * 25 * W);
+          memcpy(d_trans + z * 8 * W, src + 50 * W, sizeof(float) * 8 * W);
+        });
+      }
       CK(cudaStreamSynchronize(s));
-      const float* hs = e->adj_host.p;
-      parallel_for((size_t)n, e->host_threads, [&](size_t q) {
-        const float* src = hs + q * out_per;
-        memcpy(d_msc + (i0 + q) * 25 * W, src, sizeof(float) * 25 * W);
-        memcpy(d_isc + (i0 + q) * 25 * W, src + 25 * W, sizeof(float) * 25 * W);
-        memcpy(d_trans + (i0 + q) * 8 * W, src + 50 * W, sizeof(float) * 8 * W);
-      });
+      memcpy(lnz + i0, e->adj_lnz_host.p, sizeof(double) * (size_t)n);
       i0 = i1;
     }
   } catch (const CudaError& ce) {

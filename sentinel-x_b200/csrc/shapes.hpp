@@ -8,7 +8,6 @@
 #include <cstdint>
 
 #include "kernels.cuh"
-#include "adjoint.cuh"
 #include "envelope.cuh"
 #include "exact_rows.cuh"
 #include "wide.cuh"
@@ -118,10 +117,6 @@ typedef void (*FwdFn)(const PairRec*, const unsigned*, const BinRegion*, int, Pa
                       const int32_t*, const float4*, float);
 typedef void (*XRowsFn)(const sxk::RowRec*, int, const DevProfile*, const float*, const uint8_t*, const int64_t*,
                         const int32_t*, const float4*, float*);
-typedef void (*AdjFFn)(const sxk::AdjPair*, int, const DevProfile*, const float*, const uint8_t*, const int64_t*,
-                       const int32_t*, const float4*, float*, double*, double*);
-typedef void (*AdjBFn)(const sxk::AdjPair*, int, const DevProfile*, const float*, const uint8_t*, const int64_t*,
-                       const int32_t*, const float4*, float*, const double*, const double*, float*);
 typedef void (*EnvRowsFn)(const sxk::EnvRec*, int, const DevProfile*, const float*, const uint8_t*, const int64_t*,
                           float*, float*);
 typedef void (*EnvOaFn)(const sxk::EnvRec*, int, const DevProfile*, const float*, float*, float*, const double*,
@@ -140,8 +135,6 @@ struct KernelTables {
   FwdFn fwd_scan[kNumVbins];  // the F3 pre-screen
   XRowsFn xrows[kNumXShapes];  // exact Forward and Backward rows
   WideFn wmsv[kNumXShapes], wvit[kNumXShapes];  // M > kMaxM: MSV and Viterbi scores (nullptr for narrow shapes)
-  AdjFFn adjf[kNumVbins];
-  AdjBFn adjb[kNumVbins];
   VitGFn vitg[kNumVitShapes];
   Vit16Fn vit16[kNumVit16Shapes];  // the packed Viterbi pre-screen
 };
