@@ -62,6 +62,11 @@ __global__ void __launch_bounds__(team_threads(IN)) env_rows_kernel(const EnvRec
                                                        float* __restrict__ rows) {
   extern __shared__ float4 sm_row[];
   __shared__ XShared sh;
+  XSumShared* ss = nullptr;
+  if constexpr (MULTI) {
+    __shared__ XSumShared sum_sh;
+    ss = &sum_sh;
+  }
   const int w = MULTI ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= n) return;  // uniform over the team
   float* T = reinterpret_cast<float*>(sm_row) + (MULTI ? 0 : (threadIdx.x >> 5) * 32 * C);
@@ -72,12 +77,12 @@ __global__ void __launch_bounds__(team_threads(IN)) env_rows_kernel(const EnvRec
   float* pl = planes + r.plane_off;
   float* orow = rows + r.row_off;
   if constexpr (DIAG) {
-    exact_forward<C, MULTI, IN, kKeepDiag>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move, orow, pl, T, sh);
+    exact_forward<C, MULTI, IN, kKeepDiag>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move, orow, pl, T, sh, ss);
   } else if (blockIdx.y == 0) {
-    exact_forward<C, MULTI, IN, kKeepMI>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move, orow, pl, T, sh);
+    exact_forward<C, MULTI, IN, kKeepMI>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move, orow, pl, T, sh, ss);
   } else {
     exact_backward<C, MULTI, IN, kKeepMI>(img, M, s, r.lr, r.ploop, r.pmove, r.pe_loop, r.pe_move,
-                                      orow + 6 * (int64_t)(r.lr + 1), pl + 2 * (int64_t)(r.lr + 1) * r.width, T, sh);
+                                      orow + 6 * (int64_t)(r.lr + 1), pl + 2 * (int64_t)(r.lr + 1) * r.width, T, sh, ss);
   }
 }
 

@@ -8,9 +8,12 @@
 // bounds a pass is the latency of one row, because the B state of a row needs
 // the row's E (Forward) or B (Backward) sum, a sum the reference takes in
 // column order.  Three parts of a row are sequential in the reference:
-//   * the row sum.  It stays sequential, but as one chain of adds over a row
-//     laid out in shared memory (4 cycles a term, loads 16 terms ahead),
-//     not as a baton handed from lane to lane;
+//   * the row sum.  Up to 512 columns it stays sequential, but as one chain of
+//     adds over a row laid out in shared memory (4 cycles a term, loads 16
+//     terms ahead), not as a baton handed from lane to lane.  Above, most of it
+//     runs in parallel (team_sum_wide): while the running sum stays within one
+//     binade an add changes it by the term rounded to the sum's ulp, whatever
+//     the sum, except that a tie goes by the parity of its last bit;
 //   * the D chain D[k] = a_k + p_k D[k-1].  Every lane runs its own columns
 //     at once from a guessed carry, then takes the carry its left neighbour
 //     computed and runs them again until no lane's carry changes.  A state
@@ -56,6 +59,13 @@ constexpr int kXMaxWarps = 16;
 struct RowRec {
   int32_t p, t;
   int64_t row_off;
+};
+
+// team_sum_wide's exchange, by warp and by thread.
+struct XSumShared {
+  float total[kXMaxWarps];
+  unsigned odd[kXMaxWarps];        // threads that need their exact start
+  int inc[2][32 * kXMaxWarps];     // at the last thread of each run: what the run adds to an even / odd sum
 };
 
 struct XShared {  // exchange between the warps of a team
@@ -184,6 +194,108 @@ __device__ __forceinline__ float team_sum(const float* t, int n, XShared& sh) {
   }
 }
 
+// The team's sum of every thread's terms t[0..C), in thread order, bit for bit
+// as one chain of adds from 0 would give it; T holds the terms (written by the
+// caller, ordered by this function's barriers).
+// An approximate prefix sum tells each thread the binades of the running sum at
+// its first and after its last term, with a margin (2^-10) well above the
+// difference between any two orders of adding 8192 non-negative terms.  Where
+// both are one binade, the thread's effect on the sum's bit pattern is an
+// integer that depends on the last bit of the sum alone: it runs its chain from
+// the binade's first even and first odd value and takes the differences.  These
+// compose across the lanes of a run of such threads in a scan.  The other
+// threads, a dozen a row where the sum crosses a power of two (in the subnormal
+// range there is one "binade", without rounding), are walked in order: the run
+// before the thread, an integer, then the thread's own chain of C adds.
+// A sum that is infinite or not a number is walked too.
+// Measured at M = 1,500 (12 warps): the row passes of 1,800 targets 6.64 ->
+// 4.57 ms, their envelope matrices 7.47 -> 5.32 ms; at M = 500 (4 warps) 3.29 ->
+// 2.90 and 3.65 -> 2.95 ms.
+template <int C>
+__device__ __forceinline__ float team_sum_wide(const float (&t)[C], const float* T, XShared& sh, XSumShared& ss) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  float own = t[0];
+#pragma unroll
+  for (int c = 1; c < C; c++) own = fadd(own, t[c]);
+  float inc = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float v = __shfl_up_sync(kFull, inc, o);
+    if (lane >= o) inc = fadd(inc, v);
+  }
+  if (lane == 31) ss.total[warp] = inc;
+  __syncthreads();
+  float before = 0.f;
+  for (int q = 0; q < warp; q++) before = fadd(before, ss.total[q]);
+  const float up = __shfl_up_sync(kFull, inc, 1);
+  const float first = fadd(before, lane ? up : 0.f), last = fadd(before, inc);
+  const int e0 = __float_as_int(fmul(first, 0.9990234375f)) >> 23, e1 = __float_as_int(fmul(last, 1.0009765625f)) >> 23;
+  const bool odd = e0 != e1 || (unsigned)e1 >= 255u;
+  const unsigned om = __ballot_sync(kFull, odd);
+  int n0 = 0, n1 = 0;
+  {
+    const int s0 = e0 << 23, s1 = s0 + 1;
+    float a = __int_as_float(s0), b = __int_as_float(s1);
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      a = fadd(a, t[c]);
+      b = fadd(b, t[c]);
+    }
+    n0 = __float_as_int(a) - s0;
+    n1 = __float_as_int(b) - s1;
+  }
+  const unsigned upto = om & ((2u << lane) - 1u);
+  const int head = upto ? 32 - __clz(upto) : 0;  // first lane of this lane's run
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {  // earlier lanes' effect, then this one's
+    const int p0 = __shfl_up_sync(kFull, n0, o), p1 = __shfl_up_sync(kFull, n1, o);
+    if (lane - o >= head) {
+      const int m0 = p0 + (p0 & 1 ? n1 : n0), m1 = p1 + (p1 & 1 ? n0 : n1);
+      n0 = m0;
+      n1 = m1;
+    }
+  }
+  ss.inc[0][threadIdx.x] = n0;
+  ss.inc[1][threadIdx.x] = n1;
+  if (lane == 0) ss.odd[warp] = om;
+  __syncthreads();
+  if (warp == 0) {
+    int s = 0;  // the sum's bits
+    for (int q = 0; q < nw; q++) {
+      unsigned m = ss.odd[q];
+      int at = 0;
+      while (m) {
+        const int jn = __ffs(m) - 1, id = 32 * q + jn;
+        m &= m - 1;
+        const float4* p = reinterpret_cast<const float4*>(T + id * C);
+        float4 x[C / 4];
+#pragma unroll
+        for (int u = 0; u < C / 4; u++) x[u] = p[u];
+        if (jn > at) s += ss.inc[s & 1][id - 1];
+        float v = __int_as_float(s);
+#pragma unroll
+        for (int u = 0; u < C / 4; u++) v = fadd(fadd(fadd(fadd(v, x[u].x), x[u].y), x[u].z), x[u].w);
+        s = __float_as_int(v);
+        at = jn + 1;
+      }
+      if (at < 32) s += ss.inc[s & 1][32 * q + 31];
+    }
+    if (lane == 0) sh.sum = __int_as_float(s);
+  }
+  __syncthreads();
+  return sh.sum;
+}
+// Teams from kWideSumWarps on take it: about 1,800 cycles at six warps, the chain
+// 4 a column.
+constexpr int kWideSumWarps = 3;
+template <int C, bool MULTI>
+__device__ __forceinline__ float row_sum(const float (&t)[C], const float* T, int n, XShared& sh, XSumShared* ss) {
+  if constexpr (MULTI) {
+    if ((blockDim.x >> 5) >= kWideSumWarps) return team_sum_wide<C>(t, T, sh, *ss);
+  }
+  return team_sum<MULTI>(T, n, sh);
+}
+
 // Products of the lanes' p_dd for the guess scan: after the call bs[s] is the
 // product over the 2^s lanes that end at this one (UP: ascending lanes) and
 // `all` the product up to and including this lane; returns the number of scan
@@ -267,7 +379,7 @@ __host__ __device__ __forceinline__ int64_t diag_plane(int64_t lr, int M) { retu
 template <int C, bool MULTI, TransIn IN, Keep KEEP>
 __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int M, const uint8_t* __restrict__ s, int L,
                                               float ploop, float pmove, float pe_loop, float pe_move, float* orow,
-                                              float* planes, float* T, XShared& sh) {
+                                              float* planes, float* T, XShared& sh, XSumShared* ss) {
   const int lane = threadIdx.x & 31;
   const int warp = MULTI ? threadIdx.x >> 5 : 0;
   const int width = (MULTI ? blockDim.x : 32) * C;
@@ -350,8 +462,8 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
         if (lane == 31 && !same_bits(end, own)) sh.flag = 1;
       }
     }
+    float t[C];
     auto publish = [&]() {
-      float t[C];
 #pragma unroll
       for (int c = 0; c < C; c++) t[c] = fadd(mv[c], dv[c]);
       store_cols<C>(T + k0, t);
@@ -377,7 +489,7 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
         publish();
       }
     }
-    float xe = team_sum<MULTI>(T, nsum, sh);
+    float xe = row_sum<C, MULTI>(t, T, nsum, sh, ss);
     if (MULTI && lead) sh.flag = 0;  // read by all before the sum's barrier, set again after the next row's
     if (MULTI && lane == 0 && warp) {
       lm = sh.prev[0][warp - 1];
@@ -443,7 +555,7 @@ __device__ __forceinline__ void exact_forward(const float* __restrict__ img, int
 template <int C, bool MULTI, TransIn IN, Keep KEEP>
 __device__ __forceinline__ void exact_backward(const float* __restrict__ img, int M, const uint8_t* __restrict__ s,
                                                int L, float ploop, float pmove, float pe_loop, float pe_move,
-                                               float* orow, float* planes, float* T, XShared& sh) {
+                                               float* orow, float* planes, float* T, XShared& sh, XSumShared* ss) {
   static_assert(KEEP != kKeepDiag, "only the Forward matrix is kept in the diagonal layout");
   const int lane = threadIdx.x & 31;
   const int warp = MULTI ? threadIdx.x >> 5 : 0;
@@ -545,8 +657,8 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
   }
   // B sum of row i from M(i+1) and the odds of residue i+1; leaves M(i+1) e in me
   float me[C];
+  float bt[C];
   auto b_terms = [&](const float (&eo)[C]) {
-    float bt[C];
     const auto bm = tr.row(7);
 #pragma unroll
     for (int c = 0; c < C; c++) {
@@ -568,7 +680,7 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
     b_terms(eo);
     float me_up = __shfl_down_sync(kFull, me[0], 1);
     if (lane == 31) me_up = MULTI && warp + 1 < nw ? sh.mv[warp + 1] : 0.f;
-    const float xb = team_sum<MULTI>(T, nsum, sh);
+    const float xb = row_sum<C, MULTI>(bt, T, nsum, sh, ss);
     xj = fadd(fmul(xj, ploop), fmul(xb, pmove));
     xc = fmul(xc, ploop);
     xe = fadd(fmul(xj, pe_loop), fmul(xc, pe_move));
@@ -642,7 +754,7 @@ __device__ __forceinline__ void exact_backward(const float* __restrict__ img, in
   }
   // row 0: the B sum with residue 1
   b_terms(eo);
-  const float b0 = team_sum<MULTI>(T, nsum, sh);
+  const float b0 = row_sum<C, MULTI>(bt, T, nsum, sh, ss);
   if (lead) orow[1] = b0;
 }
 
@@ -662,6 +774,11 @@ __global__ void __launch_bounds__(team_threads(IN)) exact_rows_kernel(const RowR
                                                          const float4* __restrict__ xsc, float* __restrict__ rows) {
   extern __shared__ float4 sm_row[];
   __shared__ XShared sh;
+  XSumShared* ss = nullptr;
+  if constexpr (MULTI) {
+    __shared__ XSumShared sum_sh;
+    ss = &sum_sh;
+  }
   const int w = MULTI ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= n) return;  // uniform over the team
   float* T = reinterpret_cast<float*>(sm_row) + (MULTI ? 0 : (threadIdx.x >> 5) * 32 * C);
@@ -672,10 +789,10 @@ __global__ void __launch_bounds__(team_threads(IN)) exact_rows_kernel(const RowR
   const uint8_t* s = res + toff[r.t];
   const float4 xs = xsc[r.t];
   if (blockIdx.y == 0)
-    exact_forward<C, MULTI, IN, kKeepNone>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off, nullptr, T, sh);
+    exact_forward<C, MULTI, IN, kKeepNone>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off, nullptr, T, sh, ss);
   else
     exact_backward<C, MULTI, IN, kKeepNone>(img, M, s, L, xs.z, xs.w, 0.5f, 0.5f, rows + r.row_off + 6 * (int64_t)(L + 1),
-                                        nullptr, T, sh);
+                                        nullptr, T, sh, ss);
 }
 
 }  // namespace sxk
