@@ -157,7 +157,7 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
     CK(cudaStreamSynchronize(s));
     if (plog) plog->add("env_fb_pass", tb0);
     const auto tb1 = std::chrono::steady_clock::now();
-    parallel_for(n, nthr, [&](size_t x) {
+    E->pool->run(n, nthr, [&](size_t x) {
       const sxk::EnvRec& r = recs[x];
       const auto& it = items[order[a + x]];
       srcs[it.first].db->factors(it.second, hrows.data() + r.row_off,
@@ -359,7 +359,7 @@ RegionPassStats region_passes(sx_engine* E, const sx_profiles* P, const sx_targe
       per[(size_t)o[0]].push_back({o[1], (int64_t)o[2], (int64_t)o[3], o[4], o[5]});
     }
     std::atomic<int64_t> redone{0};
-    parallel_for(n, nthr, [&](size_t x) {
+    E->pool->run(n, nthr, [&](size_t x) {
       const auto& it = items[order[a + x]];
       const bool ok = hstatus[x] == 0;
       if (!ok) redone++;

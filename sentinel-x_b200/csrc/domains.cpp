@@ -958,20 +958,30 @@ bool is_multidomain(const std::vector<float>& btot, const std::vector<float>& et
 
 }  // namespace
 
+// The scores alone: the row logs they do not use are not taken.
 float forward_score_from_rows(const ProfileHost& p, int64_t l, const float* fwd_rows) {
+  (void)p;
   if (l <= 0) return kNegInf;  // no row was computed; the reference's xc stays 0
-  LogRows sp;
-  double lnscale;
-  forward_log_rows(p, l, fwd_rows, sp, lnscale);
   const SpecialTr st = special_transitions(l, true);
-  const float xc = fwd_rows[6 * l + 4];
-  return (float)((double)lnpos(xc * st.pmove) + lnscale);
+  double lnscale = 0.0;
+  for (int64_t i = 1; i <= l; i++) {
+    const float scale = fwd_rows[6 * i + 5];
+    if (scale > 0.0f) lnscale += std::log((double)scale);
+  }
+  return (float)((double)lnpos(fwd_rows[6 * l + 4] * st.pmove) + lnscale);
 }
 
 float backward_score_from_rows(int64_t l, const float* bwd_rows) {
   if (l <= 0) return kNegInf;
-  LogRows sp;
-  return backward_log_rows(l, bwd_rows, sp);
+  const SpecialTr st = special_transitions(l, true);
+  double lnscale = 0.0;
+  for (int64_t i = l - 1; i >= 1; i--) {
+    const float scale = bwd_rows[6 * i + 5];
+    if (scale > 0.0f) lnscale += std::log((double)scale);
+  }
+  const float ls = (float)lnscale;
+  const float n1 = l > 1 ? lnpos(bwd_rows[6]) + ls : kNegInf;  // N of row 1
+  return logsum2(n1 + st.loop, lnpos(bwd_rows[1]) + ls + st.move);
 }
 
 namespace {

@@ -62,6 +62,7 @@ int sx_create(const sx_opts* opts, sx_engine** out) {
   e->flags = opts ? opts->flags : 0;
   e->host_threads = (opts && opts->host_threads > 0) ? opts->host_threads : (int)std::thread::hardware_concurrency();
   e->host_threads = std::max(1, e->host_threads);
+  e->pool = std::make_unique<WorkerPool>(e->host_threads);
   e->batch_bytes = (opts && opts->batch_bytes > 0) ? opts->batch_bytes : (2LL << 30);
   e->pipeline_blocks = (opts && opts->pipeline_blocks > 0) ? opts->pipeline_blocks : 0;
   try {
@@ -147,7 +148,9 @@ int sx_profiles_load_text(sx_engine* e, const char* text, size_t len, const char
   auto p = std::make_unique<sx_profiles>();
   p->eng = e;
   std::string err;
-  if (!load_profiles_text(text ? text : "", len, source ? source : "<stream>", p->h, err)) return fail(SX_EINVAL, err);
+  std::vector<ProfileHost> h;
+  if (!load_profiles_text(text ? text : "", len, source ? source : "<stream>", h, err)) return fail(SX_EINVAL, err);
+  p->h.assign(std::move(h));
   return finish_profiles(e, std::move(p), out);
 }
 
@@ -157,13 +160,13 @@ int sx_profiles_from_arrays(sx_engine* e, const sx_profile_arrays* a, size_t n, 
   std::lock_guard<std::mutex> lk(e->mu);
   auto p = std::make_unique<sx_profiles>();
   p->eng = e;
-  p->h.resize(n);
+  std::vector<ProfileHost> hs(n);
   for (size_t i = 0; i < n; i++) {
     const sx_profile_arrays& s = a[i];
     const std::string at = "sx_profiles_from_arrays: profile " + std::to_string(i);
     if (!s.name || !s.msc || !s.mo || !s.t || !s.p || !s.compo) return fail(SX_EINVAL, at + ": NULL field");
     if (s.m < 1) return fail(SX_EINVAL, at + ": M must be at least 1");
-    ProfileHost& h = p->h[i];
+    ProfileHost& h = hs[i];
     const size_t w = (size_t)s.m + 1;
     h.name = s.name;
     h.has_acc = s.acc != nullptr;
@@ -196,6 +199,7 @@ int sx_profiles_from_arrays(sx_engine* e, const sx_profile_arrays* a, size_t n, 
       h.fwd[q] = h.has_fwd ? s.forward[q] : NAN;
     }
   }
+  p->h.assign(std::move(hs));
   return finish_profiles(e, std::move(p), out);
 }
 
@@ -207,7 +211,9 @@ int sx_profiles_load_file(sx_engine* e, const char* path, sx_profiles** out) {
   p->eng = e;
   std::string err;
   bool io = false;
-  if (!load_profiles_file(path, p->h, err, io)) return fail(io ? SX_EIO : SX_EINVAL, err);
+  std::vector<ProfileHost> h;
+  if (!load_profiles_file(path, h, err, io)) return fail(io ? SX_EIO : SX_EINVAL, err);
+  p->h.assign(std::move(h));
   return finish_profiles(e, std::move(p), out);
 }
 
@@ -226,7 +232,9 @@ int sx_profiles_load_binary(sx_engine* e, const char* path, sx_profiles** out) {
   p->eng = e;
   std::string err;
   bool io = false;
-  if (!load_profiles_binary(path, p->h, err, io)) return fail(io ? SX_EIO : SX_EINVAL, "sx_profiles_load_binary: " + err);
+  std::vector<ProfileHost> h;
+  if (!load_profiles_binary(path, h, err, io)) return fail(io ? SX_EIO : SX_EINVAL, "sx_profiles_load_binary: " + err);
+  p->h.assign(std::move(h));
   return finish_profiles(e, std::move(p), out);
 }
 
@@ -326,7 +334,7 @@ int sx_targets_create_digital(sx_engine* e, const uint8_t* dsq, const int64_t* o
   uint8_t* out8 = t->dsq.data();
   std::atomic<size_t> bad{SIZE_MAX};
   const size_t nchunk = o >= (1 << 22) ? std::min<size_t>(n, 8 * (size_t)e->host_threads) : 1;
-  parallel_for(nchunk, e->host_threads, [&](size_t c) {
+  e->pool->run(nchunk, e->host_threads, [&](size_t c) {
     for (size_t i = n * c / nchunk; i < n * (c + 1) / nchunk; i++) {
       const uint8_t* d = dsq + offsets[i];
       uint8_t hi = 0;  // max code, a loop the compiler vectorises; positions only on failure
@@ -402,20 +410,16 @@ int sx_search_many(sx_engine* e, const sx_profiles* const* sets, size_t n, const
   // (per-profile thresholds, E-values over the same targets, per-profile
   // domain Z), so slicing the combined hits by profile range is exact.
   std::vector<size_t> first(n + 1, 0);
-  auto all = std::make_unique<sx_profiles>();
-  all->eng = e;
-  for (size_t i = 0; i < n; i++) {
-    first[i] = all->h.size();
-    all->h.insert(all->h.end(), sets[i]->h.begin(), sets[i]->h.end());
-  }
-  first[n] = all->h.size();
+  for (size_t i = 0; i < n; i++) first[i + 1] = first[i] + sets[i]->h.size();
   std::vector<std::unique_ptr<sx_hits>> parts(n);
   try {
     CK(cudaSetDevice(e->device));
     sx_hits hits;
-    if (!all->h.empty()) {
-      pack_profiles(all.get());
-      const int rc = run_search(e, all.get(), t, cfg, &hits);
+    if (first[n]) {
+      sx_profiles all;
+      all.eng = e;
+      combine_profiles(&all, sets, n, search_opts(cfg));
+      const int rc = run_search(e, &all, t, cfg, &hits);
       if (rc) return rc;
     }
     size_t q = 0;

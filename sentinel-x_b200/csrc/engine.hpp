@@ -18,7 +18,10 @@
 #include <condition_variable>
 #include <cstring>
 #include <deque>
+#include <exception>
+#include <system_error>
 #include <functional>
+#include <list>
 #include <memory>
 #include <mutex>
 #include <numeric>
@@ -170,24 +173,100 @@ struct PinnedBuf {
 // Launch tables of every kernel instantiation (filled once).
 const KernelTables& kernels();
 
-// ---- thread pool helper ----------------------------------------------------
-template <typename F>
-void parallel_for(size_t n, int nthreads, F&& f) {
-  if (n == 0) return;
-  const int nt = std::max(1, std::min<int>(nthreads, (int)n));
-  std::atomic<size_t> next{0};
-  auto work = [&]() {
-    for (;;) {
-      const size_t i = next.fetch_add(1);
-      if (i >= n) break;
-      f(i);
+// ---- host workers ------------------------------------------------------------
+// The engine's host threads, started with the first loop that needs them and
+// joined with the engine: a search runs several short loops, and fresh threads
+// for each cost it more than the work (15 threads: ~0.2 ms).  Loops of several
+// threads may run at once (the engine thread's and the domain-definition
+// driver's); every caller works on its own loop until it is done.  An exception
+// of a body ends its loop and is thrown to the loop's caller.
+class WorkerPool {
+ public:
+  explicit WorkerPool(int threads) : most_(std::max(0, threads - 1)) {}
+  ~WorkerPool() {
+    {
+      std::lock_guard<std::mutex> g(mu_);
+      stop_ = true;
+    }
+    wake_.notify_all();
+    for (auto& t : th_) t.join();
+  }
+  // f(i) for every i < n on at most `threads` threads, the caller among them.
+  template <typename F>
+  void run(size_t n, int threads, F&& f) {
+    if (n == 0) return;
+    const int helpers = (int)std::min<size_t>({(size_t)std::max(0, threads - 1), (size_t)most_, n - 1});
+    if (helpers == 0) {
+      for (size_t i = 0; i < n; i++) f(i);
+      return;
+    }
+    Loop loop;
+    loop.n = n;
+    loop.room = helpers;
+    loop.body = [&f](size_t i) { f(i); };
+    {
+      std::lock_guard<std::mutex> g(mu_);
+      try {
+        while ((int)th_.size() < most_) th_.emplace_back([this] { work(); });
+      } catch (const std::system_error&) {  // no more threads to be had: fewer help
+      }
+      open_.push_back(&loop);
+    }
+    if (helpers == 1) wake_.notify_one();
+    else wake_.notify_all();
+    loop.drain();
+    std::unique_lock<std::mutex> g(mu_);
+    open_.remove(&loop);  // no helper joins any more
+    idle_.wait(g, [&] { return loop.inside == 0; });
+    if (loop.error) std::rethrow_exception(loop.error);
+  }
+
+ private:
+  struct Loop {
+    size_t n = 0;
+    int room = 0, inside = 0;  // helpers that may still join, helpers at work (under the pool's mutex)
+    std::function<void(size_t)> body;
+    std::atomic<size_t> next{0};
+    std::mutex err_mu;
+    std::exception_ptr error;
+    void drain() {
+      try {
+        for (size_t i; (i = next.fetch_add(1)) < n;) body(i);
+      } catch (...) {
+        next.store(n);
+        std::lock_guard<std::mutex> g(err_mu);
+        if (!error) error = std::current_exception();
+      }
     }
   };
-  std::vector<std::thread> th;
-  for (int t = 1; t < nt; t++) th.emplace_back(work);
-  work();
-  for (auto& t : th) t.join();
-}
+  void work() {
+    std::unique_lock<std::mutex> g(mu_);
+    for (;;) {
+      Loop* l = nullptr;
+      wake_.wait(g, [&] {
+        for (Loop* o : open_)
+          if (o->room > 0 && o->next.load() < o->n) {
+            l = o;
+            return true;
+          }
+        return stop_;
+      });
+      if (!l) return;
+      l->room--;
+      l->inside++;
+      g.unlock();
+      l->drain();
+      g.lock();
+      if (--l->inside == 0) idle_.notify_all();
+    }
+  }
+  const int most_;
+  std::mutex mu_;
+  std::condition_variable wake_, idle_;
+  std::list<Loop*> open_;
+  std::vector<std::thread> th_;
+  bool stop_ = false;
+};
 
 // Smallest f32 statistic s with pass(s) true, assuming pass is monotone
 // (false below the boundary, true above); +inf if it never passes, -inf if it
@@ -485,6 +564,7 @@ using namespace sxe;
 struct sx_engine {
   int device = 0;
   int host_threads = 1;
+  std::unique_ptr<WorkerPool> pool;
   uint32_t flags = 0;
   int64_t batch_bytes = 0;
   int num_sms = 148;
@@ -543,8 +623,9 @@ struct sx_engine {
 
 struct sx_profiles {
   sx_engine* eng = nullptr;
-  std::vector<ProfileHost> h;
+  ProfileList h;
   std::vector<DevProfile> dp;
+  std::vector<int64_t> plain_off;  // float offsets of the plain images
   std::vector<int> msv_shape;
   DevBuf<DevProfile> d_prof;
   DevBuf<sxk::PlainProfile> d_pprof;  // plain one-pair-per-block layout
@@ -660,7 +741,9 @@ int shape_for(const sx_engine* E, int kind, int m);
 void pack_profiles(sx_profiles* P);
 void pack_targets(sx_targets* T);
 void append_target(sx_targets* T, const uint8_t* dig, size_t l);
-std::vector<Thresholds> make_thresholds(const std::vector<ProfileHost>& H, const SearchOpts& o);
+std::vector<Thresholds> make_thresholds(const ProfileList& H, const SearchOpts& o);
+std::vector<Thresholds> thresholds_of(const sx_profiles* P, const SearchOpts& o);
+void combine_profiles(sx_profiles* P, const sx_profiles* const* sets, size_t n, const SearchOpts& o);
 void allow_smem(const void* kernel, size_t bytes);
 void fork_aux(Streams& X);
 void join_aux(Streams& X);
@@ -678,6 +761,7 @@ int long_grid(const sx_engine* E, size_t n);
 int64_t long_stride(const sx_profiles* P, const std::vector<sxk::LongPair>& v, size_t a, size_t b);
 void long_scores(sx_engine* E, const sx_profiles* P, const sx_targets* T, const std::vector<sxk::LongPair>& v,
                  bool viterbi, std::vector<float>& out);  // v: any profiles of M > kMaxM
+SearchOpts search_opts(const sx_search_cfg* cfg);
 int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx_search_cfg* cfg, sx_hits* out);
 int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T, std::vector<EnvSource>& srcs,
                         int nthr, PhaseLog* plog = nullptr);
@@ -696,7 +780,7 @@ template <typename Sink>
 void rows_pass_sync(sx_engine* E, const sx_profiles* P, const sx_targets* T, const std::vector<FinalPair>& pairs,
                     Sink&& sink) {
   rows_pass(E, E->sl[0], P, T, pairs, [&](RowsChunk&& c) {
-    parallel_for(c.which.size(), E->host_threads, [&](size_t q) { sink(c.which[q], c.fwd(q), c.bwd(q)); });
+    E->pool->run(c.which.size(), E->host_threads, [&](size_t q) { sink(c.which[q], c.fwd(q), c.bwd(q)); });
   });
 }
 

@@ -578,7 +578,7 @@ class ByteReader {
 
 }  // namespace
 
-bool save_profiles_binary(const std::vector<ProfileHost>& in, const std::string& path, std::string& err) {
+bool save_profiles_binary(const ProfileList& in, const std::string& path, std::string& err) {
   ByteWriter w;
   w.put<uint32_t>(kBinVersion);
   w.put<uint32_t>((uint32_t)in.size());

@@ -52,6 +52,32 @@ struct ProfileHost {
   const float* mo_row(int x) const { return mo.data() + (size_t)x * (m + 1); }
 };
 
+// Configured profiles, shared between the sets that list them (a combined set
+// of sx_search_many names the profiles of its parts without copying them).
+class ProfileList {
+ public:
+  struct Iter {
+    const std::shared_ptr<ProfileHost>* p;
+    const ProfileHost& operator*() const { return **p; }
+    Iter& operator++() { ++p; return *this; }
+    bool operator!=(const Iter& o) const { return p != o.p; }
+  };
+  size_t size() const { return v_.size(); }
+  bool empty() const { return v_.empty(); }
+  const ProfileHost& operator[](size_t i) const { return *v_[i]; }
+  Iter begin() const { return {v_.data()}; }
+  Iter end() const { return {v_.data() + v_.size()}; }
+  void assign(std::vector<ProfileHost>&& in) {
+    v_.clear();
+    v_.reserve(in.size());
+    for (ProfileHost& h : in) v_.push_back(std::make_shared<ProfileHost>(std::move(h)));
+  }
+  void append(const ProfileList& o) { v_.insert(v_.end(), o.v_.begin(), o.v_.end()); }
+
+ private:
+  std::vector<std::shared_ptr<ProfileHost>> v_;
+};
+
 // Parse (plain or gzip) HMMER3 text and configure every profile.  Returns
 // false with `err` set (messages follow src/hmmer/parse.rs: "<source> line N: ...").
 bool load_profiles_text(const char* text, size_t len, const std::string& source, std::vector<ProfileHost>& out,
@@ -60,7 +86,7 @@ bool load_profiles_file(const std::string& path, std::vector<ProfileHost>& out, 
 
 // Binary cache of configured profiles (hmmfile.cpp): magic, version, count,
 // the ProfileHost fields of every profile, FNV-1a checksum of the payload.
-bool save_profiles_binary(const std::vector<ProfileHost>& in, const std::string& path, std::string& err);
+bool save_profiles_binary(const ProfileList& in, const std::string& path, std::string& err);
 bool load_profiles_binary(const std::string& path, std::vector<ProfileHost>& out, std::string& err, bool& io_error);
 
 // Length-dependent special transitions (p7_ReconfigLength; src/hmmer/model.rs:284-312).

@@ -413,7 +413,7 @@ void pack_profiles(sx_profiles* P) {
   std::vector<double> bias(np * 54);
   std::vector<uint2> qimg((size_t)std::max<int64_t>(q_total, 1));
   std::vector<uint4> qvimg((size_t)std::max<int64_t>(qv_total, 1));
-  for (size_t i = 0; i < np; i++) {
+  P->eng->pool->run(np, P->eng->host_threads, [&](size_t i) {
     if (P->dp[i].xshape >= 0) pack_ximage(P->h[i], P->dp[i], ximg.data());
     if (P->dp[i].vbin >= 0) {
       pack_images(P->h[i], P->dp[i], msv.data(), vit.data(), vfb.data());
@@ -435,7 +435,7 @@ void pack_profiles(sx_profiles* P) {
       }
     }
     pack_bias(P->h[i], bias.data() + i * 54);
-  }
+  });
   // plain layout: 25 msc rows then mm mi md im ii dm dd bm, each M+1 long;
   // profiles past the exact row shapes add the 25 odds rows and the 8
   // probability rows (same order), the image of the long kernels
@@ -461,6 +461,8 @@ void pack_profiles(sx_profiles* P) {
       for (int q = 0; q < 8; q++) memcpy(b + (sxk::kLP + q) * w, h.p[order[q]].data(), sizeof(float) * w);
     }
   }
+  P->plain_off.resize(np);
+  for (size_t i = 0; i < np; i++) P->plain_off[i] = pprof[i].off;
   cudaStream_t s = P->eng->stream;
   P->d_pprof.upload(pprof.data(), np, s);
   P->d_plain.upload(plain.data(), plain.size(), s);
@@ -471,6 +473,67 @@ void pack_profiles(sx_profiles* P) {
   P->d_vit.upload(vit.data(), vit.size(), s);
   P->d_vfb.upload(vfb.data(), vfb.size(), s);
   P->d_x.upload(ximg.data(), ximg.size(), s);
+  P->d_bias.upload(bias.data(), bias.size(), s);
+  CK(cudaStreamSynchronize(s));
+}
+
+// A set that lists the profiles of several sets, in order, without copying
+// them: it shares their host profiles and reads their device images where they
+// are -- every image is addressed by an offset from one base, so the parts'
+// offsets are moved by the distance of their images from the lowest.  Only the
+// records, the bias tables (432 bytes a profile) and the thresholds are new.
+// The parts must outlive it.
+void combine_profiles(sx_profiles* P, const sx_profiles* const* sets, size_t n, const SearchOpts& o) {
+  for (size_t i = 0; i < n; i++) P->h.append(sets[i]->h);
+  const size_t np = P->h.size();
+  std::vector<sxk::PlainProfile> pprof(np);
+  std::vector<double> bias(np * 54);
+  P->dp.reserve(np);
+  P->plain_off.resize(np);
+  size_t at = 0;
+  for (size_t i = 0; i < n; i++) {
+    P->dp.insert(P->dp.end(), sets[i]->dp.begin(), sets[i]->dp.end());
+    P->msv_shape.insert(P->msv_shape.end(), sets[i]->msv_shape.begin(), sets[i]->msv_shape.end());
+    std::copy(sets[i]->plain_off.begin(), sets[i]->plain_off.end(), P->plain_off.begin() + (std::ptrdiff_t)at);
+    const std::vector<Thresholds> th = thresholds_of(sets[i], o);
+    P->th_cache.insert(P->th_cache.end(), th.begin(), th.end());
+    at += sets[i]->h.size();
+  }
+  const double key[4] = {o.filters ? 1.0 : 0.0, o.f1, o.f2, o.f3};
+  std::memcpy(P->th_key, key, sizeof key);
+  // moves one image's offsets to the lowest buffer of the parts, which P views
+  auto rebase = [&](auto member, auto&& move) {
+    uintptr_t low = UINTPTR_MAX;
+    for (size_t i = 0; i < n; i++)
+      if (!sets[i]->h.empty()) low = std::min(low, reinterpret_cast<uintptr_t>((sets[i]->*member).p));
+    size_t q = 0;
+    for (size_t i = 0; i < n; i++) {
+      const auto* p = (sets[i]->*member).p;
+      const int64_t by = (int64_t)((reinterpret_cast<uintptr_t>(p) - low) / sizeof(*p));
+      for (size_t k = 0; k < sets[i]->h.size(); k++, q++) move(q, by);
+    }
+    (P->*member).view(reinterpret_cast<void*>(low), 1);
+  };
+  rebase(&sx_profiles::d_msv, [&](size_t q, int64_t by) { P->dp[q].msv_off += by; });
+  rebase(&sx_profiles::d_vit, [&](size_t q, int64_t by) { P->dp[q].vit_off += by; });
+  rebase(&sx_profiles::d_vfb, [&](size_t q, int64_t by) { P->dp[q].vfb_off += by; });
+  rebase(&sx_profiles::d_x, [&](size_t q, int64_t by) { P->dp[q].x_off += by; });
+  rebase(&sx_profiles::d_plain, [&](size_t q, int64_t by) { P->plain_off[q] += by; });
+  rebase(&sx_profiles::d_qimg, [&](size_t q, int64_t by) {
+    if (P->dp[q].q_off >= 0) P->dp[q].q_off += by;  // -1: not pre-screened
+  });
+  rebase(&sx_profiles::d_qvimg, [&](size_t q, int64_t by) {
+    if (P->dp[q].qv_off >= 0) P->dp[q].qv_off += by;
+  });
+  for (size_t i = 0; i < np; i++) {
+    pprof[i].off = P->plain_off[i];
+    pprof[i].m = P->h[i].m;
+    pprof[i].pad = 0;
+    pack_bias(P->h[i], bias.data() + i * 54);
+  }
+  cudaStream_t s = P->eng->stream;
+  P->d_pprof.upload(pprof.data(), np, s);
+  P->d_prof.upload(P->dp.data(), np, s);
   P->d_bias.upload(bias.data(), bias.size(), s);
   CK(cudaStreamSynchronize(s));
 }
@@ -548,12 +611,23 @@ void append_target(sx_targets* T, const uint8_t* dig, size_t l) {
   T->dsq.resize(padded, SYM_STAR);
 }
 
+// A set's thresholds for the search options, computed once per options.
+std::vector<Thresholds> thresholds_of(const sx_profiles* P, const SearchOpts& o) {
+  const double key[4] = {o.filters ? 1.0 : 0.0, o.f1, o.f2, o.f3};
+  std::lock_guard<std::mutex> g(P->th_mu);
+  if (P->th_cache.size() != P->h.size() || std::memcmp(key, P->th_key, sizeof key) != 0) {
+    P->th_cache = make_thresholds(P->h, o);
+    std::memcpy(P->th_key, key, sizeof key);
+  }
+  return P->th_cache;
+}
+
 // ---- thresholds ---------------------------------------------------------------
 // Per profile, the smallest f32 bit statistic that passes each filter
 // (pipeline.rs:164-183).  The tails are monotone in the statistic, except the
 // Gumbel survival around its branch at 1e-5; a threshold within 2% of that
 // point disables device filtering for the stage (the host still decides).
-std::vector<Thresholds> make_thresholds(const std::vector<ProfileHost>& H, const SearchOpts& o) {
+std::vector<Thresholds> make_thresholds(const ProfileList& H, const SearchOpts& o) {
   std::vector<Thresholds> th(H.size());
   auto near_branch = [](double f) { return f > 0.98e-5 && f < 1.02e-5; };
   for (size_t i = 0; i < H.size(); i++) {

@@ -1031,7 +1031,7 @@ bool cascade_finish(sx_engine* E, Slot& S, const sx_profiles* P, const sx_target
   CK(cudaStreamSynchronize(s));
   // exact host re-check of F1 / bias / F2 with the reference's libm
   std::vector<char> keep(surv.size(), 0);
-  parallel_for(surv.size(), E->host_threads, [&](size_t i) {
+  E->pool->run(surv.size(), E->host_threads, [&](size_t i) {
     PairRec& r = surv[i];
     const ProfileHost& h = P->h[r.p];
     const uint8_t* d = T->dsq.data() + T->off[r.t];
@@ -1049,28 +1049,24 @@ bool cascade_finish(sx_engine* E, Slot& S, const sx_profiles* P, const sx_target
   return true;
 }
 
-int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx_search_cfg* cfg, sx_hits* out) {
-  int rc = check_cutoffs(P, cfg->cutoff_kind);
-  if (rc) return rc;
-  E->stats = sx_search_stats{};
+SearchOpts search_opts(const sx_search_cfg* cfg) {
   SearchOpts o;
   o.filters = cfg->filters != 0;
   o.null2 = cfg->null2 != 0;
   o.f1 = cfg->f1;
   o.f2 = cfg->f2;
   o.f3 = cfg->f3;
+  return o;
+}
+
+int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx_search_cfg* cfg, sx_hits* out) {
+  int rc = check_cutoffs(P, cfg->cutoff_kind);
+  if (rc) return rc;
+  E->stats = sx_search_stats{};
+  const SearchOpts o = search_opts(cfg);
   const size_t np = P->h.size(), nt = T->len.size();
   cudaStream_t s = E->stream;
-  std::vector<Thresholds> th;
-  {
-    const double key[4] = {o.filters ? 1.0 : 0.0, o.f1, o.f2, o.f3};
-    std::lock_guard<std::mutex> g(P->th_mu);
-    if (P->th_cache.size() != np || std::memcmp(key, P->th_key, sizeof key) != 0) {
-      P->th_cache = make_thresholds(P->h, o);
-      std::memcpy(P->th_key, key, sizeof key);
-    }
-    th = P->th_cache;
-  }
+  std::vector<Thresholds> th = thresholds_of(P, o);
   // profiles longer than kMaxM take the long pass instead of the cascade
   std::vector<int> longs;
   std::vector<char> long_exact(np, 0);
@@ -1190,7 +1186,7 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
           };
           std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) { return cost(a) > cost(b); });
           if (!dev_env) {  // F3 and the whole domain definition on the host (pipeline.rs:179-293)
-            parallel_for(ord.size(), nthr, [&](size_t rr) {
+            E->pool->run(ord.size(), nthr, [&](size_t rr) {
               const size_t q = ord[rr];
               const size_t i = ch->which[q];
               const FinalPair& f = B->finals[i];
@@ -1215,7 +1211,7 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
           pb->db = std::make_unique<DomainBatch>(o, nq);
           DomainBatch& db = *pb->db;
           std::vector<char>& begun = pb->begun;
-          parallel_for(ord.size(), nthr, [&](size_t rr) {
+          E->pool->run(ord.size(), nthr, [&](size_t rr) {
             const size_t q = ord[rr];
             const FinalPair& f = B->finals[ch->which[q]];
             const ProfileHost& h = P->h[f.p];
@@ -1231,7 +1227,7 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
           const std::vector<RegionRequest>& regs = db.regions();
           pb->dev_regions = !regs.empty() && device_traces(regs, nthr);
           if (!regs.empty() && !pb->dev_regions)
-            parallel_for(regs.size(), nthr, [&](size_t r) { db.expand(r, {}, nullptr, false); });
+            E->pool->run(regs.size(), nthr, [&](size_t r) { db.expand(r, {}, nullptr, false); });
           pending.push_back(std::move(pb));
         } catch (const CudaError& ce) {
           std::lock_guard<std::mutex> g(host_err_mu);
@@ -1318,7 +1314,7 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
     std::vector<float> usc, vsc, fsc(filt.size(), 0.f);
     long_scores(E, P, T, filt, false, usc);
     std::vector<char> pass1(filt.size(), 0);
-    parallel_for(filt.size(), E->host_threads, [&](size_t i) {
+    E->pool->run(filt.size(), E->host_threads, [&](size_t i) {
       const ProfileHost& h = P->h[filt[i].p];
       const int64_t l = T->len[filt[i].t];
       const float nullsc = null1_score(l);
@@ -1357,7 +1353,7 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
       std::vector<sxk::LongPair> lp;
       for (const FinalPair& f : H->finals) lp.push_back({f.p, f.t});
       long_rows(E, P, T, lp, [&](size_t first, size_t n, const float* f, const float* b, const std::vector<int64_t>& off) {
-        parallel_for(n, E->host_threads, [&](size_t q) {
+        E->pool->run(n, E->host_threads, [&](size_t q) {
           const size_t i = first + q;
           const FinalPair& fp = H->finals[i];
           const ProfileHost& h = P->h[fp.p];
@@ -1404,7 +1400,7 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
     for (auto& pb : pending)
       for (size_t q = 0; q < pb->which.size(); q++)
         if (pb->begun[q]) todo.emplace_back(pb.get(), q);
-    parallel_for(todo.size(), E->host_threads, [&](size_t x) {
+    E->pool->run(todo.size(), E->host_threads, [&](size_t x) {
       PendingBatch& pb = *todo[x].first;
       const size_t q = todo[x].second;
       const size_t i = pb.which[q];

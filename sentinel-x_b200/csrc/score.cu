@@ -441,7 +441,7 @@ int sx_posterior_grad(sx_engine* e, const sx_profiles* p, const sx_targets* t, c
       for (int q = 0; q < parts; q++) {
         CK(cudaEventSynchronize(e->ev[q]));
         const float* hs = e->adj_host.p + at[q] * out_per;
-        parallel_for((size_t)(at[q + 1] - at[q]), e->host_threads, [&](size_t y) {
+        e->pool->run((size_t)(at[q + 1] - at[q]), e->host_threads, [&](size_t y) {
           const size_t z = i0 + (size_t)at[q] + y;
           const float* src = hs + y * out_per;
           memcpy(d_msc + z * 25 * W, src, sizeof(float) * 25 * W);

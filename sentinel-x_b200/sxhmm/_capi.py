@@ -308,19 +308,20 @@ class Engine:
 
 def _take_hits(out):
     try:
-        nh = _lib.sx_hits_count(out)
-        nd = _lib.sx_hits_domain_count(out)
-        hits = [_copy(_lib.sx_hits_array(out)[i]) for i in range(nh)]
-        doms = [_copy(_lib.sx_hits_domains(out)[i]) for i in range(nd)]
+        hits = _records(SxHit, _lib.sx_hits_array(out), _lib.sx_hits_count(out))
+        doms = _records(SxDomain, _lib.sx_hits_domains(out), _lib.sx_hits_domain_count(out))
     finally:
         _lib.sx_hits_free(out)
     return hits, doms
 
 
-def _copy(s):
-    c = type(s)()
-    C.pointer(c)[0] = s
-    return c
+def _records(kind, ptr, n):
+    """The library's n records copied at once, as a list."""
+    if not n:
+        return []
+    a = (kind * n)()
+    C.memmove(a, ptr, C.sizeof(a))
+    return list(a)
 
 
 class Profiles:
