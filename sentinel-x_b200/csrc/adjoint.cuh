@@ -66,9 +66,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // A team's view of its profile: transitions at the thread's columns, those of
 // the column left of them, and the factors of the D scans.
-template <bool MULTI>
+template <bool MULTI, int C = kAdjC>
 struct AdjTeam {
-  static constexpr int C = kAdjC;
   int lane, warp, nw, k0, M, width;
   const float* im;  // the row image at the thread's first column
   float mm[C], mi[C], md[C], imr[C], ii[C], dm[C], dd[C], bm[C];
@@ -229,6 +228,7 @@ struct AdjTeam {
   }
   __device__ __forceinline__ void load_row(const float* base, int tw, float (&m)[C], float (&i)[C], float (&d)[C]) const {
     auto get = [&](const float* p, float (&v)[C]) {  // plain loads: this kernel wrote them
+      static_assert(C == 4, "a float4 a row");
       const float4 x = *reinterpret_cast<const float4*>(p);
       v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
     };

@@ -735,7 +735,7 @@ struct RegionPassStats {
 };
 
 int vit_blocks(int num_sms, int shape, unsigned n);
-int warp_ctas(int num_sms, unsigned n);
+unsigned scan_ctas(unsigned n);
 std::vector<int16_t> default_shape_table(int kind);
 int shape_for(const sx_engine* E, int kind, int m);
 void pack_profiles(sx_profiles* P);

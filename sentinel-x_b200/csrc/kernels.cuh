@@ -20,7 +20,7 @@ constexpr float kLn2 = 0.693147182464599609375f;
 constexpr unsigned kFull = 0xffffffffu;
 
 // ---- device records ------------------------------------------------------
-struct DevProfile {  // 88 bytes
+struct DevProfile {  // 96 bytes
   int32_t m;
   int32_t vc;        // columns per lane in the warp-chunked layout (32 lanes)
   int32_t vbin;      // survivor-list bin of vc
@@ -39,6 +39,8 @@ struct DevProfile {  // 88 bytes
   int32_t qv_cap;    // its row maxima above this (int16 units) pass at once
   int32_t xshape;    // shape of the exact row passes (index into kXShapes)
   int64_t x_off;     // float offset of its row image
+  int32_t x_width;   // columns of a row of it
+  int32_t pad;
 };
 struct Thresholds {  // per profile, per search: pass iff statistic >= threshold (bits)
   float s1, s2, s3;
@@ -63,10 +65,7 @@ struct MsvTile {
 enum : int {
   kRowMsc = 0,    // 25 rows: log-odds match scores msc[x][k]
   kRowVit = 25,   // 8 rows: t_mm[k-1], t_im[k-1], t_dm[k-1], t_bm[k], t_mi[k], t_ii[k], t_md[k-1], t_dd[k-1]
-  kRowMo = 33,    // 25 rows: match odds mo[x][k]
-  kRowFwd = 58,   // 8 rows: p_bm[k], p_mm[k-1], p_im[k-1], p_dm[k-1], p_mi[k], p_ii[k], p_md[k-1], p_dd[k-1]
-  kRowBwd = 66,   // 8 rows: p_mm[k], p_mi[k], p_md[k], p_im[k], p_ii[k], p_dm[k], p_dd[k], p_bm[k]
-  kImgRows = 74
+  kImgRows = 33
 };
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
@@ -507,154 +506,6 @@ __global__ void __launch_bounds__(256) viterbi_kernel(
       r.vsc = vsc;
       if (score_out) score_out[r.slot] = vsc;
       else if (bits_stat(vsc, r.filtersc) >= thr[r.p].s2 - slack) push_pair(r, bin, out, out_bins, out_counts, overflow);
-    }
-  }
-}
-
-// ===========================================================================
-// Forward pre-screen of F3 (src/hmmer/dp.rs:229-298), one warp per pair,
-// probability space with the reference's sparse rescaling; the pair passes when
-// the device estimate of the F3 statistic clears the threshold minus `slack`.
-//
-// The D chain is an affine recurrence D[k] = a_k + D[k-1] p_k, so each lane
-// forms its transfer (A, B) over its columns, a Kogge-Stone scan of 5 shuffles
-// composes them across lanes, each lane re-runs its columns from the true
-// carry-in, and the row sum is a butterfly.  The rounding differs from the
-// reference's order, so the pass test adds a bound on the difference: for sums
-// and products of non-negative numbers the relative errors of two evaluation
-// orders add up along their longest paths, at most 2^-24 per operation, i.e.
-// |ln F_scan - ln F_ref| <= (L+1)(2M + 6 VC + 64) 2^-24, taken twice.  The
-// pre-screen therefore passes every pair the exact F3 test (on the host, from
-// the exact rows of exact_rows.cuh) passes.
-// ===========================================================================
-template <int VC>
-__global__ void __launch_bounds__(256) forward_scan_kernel(
-    const PairRec* __restrict__ in, const unsigned* __restrict__ in_counts, const BinRegion* __restrict__ in_bins,
-    int bin, PairRec* __restrict__ out, const BinRegion* __restrict__ out_bins, unsigned* __restrict__ out_counts,
-    unsigned* __restrict__ overflow, const DevProfile* __restrict__ profs, const Thresholds* __restrict__ thr,
-    const float* __restrict__ vfb, const uint8_t* __restrict__ res, const int64_t* __restrict__ toff,
-    const int32_t* __restrict__ tlen, const float4* __restrict__ xsc, float slack) {
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  const unsigned n = min(in_counts[bin], in_bins[bin].cap);
-  for (unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += warps) {
-    PairRec r = in[in_bins[bin].off + w];
-    const DevProfile P = profs[r.p];
-    const Img<VC> img{vfb + P.vfb_off};
-    const int M = P.m;
-    const int nl = (M + VC - 1) / VC;  // lanes holding columns 1..M
-    const uint8_t* s = res + toff[r.t];
-    const int L = tlen[r.t];
-    const float4 xs = xsc[r.t];
-    const float ploop = xs.z, pmove = xs.w;
-    TransRows<VC> tr;
-    tr.load(img, kRowFwd, lane);
-    float mp[VC], ip[VC], dp[VC], eo[VC];
-#pragma unroll
-    for (int c = 0; c < VC; c++) mp[c] = ip[c] = dp[c] = 0.f;
-    float xn = 1.f, xb = pmove, xj = 0.f, xc = 0.f;
-    double lnscale = 0.0;
-    int x = L > 0 ? __ldg(s) : 24;
-#pragma unroll
-    for (int c = 0; c < VC; c++) eo[c] = img.at(kRowMo + x, c, lane);
-    for (int i = 0; i < L; i++) {
-      const int xnext = (i + 1 < L) ? __ldg(s + i + 1) : 24;
-      float eon[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) eon[c] = img.at(kRowMo + xnext, c, lane);
-      const float ins = x != 24 ? 1.f : 0.f;
-      const float mpl0 = __shfl_up_sync(kFull, mp[VC - 1], 1);
-      const float ipl0 = __shfl_up_sync(kFull, ip[VC - 1], 1);
-      const float dpl0 = __shfl_up_sync(kFull, dp[VC - 1], 1);
-      const float mpl = lane ? mpl0 : 0.f, ipl = lane ? ipl0 : 0.f, dpl = lane ? dpl0 : 0.f;
-      float mv[VC], iv[VC], a[VC], dv[VC], pdd[VC];
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        const int k = lane * VC + c + 1;
-        const float mpv = c ? mp[c - 1] : mpl, ipv = c ? ip[c - 1] : ipl, dpv = c ? dp[c - 1] : dpl;
-        float t = fmul(xb, tr.get(img, kRowFwd, 0, c, lane));
-        t = fadd(t, fmul(mpv, tr.get(img, kRowFwd, 1, c, lane)));
-        t = fadd(t, fmul(ipv, tr.get(img, kRowFwd, 2, c, lane)));
-        t = fadd(t, fmul(dpv, tr.get(img, kRowFwd, 3, c, lane)));
-        mv[c] = fmul(t, eo[c]);
-        iv[c] = k < M ? fmul(fadd(fmul(mp[c], tr.get(img, kRowFwd, 4, c, lane)), fmul(ip[c], tr.get(img, kRowFwd, 5, c, lane))), ins)
-                      : 0.f;
-      }
-      const float mcl0 = __shfl_up_sync(kFull, mv[VC - 1], 1);
-      const float mcl = lane ? mcl0 : 0.f;
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        a[c] = fmul(c ? mv[c - 1] : mcl, tr.get(img, kRowFwd, 6, c, lane));
-        pdd[c] = tr.get(img, kRowFwd, 7, c, lane);
-      }
-      float dcar = 0.f, xe = 0.f;
-      {
-        // lane transfer D_out = A + B D_in, then an inclusive scan over lanes
-        float A = 0.f, B = 1.f;
-#pragma unroll
-        for (int c = 0; c < VC; c++) {
-          A = fadd(a[c], fmul(A, pdd[c]));
-          B = fmul(B, pdd[c]);
-        }
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const float Au = __shfl_up_sync(kFull, A, o), Bu = __shfl_up_sync(kFull, B, o);
-          if (lane >= o) {
-            A = fadd(A, fmul(B, Au));
-            B = fmul(B, Bu);
-          }
-        }
-        const float din = __shfl_up_sync(kFull, A, 1);
-        dcar = lane ? din : 0.f;
-        float xl = 0.f;
-#pragma unroll
-        for (int c = 0; c < VC; c++) {
-          const float d = fadd(a[c], fmul(dcar, pdd[c]));
-          dv[c] = d;
-          xl = fadd(xl, fadd(mv[c], d));
-          dcar = d;
-        }
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) xl = fadd(xl, __shfl_xor_sync(kFull, xl, o));
-        xe = xl;
-      }
-      if (lane >= nl) {
-#pragma unroll
-        for (int c = 0; c < VC; c++) dv[c] = 0.f;
-      }
-      xj = fadd(fmul(xj, ploop), fmul(xe, 0.5f));
-      xc = fadd(fmul(xc, ploop), fmul(xe, 0.5f));
-      xn = fmul(xn, ploop);
-      xb = fadd(fmul(xn, pmove), fmul(xj, pmove));
-      if (xe > 1.0e4f) {
-        const float inv = __fdiv_rn(1.0f, xe);
-#pragma unroll
-        for (int c = 0; c < VC; c++) {
-          mv[c] = fmul(mv[c], inv);
-          iv[c] = fmul(iv[c], inv);
-          dv[c] = fmul(dv[c], inv);
-        }
-        xn = fmul(xn, inv);
-        xb = fmul(xb, inv);
-        xj = fmul(xj, inv);
-        xc = fmul(xc, inv);
-        lnscale += log((double)xe);
-      }
-#pragma unroll
-      for (int c = 0; c < VC; c++) {
-        mp[c] = mv[c];
-        ip[c] = iv[c];
-        dp[c] = dv[c];
-        eo[c] = eon[c];
-      }
-      x = xnext;
-    }
-    if (lane == 0) {
-      const float v = fmul(xc, pmove);
-      const float fsc = (L > 0 && M > 0) ? (float)((double)(v > 0.f ? logf(v) : SX_NEG_INF) + lnscale) : SX_NEG_INF;
-      r.fwd = fsc;
-      const float sl = slack + 2.0f * (float)(L + 1) * (float)(2 * M + 6 * VC + 64) * 5.9604645e-8f / kLn2;
-      if (bits_stat(fsc, r.filtersc) >= thr[r.p].s3 - sl) push_pair(r, bin, out, out_bins, out_counts, overflow);
     }
   }
 }

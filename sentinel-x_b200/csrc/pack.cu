@@ -63,12 +63,9 @@ int choose_vit16_shape(int m) {
   return -1;
 }
 
-// Forward/Backward pass kernels run one warp per pair in one-warp CTAs, so a
-// warp that finishes frees its SM slot at once instead of holding it until
-// the longest pair of a larger CTA is done.
-int warp_ctas(int num_sms, unsigned n) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)n, (int64_t)num_sms * 32));
-}
+// A CTA per pair: one that finishes frees its place on the SM at once.  (The
+// kernel strides over what a capped grid leaves.)
+unsigned scan_ctas(unsigned n) { return std::max(1u, std::min(n, 1u << 20)); }
 
 // Exact row pass shape of a profile: the narrowest that covers M.
 int choose_xshape(int m) {
@@ -169,12 +166,8 @@ void pack_images(const ProfileHost& h, const DevProfile& d, float4* msv, float4*
           base[((size_t)r * vc + c) * 32 + l] = k <= m ? f(k) : pad;
         }
     };
-    for (int x = 0; x < 25; x++) {
-      put(sxk::kRowMsc + x, [&](int k) { return h.msc_row(x)[k]; }, kNegInf);
-      put(sxk::kRowMo + x, [&](int k) { return h.mo_row(x)[k]; }, 0.0f);
-    }
+    for (int x = 0; x < 25; x++) put(sxk::kRowMsc + x, [&](int k) { return h.msc_row(x)[k]; }, kNegInf);
     const auto& t = h.t;
-    const auto& p = h.p;
     auto shl = [&](const std::vector<float>& v) { return [&v](int k) { return v[k - 1]; }; };
     auto at = [&](const std::vector<float>& v) { return [&v](int k) { return v[k]; }; };
     put(sxk::kRowVit + 0, shl(t[TMM]), kNegInf);
@@ -185,22 +178,6 @@ void pack_images(const ProfileHost& h, const DevProfile& d, float4* msv, float4*
     put(sxk::kRowVit + 5, at(t[TII]), kNegInf);
     put(sxk::kRowVit + 6, shl(t[TMD]), kNegInf);
     put(sxk::kRowVit + 7, shl(t[TDD]), kNegInf);
-    put(sxk::kRowFwd + 0, at(p[TBM]), 0.0f);
-    put(sxk::kRowFwd + 1, shl(p[TMM]), 0.0f);
-    put(sxk::kRowFwd + 2, shl(p[TIM]), 0.0f);
-    put(sxk::kRowFwd + 3, shl(p[TDM]), 0.0f);
-    put(sxk::kRowFwd + 4, at(p[TMI]), 0.0f);
-    put(sxk::kRowFwd + 5, at(p[TII]), 0.0f);
-    put(sxk::kRowFwd + 6, shl(p[TMD]), 0.0f);
-    put(sxk::kRowFwd + 7, shl(p[TDD]), 0.0f);
-    put(sxk::kRowBwd + 0, at(p[TMM]), 0.0f);
-    put(sxk::kRowBwd + 1, at(p[TMI]), 0.0f);
-    put(sxk::kRowBwd + 2, at(p[TMD]), 0.0f);
-    put(sxk::kRowBwd + 3, at(p[TIM]), 0.0f);
-    put(sxk::kRowBwd + 4, at(p[TII]), 0.0f);
-    put(sxk::kRowBwd + 5, at(p[TDM]), 0.0f);
-    put(sxk::kRowBwd + 6, at(p[TDD]), 0.0f);
-    put(sxk::kRowBwd + 7, at(p[TBM]), 0.0f);
   }
 }
 
@@ -369,6 +346,7 @@ void pack_profiles(sx_profiles* P) {
       d.vbin = d.vshape = -1;
       d.xshape = choose_xshape(h.m);
       d.x_off = x_total;
+      d.x_width = d.xshape >= 0 ? xwidth(d.xshape) : 0;
       if (d.xshape >= 0) x_total += (int64_t)ximage_rows(h.m) * xwidth(d.xshape);
       d.msv_off = msv_total;
       d.vfb_off = vfb_total;
@@ -395,6 +373,7 @@ void pack_profiles(sx_profiles* P) {
     vfb_total += (int64_t)sxk::kImgRows * 32 * d.vc;
     d.xshape = choose_xshape(h.m);
     d.x_off = x_total;
+    d.x_width = xwidth(d.xshape);
     x_total += (int64_t)ximage_rows(h.m) * xwidth(d.xshape);
     d.vshape = shape_for(P->eng, 1, h.m);
     if (d.vshape < 0) throw CudaError{SX_EINVAL, "profile '" + h.name + "' too long for the Viterbi shapes"};

@@ -582,9 +582,9 @@ void launch_stage(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets*
                                           S.overflow.p, P->d_prof.p, E->thr.p, P->d_vit.p, T->d_res.p, T->d_off.p,
                                           T->d_len.p, T->d_xsc.p, kSlackBits, nullptr, S.cursor.p);
       } else
-        K.fwd_scan[b]<<<warp_ctas(E->num_sms, nin[b]), 32, 0, s>>>(S.lists[2].p, cin, S.bins[2].p, b, S.lists[3].p,
+        K.fwd_scan[b]<<<scan_ctas(nin[b]), 32 * scan_warps(b), 0, s>>>(S.lists[2].p, cin, S.bins[2].p, b, S.lists[3].p,
                                                                S.bins[3].p, cout,
-                                        S.overflow.p, P->d_prof.p, E->thr.p, P->d_vfb.p, T->d_res.p, T->d_off.p,
+                                        S.overflow.p, P->d_prof.p, E->thr.p, P->d_x.p, T->d_res.p, T->d_off.p,
                                         T->d_len.p, T->d_xsc.p, kSlackBits);
       E->stats.kernel_launches++;
     }

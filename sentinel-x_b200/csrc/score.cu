@@ -306,9 +306,9 @@ int sx_score_prescreens(sx_engine* e, const sx_profiles* p, const sx_targets* t,
         CK(cudaMemsetAsync(e->counts.p + 3 * kMaxBins, 0, sizeof(unsigned) * kMaxBins, s));
         for (int b = 0; b < kNumVbins; b++) {
           if (!cnt[b]) continue;
-          K.fwd_scan[b]<<<warp_ctas(e->num_sms, cnt[b]), 32, 0, s>>>(
+          K.fwd_scan[b]<<<scan_ctas(cnt[b]), 32 * scan_warps(b), 0, s>>>(
               S.lists[2].p, e->counts.p + 2 * kMaxBins, S.bins[2].p, b, S.lists[3].p, S.bins[3].p,
-              e->counts.p + 3 * kMaxBins, e->overflow.p, p->d_prof.p, e->thr.p, p->d_vfb.p, t->d_res.p, t->d_off.p,
+              e->counts.p + 3 * kMaxBins, e->overflow.p, p->d_prof.p, e->thr.p, p->d_x.p, t->d_res.p, t->d_off.p,
               t->d_len.p, t->d_xsc.p, kSlackBits);
         }
         CK(cudaGetLastError());

@@ -75,6 +75,10 @@ constexpr int vit16_threads(const Vit16Shape&) { return 128; }
 // Warp-chunked column counts (columns per lane, 32 lanes per pair).
 constexpr int kVcBins[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
 constexpr int kNumVbins = sizeof(kVcBins) / sizeof(kVcBins[0]);
+// Forward pre-screen: four columns a thread of one warp up to 128 columns, eight
+// a thread above
+constexpr int kScanNarrow = 4;
+constexpr int scan_warps(int b) { return (kVcBins[b] + 7) / 8; }
 
 // Exact row passes (exact_rows.cuh): columns per thread and warps per team; a
 // profile takes the narrowest shape that covers M.  A row's latency is its
