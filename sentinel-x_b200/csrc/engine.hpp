@@ -734,7 +734,8 @@ struct RegionPassStats {
   double cells = 0;
 };
 
-int vit_blocks(int num_sms, int shape, unsigned n);
+int vit_threads(int num_sms, int shape, unsigned n);
+int vit_blocks(int num_sms, int shape, unsigned n, int threads);
 unsigned scan_ctas(unsigned n);
 std::vector<int16_t> default_shape_table(int kind);
 int shape_for(const sx_engine* E, int kind, int m);

@@ -47,12 +47,20 @@ int choose_vit_shape(int m) {
   }
   return best;
 }
-// Persistent grid for a lane-group Viterbi launch of `n` pairs: the CTAs that
-// fit on the GPU at once (two per SM for C <= 16, whose registers are capped
-// at 128, one otherwise), fewer if the pairs need fewer groups.
-int vit_blocks(int num_sms, int shape, unsigned n) {
+// Threads of a CTA of a lane-group Viterbi launch of `n` pairs: as few warps as
+// put the pairs on all SMs, up to eight.  A few pairs' rows are one chain each,
+// and warps on one SM wait for one another's issue slots (50 pairs of
+// 100 columns 0.50 -> 0.47 ms).
+int vit_threads(int num_sms, int shape, unsigned n) {
+  const int64_t warps = ((int64_t)n * kVitShapes[shape].g + 31) / 32;
+  return 32 * (int)std::max<int64_t>(1, std::min<int64_t>(8, (warps + num_sms - 1) / num_sms));
+}
+// Its persistent grid: the CTAs that fit on the GPU at once (two per SM for
+// C <= 16, whose registers are capped at 128, one otherwise), fewer if the
+// pairs need fewer groups.
+int vit_blocks(int num_sms, int shape, unsigned n, int threads) {
   const int g = kVitShapes[shape].g, per_sm = vit_ctas_per_sm(kVitShapes[shape]);
-  return (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n * g + 255) / 256, (int64_t)num_sms * per_sm));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n * g + threads - 1) / threads, (int64_t)num_sms * per_sm));
 }
 
 // Packed Viterbi pre-screen shape of a profile: the narrowest that covers M;

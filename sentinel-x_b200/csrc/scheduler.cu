@@ -577,8 +577,9 @@ void launch_stage(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets*
         continue;
       }
       if (si == 1) {
-        const int vblocks = vit_blocks(E->num_sms, b, nin[b]);
-        K.vitg[b]<<<vblocks, 256, 0, s>>>(S.lists[1].p, cin, S.bins[1].p, b, S.lists[2].p, S.bins[2].p, cout,
+        const int vthreads = vit_threads(E->num_sms, b, nin[b]);
+        const int vblocks = vit_blocks(E->num_sms, b, nin[b], vthreads);
+        K.vitg[b]<<<vblocks, vthreads, 0, s>>>(S.lists[1].p, cin, S.bins[1].p, b, S.lists[2].p, S.bins[2].p, cout,
                                           S.overflow.p, P->d_prof.p, E->thr.p, P->d_vit.p, T->d_res.p, T->d_off.p,
                                           T->d_len.p, T->d_xsc.p, kSlackBits, nullptr, S.cursor.p);
       } else
@@ -593,12 +594,15 @@ void launch_stage(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets*
   CK(cudaGetLastError());
 }
 
+constexpr double kVitCtas = 4;
 // Packed Viterbi pre-screen of a block's bias-filter survivors (profiles
 // `prof`, per-profile lists in `vs`, `count[p - p0]` pairs in each): a
-// profile's list is cut into strided sub-tiles of about 8 rounds of the pairs a
+// profile's list is cut into strided sub-tiles of at most 8 rounds of the pairs a
 // CTA holds at once (with the longest targets of a tile first, 4 to 24 rounds
 // differ by 3% on the Pfam-scale search; a marker-set genome, whose lists are
-// short, takes 6.1 ms at 8 and 7.2 at 24), larger M first, one launch per shape
+// short, takes 6.1 ms at 8 and 7.2 at 24), of fewer when 8 would leave the GPU
+// without kVitCtas CTAs an SM (50 pairs of one profile 0.43 -> 0.27 ms, spread over
+// the SMs), larger M first, one launch per shape
 // on the slot's high-priority auxiliary streams; pairs whose bound passes F2 go
 // to the Viterbi lists (lists[1]), S.vstats collects cells and passes.
 void launch_vprescreen(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T, const std::vector<int>& prof,
@@ -607,11 +611,17 @@ void launch_vprescreen(sx_engine* E, Slot& S, const sx_profiles* P, const sx_tar
   std::vector<std::vector<sxk::VitTile>> by_shape(kNumVit16Shapes);
   std::vector<int> order(prof);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return P->h[a].m > P->h[b].m; });
+  auto round_of = [&](int pi) {  // pairs a CTA holds at once
+    const Vit16Shape& v = kVit16Shapes[P->dp[pi].qv_shape];
+    return (unsigned)(vit16_threads(v) / 32) * (unsigned)(32 / v.g) * 2u * (unsigned)v.w;
+  };
+  double rounds = 0;
+  for (int pi : order) rounds += std::ceil((double)std::min(count[pi - vs.p0], vs.cap) / round_of(pi));
+  const unsigned deep = (unsigned)std::min(8.0, std::max(1.0, rounds / (kVitCtas * E->num_sms)));
   for (int pi : order) {
     const unsigned n = std::min(count[pi - vs.p0], vs.cap);
     if (!n) continue;
-    const Vit16Shape& v = kVit16Shapes[P->dp[pi].qv_shape];
-    const unsigned per = 8u * (unsigned)(vit16_threads(v) / 32) * (unsigned)(32 / v.g) * 2u * (unsigned)v.w;  // pairs per sub-tile
+    const unsigned per = deep * round_of(pi);  // pairs per sub-tile
     const int nsub = (int)std::min<unsigned>(256u, (n + per - 1) / per);
     for (int q = 0; q < nsub; q++) by_shape[P->dp[pi].qv_shape].push_back({pi, q, nsub, 0});
   }

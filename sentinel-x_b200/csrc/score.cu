@@ -109,8 +109,9 @@ int sx_score_pairs(sx_engine* e, const sx_profiles* p, const sx_targets* t, cons
         CK(cudaEventRecord(e->ev[0], s));
         for (int b = 0; b < kNumVitShapes; b++) {
           if (!cnt[b]) continue;
-          const int blocks = vit_blocks(e->num_sms, b, cnt[b]);
-          K.vitg[b]<<<blocks, 256, 0, s>>>(e->lists[0].p, e->counts.p, e->bins[0].p, b, nullptr, nullptr, nullptr,
+          const int threads = vit_threads(e->num_sms, b, cnt[b]);
+          const int blocks = vit_blocks(e->num_sms, b, cnt[b], threads);
+          K.vitg[b]<<<blocks, threads, 0, s>>>(e->lists[0].p, e->counts.p, e->bins[0].p, b, nullptr, nullptr, nullptr,
                                            e->overflow.p, p->d_prof.p, e->thr.p, p->d_vit.p, t->d_res.p, t->d_off.p,
                                            t->d_len.p, t->d_xsc.p, 0.f, e->scores.p, e->sl[0].cursor.p);
         }
