@@ -551,7 +551,9 @@ namespace sxk {
 // I descending (each needs the old values at k and k-1), then the D chain
 // ascending with carry -inf at the lane boundary, then carries are pushed
 // across the group's lanes until nothing changes (exact, as fl(x+t) is
-// monotone in x).  All groups step rows in lock step; a group that finishes a
+// monotone in x, and so is running the carry's own chain beside the lane's D and
+// taking the larger, four columns at a time; one column at a time, with a test
+// and a branch each, took more than the rest of the row).  All groups step rows in lock step; a group that finishes a
 // pair takes the next one, and the score is latched at its last row.
 // ===========================================================================
 template <int G, int C, bool RT>
@@ -719,24 +721,23 @@ __global__ void __launch_bounds__(256, (C <= 16 && !(RT && C > 8)) ? 2 : 1) vite
         settled = true;
         break;
       }
-      bool go = true;
+      // Measured on B200, column by column -> as here (296 profiles of one length x
+      // 12,000 targets, ms): M = 100 2.12 -> 1.55, 250 2.53 -> 1.40, 600 4.66 ->
+      // 3.37, 1500 8.8 -> 7.3; the Pfam-scale search's exact Viterbi 9.2 -> 6.4.
+      // D[c] = max(own D, the carry's chain), four columns at a time: a carry that
+      // does not win the fourth wins none after it
+      bool go = need;
 #pragma unroll
       for (int c4 = 0; c4 < NC4; c4++) {
         if (go) {
           const float4 tdd = T(7, c4);
+          float x[4];
 #pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const int c = 4 * c4 + e;
-            if (go) {
-              const float cand = fadd(cin, pick(tdd, e));
-              if (cand > dp[c]) {
-                dp[c] = cand;
-                cin = cand;
-              } else {
-                go = false;
-              }
-            }
-          }
+          for (int e = 0; e < 4; e++) x[e] = fadd(e ? x[e - 1] : cin, pick(tdd, e));
+          cin = x[3];
+          go = cin > dp[4 * c4 + 3];
+#pragma unroll
+          for (int e = 0; e < 4; e++) dp[4 * c4 + e] = fmx(dp[4 * c4 + e], x[e]);
         }
       }
     }
