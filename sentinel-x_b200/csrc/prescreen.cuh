@@ -392,9 +392,9 @@ namespace sxk {
 // operation on two cells, W words share the transitions read from shared
 // memory and fill each other's latency, and rows run in blocks of four without
 // control flow:
-//   * the D chain runs in every lane at once, first without a carry, then from
-//     the carry its left neighbour ended with, until no lane's carry changes
-//     (integers: the fixed point is the sequential chain);
+//   * the D chain runs in every lane at once, first without a carry, then the
+//     carries their left neighbours ended with run beside it until none changes
+//     a lane's first column (integers: the fixed point is the sequential chain);
 //   * N, J and B as in the MSV pre-screen: base = max(N, J) decays, a vote finds
 //     the rows whose E raises it, J is kept per lane and combined at the end;
 //   * rows past a target's end in its last block read a score row of -24 nats
@@ -406,8 +406,9 @@ namespace sxk {
 // survivors of 12,000 targets; before: one word, carries pushed column by
 // column, specials and a butterfly every row, list order): M = 60 4.3 -> 1.5
 // ms, 100 5.2 -> 2.4, 208 7.5 -> 3.7, 300 14.2 -> 5.5, and the Pfam-scale
-// search's 61 -> 34 ms.  M = 513 to 1536, exact before (600: 35 ms, 1000: 44),
-// is pre-screened with one word: 1000 11.7 + 6.0 ms exact; 48 columns a lane
+// search's 61 -> 33 ms (34 with the chains of all terms run again from every
+// carry, 36 with a branch around lanes whose carry does not win).  M = 513 to 1536, exact before (600: 35 ms, 1000: 44),
+// is pre-screened with one word: 1000 11.7 + 4.7 ms exact; 48 columns a lane
 // spill, but still run 1.8 times the exact kernel's cells (a marker-set
 // genome's Viterbi stage 18.3 -> 10.5 ms).
 //
@@ -693,9 +694,7 @@ __global__ void __launch_bounds__(128, (C * W <= 16 ? 3 : 2)) vit16_kernel(
         if (j == 0) ml[w] = il[w] = kV16Init2;
         cin[w] = j ? kV16Low2 : kV16Init2;
       }
-      bool again;
-      int it = 0;
-      do {
+      {
         unsigned d[W];
 #pragma unroll
         for (int w = 0; w < W; w++) d[w] = cin[w];
@@ -710,15 +709,31 @@ __global__ void __launch_bounds__(128, (C * W <= 16 ? 3 : 2)) vit16_kernel(
               dp[w][c] = d[w] = __viaddmax_s16x2(d[w], pick(tdd, e), add2s16(c ? m[w][c - 1] : ml[w], pick(tmd, e)));
           }
         }
-        again = false;
+      }
+      // a lane's D is the larger of its own chain and its carry's; every round that changes a
+      // lane's end moves the carries one lane on, so the vote ends the loop.
+      for (int it = 0; it < G; it++) {
+        const unsigned t0 = T(7, 0).x;
+        bool need = false;
 #pragma unroll
         for (int w = 0; w < W; w++) {
-          const unsigned up = __shfl_up_sync(kFull, d[w], 1, G);
-          const unsigned nc = j ? up : kV16Init2;
-          again |= nc != cin[w];
-          cin[w] = nc;
+          const unsigned up = __shfl_up_sync(kFull, dp[w][C - 1], 1, G);
+          cin[w] = j ? up : kV16Init2;
+          need |= __viaddmax_s16x2(cin[w], t0, dp[w][0]) != dp[w][0];
         }
-      } while (__any_sync(kFull, again) && ++it < G);
+        if (!__any_sync(kFull, need)) break;
+        unsigned d[W];
+#pragma unroll
+        for (int w = 0; w < W; w++) d[w] = cin[w];
+#pragma unroll
+        for (int c4 = 0; c4 < NC4; c4++) {
+          const uint4 tdd = T(7, c4);
+#pragma unroll
+          for (int e = 0; e < 4; e++)
+#pragma unroll
+            for (int w = 0; w < W; w++) dp[w][4 * c4 + e] = d[w] = __viaddmax_s16x2(d[w], pick(tdd, e), dp[w][4 * c4 + e]);
+        }
+      }
 #pragma unroll
       for (int w = 0; w < W; w++) dpl[w] = cin[w];
       // ---- the next row's pre and I, in place ----
