@@ -210,7 +210,10 @@ __device__ __forceinline__ float team_sum(const float* t, int n, XShared& sh) {
 // A sum that is infinite or not a number is walked too.
 // Measured at M = 1,500 (12 warps): the row passes of 1,800 targets 6.64 ->
 // 4.57 ms, their envelope matrices 7.47 -> 5.32 ms; at M = 500 (4 warps) 3.29 ->
-// 2.90 and 3.65 -> 2.95 ms.
+// 2.90 and 3.65 -> 2.95 ms.  With a run's two integers loaded beside the thread's
+// terms, not after the sum's last bit is known, M = 2,100 to 2,500: 10.5 -> 9.5
+// and 12.9 -> 11.7 ms (a software pipeline over the walk's steps: slower, 42
+// against 37 ms for that search).
 template <int C>
 __device__ __forceinline__ float team_sum_wide(const float (&t)[C], const float* T, XShared& sh, XSumShared& ss) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -260,9 +263,13 @@ __device__ __forceinline__ float team_sum_wide(const float (&t)[C], const float*
   if (lane == 0) ss.odd[warp] = om;
   __syncthreads();
   if (warp == 0) {
+    // lane q: warp q's odd threads and the run up to its end
+    const unsigned masks = lane < nw ? ss.odd[lane] : 0u;
+    const int r0 = lane < nw ? ss.inc[0][32 * lane + 31] : 0, r1 = lane < nw ? ss.inc[1][32 * lane + 31] : 0;
     int s = 0;  // the sum's bits
     for (int q = 0; q < nw; q++) {
-      unsigned m = ss.odd[q];
+      unsigned m = __shfl_sync(kFull, masks, q);
+      const int t0 = __shfl_sync(kFull, r0, q), t1 = __shfl_sync(kFull, r1, q);
       int at = 0;
       while (m) {
         const int jn = __ffs(m) - 1, id = 32 * q + jn;
@@ -271,22 +278,25 @@ __device__ __forceinline__ float team_sum_wide(const float (&t)[C], const float*
         float4 x[C / 4];
 #pragma unroll
         for (int u = 0; u < C / 4; u++) x[u] = p[u];
-        if (jn > at) s += ss.inc[s & 1][id - 1];
+        if (jn > at) {
+          const int i0 = ss.inc[0][id - 1], i1 = ss.inc[1][id - 1];
+          s += s & 1 ? i1 : i0;
+        }
         float v = __int_as_float(s);
 #pragma unroll
         for (int u = 0; u < C / 4; u++) v = fadd(fadd(fadd(fadd(v, x[u].x), x[u].y), x[u].z), x[u].w);
         s = __float_as_int(v);
         at = jn + 1;
       }
-      if (at < 32) s += ss.inc[s & 1][32 * q + 31];
+      if (at < 32) s += s & 1 ? t1 : t0;
     }
     if (lane == 0) sh.sum = __int_as_float(s);
   }
   __syncthreads();
   return sh.sum;
 }
-// Teams from kWideSumWarps on take it: about 1,800 cycles at six warps, the chain
-// 4 a column.
+// Teams from kWideSumWarps on take it; two warps are faster with the chain, 4
+// cycles a column (M = 300, 2,048 pairs: 6.8 ms, 7.7 in parallel).
 constexpr int kWideSumWarps = 3;
 template <int C, bool MULTI>
 __device__ __forceinline__ float row_sum(const float (&t)[C], const float* T, int n, XShared& sh, XSumShared* ss) {
