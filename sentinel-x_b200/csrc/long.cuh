@@ -126,8 +126,8 @@ static __global__ void __launch_bounds__(kPlainThreads) long_viterbi_kernel(
 }
 
 // Forward (src/hmmer/dp.rs:229-298) then Backward (dp.rs:301-392) of every
-// pair, multihit, writing the raw special rows exactly as forward_kernel and
-// backward_kernel do: fwd rows 1..L (N B E J C, rescale factor or 0); bwd
+// pair, multihit, writing the raw special rows exactly as exact_rows_kernel
+// does: fwd rows 1..L (N B E J C, rescale factor or 0); bwd
 // row L (E, C), rows L-1..1 (N B E J C, factor) and the B sum in slot 1 of row 0.
 static __global__ void __launch_bounds__(kPlainThreads) long_rows_kernel(
     const LongPair* __restrict__ pairs, int n, const PlainProfile* __restrict__ pprof, const float* __restrict__ pimg,
