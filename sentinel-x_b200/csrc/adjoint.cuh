@@ -17,7 +17,8 @@
 //   to row i+1 F_M/F_I(i,k) t ins(x_{i+1}) B_I(i+1,k)  (MI II)
 // Every accumulator belongs to one thread (the owner of the transition's target
 // column), so the sums have one order.  D chains are affine scans and row sums
-// butterflies (the adjoint is checked against FP64, not bit for bit).
+// butterflies (the adjoint is checked against FP64, not bit for bit; Backward and
+// the counts take fused multiply-adds, half the roundings).
 //
 // What bounds it: the latency of a row, two barriers each for a Backward and a
 // recomputed Forward row.  Four columns a thread keep the transitions and
@@ -28,7 +29,8 @@
 // compiler not knowing them apart.  adjoint_out_kernel turns the scratch rows
 // into the caller's.  Measured on B200, 4,096 pairs of M = 300, L 400-950, in
 // one launch: kernel B 59.5 -> 11.4 ms, kernel A 2.8 -> 2.6; the call, whose
-// copies and host split now run beside the kernels, 75 -> 17 ms.
+// copies and host split now run beside the kernels, 75 -> 16.4 ms (16.9 without
+// the fused operations).
 #pragma once
 #include "exact_rows.cuh"
 
@@ -58,6 +60,7 @@ struct AdjShared {  // exchange between the warps of a team, by use
 __device__ __forceinline__ void adj_add4(float* p, const float (&v)[4]) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]));
 }
+__device__ __forceinline__ float ffma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) v = fadd(v, __shfl_xor_sync(kFull, v, o));
@@ -343,11 +346,11 @@ __global__ void __launch_bounds__(32 * kAdjMaxWarps) adjoint_backward_kernel(
   auto d_chain = [&](const float (&al)[C], float e, float (&dc)[C]) -> float {
     float a = 0.f;
 #pragma unroll
-    for (int c = C - 1; c >= 0; c--) a = fadd(fadd(al[c], e), fmul(T.dd[c], a));
+    for (int c = C - 1; c >= 0; c--) a = ffma(T.dd[c], a, fadd(al[c], e));
 #pragma unroll
     for (int q = 0; q < 5; q++) {
       const float n = __shfl_down_sync(kFull, a, 1 << q);
-      if (lane + (1 << q) < 32) a = fadd(a, fmul(T.dn[q], n));
+      if (lane + (1 << q) < 32) a = ffma(T.dn[q], n, a);
     }
     float cin = __shfl_down_sync(kFull, a, 1);
     if (lane == 31) cin = 0.f;
@@ -358,12 +361,12 @@ __global__ void __launch_bounds__(32 * kAdjMaxWarps) adjoint_backward_kernel(
       }
       __syncthreads();
       float in = 0.f;  // D right of the warp's last column
-      for (int q = nw - 1; q > warp; q--) in = fadd(sh.a[q], fmul(in, sh.edge[0][q]));
-      cin = fadd(cin, fmul(T.dn_in, in));
+      for (int q = nw - 1; q > warp; q--) in = ffma(in, sh.edge[0][q], sh.a[q]);
+      cin = ffma(T.dn_in, in, cin);
     }
     float v = cin;
 #pragma unroll
-    for (int c = C - 1; c >= 0; c--) dc[c] = v = fadd(fadd(al[c], fmul(v, T.dd[c])), e);
+    for (int c = C - 1; c >= 0; c--) dc[c] = v = ffma(v, T.dd[c], fadd(al[c], e));
     return cin;
   };
   for (int i = rows; i >= 1; i--) {
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(32 * kAdjMaxWarps) adjoint_backward_kernel(
       for (int c = 0; c < C; c++) al[c] = ic[c] = inn[c] = 0.f;
       const float dnr = d_chain(al, bxe, dc);
 #pragma unroll
-      for (int c = 0; c < C; c++) mc[c] = fadd(bxe, fmul(c < C - 1 ? dc[c + 1] : dnr, T.md[c]));
+      for (int c = 0; c < C; c++) mc[c] = ffma(c < C - 1 ? dc[c + 1] : dnr, T.md[c], bxe);
     } else {
       const float ins = x != 24 ? 1.f : 0.f;
       float me[C];
@@ -419,7 +422,7 @@ __global__ void __launch_bounds__(32 * kAdjMaxWarps) adjoint_backward_kernel(
 #pragma unroll
       for (int c = 0; c < C; c++) {
         me[c] = fmul(mn[c], eo[c]);
-        b = fadd(b, fmul(fmul(mn[c], T.bm[c]), eo[c]));
+        b = ffma(me[c], T.bm[c], b);
         if (k0 + c < M) top = fmaxf(top, mn[c]);
       }
       if (MULTI && lane == 0) sh.edge[1][warp] = me[0];
@@ -440,10 +443,10 @@ __global__ void __launch_bounds__(32 * kAdjMaxWarps) adjoint_backward_kernel(
         bxc = fmul(bxc, inv);
         lnsb += log((double)top);
       }
-      bxj = fadd(fmul(bxj, ploop), fmul(bxb, pmove));
+      bxj = ffma(bxj, ploop, fmul(bxb, pmove));
       bxc = fmul(bxc, ploop);
-      bxe = fadd(fmul(bxj, 0.5f), fmul(bxc, 0.5f));
-      bxn = fadd(fmul(bxn, ploop), fmul(bxb, pmove));
+      bxe = ffma(bxj, 0.5f, fmul(bxc, 0.5f));
+      bxn = ffma(bxn, ploop, fmul(bxb, pmove));
       float al[C];
 #pragma unroll
       for (int c = 0; c < C; c++) {
@@ -454,8 +457,8 @@ __global__ void __launch_bounds__(32 * kAdjMaxWarps) adjoint_backward_kernel(
 #pragma unroll
       for (int c = 0; c < C; c++) {
         const float mnext = c < C - 1 ? me[c + 1] : me_up, dnext = c < C - 1 ? dc[c + 1] : dnr;
-        mc[c] = fadd(fadd(fadd(fmul(mnext, T.mm[c]), fmul(inn[c], T.mi[c])), bxe), fmul(dnext, T.md[c]));
-        ic[c] = fadd(fmul(mnext, T.imr[c]), fmul(inn[c], T.ii[c]));
+        mc[c] = ffma(dnext, T.md[c], ffma(mnext, T.mm[c], ffma(inn[c], T.mi[c], bxe)));
+        ic[c] = ffma(mnext, T.imr[c], fmul(inn[c], T.ii[c]));
       }
     }
     // ---- accumulate counts (columns past M hold zeros in every Forward row) ----
@@ -479,14 +482,14 @@ __global__ void __launch_bounds__(32 * kAdjMaxWarps) adjoint_backward_kernel(
       gm[c] = fm1[c] * mc[c] * f_ii;
       gi[c] = fi1[c] * ic[c] * f_ii;
       const float bme = ei[c] * mc[c] * f_i0;
-      cbm[c] += fb0 * T.bm[c] * bme;  // B -> M_k
-      cmm[c] += (c ? fm0[c - 1] : l[0]) * (c ? T.mm[c - 1] : T.mm0) * bme;
-      cim[c] += (c ? fi0[c - 1] : l[1]) * (c ? T.imr[c - 1] : T.im0) * bme;
-      cdm[c] += (c ? fd0[c - 1] : l[2]) * (c ? T.dm[c - 1] : T.dm0) * bme;
-      cmd[c] += (c ? fm1[c - 1] : l[3]) * (c ? T.md[c - 1] : md0) * dc[c] * f_ii;
-      cdd[c] += (c ? fd1[c - 1] : l[4]) * (c ? T.dd[c - 1] : dd0) * dc[c] * f_ii;
-      cmi[c] += fm1[c] * T.mi[c] * inn[c] * f_ii;
-      cii[c] += fi1[c] * T.ii[c] * inn[c] * f_ii;
+      cbm[c] = ffma(fb0 * T.bm[c], bme, cbm[c]);  // B -> M_k
+      cmm[c] = ffma((c ? fm0[c - 1] : l[0]) * (c ? T.mm[c - 1] : T.mm0), bme, cmm[c]);
+      cim[c] = ffma((c ? fi0[c - 1] : l[1]) * (c ? T.imr[c - 1] : T.im0), bme, cim[c]);
+      cdm[c] = ffma((c ? fd0[c - 1] : l[2]) * (c ? T.dm[c - 1] : T.dm0), bme, cdm[c]);
+      cmd[c] = ffma((c ? fm1[c - 1] : l[3]) * (c ? T.md[c - 1] : md0) * dc[c], f_ii, cmd[c]);
+      cdd[c] = ffma((c ? fd1[c - 1] : l[4]) * (c ? T.dd[c - 1] : dd0) * dc[c], f_ii, cdd[c]);
+      cmi[c] = ffma(fm1[c] * T.mi[c] * inn[c], f_ii, cmi[c]);
+      cii[c] = ffma(fi1[c] * T.ii[c] * inn[c], f_ii, cii[c]);
     }
     adj_add4(acc + (int64_t)xi * tw, gm);
     adj_add4(acc + (int64_t)(25 + xi) * tw, gi);
