@@ -49,10 +49,6 @@ TeamLaunch team_launch(const sx_engine* E, int shape, int n, int directions) {
   return {dim3((unsigned)((n + t - 1) / t), (unsigned)directions), (unsigned)(32 * t * kXShapes[shape].warps),
           xsmem(shape, t)};
 }
-// Rows the insert-sum kernel prepares at once: as many as its lists have shared
-// memory for.
-int insert_rows(int width) { return std::min<int>(sxk::kInsertRows, (200 << 10) / (2 * 4 * width)); }
-
 // The device passes of a DomainBatch: for every envelope request the
 // full-matrix Forward and Backward (their raw special rows come back to the
 // host), the host's posterior factors, then the posterior / null2 /
@@ -144,7 +140,6 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
       FanOut fan(E, s);
       each_shape([&](int sh, int x0, int cnt) {
         const TeamLaunch t = team_launch(E, sh, cnt, 2);
-        allow_smem((const void*)K.envr[sh], t.smem);
         K.envr[sh]<<<t.grid, t.threads, t.smem, fan.take()>>>(E->env_recs.p + x0, cnt, P->d_prof.p, P->d_x.p, T->d_res.p,
                                                               T->d_off.p, E->env_planes.p, E->env_rows.p);
         launches += 1;
@@ -182,13 +177,9 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
     FanOut fan(E, s);
     each_shape([&](int sh, int x0, int cnt) {
       const TeamLaunch t = team_launch(E, sh, cnt, 1);
-      allow_smem((const void*)K.envoa[sh], t.smem);
       K.envoa[sh]<<<t.grid, t.threads, t.smem, fan.take()>>>(E->env_recs.p + x0, cnt, P->d_prof.p, P->d_x.p,
                                                              E->env_planes.p, E->env_aux.p, E->env_fac.p, E->env_out.p);
-      const int ir = insert_rows(xwidth(sh));
-      const size_t ism = 2 * sizeof(float) * (size_t)ir * xwidth(sh);
-      allow_smem((const void*)sxk::env_insert_kernel, ism);
-      sxk::env_insert_kernel<<<cnt, 32 * (ir + 1), ism, fan.take()>>>(
+      K.envins<<<cnt, 32 * (insert_rows(xwidth(sh)) + 1), insert_smem(sh), fan.take()>>>(
           E->env_recs.p + x0, cnt, P->d_prof.p, E->env_planes.p, E->env_fac.p, E->env_out.p, xwidth(sh));
       launches += 2;
     });
@@ -324,7 +315,6 @@ RegionPassStats region_passes(sx_engine* E, const sx_profiles* P, const sx_targe
       size_t y = x;
       while (y < n && P->dp[reg(order[a + y]).p].xshape == sh) y++;
       const TeamLaunch t = team_launch(E, sh, (int)(y - x), 1);
-      allow_smem((const void*)K.regf[sh], t.smem);
       K.regf[sh]<<<t.grid, t.threads, t.smem, fan.take()>>>(E->env_recs.p + x, (int)(y - x), P->d_prof.p, P->d_x.p,
                                                             T->d_res.p, T->d_off.p, E->env_planes.p, E->env_rows.p);
       st.launches += 1;

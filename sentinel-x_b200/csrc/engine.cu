@@ -87,7 +87,7 @@ int sx_create(const sx_opts* opts, sx_engine** out) {
     }
     note_free_memory(e.get());
     for (int kind = 0; kind < 2; kind++) e->shape_table[kind] = default_shape_table(kind);
-    (void)kernels();
+    allow_shared_memory();
   } catch (const CudaError& ce) {
     return fail(ce.code, ce.msg);
   }

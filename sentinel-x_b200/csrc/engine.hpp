@@ -745,7 +745,7 @@ void append_target(sx_targets* T, const uint8_t* dig, size_t l);
 std::vector<Thresholds> make_thresholds(const ProfileList& H, const SearchOpts& o);
 std::vector<Thresholds> thresholds_of(const sx_profiles* P, const SearchOpts& o);
 void combine_profiles(sx_profiles* P, const sx_profiles* const* sets, size_t n, const SearchOpts& o);
-void allow_smem(const void* kernel, size_t bytes);
+void allow_shared_memory();
 void fork_aux(Streams& X);
 void join_aux(Streams& X);
 void note_free_memory(sx_engine* E);

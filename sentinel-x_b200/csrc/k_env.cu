@@ -19,6 +19,7 @@ void fill_env_tables(KernelTables& t) {
     else if (kXShapes[s].c == 8) put<8, false, sxk::kTrReg>(t, s);
     else put<4, false, sxk::kTrReg>(t, s);
   }
+  t.envins = sxk::env_insert_kernel;
 }
 
 }  // namespace sx

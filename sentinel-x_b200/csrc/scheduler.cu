@@ -9,10 +9,27 @@
 namespace sxe {
 
 
-// Lets a kernel take more shared memory than the default 48 KB (which the
-// dynamic part shares with the kernel's static arrays).
-void allow_smem(const void* kernel, size_t bytes) {
-  if (bytes > (32u << 10)) CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+// Lets the kernels that several row shapes share take the most dynamic shared
+// memory any of their shapes asks for.  The limit belongs to the function in the
+// device's context, which all engines of a process share: set to a shape's own
+// size before each launch, one engine's thread lowered it between another's
+// setting and launch.  Up to 32 KB fit beside a kernel's static arrays unasked.
+void allow_shared_memory() {
+  const auto& K = kernels();
+  std::unordered_map<const void*, size_t> most;
+  auto want = [&](const void* kernel, size_t bytes) { most[kernel] = std::max(most[kernel], bytes); };
+  for (int x = 0; x < kNumXShapes; x++) {
+    const size_t rows = xsmem(x, 1);  // a one-warp shape's CTA of eight teams stays below 32 KB
+    want((const void*)K.xrows[x], rows);
+    want((const void*)K.envr[x], rows);
+    want((const void*)K.regf[x], rows);
+    want((const void*)K.envoa[x], rows);
+    want((const void*)K.envins, insert_smem(x));
+    if (K.wvit[x]) want((const void*)K.wvit[x], wide_viterbi_smem(x));
+  }
+  for (const auto& k : most)
+    if (k.second > (32u << 10))
+      CK(cudaFuncSetAttribute(k.first, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.second));
 }
 
 // Fan independent launches out over the auxiliary streams and join them back
@@ -118,7 +135,6 @@ void queue_rows(sx_engine* E, Slot& S, const sx_profiles* P, const sx_targets* T
     load[a] += o.first;
     const int teams = sh.warps > 1 ? 1 : kRowsWarps;  // per CTA
     const dim3 grid((unsigned)((n + teams - 1) / teams), 2);
-    allow_smem((const void*)K.xrows[x], xsmem(x, teams));
     K.xrows[x]<<<grid, 32 * teams * sh.warps, xsmem(x, teams), S.hi.aux[a]>>>(
         S.rrecs.p + c.first[x], n, P->d_prof.p, P->d_x.p, T->d_res.p, T->d_off.p, T->d_len.p, T->d_xsc.p, S.rows.p);
     E->stats.kernel_launches++;
@@ -696,8 +712,7 @@ void long_scores(sx_engine* E, const sx_profiles* P, const sx_targets* T, const 
     float* to = E->long_out.p + a;
     if (x >= 0) {
       const int threads = 32 * kXShapes[x].warps;
-      const size_t smem = xtrans(x) == sxk::kTrShared ? 8 * sizeof(float) * (size_t)xwidth(x) : 0;
-      allow_smem((const void*)K.wvit[x], smem);
+      const size_t smem = wide_viterbi_smem(x);
       if (viterbi)
         K.wvit[x]<<<n, threads, smem, s>>>(pairs, P->d_prof.p, P->d_x.p, T->d_res.p, T->d_off.p, T->d_len.p, T->d_xsc.p, to);
       else

@@ -100,6 +100,16 @@ constexpr sxk::TransIn xtrans(int s) {
 constexpr size_t xsmem(int s, int teams) {
   return sizeof(float) * (size_t)xwidth(s) * (size_t)(teams + (xtrans(s) == sxk::kTrShared ? 8 : 0));
 }
+// of wide_viterbi_kernel: the transitions
+constexpr size_t wide_viterbi_smem(int s) {
+  return xtrans(s) == sxk::kTrShared ? 8 * sizeof(float) * (size_t)xwidth(s) : 0;
+}
+// Rows the insert-sum kernel prepares at once, as many as its lists have shared
+// memory for, and those lists' bytes.
+constexpr int insert_rows(int width) {
+  return (200 << 10) / (2 * 4 * width) < sxk::kInsertRows ? (200 << 10) / (2 * 4 * width) : sxk::kInsertRows;
+}
+constexpr size_t insert_smem(int s) { return 2 * sizeof(float) * (size_t)insert_rows(xwidth(s)) * (size_t)xwidth(s); }
 
 typedef void (*MsvFn)(const MsvTile*, const DevProfile*, const Thresholds*, const float4*, const uint8_t*,
                       const int64_t*, const int32_t*, const float4*, const int32_t*, float*, const int32_t*, PairRec*,
@@ -125,6 +135,7 @@ typedef void (*EnvRowsFn)(const sxk::EnvRec*, int, const DevProfile*, const floa
                           float*, float*);
 typedef void (*EnvOaFn)(const sxk::EnvRec*, int, const DevProfile*, const float*, float*, float*, const double*,
                         float*);
+typedef void (*EnvInsertFn)(const sxk::EnvRec*, int, const DevProfile*, const float*, const double*, float*, int);
 
 typedef void (*WideFn)(const sxk::LongPair*, const DevProfile*, const float*, const uint8_t*, const int64_t*,
                        const int32_t*, const float4*, float*);
@@ -135,6 +146,7 @@ struct KernelTables {
   EnvRowsFn envr[kNumXShapes];  // envelopes: Forward and Backward matrices
   EnvRowsFn regf[kNumXShapes];  // regions: Forward matrix in the diagonal layout
   EnvOaFn envoa[kNumXShapes];   // envelopes: posteriors, null2, optimal accuracy
+  EnvInsertFn envins;           // envelopes: insert sums, every shape
   VitFn vit[kNumVbins];
   FwdFn fwd_scan[kNumVbins];  // the F3 pre-screen
   XRowsFn xrows[kNumXShapes];  // exact Forward and Backward rows
