@@ -21,7 +21,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 # compile in parallel
 SOURCES = ["engine.cu", "pack.cu", "scheduler.cu", "domain_passes.cu", "score.cu", "static_entry.cu", "k_msv.cu",
            "k_msv16.cu", "k_vit16.cu", "k_vit.cu", "k_vbin.cu", "k_exact.cu", "k_env.cu", "hmmfile.cpp", "domains.cpp"]
-HEADERS = ["engine.hpp", "kernels.cuh", "adjoint.cuh", "forward_scan.cuh", "plain.cuh", "long.cuh", "envelope.cuh", "exact_rows.cuh", "wide.cuh", "internal.hpp", "shapes.hpp", "prescreen.cuh",
+HEADERS = ["engine.hpp", "kernels.cuh", "adjoint.cuh", "forward_scan.cuh", "plain.cuh", "long.cuh", "envelope.cuh", "exact_rows.cuh", "wide.cuh", "host_pools.hpp", "internal.hpp", "shapes.hpp", "prescreen.cuh",
            "tuned_shapes.inc"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 

@@ -1,0 +1,209 @@
+// Host resources an engine keeps between calls: its worker threads, and the
+// page-locked buffers of target sets and row copies.
+#pragma once
+
+#include <cuda_runtime_api.h>
+
+#include <algorithm>
+#include <atomic>
+#include <condition_variable>
+#include <cstddef>
+#include <cstdint>
+#include <cstdlib>
+#include <cstring>
+#include <exception>
+#include <functional>
+#include <list>
+#include <mutex>
+#include <new>
+#include <system_error>
+#include <thread>
+#include <utility>
+#include <vector>
+
+namespace sxe {
+
+// ---- host workers ------------------------------------------------------------
+// The engine's host threads, started with the first loop that needs them and
+// joined with the engine: a search runs several short loops, and fresh threads
+// for each cost it more than the work (15 threads: ~0.2 ms).  Loops of several
+// threads may run at once (the engine thread's and the domain-definition
+// driver's); every caller works on its own loop until it is done.  An exception
+// of a body ends its loop and is thrown to the loop's caller.
+class WorkerPool {
+ public:
+  explicit WorkerPool(int threads) : most_(std::max(0, threads - 1)) {}
+  ~WorkerPool() {
+    {
+      std::lock_guard<std::mutex> g(mu_);
+      stop_ = true;
+    }
+    wake_.notify_all();
+    for (auto& t : th_) t.join();
+  }
+  // f(i) for every i < n on at most `threads` threads, the caller among them.
+  template <typename F>
+  void run(size_t n, int threads, F&& f) {
+    if (n == 0) return;
+    const int helpers = (int)std::min<size_t>({(size_t)std::max(0, threads - 1), (size_t)most_, n - 1});
+    if (helpers == 0) {
+      for (size_t i = 0; i < n; i++) f(i);
+      return;
+    }
+    Loop loop;
+    loop.n = n;
+    loop.room = helpers;
+    loop.body = [&f](size_t i) { f(i); };
+    {
+      std::lock_guard<std::mutex> g(mu_);
+      try {
+        while ((int)th_.size() < most_) th_.emplace_back([this] { work(); });
+      } catch (const std::system_error&) {  // no more threads to be had: fewer help
+      }
+      open_.push_back(&loop);
+    }
+    if (helpers == 1) wake_.notify_one();
+    else wake_.notify_all();
+    loop.drain();
+    std::unique_lock<std::mutex> g(mu_);
+    open_.remove(&loop);  // no helper joins any more
+    idle_.wait(g, [&] { return loop.inside == 0; });
+    if (loop.error) std::rethrow_exception(loop.error);
+  }
+
+ private:
+  struct Loop {
+    size_t n = 0;
+    int room = 0, inside = 0;  // helpers that may still join, helpers at work (under the pool's mutex)
+    std::function<void(size_t)> body;
+    std::atomic<size_t> next{0};
+    std::mutex err_mu;
+    std::exception_ptr error;
+    void drain() {
+      try {
+        for (size_t i; (i = next.fetch_add(1)) < n;) body(i);
+      } catch (...) {
+        next.store(n);
+        std::lock_guard<std::mutex> g(err_mu);
+        if (!error) error = std::current_exception();
+      }
+    }
+  };
+  void work() {
+    std::unique_lock<std::mutex> g(mu_);
+    for (;;) {
+      Loop* l = nullptr;
+      wake_.wait(g, [&] {
+        for (Loop* o : open_)
+          if (o->room > 0 && o->next.load() < o->n) {
+            l = o;
+            return true;
+          }
+        return stop_;
+      });
+      if (!l) return;
+      l->room--;
+      l->inside++;
+      g.unlock();
+      l->drain();
+      g.lock();
+      if (--l->inside == 0) idle_.notify_all();
+    }
+  }
+  const int most_;
+  std::mutex mu_;
+  std::condition_variable wake_, idle_;
+  std::list<Loop*> open_;
+  std::vector<std::thread> th_;
+  bool stop_ = false;
+};
+
+// ---- page-locked buffers -------------------------------------------------------
+// Page-locked host memory for the packed residues of target sets, so their
+// copy to the device runs at the bus's rate rather than through the driver's
+// pageable staging; plain heap memory when the pinned allocation fails.
+// Growing a vector leaves the new elements uninitialised (the packers write
+// every byte).
+template <typename T>
+struct PinnedAlloc {
+  using value_type = T;
+  PinnedAlloc() = default;
+  template <typename U>
+  PinnedAlloc(const PinnedAlloc<U>&) {}
+  // Each block starts with a 64-byte header recording how it was obtained,
+  // so it is freed the same way even after the CUDA context is gone.
+  static constexpr size_t kHead = 64;
+  T* allocate(size_t n) {
+    const size_t bytes = std::max<size_t>(n, 1) * sizeof(T) + kHead;
+    void* p = nullptr;
+    uint32_t pinned = 1;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      pinned = 0;
+      p = std::malloc(bytes);
+      if (!p) throw std::bad_alloc();
+    }
+    std::memcpy(p, &pinned, sizeof pinned);
+    return reinterpret_cast<T*>(static_cast<char*>(p) + kHead);
+  }
+  void deallocate(T* q, size_t) {
+    void* p = reinterpret_cast<char*>(q) - kHead;
+    uint32_t pinned = 0;
+    std::memcpy(&pinned, p, sizeof pinned);
+    if (pinned) {
+      if (cudaFreeHost(p) != cudaSuccess) cudaGetLastError();
+    } else {
+      std::free(p);
+    }
+  }
+  template <typename U>
+  void construct(U* p) noexcept {}  // default-initialise: no fill
+  template <typename U, typename... A>
+  void construct(U* p, A&&... a) {
+    ::new ((void*)p) U(std::forward<A>(a)...);
+  }
+  template <typename U>
+  bool operator==(const PinnedAlloc<U>&) const { return true; }
+  template <typename U>
+  bool operator!=(const PinnedAlloc<U>&) const { return false; }
+};
+using HostBytes = std::vector<uint8_t, PinnedAlloc<uint8_t>>;
+
+// Host buffers of packed residues, recycled across target sets so that a
+// caller streaming batches of targets writes into pages already touched.
+class HostBytePool {
+ public:
+  HostBytes take(size_t bytes) {
+    std::lock_guard<std::mutex> g(mu_);
+    for (size_t i = 0; i < free_.size(); i++)
+      if (free_[i].capacity() >= bytes) {
+        HostBytes v = std::move(free_[i]);
+        free_.erase(free_.begin() + (std::ptrdiff_t)i);
+        v.clear();
+        return v;
+      }
+    HostBytes v;
+    v.reserve(bytes + bytes / 4);  // sizes vary from call to call: grow seldom
+    return v;
+  }
+  // Page-locked memory is not kept without bound: larger buffers are freed.
+  static constexpr size_t kMaxKept = 256u << 20;
+  void give(HostBytes&& v) {
+    if (!v.capacity()) return;
+    if (v.capacity() > kMaxKept) {
+      HostBytes().swap(v);
+      return;
+    }
+    std::lock_guard<std::mutex> g(mu_);
+    free_.push_back(std::move(v));
+    if (free_.size() > 2)  // keep the two largest
+      free_.erase(std::min_element(free_.begin(), free_.end(),
+                                   [](const auto& x, const auto& y) { return x.capacity() < y.capacity(); }));
+  }
+
+ private:
+  std::mutex mu_;
+  std::vector<HostBytes> free_;
+};
+
+}  // namespace sxe
