@@ -413,7 +413,7 @@ struct sx_engine {
   bool destroyed = false;
   BlockPool target_blocks;  // device memory of freed target sets
   HostBytePool target_bytes;  // host residue buffers of freed target sets
-  HostBytePool row_bytes;     // host copies of the row passes
+  HostBytePool row_bytes{256u << 20};  // host copies of the row passes (a chunk, or one very long pair)
   // envelope passes of the host domain definition (used by the host pool's
   // driver thread, one batch at a time)
   cudaStream_t env_stream = nullptr;  // the passes' copies; their launches fan out over the slots' streams
