@@ -3,6 +3,8 @@
 #pragma once
 
 #include <cuda_runtime_api.h>
+#include <sys/types.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
@@ -14,6 +16,7 @@
 #include <exception>
 #include <functional>
 #include <list>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <system_error>
@@ -30,23 +33,30 @@ namespace sxe {
 // threads may run at once (the engine thread's and the domain-definition
 // driver's); every caller works on its own loop until it is done.  An exception
 // of a body ends its loop and is thrown to the loop's caller.
+// The threads belong to the process that started them.  In a child forked from
+// it they do not exist, though the pool's state says so: there a loop runs on its
+// caller alone, and the state is left behind rather than joined.
 class WorkerPool {
  public:
-  explicit WorkerPool(int threads) : most_(std::max(0, threads - 1)) {}
+  explicit WorkerPool(int threads) : most_(std::max(0, threads - 1)), st_(new State) {}
   ~WorkerPool() {
-    {
-      std::lock_guard<std::mutex> g(mu_);
-      stop_ = true;
+    if (foreign()) {
+      (void)st_.release();
+      return;
     }
-    wake_.notify_all();
-    for (auto& t : th_) t.join();
+    {
+      std::lock_guard<std::mutex> g(st_->mu);
+      st_->stop = true;
+    }
+    st_->wake.notify_all();
+    for (auto& t : st_->th) t.join();
   }
   // f(i) for every i < n on at most `threads` threads, the caller among them.
   template <typename F>
   void run(size_t n, int threads, F&& f) {
     if (n == 0) return;
     const int helpers = (int)std::min<size_t>({(size_t)std::max(0, threads - 1), (size_t)most_, n - 1});
-    if (helpers == 0) {
+    if (helpers == 0 || foreign()) {
       for (size_t i = 0; i < n; i++) f(i);
       return;
     }
@@ -54,20 +64,24 @@ class WorkerPool {
     loop.n = n;
     loop.room = helpers;
     loop.body = [&f](size_t i) { f(i); };
+    State& st = *st_;
     {
-      std::lock_guard<std::mutex> g(mu_);
+      std::lock_guard<std::mutex> g(st.mu);
       try {
-        while ((int)th_.size() < most_) th_.emplace_back([this] { work(); });
+        while ((int)st.th.size() < most_) {
+          owner_.store(getpid());
+          st.th.emplace_back([&st] { work(st); });
+        }
       } catch (const std::system_error&) {  // no more threads to be had: fewer help
       }
-      open_.push_back(&loop);
+      st.open.push_back(&loop);
     }
-    if (helpers == 1) wake_.notify_one();
-    else wake_.notify_all();
+    if (helpers == 1) st.wake.notify_one();
+    else st.wake.notify_all();
     loop.drain();
-    std::unique_lock<std::mutex> g(mu_);
-    open_.remove(&loop);  // no helper joins any more
-    idle_.wait(g, [&] { return loop.inside == 0; });
+    std::unique_lock<std::mutex> g(st.mu);
+    st.open.remove(&loop);  // no helper joins any more
+    st.idle.wait(g, [&] { return loop.inside == 0; });
     if (loop.error) std::rethrow_exception(loop.error);
   }
 
@@ -89,17 +103,24 @@ class WorkerPool {
       }
     }
   };
-  void work() {
-    std::unique_lock<std::mutex> g(mu_);
+  struct State {
+    std::mutex mu;
+    std::condition_variable wake, idle;
+    std::list<Loop*> open;
+    std::vector<std::thread> th;
+    bool stop = false;
+  };
+  static void work(State& st) {
+    std::unique_lock<std::mutex> g(st.mu);
     for (;;) {
       Loop* l = nullptr;
-      wake_.wait(g, [&] {
-        for (Loop* o : open_)
+      st.wake.wait(g, [&] {
+        for (Loop* o : st.open)
           if (o->room > 0 && o->next.load() < o->n) {
             l = o;
             return true;
           }
-        return stop_;
+        return st.stop;
       });
       if (!l) return;
       l->room--;
@@ -107,15 +128,16 @@ class WorkerPool {
       g.unlock();
       l->drain();
       g.lock();
-      if (--l->inside == 0) idle_.notify_all();
+      if (--l->inside == 0) st.idle.notify_all();
     }
   }
+  bool foreign() const {
+    const pid_t o = owner_.load();
+    return o && o != getpid();
+  }
   const int most_;
-  std::mutex mu_;
-  std::condition_variable wake_, idle_;
-  std::list<Loop*> open_;
-  std::vector<std::thread> th_;
-  bool stop_ = false;
+  std::unique_ptr<State> st_;
+  std::atomic<pid_t> owner_{0};  // of the threads; 0 before the first
 };
 
 // ---- page-locked buffers -------------------------------------------------------

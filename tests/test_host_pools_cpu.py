@@ -13,6 +13,8 @@ CUDA_INCLUDE = os.path.join(os.path.dirname(os.path.dirname(os.environ.get("NVCC
 PRELUDE = r"""
 #include "host_pools.hpp"
 #include <cstdio>
+#include <sys/wait.h>
+#include <unistd.h>
 #include <cstdlib>
 static size_t locks = 0, locked = 0;
 extern "C" cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
@@ -68,3 +70,46 @@ def test_row_copies_keep_a_bounded_amount(tmp_path):
   CHECK(locks == 3);
   pool.give(pool.take(128 * MB));
   CHECK(locks == 3);""")
+
+
+def test_workers_in_a_forked_child(tmp_path):
+    """A forked child has none of the pool's threads: its loops still run, and
+    the pool (freed with the engine when the child's interpreter exits) waits
+    for nobody.  The parent's pool goes on as before."""
+    _run(tmp_path, r"""
+  WorkerPool pool(4);
+  std::atomic<int> sum{0};
+  pool.run(1000, 4, [&](size_t) { sum++; });
+  CHECK(sum == 1000);
+  const pid_t child = fork();
+  if (child == 0) {
+    alarm(20);
+    {
+      WorkerPool* p = &pool;
+      p->run(1000, 4, [&](size_t) { sum++; });
+      p->~WorkerPool();
+    }
+    _exit(sum == 2000 ? 0 : 2);
+  }
+  int status = 0;
+  CHECK(waitpid(child, &status, 0) == child);
+  CHECK(WIFEXITED(status) && WEXITSTATUS(status) == 0);
+  pool.run(1000, 4, [&](size_t) { sum++; });
+  CHECK(sum == 2000);""")
+
+
+def test_workers_started_after_a_fork(tmp_path):
+    """A pool whose threads a child starts itself is the child's own."""
+    _run(tmp_path, r"""
+  WorkerPool pool(4);
+  std::atomic<int> sum{0};
+  const pid_t child = fork();
+  if (child == 0) {
+    alarm(20);
+    pool.run(1000, 4, [&](size_t) { sum++; });
+    pool.~WorkerPool();
+    _exit(sum == 1000 ? 0 : 2);
+  }
+  int status = 0;
+  CHECK(waitpid(child, &status, 0) == child);
+  CHECK(WIFEXITED(status) && WEXITSTATUS(status) == 0);""")
