@@ -44,7 +44,10 @@ extern "C" {
 #define SX_FLAG_PLAIN 1u /* run the plain one-pair-per-block kernels instead of the batched cascade */
 /* Where the envelope rescoring of domain definition runs (default: chosen per
  * profile block; the device unless the host's share is below what a device
- * pass costs).  Results are identical either way. */
+ * pass costs).  An envelope whose matrices alone exceed the scratch budget (4 x
+ * batch_bytes, at most half of the device memory that was free when the engine
+ * was created) is rescored on the host in any case, and so is the ensemble of a
+ * region above 2 x batch_bytes below.  Results are identical either way. */
 #define SX_FLAG_ENV_DEVICE 2u /* always on the device */
 #define SX_FLAG_ENV_HOST 4u   /* always on the host */
 /* Where the stochastic-trace ensembles of multi-domain regions (200 sampled

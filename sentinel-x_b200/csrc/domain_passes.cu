@@ -56,13 +56,22 @@ TeamLaunch team_launch(const sx_engine* E, int shape, int n, int directions) {
 // bounded by the memory of their matrix planes.  Runs on the host pool's driver thread.
 int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T, std::vector<EnvSource>& srcs,
                         int nthr, PhaseLog* plog) {
-  // every request of every batch, as (batch, request)
+  // Planes of every envelope of a search at once when they fit: each batch
+  // is one round of latency-bound passes (the longest envelope sets its
+  // time) plus a host round trip, so fewer, larger batches finish sooner.
+  const int64_t budget = scratch_budget(E, std::max<int64_t>(4 * E->batch_bytes, 256LL << 20));
+  auto plane_floats = [&](const EnvRequest& q) { return sxk::env_plane_floats(q.j - q.i + 1, xwidth(P->dp[q.p].xshape)); };
+  // every request of every batch, as (batch, request); one whose planes alone
+  // exceed the budget (M = 8,000 x 35,000 residues: 5.7 GB) stays on the host
   std::vector<std::pair<uint32_t, uint32_t>> items;
   for (size_t b = 0; b < srcs.size(); b++) {
     const size_t nr = srcs[b].reqs->size();
     srcs[b].F->assign(nr, EnvFactors{});
     srcs[b].D->assign(nr, EnvDeviceOut{});
-    for (size_t r = 0; r < nr; r++) items.emplace_back((uint32_t)b, (uint32_t)r);
+    for (size_t r = 0; r < nr; r++) {
+      if (plane_floats((*srcs[b].reqs)[r]) * (int64_t)sizeof(float) > budget) (*srcs[b].F)[r].host = true;
+      else items.emplace_back((uint32_t)b, (uint32_t)r);
+    }
   }
   const size_t nr = items.size();
   int64_t launches = 0;
@@ -72,10 +81,6 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
   auto out_of = [&](size_t x) -> EnvDeviceOut& { return (*srcs[items[x].first].D)[items[x].second]; };
   const auto& K = kernels();
   cudaStream_t s = E->env_stream;
-  // Planes of every envelope of a search at once when they fit: each batch
-  // is one round of latency-bound passes (the longest envelope sets its
-  // time) plus a host round trip, so fewer, larger batches finish sooner.
-  const int64_t budget = scratch_budget(E, std::max<int64_t>(4 * E->batch_bytes, 256LL << 20));
   std::vector<size_t> order(nr);
   std::iota(order.begin(), order.end(), (size_t)0);
   std::stable_sort(order.begin(), order.end(),
@@ -92,7 +97,7 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
       const EnvRequest& q = req(order[b]);
       const int width = xwidth(P->dp[q.p].xshape);
       const int64_t lr = q.j - q.i + 1;
-      const int64_t need = sxk::env_plane_floats(lr, width);
+      const int64_t need = plane_floats(q);
       if (b > a && (planes + need) * (int64_t)sizeof(float) > budget) break;
       sxk::EnvRec r{};
       r.p = q.p;
@@ -214,9 +219,15 @@ int64_t envelope_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
 RegionPassStats region_passes(sx_engine* E, const sx_profiles* P, const sx_targets* T,
                               std::vector<RegionSource>& srcs, int nthr) {
   RegionPassStats st;
-  std::vector<std::pair<uint32_t, uint32_t>> items;
+  // a batch is one latency-bound wave of 200-trace chains: keep the batches few
+  const int64_t budget = scratch_budget(E, std::max<int64_t>(E->batch_bytes * 2, 1LL << 30));
+  auto plane_floats = [&](const RegionRequest& g) { return 3 * sxk::diag_plane(g.j - g.i + 1, P->h[g.p].m); };
+  std::vector<std::pair<uint32_t, uint32_t>> items, beyond;  // (batch, region); planes within / above the budget
   for (size_t b = 0; b < srcs.size(); b++)
-    for (size_t r = 0; r < srcs[b].regs->size(); r++) items.emplace_back((uint32_t)b, (uint32_t)r);
+    for (size_t r = 0; r < srcs[b].regs->size(); r++)
+      (plane_floats((*srcs[b].regs)[r]) * (int64_t)sizeof(float) > budget ? beyond : items)
+          .emplace_back((uint32_t)b, (uint32_t)r);
+  E->pool->run(beyond.size(), nthr, [&](size_t x) { srcs[beyond[x].first].db->expand(beyond[x].second, {}, nullptr, false); });
   const size_t nr = items.size();
   if (!nr) return st;
   auto reg = [&](size_t x) -> const RegionRequest& { return (*srcs[items[x].first].regs)[items[x].second]; };
@@ -229,8 +240,6 @@ RegionPassStats region_passes(sx_engine* E, const sx_profiles* P, const sx_targe
   }
   const auto& K = kernels();
   cudaStream_t s = E->env_stream;
-  // a batch is one latency-bound wave of 200-trace chains: keep the batches few
-  const int64_t budget = scratch_budget(E, std::max<int64_t>(E->batch_bytes * 2, 1LL << 30));
   constexpr int64_t kPoolPerRegion = 1024;
   // column tables of the profiles that have regions (exact copies of the host's
   // probabilities and match odds), uploaded once
@@ -262,7 +271,7 @@ RegionPassStats region_passes(sx_engine* E, const sx_profiles* P, const sx_targe
     while (b < nr) {
       const RegionRequest& g = reg(order[b]);
       const int64_t lr = g.j - g.i + 1;
-      const int64_t need = 3 * sxk::diag_plane(lr, P->h[g.p].m);
+      const int64_t need = plane_floats(g);
       if (b > a && (planes + need) * (int64_t)sizeof(float) > budget) break;
       sxk::EnvRec f{};
       f.p = g.p;

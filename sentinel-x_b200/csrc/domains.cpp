@@ -1307,6 +1307,11 @@ bool DomainBatch::finish(size_t q, const std::vector<EnvFactors>& F, const std::
   for (const Impl::Pending& e : st.pend) {
     if (e.req < 0) continue;
     const EnvFactors& f = F[(size_t)e.req];
+    if (f.host) {
+      Env v;
+      if (es.rescore(e.i, e.j, st.n2sc, e.null2_done, v.d, v.envsc, v.domcorr)) envs.push_back(v);
+      continue;
+    }
     if (!f.ok) continue;
     const EnvDeviceOut& d = D[(size_t)e.req];
     const int64_t lr = e.j - e.i + 1;

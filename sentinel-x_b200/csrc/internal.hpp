@@ -140,7 +140,8 @@ float backward_score_from_rows(int64_t l, const float* bwd_rows);
 // caller: regions() -> device trace passes -> expand() per region, which
 // clusters the samples on the host) -> requests() -> the caller runs the
 // Forward and Backward envelope passes -> factors() per request -> the caller
-// runs the posterior / null2 / optimal-accuracy pass -> finish() per pair.
+// runs the posterior / null2 / optimal-accuracy pass -> finish() per pair, which
+// also rescores the envelopes whose matrices the caller had no room for.
 struct EnvRequest {
   int32_t pair;     // index of the pair in the batch
   int32_t p, t;     // profile and target indices
@@ -150,6 +151,7 @@ struct EnvRequest {
 };
 struct EnvFactors {
   bool ok = false;  // Forward and Backward envelope scores finite
+  bool host = false;  // left to finish(), which rescores the envelope itself
   float envsc = 0;
   std::vector<double> fac;        // exp(lnF[i] + lnB[i] - lnZ), rows 0..lr
   std::vector<float> pn, pj, pc;  // N/J/C posteriors, rows 0..lr

@@ -1411,15 +1411,14 @@ int run_search(sx_engine* E, const sx_profiles* P, const sx_targets* T, const sx
     rstats = region_passes(E, P, T, rsrc, E->host_threads);
     plog.add("region_passes", t_env);
     env_launches += rstats.launches;
-    for (auto& pb : pending) {
-      pb->reqs = pb->db->requests();
-      n_env += (int64_t)pb->reqs.size();
-    }
+    for (auto& pb : pending) pb->reqs = pb->db->requests();
     std::vector<EnvSource> srcs;
     for (auto& pb : pending) srcs.push_back({pb->db.get(), &pb->reqs, &pb->F, &pb->D});
     const auto t_ep = std::chrono::steady_clock::now();
     env_launches += envelope_passes(E, P, T, srcs, E->host_threads, &plog);
     plog.add("envelope_passes", t_ep);
+    for (auto& pb : pending)
+      for (const EnvFactors& f : pb->F) n_env += !f.host;
     const auto t_fin = std::chrono::steady_clock::now();
     std::vector<std::pair<PendingBatch*, size_t>> todo;
     for (auto& pb : pending)
