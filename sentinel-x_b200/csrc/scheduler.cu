@@ -781,6 +781,15 @@ void long_rows(sx_engine* E, const sx_profiles* P, const sx_targets* T, const st
   }
 }
 
+// Pairs a profile's survivor lists hold at first, of nt targets: after MSV and
+// after the bias filter, into and out of the Forward pre-screen, and the two
+// pre-screens' lists.
+constexpr double kMsvKept = 0.06, kVitKept = 0.01, kScreenKept = 0.05, kScreenLeast = 1024;
+double list_bytes(double nt) {
+  const double screened = std::min(nt, kScreenKept * nt + kScreenLeast);
+  return sizeof(PairRec) * (2 * kMsvKept + 2 * kVitKept) * nt + (sizeof(int32_t) + sizeof(PairRec)) * screened;
+}
+
 // Contiguous ranges of profile indices with about equal filtered DP cells.
 // Each range runs through the device cascade as one block; the host domain
 // definition of a block overlaps the device work of the blocks after it.
@@ -789,8 +798,10 @@ std::vector<std::pair<int, int>> profile_blocks(const sx_engine* E, const sx_pro
   // With the envelopes on the device little host work is left to hide behind a
   // later block, and each block adds its own last waves: Pfam-scale (3e12
   // cells) 342 ms in one block, 351 in two, 367 in three, 395 in five; 800
-  // viral profiles 80 / 82 / 86 / 93.  Larger searches are split to bound the
-  // survivor lists.
+  // viral profiles 80 / 82 / 86 / 93.  From 1.2e13 cells on a search is split all
+  // the same, in two to five, so that a block's decoding on the host does not
+  // wait for the last profile (2.4e13 cells with few hits: 2,197 ms in one block
+  // or two, 2,267 in four equal ones, 2,234 in the four below).
   constexpr double kCellsPerBlock = 6e12;
   constexpr int kMaxBlocks = 5;
   const int np = (int)P->h.size();
@@ -808,9 +819,16 @@ std::vector<std::pair<int, int>> profile_blocks(const sx_engine* E, const sx_pro
   int nb = E->pipeline_blocks > 0 ? E->pipeline_blocks
                                   : (int)std::min<double>(kMaxBlocks, std::max(1.0, std::floor(total / kCellsPerBlock)));
   nb = std::max(1, std::min(nb, nfilt));
+  // filtered profiles of a block: the survivor lists of the two blocks in flight
+  // stay within the scratch budget (unless those of two profiles exceed it)
+  int most = nfilt;
+  if (E->pipeline_blocks <= 0) {
+    const double each = list_bytes((double)T->len.size()), budget = (double)scratch_budget(E, E->batch_bytes);
+    if (nb > 1 || each * nfilt > budget) most = (int)std::min<double>(nfilt, std::max(1.0, budget / 2 / each));
+  }
   // relative block sizes: the last two blocks of an automatic partition of
   // four or more are smaller (0.7 and 0.4 of the others), so the work left
-  // after the last MSV stage is short
+  // after the last MSV stage is short (the figures above)
   std::vector<double> rel(nb, 1.0);
   if (E->pipeline_blocks <= 0 && nb >= 4) {
     rel[nb - 2] = 0.7;
@@ -818,16 +836,21 @@ std::vector<std::pair<int, int>> profile_blocks(const sx_engine* E, const sx_pro
   }
   std::vector<double> cum(nb + 1, 0.0);
   for (int b = 0; b < nb; b++) cum[b + 1] = cum[b] + rel[b];
-  int p0 = 0;
+  int p0 = 0, filtered = 0, cut = 0;
   double acc = 0;
   for (int pi = 0; pi < np; pi++) {
     acc += w[pi];
-    if ((int)out.size() < nb - 1 && acc >= total * cum[out.size() + 1] / cum[nb]) {
+    filtered += th[pi].exact != 0;
+    const bool end = cut < nb - 1 && acc >= total * cum[cut + 1] / cum[nb];
+    if (end) cut++;
+    if (end || filtered == most) {
       out.emplace_back(p0, pi + 1);
       p0 = pi + 1;
+      filtered = 0;
     }
   }
-  if (p0 < np) out.emplace_back(p0, np);
+  if (filtered) out.emplace_back(p0, np);
+  else if (!out.empty()) out.back().second = np;
   return out;
 }
 
@@ -867,9 +890,9 @@ void cascade_launch(sx_engine* E, Slot& S, const sx_profiles* P, const sx_target
   std::vector<double> w1(kMaxBins), w1v(kMaxBins), w3(kMaxBins);
   for (int b = 0; b < kMaxBins; b++) {
     const double pb = R.pairs_in_bin[b], pv = R.pairs_in_vs[b];
-    w1[b] = full ? pb : std::min(pb, scale * (0.06 * pb + 8192));
-    w1v[b] = full ? pv : std::min(pv, scale * (0.06 * pv + 8192));
-    w3[b] = full ? pb : std::min(pb, scale * (0.01 * pb + 4096));
+    w1[b] = full ? pb : std::min(pb, scale * (kMsvKept * pb + 8192));
+    w1v[b] = full ? pv : std::min(pv, scale * (kMsvKept * pv + 8192));
+    w3[b] = full ? pb : std::min(pb, scale * (kVitKept * pb + 4096));
   }
   R.L[0] = make_regions(w1);
   R.L[1] = make_regions(w1v);
@@ -904,7 +927,7 @@ void cascade_launch(sx_engine* E, Slot& S, const sx_profiles* P, const sx_target
     if (!(E->flags & SX_FLAG_NO_PRESCREEN) && nt > 0)
       for (int pi = R.p0; pi < R.p1; pi++)
         if (th[pi].exact && P->dp[pi].q_off >= 0) R.screened.push_back(pi);
-    R.rcap = (unsigned)(full ? nt : std::min<double>((double)nt, scale * (0.05 * (double)nt + 1024)));
+    R.rcap = (unsigned)(full ? nt : std::min<double>((double)nt, scale * (kScreenKept * (double)nt + kScreenLeast)));
     if ((int64_t)(R.p1 - R.p0) * (int64_t)R.rcap >= (int64_t)INT32_MAX) R.screened.clear();
     std::vector<char> scr(R.p1 - R.p0, 0);
     for (int pi : R.screened) scr[pi - R.p0] = 1;

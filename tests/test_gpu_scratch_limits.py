@@ -58,3 +58,34 @@ def test_region_above_the_budget():
     roomy, _, regions_all = _search(m, targets, envelopes="device", traces="device")
     assert regions_all == 2 and regions == 1
     assert small == roomy and len(small[1]) == 4
+
+
+def test_survivor_lists_within_the_budget(capfd, monkeypatch):
+    """420 small profiles x 20,000 short targets reserve 68 MB of survivor
+    lists: more than an engine with the smallest budget (64 MB) holds at once,
+    so it searches in blocks, with the same hits."""
+    rng = np.random.default_rng(3)
+    profs = [synth.sample_profile(rng, 12, f"s{q}") for q in range(420)]
+    targets = [synth.background_seq(rng, int(n)) for n in rng.integers(10, 40, 19900)]
+    targets += [synth.plant(rng, 40, [synth.emit_homolog(rng, profs[4 * q])]) for q in range(100)]
+    lens = np.array([len(t) for t in targets])
+    offs = np.concatenate([[0], np.cumsum(lens)[:-1]])
+    cfg = sxhmm.SearchConfig(sxhmm.Cutoff.evalue(10.0, 10.0)).to_c()
+    text, got, blocks = None, [], []
+    for opts in ({}, {"batch_bytes": 1}):
+        e = sxhmm.Engine(**opts)
+        try:
+            if text is None:
+                synth.calibrate(profs, synth.engine_scorer(e), np.random.default_rng(7), nseq=40)
+                text = "".join(synth.profile_text(p) for p in profs)
+            ps, ts = e.load_text(text), e.targets_digital(np.concatenate(targets), offs, lens)
+            capfd.readouterr()
+            monkeypatch.setenv("SXHMM_PROFILE", "1")
+            hits, doms = e.search(ps, ts, cfg)
+            monkeypatch.delenv("SXHMM_PROFILE")
+            blocks.append(capfd.readouterr().err.count("_cascade="))
+            got.append(([bytes(h) for h in hits], [bytes(d) for d in doms], e.stats()["pairs_out"][:4]))
+        finally:
+            e.close()
+    assert blocks[0] == 1 and blocks[1] >= 3
+    assert got[0] == got[1] and len(got[0][0]) > 0
