@@ -269,14 +269,14 @@ int sx_score_pairs(sx_engine* e, const sx_profiles* p, const sx_targets* t, cons
  *     match scores above +16 nats).
  *   fwd_scan: the F3 pre-screen's Forward score (nats), evaluated in a
  *     parallel order that differs from the reference's; its difference from
- *     the exact Forward score is bounded by (L+1)(2M + 6 VC + 64) 2^-24 nats,
- *     taken twice (VC = columns per lane of the profile's warp-chunked image);
- *     NaN for M > 2048.
+ *     the exact Forward score is bounded by (L+1)(2M + 6 ceil(M/32) + 64) 2^-24
+ *     nats, taken twice; NaN for M > 2048.
  *   vit_bound: the packed int16x2 Viterbi pre-screen's upper bound of the
  *     f32 Viterbi score (nats; +inf when capped).  It is >= the viterbi score
- *     of sx_score_pairs for every pair; NaN for empty targets and for
- *     profiles the pre-screen does not handle (M > 512, profiles outside the
- *     MSV pre-screen, match scores above +16 nats).
+ *     of sx_score_pairs for every pair; NaN for empty targets, for profiles
+ *     the pre-screen does not handle (outside the MSV pre-screen, match scores
+ *     above +16 nats) and for M > 512: a search pre-screens profiles of up to
+ *     1536 nodes, this call reports its bounds up to 512.
  * Any output pointer may be NULL to skip that screen. */
 int sx_score_prescreens(sx_engine* e, const sx_profiles* p, const sx_targets* t, const int32_t* pair_profile,
                         const int32_t* pair_target, size_t npairs, float* msv_bound, float* fwd_scan,

@@ -64,7 +64,9 @@ struct Vit16Shape {
 };
 constexpr Vit16Shape kVit16Shapes[] = {{4, 8, 2}, {8, 8, 2}, {16, 8, 2}, {32, 8, 2}, {32, 16, 2}, {32, 32, 1}, {32, 48, 1}};
 constexpr int kNumVit16Shapes = sizeof(kVit16Shapes) / sizeof(kVit16Shapes[0]);
-constexpr int kVit16BoundM = 512;  // sx_score_prescreens reports bounds up to here
+// sx_score_prescreens reports bounds up to here (its callers expect NaN above);
+// the wider shapes' bounds are checked through searches
+constexpr int kVit16BoundM = 512;
 // dynamic shared memory of one tile: 8 transition rows of 4 bytes per column
 // and kV16Rows score rows of 2 bytes per column
 constexpr int vit16_smem(const Vit16Shape& v) { return (32 + 2 * sxk::kV16Rows) * v.g * v.c; }
