@@ -4,8 +4,9 @@
 // Why: the exact f32 MSV kernel is bound by its ALU pipe and by the 4 bytes of
 // shared memory each DP cell reads.  Here every 32-bit word carries the same
 // column of two profiles (profile a in the low half, b in the high half), so
-// one LDS.128 feeds 8 cells, one max.s16x2 / add.s16x2 pair does 2 cells, and
-// the pair shares the target's residues and the diagonal shuffle.
+// one LDS.128 feeds 8 cells, a fused max(a + b, c) and half a three-input
+// maximum do 2 cells, and the pair shares the target's residues and the diagonal
+// shuffle.
 //
 // Exactness.  The pre-screen never decides a pair; it only rejects pairs whose
 // bound fails F1, and every pair it passes is rescored by the exact kernel.
@@ -25,7 +26,8 @@
 //     bounds of the reference's f32 specials row by row;
 //   * the final bound (xC + tmove, rounded up to f32) goes through the same
 //     f32 bit statistic as the exact kernel, which is monotone.
-// int16 headroom: cells stay in [-32768, cap + emax]; a row maximum above the
+// int16 headroom: cells stay in [-32768, cap + emax] (the entry's floor and a
+// padding column's score add up to -32768); a row maximum above the
 // profile's cap (32767 minus its largest rounded score) marks the pair as
 // passing before any cell can wrap, and the flag is sticky.
 #pragma once
@@ -43,6 +45,7 @@ constexpr int kQ16EPad = -16384;    // columns past M
 constexpr int kQ16BeFloor = -16384; // -32 nats: lowest entry score
 constexpr int kQ32Neg = -(1 << 30); // f32 -inf of the special states
 constexpr unsigned kQ16Neg2 = 0x80008000u;  // (-32768, -32768)
+static_assert(kQ16BeFloor + kQ16EPad >= -32768 && kQ16BeFloor + kQ16EFloor >= -32768, "MSV sums leave int16");
 
 // A pair of profiles of one MSV shape x a slice [begin, end) of the target list
 // (pb = -1: the high half is padding and produces no decisions).
@@ -79,9 +82,6 @@ __device__ __forceinline__ int q32_up(float x) {
 // lanes vote on whether any E lies above the threshold at which it raises base,
 // and only then the group takes its maximum, updates base and raises w to the
 // row's B (w' = max(cell, B') and B >= B', so max(w', B) = max(cell, B)).
-// J itself matters only at the target's end: each lane keeps its own J from its
-// own columns' maximum and the group combines them once, which is exact, as
-// max and the common decay commute.
 // The two profiles' base and constants are int32 in units of 2^-25 nat here,
 // so the int16 value of a state is the upper half of its word.  J itself
 // matters only at the target's end: above N it is base; below N the pair's
@@ -94,8 +94,8 @@ __device__ __forceinline__ int q32_up(float x) {
 //   * a target long enough to reach the entry floor or to have tloop rounded
 //     up to 0 (L > 390,000) is recomputed by the plain recurrence.
 //   * a tile that tracks J keeps it per lane, of the lane's own columns, and
-//     the group combines them once, which is exact, as max and the common decay commute;
-//     a final J at or below the final B's level may come from B' and is
+//     the group combines them once, which is exact, as max and the common decay
+//     commute; a final J at or below the final B's level may come from B' and is
 //     recomputed by the plain recurrence too (no row of the target scored above
 //     its entry: all '*', say).
 // Bound now: the ALU pipe, about 70 operations per row of 40 columns, and 2
@@ -201,7 +201,9 @@ __global__ void __launch_bounds__(256, 2) msv16_kernel(
   const int base_idle = 32767 * 65536 + nln2_25;       // a base no E raises
   const float s1a = thr[tile.pa].s1, s1b = has_b ? thr[tile.pb].s1 : __int_as_float(0x7f800000);
   // J below N matters where the bound is asked for and where a bound at N's
-  // level, -2.4 to -0.4 bits at any length, might pass
+  // level might pass: that is -1.3 to -0.4 bits, and above 0.5 only from about
+  // 150,000 residues on, when tloop's rounding has eaten its decay (such a pair
+  // may then pass at N's level, which costs a rescoring and loses nothing)
   const bool track = bound_out != nullptr || !(s1a >= 0.5f) || !(s1b >= 0.5f);
 
   unsigned w[C];
@@ -433,11 +435,13 @@ namespace sxk {
 //     rounded up after adding 2^-17 nat, as in the MSV pre-screen;
 //   * the final bound (xJ + tmove at row L, rounded up to f32) goes through
 //     the exact kernel's f32 bit statistic, which is monotone.
-// int16 range: the floors keep every sum >= -28672 (B + t_bm >= -12 nats so
-// M >= -32 nats, D, I >= -40 nats, pre >= -48 nats, plus one more
-// transition); every value is <= the previous rows' maximum plus the largest
-// match score, so a row maximum above the profile's cap (32767 minus that
-// score) marks the pair as passing before anything can wrap (sticky).
+// int16 range: B + t_bm >= -24 nats, so M >= -32 nats in a row of real scores
+// and -48 in a row past a target's end (at -24 nats a score; the three rows
+// after a target at most, before its words are set anew), D, I and pre one
+// transition below, and no sum more than one transition below those: -64 nats,
+// the least an int16 holds.  Every value is <= the previous rows' maximum plus
+// the largest match score, so a row maximum above the profile's cap (32767 minus
+// that score) marks the pair as passing before anything can wrap (sticky).
 // Columns past M carry the floor scores; the profile's quantized image has
 // the kernel's width G*C and the CPU model follows the same columns.
 // ---------------------------------------------------------------------------
@@ -449,6 +453,9 @@ constexpr unsigned kV16Init2 = 0xc000c000u;  // (-16384, -16384): -inf before ro
 constexpr unsigned kV16Low2 = 0xa000a000u;   // (-24576, -24576): no D carry into a lane
 constexpr int kV16EPast = -12288;    // -24 nats: scores of the rows past a target's end
 constexpr unsigned kV16BFloor2 = 0xf000f000u;
+// B + t_bm + e, then D, I or pre from it, then a further transition
+static_assert(kV16BFloor + kV16BmFloor + kV16EPast + 2 * kV16TFloor >= -32768 && kV16EPast <= kV16EFloor,
+              "Viterbi sums leave int16");
 constexpr int kV16Rows = 26;         // score rows of an image: 25 residue codes and the row past the end
 
 constexpr int kV16Tile = 1024;       // entries of a tile that are ordered by length
