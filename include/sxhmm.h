@@ -150,7 +150,7 @@ typedef struct {
   const char* name;     /* required */
   const char* acc;      /* NULL if absent */
   const char* desc;     /* NULL if absent */
-  int32_t m;            /* model length M, 1..2048 */
+  int32_t m;            /* model length M, at least 1 */
   int32_t has_cutoffs;  /* bit 0 GA, bit 1 TC, bit 2 NC */
   const float* msc;     /* [25][w] match log-odds msc[x*w+k] (column 0 -inf) */
   const float* mo;      /* [25][w] match odds */

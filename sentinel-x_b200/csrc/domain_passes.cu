@@ -240,7 +240,7 @@ RegionPassStats region_passes(sx_engine* E, const sx_profiles* P, const sx_targe
   }
   const auto& K = kernels();
   cudaStream_t s = E->env_stream;
-  constexpr int64_t kPoolPerRegion = 1024;
+  constexpr int64_t kPoolPerRegion = 1024;  // sampled domains per region, on average, before regions are redone
   // column tables of the profiles that have regions (exact copies of the host's
   // probabilities and match odds), uploaded once
   std::unordered_map<int32_t, int64_t> col_of;
@@ -257,7 +257,7 @@ RegionPassStats region_passes(sx_engine* E, const sx_profiles* P, const sx_targe
       for (int x2 = 0; x2 < sxk::kTraceRes; x2++) hcols.push_back(h.mo_row(x2)[k]);
     }
   }
-  E->trc_cols.upload(hcols.data(), hcols.size(), s);  // sampled domains per region, on average, before regions are redone
+  E->trc_cols.upload(hcols.data(), hcols.size(), s);
   std::vector<size_t> order(nr);
   std::iota(order.begin(), order.end(), (size_t)0);
   std::stable_sort(order.begin(), order.end(),
